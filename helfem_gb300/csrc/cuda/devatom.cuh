@@ -149,23 +149,28 @@ struct Profiler {
 
 // Device tables of the atomic DFT grid (host layout in host/atom.hpp)
 struct DevXC {
-  int nquad = 0, nap = 0;
-  const double* wang = nullptr;  // [nap]
-  const double* isin = nullptr;  // [nap]
-  const double* W = nullptr;     // [(alpha + beta*nang)*nap + a]
+  int nquad = 0, nth = 0, mdft = 0, nphi = 0, npair = 0, kmax = 0;
+  const double* wth = nullptr;   // [nth]
+  const double* isin = nullptr;  // [nth]
+  const int* pair = nullptr;     // [3*npair]
+  const int* kptr = nullptr;     // [kmax+2]
+  const double* W = nullptr;     // [p*nth + i]
   const double* Wt = nullptr;
-  const double* Wp = nullptr;
+  const double* Wd = nullptr;
+  const double* phw = nullptr;   // [nphi]
+  const double* cosk = nullptr;  // [k*nphi + j]
+  const double* sink = nullptr;
   const double* r = nullptr;     // [e*nquad + q]
   const double* wr = nullptr;    // radial weight times r^2
   const double* R = nullptr;     // [(e*nquad + q)*nn + p]
   const double* dR = nullptr;
 };
+// radial points per CTA of the point kernel (at most)
+#define XC_QB 4
 struct XcScratch {
-  double* D;      // [2][nel][nang^2][nquad]
-  double* Dr;     // same
-  double* F;      // [2][4][nel][nquad][nap]
-  double* U;      // [2][4][nel][nang^2][nquad]
-  double* epart;  // [nel*nquad][2]
+  double* D;      // [2][nel][nquad][3][npair]: D, Dr and the antisymmetric D (xc.cu)
+  double* U;      // [2][nel][npair][2][nquad]
+  double* epart;  // [nel*nquad][2] (at most)
 };
 bool xc_func_supported(int id);
 bool xc_func_is_gga(int id);

@@ -161,25 +161,27 @@ __global__ void dxc_point(DevDiatomic D, DevDiatomicXC X, DiatomicXcScratch S, i
     }
     double ra = rho[0], rb = rho[1];
     const double n = ra + rb;
-    double ev = 0.0, v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    xcf::XcOut v = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     if (n >= thr) {  // density threshold: below it the point contributes nothing
       ra = fmax(ra, 0.5 * thr);
       rb = fmax(rb, 0.5 * thr);
-      const double saa = g[0][0] * g[0][0] + g[0][1] * g[0][1];
-      const double sab = g[0][0] * g[1][0] + g[0][1] * g[1][1];
-      const double sbb = g[1][0] * g[1][0] + g[1][1] * g[1][1];
-      if (gga) eval_func<5>(xid, cid, ra, rb, saa, sab, sbb, ev, v);
-      else eval_func<2>(xid, cid, ra, rb, 0.0, 0.0, 0.0, ev, v);
+      double saa = 0.0, sab = 0.0, sbb = 0.0;
+      if (gga) {
+        saa = g[0][0] * g[0][0] + g[0][1] * g[0][1];
+        sab = g[0][0] * g[1][0] + g[0][1] * g[1][1];
+        sbb = g[1][0] * g[1][0] + g[1][1] * g[1][1];
+      }
+      v = polarized ? xc_eval<true>(xid, cid, ra, rb, saa, sab, sbb) : xc_eval<false>(xid, cid, ra, rb, saa, sab, sbb);
     }
-    esum = w * ev;
+    esum = w * v.e;
     nsum = w * n;
     const int nout = polarized ? 2 : 1;
     for (int s = 0; s < nout; ++s) {
       const size_t cstride = (size_t)D.nel * nq * na;
       const size_t base = (size_t)s * 3 * cstride + ((size_t)e * nq + q) * na + a;
-      S.F[base] = w * v[s];
+      S.F[base] = w * (s ? v.vb : v.va);
       if (gga) {
-        const double vss = v[s == 0 ? 2 : 4], vab = v[3];
+        const double vss = s ? v.vbb : v.vaa, vab = v.vab;
         for (int c = 0; c < 2; ++c)
           S.F[base + (size_t)(c + 1) * cstride] = w * (2.0 * vss * g[s][c] + vab * g[1 - s][c]) * hinv;
       }

@@ -450,7 +450,7 @@ struct hfg_atom {
   hfg::DevXC xc{};
   hfg::XcScratch xs{};
   bool xc_ready = false;
-  DBuf x_wang, x_isin, x_W, x_Wt, x_Wp, x_r, x_wr, x_R, x_dR, xs_D, xs_Dr, xs_F, xs_U, xs_ep;
+  DBuf x_wth, x_isin, x_pair, x_kptr, x_W, x_Wt, x_Wd, x_phw, x_cos, x_sin, x_r, x_wr, x_R, x_dR, xs_D, xs_U, xs_ep;
   hfg::Profiler prof;
   std::vector<cudaEvent_t> prof_ev;
   std::vector<int> prof_cls;
@@ -775,25 +775,30 @@ struct hfg_atom {
     host.build_dft_grid(ldft, mdft);
     const hfg::AtomHost& H = host;
     xc.nquad = H.nquad;
-    xc.nap = H.nap;
-    xc.wang = x_wang.upload(H.xc_wang);
+    xc.nth = H.ldft;
+    xc.mdft = H.mdft;
+    xc.nphi = H.xc_nphi;
+    xc.npair = H.xc_npair;
+    xc.kmax = H.xc_kmax;
+    xc.wth = x_wth.upload(H.xc_wth);
     xc.isin = x_isin.upload(H.xc_isin);
+    xc.pair = x_pair.upload(H.xc_pair);
+    xc.kptr = x_kptr.upload(H.xc_kptr);
     xc.W = x_W.upload(H.xc_W);
     xc.Wt = x_Wt.upload(H.xc_Wt);
-    xc.Wp = x_Wp.upload(H.xc_Wp);
+    xc.Wd = x_Wd.upload(H.xc_Wd);
+    xc.phw = x_phw.upload(H.xc_phw);
+    xc.cosk = x_cos.upload(H.xc_cos);
+    xc.sink = x_sin.upload(H.xc_sin);
     xc.r = x_r.upload(H.xc_r);
     xc.wr = x_wr.upload(H.xc_wr);
     xc.R = x_R.upload(H.xc_R);
     xc.dR = x_dR.upload(H.xc_dR);
-    const size_t nel = H.rad.nel, nq = H.nquad, nab = (size_t)H.nang * H.nang, nap = H.nap;
-    xs_D.alloc(sizeof(double) * 2 * nel * nab * nq);
-    xs_Dr.alloc(sizeof(double) * 2 * nel * nab * nq);
-    xs_F.alloc(sizeof(double) * 8 * nel * nq * nap);
-    xs_U.alloc(sizeof(double) * 8 * nel * nab * nq);
+    const size_t nel = H.rad.nel, nq = H.nquad, np = H.xc_npair;
+    xs_D.alloc(sizeof(double) * 2 * nel * nq * 3 * np);
+    xs_U.alloc(sizeof(double) * 2 * nel * np * 2 * nq);
     xs_ep.alloc(sizeof(double) * 2 * nel * nq);
     xs.D = xs_D.as<double>();
-    xs.Dr = xs_Dr.as<double>();
-    xs.F = xs_F.as<double>();
     xs.U = xs_U.as<double>();
     xs.epart = xs_ep.as<double>();
     ck(cudaStreamSynchronize(own_stream), "sync after grid upload");

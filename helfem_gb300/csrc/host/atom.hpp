@@ -123,13 +123,17 @@ struct AtomHost {
   // per element: nquad Chebyshev radial points; angular product rule of
   // ldft cos(theta) Chebyshev points x mdft uniform phi points (nap total)
   int ldft = 0, mdft = 0, nap = 0;
-  std::vector<double> xc_wang;     // [nap] angular weights
-  std::vector<double> xc_isin;     // [nap] 1/sin(theta)
-  // real angular tables, [(alpha + beta*nang)*nap + a]:
-  //   W   = Re[Y_alpha conj(Y_beta)]
-  //   Wt  = Re[dY_alpha/dtheta conj(Y_beta)]
-  //   Wp  = Re[(i m_alpha) Y_alpha conj(Y_beta)]
-  std::vector<double> xc_W, xc_Wt, xc_Wp;
+  std::vector<double> xc_wth;      // [ldft] weight of each of a theta's mdft points
+  std::vector<double> xc_isin;     // [ldft] 1/sin(theta)
+  // unordered angular pairs p = (al <= be), sorted by k = |m_al - m_be| (pairs
+  // of k: xc_kptr[k] .. xc_kptr[k+1]); xc_pair[3p..] = al, be and
+  // sign(m_al - m_be) (m_al + m_be). With Y = T(theta) e^{i m phi}:
+  //   W  = T_al T_be,  Wt, Wd = T'_al T_be +- T_al T'_be   [p*ldft + i]
+  // and cos(k phi), sin(k phi) at the xc_nphi points of [0, pi], each standing
+  // for xc_phw (1 or 2) of the mdft points
+  int xc_npair = 0, xc_kmax = 0, xc_nphi = 0;
+  std::vector<int> xc_pair, xc_kptr;
+  std::vector<double> xc_W, xc_Wt, xc_Wd, xc_phw, xc_cos, xc_sin;
   // per element e and radial point q: r, total radial weight wrad*r^2,
   // R and dR/dr of the nn primitives: [(e*nquad + q)*nn + p]
   std::vector<double> xc_r, xc_wr, xc_R, xc_dR;

@@ -2,9 +2,8 @@
 // src/general/angular.cpp:21-70): the element radial rule (modified
 // Gauss-Chebyshev, nquad points), the angular product rule (ldft Chebyshev
 // points in cos(theta) x mdft uniform phi points), the radial functions and
-// their derivatives at the radial points, and the real angular coupling
-// tables that let the device evaluate the density and the Fock matrix in
-// separable form.
+// their derivatives at the radial points, and the theta and phi factors that
+// let the device evaluate the density and the Fock matrix in separable form.
 #include <cmath>
 #include <stdexcept>
 
@@ -54,58 +53,74 @@ void AtomHost::build_dft_grid(int ld, int md) {
   cheb_rule(ldft, xc, wc);
   nap = ldft * mdft;
   const double dphi = 2.0 * M_PI / mdft;
-  std::vector<double> cth(nap), ph(nap);
-  xc_wang.assign(nap, 0.0);
-  xc_isin.assign(nap, 0.0);
-  for (int i = 0; i < ldft; ++i)
-    for (int j = 0; j < mdft; ++j) {
-      const int a = i * mdft + j;
-      cth[a] = xc[i];
-      ph[a] = j * dphi;
-      xc_wang[a] = wc[i] * dphi;
-      xc_isin[a] = 1.0 / std::sqrt((1.0 - xc[i]) * (1.0 + xc[i]));
-    }
-  // Y, dY/dtheta at every angular point
-  std::vector<double> Yr((size_t)nang * nap), Yi((size_t)nang * nap), Tr((size_t)nang * nap), Ti((size_t)nang * nap);
+  xc_wth.assign(ldft, 0.0);
+  xc_isin.assign(ldft, 0.0);
+  for (int i = 0; i < ldft; ++i) {
+    xc_wth[i] = wc[i] * dphi;
+    xc_isin[i] = 1.0 / std::sqrt((1.0 - xc[i]) * (1.0 + xc[i]));
+  }
+  // Y_l^m = T(theta) e^{i m phi}: the theta factors and their derivatives
+  // dY/dtheta = m cot(theta) Y_l^m + sqrt((l-m)(l+m+1)) e^{-i phi} Y_l^{m+1}
+  std::vector<double> T((size_t)nang * ldft), dT((size_t)nang * ldft);
   for (int al = 0; al < nang; ++al) {
     const int l = lval[al], m = mval[al];
-    for (int a = 0; a < nap; ++a) {
-      double yr, yi;
-      ylm(l, m, cth[a], ph[a], yr, yi);
-      const double s = std::sqrt((1.0 - cth[a]) * (1.0 + cth[a]));
-      const double cot = cth[a] / s;
-      // dY/dtheta = m cot(theta) Y_l^m + sqrt((l-m)(l+m+1)) e^{-i phi} Y_l^{m+1}
-      double tr = m * cot * yr, ti = m * cot * yi;
+    for (int i = 0; i < ldft; ++i) {
+      double y, im;
+      ylm(l, m, xc[i], 0.0, y, im);
+      double d = m * xc[i] * xc_isin[i] * y;
       if (m < l) {
-        double ur, ui;
-        ylm(l, m + 1, cth[a], ph[a], ur, ui);
-        const double f = std::sqrt((double)(l - m) * (l + m + 1));
-        const double cr = std::cos(ph[a]), ci = -std::sin(ph[a]);
-        tr += f * (cr * ur - ci * ui);
-        ti += f * (cr * ui + ci * ur);
+        double u;
+        ylm(l, m + 1, xc[i], 0.0, u, im);
+        d += std::sqrt((double)(l - m) * (l + m + 1)) * u;
       }
-      Yr[al * (size_t)nap + a] = yr;
-      Yi[al * (size_t)nap + a] = yi;
-      Tr[al * (size_t)nap + a] = tr;
-      Ti[al * (size_t)nap + a] = ti;
+      T[al * (size_t)ldft + i] = y;
+      dT[al * (size_t)ldft + i] = d;
     }
   }
-  const size_t n2 = (size_t)nang * nang;
-  xc_W.assign(n2 * nap, 0.0);
-  xc_Wt.assign(n2 * nap, 0.0);
-  xc_Wp.assign(n2 * nap, 0.0);
-  for (int be = 0; be < nang; ++be)
-    for (int al = 0; al < nang; ++al) {
-      const size_t o = (al + (size_t)be * nang) * nap;
-      for (int a = 0; a < nap; ++a) {
-        const double ar = Yr[al * (size_t)nap + a], ai = Yi[al * (size_t)nap + a];
-        const double br = Yr[be * (size_t)nap + a], bi = Yi[be * (size_t)nap + a];
-        const double tr = Tr[al * (size_t)nap + a], ti = Ti[al * (size_t)nap + a];
-        xc_W[o + a] = ar * br + ai * bi;   // Re[Ya conj(Yb)]
-        xc_Wt[o + a] = tr * br + ti * bi;  // Re[dYa conj(Yb)]
-        // Re[(i m) Ya conj(Yb)] = -m Im[Ya conj(Yb)] = -m (ai br - ar bi)
-        xc_Wp[o + a] = -mval[al] * (ai * br - ar * bi);
+  // unordered pairs al <= be in ascending k = |m_al - m_be|
+  xc_kmax = 0;
+  for (int al = 0; al < nang; ++al)
+    for (int be = al; be < nang; ++be) xc_kmax = std::max(xc_kmax, std::abs(mval[al] - mval[be]));
+  xc_pair.clear();
+  xc_kptr.assign(1, 0);
+  for (int k = 0; k <= xc_kmax; ++k) {
+    for (int be = 0; be < nang; ++be)
+      for (int al = 0; al <= be; ++al) {
+        const int dm = mval[al] - mval[be];
+        if (std::abs(dm) != k) continue;
+        xc_pair.push_back(al);
+        xc_pair.push_back(be);
+        xc_pair.push_back((dm > 0 ? 1 : -1) * (mval[al] + mval[be]));
       }
+    xc_kptr.push_back((int)xc_pair.size() / 3);
+  }
+  const int np = (int)xc_pair.size() / 3;
+  xc_npair = np;
+  xc_W.assign((size_t)np * ldft, 0.0);
+  xc_Wt.assign((size_t)np * ldft, 0.0);
+  xc_Wd.assign((size_t)np * ldft, 0.0);
+  for (int p = 0; p < np; ++p) {
+    const double *ta = &T[(size_t)xc_pair[3 * p] * ldft], *tb = &T[(size_t)xc_pair[3 * p + 1] * ldft];
+    const double *da = &dT[(size_t)xc_pair[3 * p] * ldft], *db = &dT[(size_t)xc_pair[3 * p + 1] * ldft];
+    for (int i = 0; i < ldft; ++i) {
+      xc_W[(size_t)p * ldft + i] = ta[i] * tb[i];
+      xc_Wt[(size_t)p * ldft + i] = da[i] * tb[i] + ta[i] * db[i];
+      xc_Wd[(size_t)p * ldft + i] = da[i] * tb[i] - ta[i] * db[i];
+    }
+  }
+  // phi = 0 .. pi: the density is even in phi, so the points beyond pi repeat
+  // those of the first half (weight 2)
+  xc_nphi = mdft / 2 + 1;
+  xc_phw.assign(xc_nphi, 2.0);
+  xc_phw[0] = 1.0;
+  if (mdft % 2 == 0) xc_phw[mdft / 2] = 1.0;
+  xc_cos.assign((size_t)(xc_kmax + 1) * xc_nphi, 0.0);
+  xc_sin.assign((size_t)(xc_kmax + 1) * xc_nphi, 0.0);
+  for (int k = 0; k <= xc_kmax; ++k)
+    for (int j = 0; j < xc_nphi; ++j) {
+      xc_cos[(size_t)k * xc_nphi + j] = std::cos(k * (j * dphi));
+      // exactly 0 at phi = 0 and pi
+      xc_sin[(size_t)k * xc_nphi + j] = xc_phw[j] == 1.0 ? 0.0 : std::sin(k * (j * dphi));
     }
   // radial side
   const int nn = rad.nn, nel = rad.nel;
