@@ -145,7 +145,7 @@ def parse_xc(method: str):
 EXCHANGE_SYMMETRIC = 1
 EXCHANGE_SPLIT = 2
 COULOMB_SPLIT = 4
-EXCHANGE_ITEMWISE = 4  # diatomic split form: diagonal tiles one output block per item (comparison schedule)
+EXCHANGE_ITEMWISE = 4  # diatomic split form: in-element recoupling one output block per item (comparison schedule)
 
 
 

@@ -47,6 +47,19 @@ struct DevDiatomic {
   const int* kent_Ma;
   const int* kent_ilm;
   const int* kent_jk;    // [nent] owning output block
+  // shells ordered by m (ascending within an m): those of m are
+  // msh[msh_ptr[m + mmax] .. msh_ptr[m + mmax + 1]); groups of at most 16 (and
+  // of at most 8) consecutive shells of one m are msh[grp_ptr[g] ..), and
+  // (L, |M|) of each multipole
+  const int* mval;
+  const int* msh;
+  const int* msh_ptr;
+  int ngrp, gmax;
+  const int* grp_ptr;
+  int ngrp8;
+  const int* grp8_ptr;
+  const int* lmL;
+  const int* lmM;
   // element pairs: off-diagonal ordered pairs (a != b) and a < b pairs
   const int2* pairs_all;
   int npairs_all;
@@ -57,7 +70,6 @@ struct DevDiatomic {
   const float2* p2s = nullptr;
   const float2* q0s = nullptr;
   const float2* q2s = nullptr;
-  const float2* txs = nullptr;
   const float2* al_c0s = nullptr;
   const float2* al_c2s = nullptr;
   const float2* lmfacs = nullptr;
@@ -66,6 +78,33 @@ struct DevDiatomic {
   // Q * 2^+k with k = kexp[ilm*nel+e] (the exponent of the element's largest
   // P entry); an element pair (inner a, outer b) restores 2^(k_a - k_b) <= 1.
   const int* kexp = nullptr;
+};
+
+// In-element tiles of the split exchange on the tensor cores (dk_tc.cu): digit
+// planes of the exchange-ordered kernel, and the scratch of one call
+#define DTC_XDIGITS 6
+#define DTC_TDIGITS 7
+#define DTC_TT 64
+struct DevDiaTC {
+  int ksteps = 0, ntt = 0;            // K steps of 16 over 4 nn^2 columns, tiles of DTC_TT rows
+  const unsigned char* tx = nullptr;  // [ilm][e][tile][K step][digit][DTC_TT x 16]
+  const int* txexp = nullptr;         // [ilm][e][tile][DTC_TT] row exponents
+  const int* cexp = nullptr;          // [ilm][e][4 nn^2] column exponents
+  int cap = 0, lparts = 1;            // units of digits held at a time, parts of the multipole sum
+  unsigned char* x = nullptr;         // [unit][ilm][K step][digit][128 x 16]
+  int* xexp = nullptr;                // [unit][ilm][128]
+  double* part = nullptr;             // [part][unit][tile][DTC_TT][128]
+  int* err = nullptr;                 // set when a completion wait ran out
+};
+
+// Scratch of the in-element tiles of the FP64 exchange (dk_share.cu): units
+// are (element, 8 output blocks)
+struct DevDia64 {
+  int cap = 0, lparts = 1;       // units of recoupled tiles held at a time, parts of the multipole sum
+  int rsplit = 1, vsplit = 1;    // parts of the tile rows, threads that share a row
+  double* x = nullptr;           // [unit][ilm][4 nn^2][8]
+  unsigned int* xact = nullptr;  // [unit][ilm] rows with an entry (bits)
+  double* part = nullptr;        // [part][unit][8][nn^2]
 };
 
 struct DevDiatomicScratch {
@@ -77,8 +116,16 @@ struct DevDiatomicScratch {
   unsigned char* ent_act; // [nent]
   unsigned char* jk_act;  // [nang^2]
   int* jk_list;           // [2*nang^2]: active output blocks, then those with j <= k
-  int* counts;            // [2]
+  int* jk_pos;            // [nang^2] position in the call's list of output blocks, or -1
+  int* kg_list;           // active (k*ngrp + g), then (k*ngrp8 + g) of the in-element items
+  // [0] active output blocks, [1] those with j <= k, [2] and [3] the lengths of
+  // the two kg lists, [4] and [5] item counters
+  int* counts;
   float2* pd2;            // [nd*nd] split copy of the density (split path)
+  // off-diagonal pairs in parts of the multipole sum: part sums of each item's
+  // tiles, [part][item][gmax][nn^2] (offparts > 1 only)
+  int offparts;
+  double* offsum;
 };
 
 #define DNORM_SPLIT 8
@@ -117,20 +164,32 @@ cudaError_t launch_diatomic_xc(const DevDiatomic& D, const DevDiatomicXC& X, con
                                int cid, const double* Pa, const double* Pb, double* Ha, double* Hb, double* energies,
                                double thr, cudaStream_t st);
 
+// exchange tiles with the recoupling shared by the output blocks of one k
+// (dk_share.cu): off-diagonal element pairs (FP64, or float pairs), and the
+// in-element tiles in FP64
+cudaError_t launch_dk_share_off(const DevDiatomic& D, const DevDiatomicScratch& S, const double* Pd, double* Kd,
+                                bool symmetric, bool split, cudaStream_t st);
+cudaError_t launch_dk_share_diag(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDia64& T,
+                                 const double* Pd, double* Kd, bool symmetric, cudaStream_t st);
+
 cudaError_t launch_diatomic_expand(const double* P, int nbf, const int* pure, double* Pd, int nd, cudaStream_t st);
 cudaError_t launch_diatomic_gather(const double* Fd, int nd, const int* pure, int nbf, double* F, cudaStream_t st);
 cudaError_t launch_diatomic_tx(const DevDiatomic& D, double* tx, cudaStream_t st);
 // J of a pure-basis density, written to the pure-basis J (overwritten)
 cudaError_t launch_diatomic_coulomb(const DevDiatomic& D, const DevDiatomicScratch& S, const double* P, double* J,
                                     cudaStream_t st);
-cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScratch& S, const double* Pd,
-                                     double* Kd, bool symmetric, cudaStream_t st);
-// split-precision exchange (float-float on the FP32 pipe, FP64 recombination);
-// inline_diag: diagonal element tiles item by item inside the tile kernel
-// instead of the grouped kernel (bitwise the same K)
-cudaError_t launch_diatomic_exchange_split(const DevDiatomic& D, const DevDiatomicScratch& S, const double* Pd,
-                                           double* Kd, bool symmetric, cudaStream_t st, bool inline_diag = false);
-// txs[i] = split(tx[i])
-cudaError_t launch_diatomic_split_tx(const double* tx, float2* txs, size_t n, cudaStream_t st);
+cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDia64& T,
+                                     const double* Pd, double* Kd, bool symmetric, cudaStream_t st);
+cudaError_t launch_dk_tc_table(const DevDiatomic& D, const DevDiaTC& T, unsigned char* tx, int* txexp, int* cexp,
+                               cudaStream_t st);
+size_t dtc_gemm_smem(const DevDiatomic& D);
+cudaError_t launch_dk_tc_diag(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDiaTC& T, double* Kd,
+                              bool symmetric, bool itemwise, cudaStream_t st);
+// split-precision exchange: off-diagonal element pairs in float pairs, the
+// in-element tiles on the tensor cores; itemwise: their recoupled tiles one
+// output block at a time (bitwise the same K)
+cudaError_t launch_diatomic_exchange_split(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDiaTC& T,
+                                           const double* Pd, double* Kd, bool symmetric, cudaStream_t st,
+                                           bool itemwise = false);
 
 }  // namespace hfg

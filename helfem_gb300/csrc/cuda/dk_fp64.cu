@@ -1,4 +1,4 @@
-// Plain-FP64 Coulomb (J) and exchange (K) builds for the diatomic basis.
+// Coulomb (J, plain FP64) and exchange (K) builds for the diatomic basis.
 //
 // J restates diatomic TwoDBasis::coulomb (src/diatomic/basis.cpp:1621-1815):
 //   dj_contract : per signed (L,M) channel and element, the two Gaunt-weighted
@@ -14,16 +14,12 @@
 //   dk_norms / dk_act : density-block screening (||P_il|| < 10 eps skipped).
 //   dk_entry_act      : which (output block, (L,|M|)) entries see an active
 //                       density block; dk_compact lists the active output
-//                       blocks on the device.
-//   dk_tiles          : persistent CTAs over (element pair, active output
-//                       block) items. Each entry recouples the four radial
-//                       matrices R00, R02, R20, R22 from the density with the
-//                       product couplings (the j-side coupling times the
-//                       k-side one, summed in that order), then
-//                       off-diagonal pairs: K -= I0 (R00 J0' + R02 J2') +
-//                       I2 (R20 J0' + R22 J2') with I/J the P- or Q-type
-//                       integrals by element order; in-element blocks: the
-//                       exchange-ordered kernel rebuilt from the factor.
+//                       blocks, and the (k, group of output rows) that hold
+//                       them, on the device.
+//   dk_share.cu       : the element-pair tiles (FP64 and float pairs) and the
+//                       in-element tiles (FP64), with the recoupling shared by
+//                       the output blocks of one k; dk_tc.cu: the in-element
+//                       tiles of the split form on the tensor cores.
 //   dk_fixup          : the shared-boundary contributions of neighbouring
 //                       tiles, added in a fixed order (bitwise reproducible).
 #include <algorithm>
@@ -31,7 +27,6 @@
 
 #include "devdiatomic.cuh"
 #include "ff.cuh"
-#include "smem_limit.hpp"
 
 namespace hfg {
 namespace {
@@ -267,6 +262,7 @@ __global__ void dk_act(DevDiatomic D, DevDiatomicScratch S) {
     double s = 0.0;
     for (int c = 0; c < DNORM_SPLIT; ++c) s += S.bnorm[idx * DNORM_SPLIT + c];
     S.act[idx] = !(sqrt(s) < 10.0 * DBL_EPSILON);
+    S.jk_act[idx] = 0;
   }
 }
 
@@ -285,514 +281,79 @@ __global__ void dk_entry_act(DevDiatomic D, DevDiatomicScratch S) {
       }
     }
     S.ent_act[ent] = any ? 1 : 0;
+    if (any) S.jk_act[jk] = 1;
   }
 }
 
-// one CTA: flags and compacted lists of the active output blocks (all, and
-// those with j <= k for the symmetric mode), in ascending jk order
-__global__ void dk_compact(DevDiatomic D, DevDiatomicScratch S) {
-  __shared__ int ca[1024], cs[1024];
+// position of this thread's first entry in a list that the threads of the
+// CTA fill in order (n entries each), and the list's length
+__device__ int dk_offset(int n, int* sh, int* length) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int v = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  __syncthreads();
+  if (lane == 31) sh[w] = v;
+  __syncthreads();
+  int base = 0, tot = 0;
+  for (int i = 0; i < nw; ++i) {
+    if (i < w) base += sh[i];
+    tot += sh[i];
+  }
+  if (threadIdx.x == 0) *length = tot;
+  return base + v - n;
+}
+
+// one CTA: compacted lists of the active output blocks (all, and those with
+// j <= k for the symmetric mode) and of the active (k, group of output rows)
+// of the shared tiles (in-element items: some j <= k in symmetric mode), in
+// ascending order
+__global__ void dk_compact(DevDiatomic D, DevDiatomicScratch S, int symmetric) {
+  __shared__ int sh[32];
   const int n = D.nang * D.nang, nt = blockDim.x;
-  const int chunk = (n + nt - 1) / nt;
-  const int lo = min(n, (int)threadIdx.x * chunk), hi = min(n, lo + chunk);
-  int na = 0, ns = 0;
-  for (int jk = lo; jk < hi; ++jk) {
-    bool a = false;
-    for (int ent = D.kjk_ptr[jk]; ent < D.kjk_ptr[jk + 1]; ++ent)
-      if (S.ent_act[ent]) { a = true; break; }
-    S.jk_act[jk] = a ? 1 : 0;
-    if (a) {
+  auto range = [&](int m, int& lo, int& hi) {
+    const int chunk = (m + nt - 1) / nt;
+    lo = min(m, (int)threadIdx.x * chunk);
+    hi = min(m, lo + chunk);
+  };
+  auto row_active = [&](int k, const int* ptr, int g, bool half) {
+    for (int x = ptr[g]; x < ptr[g + 1]; ++x)
+      if (S.jk_act[D.msh[x] + k * D.nang] && (!half || D.msh[x] <= k)) return true;
+    return false;
+  };
+  int lo, hi, na = 0, ns = 0, nk = 0, nd = 0;
+  range(n, lo, hi);
+  for (int jk = lo; jk < hi; ++jk)
+    if (S.jk_act[jk]) {
       ++na;
       if (jk % D.nang <= jk / D.nang) ++ns;
     }
+  int oa = dk_offset(na, sh, &S.counts[0]), os = dk_offset(ns, sh, &S.counts[1]);
+  for (int jk = lo; jk < hi; ++jk) {
+    const bool on = S.jk_act[jk], half = on && jk % D.nang <= jk / D.nang;
+    S.jk_pos[jk] = symmetric ? (half ? os : -1) : (on ? oa : -1);
+    if (on) S.jk_list[oa++] = jk;
+    if (half) S.jk_list[n + os++] = jk;
   }
-  ca[threadIdx.x] = na;
-  cs[threadIdx.x] = ns;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int sa = 0, ss = 0;
-    for (int t = 0; t < nt; ++t) {
-      const int a = ca[t], s = cs[t];
-      ca[t] = sa;
-      cs[t] = ss;
-      sa += a;
-      ss += s;
-    }
-    S.counts[0] = sa;
-    S.counts[1] = ss;
-  }
-  __syncthreads();
-  int oa = ca[threadIdx.x], os = cs[threadIdx.x];
-  for (int jk = lo; jk < hi; ++jk)
-    if (S.jk_act[jk]) {
-      S.jk_list[oa++] = jk;
-      if (jk % D.nang <= jk / D.nang) S.jk_list[n + os++] = jk;
-    }
+  range(D.nang * D.ngrp, lo, hi);
+  for (int x = lo; x < hi; ++x) nk += row_active(x / D.ngrp, D.grp_ptr, x % D.ngrp, false);
+  int ok = dk_offset(nk, sh, &S.counts[2]);
+  for (int x = lo; x < hi; ++x)
+    if (row_active(x / D.ngrp, D.grp_ptr, x % D.ngrp, false)) S.kg_list[ok++] = x;
+  range(D.nang * D.ngrp8, lo, hi);
+  for (int x = lo; x < hi; ++x) nd += row_active(x / D.ngrp8, D.grp8_ptr, x % D.ngrp8, symmetric != 0);
+  int od = dk_offset(nd, sh, &S.counts[3]);
+  for (int x = lo; x < hi; ++x)
+    if (row_active(x / D.ngrp8, D.grp8_ptr, x % D.ngrp8, symmetric != 0))
+      S.kg_list[(size_t)D.nang * D.ngrp + od++] = x;
+  if (threadIdx.x == 0) S.counts[4] = S.counts[5] = 0;
 }
 
 __device__ __forceinline__ size_t dhalo_idx(const DevDiatomic& D, int a, int b, int jk, int h) {
   return ((size_t)(a * D.nel + b) * (D.nang * D.nang) + jk) * (2 * D.nn - 1) + h;
-}
-
-__device__ __forceinline__ void dk_store(const DevDiatomic& D, const DevDiatomicScratch& S, double* Kd, int a, int b,
-                                         int jk, int p, int q, double y) {
-  const int nn = D.nn;
-  const int gp = dgf(D, a, p), gq = dgf(D, b, q);
-  if (gp >= D.nrad || gq >= D.nrad) return;
-  const int j = jk % D.nang, k = jk / D.nang;
-  if (p <= nn - 2 && q <= nn - 2)
-    Kd[(size_t)(k * D.nrad + gq) * D.nd + (size_t)j * D.nrad + gp] = y;
-  else if (p == nn - 1)
-    S.khalo[dhalo_idx(D, a, b, jk, q)] = y;
-  else
-    S.khalo[dhalo_idx(D, a, b, jk, nn + p)] = y;
-}
-
-// Persistent CTAs over work items. Item w < n_off: element pair
-// pairs[w / n_act], output block jk_list[w % n_act]; the rest: diagonal
-// element e, output block from the (symmetric: j <= k) list. In symmetric
-// mode (P = P^T) only a < b pairs are items and each also writes the
-// transposed partner tile, K_kj(b,a) = K_jk(a,b)^T.
-__global__ void __launch_bounds__(320) dk_tiles(DevDiatomic D, DevDiatomicScratch S, const double* __restrict__ Pd,
-                                                double* __restrict__ Kd, int symmetric) {
-  const int nn = D.nn, n2 = nn * nn, nang2 = D.nang * D.nang;
-  const int n_act = S.counts[0], n_dact = symmetric ? S.counts[1] : S.counts[0];
-  const int* dlist = symmetric ? S.jk_list + nang2 : S.jk_list;
-  const int2* pairs = symmetric ? D.pairs_sym : D.pairs_all;
-  const long npairs = symmetric ? D.npairs_sym : D.npairs_all;
-  const long n_off = npairs * n_act, total = n_off + (long)D.nel * n_dact;
-  extern __shared__ double sm[];
-  double* X = sm;            // [4*n2]: R00, R02, R20, R22 tiles
-  double* T = X + 4 * n2;    // [2*n2]
-  double* Im = T + 2 * n2;   // [2*n2] row-element integrals (channel 0, 2)
-  double* Jm = Im + 2 * n2;  // [2*n2] column-element integrals
-  unsigned char* act = reinterpret_cast<unsigned char*>(Jm + 2 * n2);
-  for (int idx = threadIdx.x; idx < nang2; idx += blockDim.x) act[idx] = S.act[idx];
-  __syncthreads();
-  const int t = threadIdx.x;
-  const bool live = t < n2;
-  const int p = live ? t % nn : 0, q = live ? t / nn : 0;
-  for (long w = blockIdx.x; w < total; w += gridDim.x) {
-    int a, b, jk;
-    if (w < n_off) {
-      const int2 pr = pairs[w / n_act];
-      a = pr.x;
-      b = pr.y;
-      jk = S.jk_list[w % n_act];
-    } else {
-      const long w2 = w - n_off;
-      a = b = (int)(w2 / n_dact);
-      jk = dlist[w2 % n_dact];
-    }
-    const bool diag = (a == b);
-    const int j = jk % D.nang, k = jk / D.nang;
-    const int gp = dgf(D, a, p), gq = dgf(D, b, q);
-    const bool vpq = live && gp < D.nrad && gq < D.nrad;
-    double y = 0.0;
-    for (int ent = D.kjk_ptr[jk]; ent < D.kjk_ptr[jk + 1]; ++ent) {
-      if (!S.ent_act[ent]) continue;  // uniform over the CTA
-      const int L = D.kent_L[ent], Ma = D.kent_Ma[ent], ilm = D.kent_ilm[ent];
-      double x00 = 0.0, x02 = 0.0, x20 = 0.0, x22 = 0.0;
-      if (vpq) {
-        for (int sgn = 0; sgn < (Ma ? 2 : 1); ++sgn) {
-          const int M = sgn ? -Ma : Ma;
-          const int xj = al_idx(D, j, L, M), xk = al_idx(D, k, L, M);
-          const int k0 = D.al_ptr[xk], k1 = D.al_ptr[xk + 1];
-          for (int uj = D.al_ptr[xj]; uj < D.al_ptr[xj + 1]; ++uj) {
-            const int i = D.al_b[uj];
-            const double* Pi = Pd + (size_t)i * D.nrad + gp;
-            double u0 = 0.0, u2 = 0.0;
-            for (int uk = k0; uk < k1; ++uk) {
-              const int l = D.al_b[uk];
-              if (!act[i + l * D.nang]) continue;
-              const double v = Pi[(size_t)(l * D.nrad + gq) * D.nd];
-              u0 += D.al_c0[uk] * v;
-              u2 += D.al_c2[uk] * v;
-            }
-            const double c0 = D.al_c0[uj], c2 = D.al_c2[uj];
-            x00 += c0 * u0;
-            x02 += c0 * u2;
-            x20 += c2 * u0;
-            x22 += c2 * u2;
-          }
-        }
-      }
-      const double fac = (Ma & 1) ? -D.lmfac[ilm] : D.lmfac[ilm];
-      if (live) {
-        X[t] = fac * x00;
-        X[n2 + t] = -fac * x02;
-        X[2 * n2 + t] = -fac * x20;
-        X[3 * n2 + t] = fac * x22;
-        if (!diag) {
-          const size_t la = ((size_t)ilm * D.nel + a) * n2 + t, lb = ((size_t)ilm * D.nel + b) * n2 + t;
-          Im[t] = (a < b) ? D.p0[la] : D.q0[la];
-          Im[n2 + t] = (a < b) ? D.p2[la] : D.q2[la];
-          Jm[t] = (a < b) ? D.q0[lb] : D.p0[lb];
-          Jm[n2 + t] = (a < b) ? D.q2[lb] : D.p2[lb];
-        }
-      }
-      __syncthreads();
-      if (diag) {
-        if (live) {
-          const double* tx = D.tx + ((size_t)ilm * D.nel + a) * 4 * n2 * n2;
-          double s = 0.0;
-          for (int ab = 0; ab < 4; ++ab) {
-            const double* txb = tx + (size_t)ab * n2 * n2;
-            const double* Xb = X + ab * n2;
-            for (int v = 0; v < n2; ++v) s += txb[t + (size_t)v * n2] * Xb[v];
-          }
-          y += s;
-        }
-      } else {
-        if (live) {
-          double s0 = 0.0, s2 = 0.0;
-          for (int c = 0; c < nn; ++c) {
-            const double j0 = Jm[q + c * nn], j2 = Jm[n2 + q + c * nn];
-            s0 += X[p + c * nn] * j0 + X[n2 + p + c * nn] * j2;
-            s2 += X[2 * n2 + p + c * nn] * j0 + X[3 * n2 + p + c * nn] * j2;
-          }
-          T[t] = s0;
-          T[n2 + t] = s2;
-        }
-        __syncthreads();
-        if (live) {
-          double s = 0.0;
-          for (int c = 0; c < nn; ++c) s += Im[p + c * nn] * T[c + q * nn] + Im[n2 + p + c * nn] * T[n2 + c + q * nn];
-          y += s;
-        }
-      }
-      __syncthreads();
-    }
-    if (live) dk_store(D, S, Kd, a, b, jk, p, q, -y);
-    if (symmetric && (!diag || j != k)) {
-      if (live) X[t] = -y;
-      __syncthreads();
-      if (live) dk_store(D, S, Kd, b, a, k + j * D.nang, p, q, X[q + p * nn]);
-      __syncthreads();
-    }
-  }
-}
-
-// Split-precision tiles: dk_tiles with every operand a (hi, lo) float pair,
-// TwoProd/TwoSum products on the FP32 pipe, the per-multipole results summed
-// as float pairs and recombined in FP64 once per output element.
-template <int NN>
-// 15-node elements: 256 threads, at most 51 registers so that five CTAs share an SM
-__global__ void __launch_bounds__(NN == 15 ? 256 : 320, NN == 15 ? 5 : 1) dk_tiles_split(DevDiatomic D, DevDiatomicScratch S, double* __restrict__ Kd,
-                                                      int symmetric, int with_diag) {
-  const int nn = NN > 0 ? NN : D.nn, n2 = nn * nn, nang2 = D.nang * D.nang;
-  const int n_act = S.counts[0], n_dact = symmetric ? S.counts[1] : S.counts[0];
-  const int* dlist = symmetric ? S.jk_list + nang2 : S.jk_list;
-  const int2* pairs = symmetric ? D.pairs_sym : D.pairs_all;
-  const long npairs = symmetric ? D.npairs_sym : D.npairs_all;
-  const long n_off = npairs * n_act, total = n_off + (with_diag ? (long)D.nel * n_dact : 0L);
-  extern __shared__ float2 sm2[];
-  float2* X = sm2;           // [4*n2]
-  float2* T = X + 4 * n2;    // [2*n2]
-  float2* Im = T + 2 * n2;   // [2*n2]
-  float2* Jm = Im + 2 * n2;  // [2*n2]
-  double* Y = reinterpret_cast<double*>(Jm + 2 * n2);
-  unsigned char* act = reinterpret_cast<unsigned char*>(Y + n2);
-  for (int idx = threadIdx.x; idx < nang2; idx += blockDim.x) act[idx] = S.act[idx];
-  __syncthreads();
-  const int t = threadIdx.x;
-  const bool live = t < n2;
-  const int p = live ? t % nn : 0, q = live ? t / nn : 0;
-  for (long w = blockIdx.x; w < total; w += gridDim.x) {
-    int a, b, jk;
-    if (w < n_off) {
-      const int2 pr = pairs[w / n_act];
-      a = pr.x;
-      b = pr.y;
-      jk = S.jk_list[w % n_act];
-    } else {
-      const long w2 = w - n_off;
-      a = b = (int)(w2 / n_dact);
-      jk = dlist[w2 % n_dact];
-    }
-    const bool diag = (a == b);
-    const int j = jk % D.nang, k = jk / D.nang;
-    const int gp = dgf(D, a, p), gq = dgf(D, b, q);
-    const bool vpq = live && gp < D.nrad && gq < D.nrad;
-    const float2* pbase = S.pd2 + (size_t)gq * D.nd + gp;
-    ffv yacc = {0.f, 0.f};
-    for (int ent = D.kjk_ptr[jk]; ent < D.kjk_ptr[jk + 1]; ++ent) {
-      if (!S.ent_act[ent]) continue;  // uniform over the CTA
-      const int L = D.kent_L[ent], Ma = D.kent_Ma[ent], ilm = D.kent_ilm[ent];
-      ffv x00 = {0.f, 0.f}, x02 = {0.f, 0.f}, x20 = {0.f, 0.f}, x22 = {0.f, 0.f};
-      if (vpq) {
-        for (int sgn = 0; sgn < (Ma ? 2 : 1); ++sgn) {
-          const int M = sgn ? -Ma : Ma;
-          const int xj = al_idx(D, j, L, M), xk = al_idx(D, k, L, M);
-          const int k0 = D.al_ptr[xk], k1 = D.al_ptr[xk + 1];
-          for (int uj = D.al_ptr[xj]; uj < D.al_ptr[xj + 1]; ++uj) {
-            const int i = D.al_b[uj];
-            ffv u0 = {0.f, 0.f}, u2 = {0.f, 0.f};
-            for (int uk = k0; uk < k1; ++uk) {
-              const int l = D.al_b[uk];
-              if (!act[i + l * D.nang]) continue;
-              const float2 v = pbase[(size_t)(l * D.nrad) * D.nd + (size_t)i * D.nrad];
-              u0 = ff_fma(u0, D.al_c0s[uk], v);
-              u2 = ff_fma(u2, D.al_c2s[uk], v);
-            }
-            const float2 U0 = ff2(u0), U2 = ff2(u2), c0 = D.al_c0s[uj], c2 = D.al_c2s[uj];
-            x00 = ff_fma(x00, c0, U0);
-            x02 = ff_fma(x02, c0, U2);
-            x20 = ff_fma(x20, c2, U0);
-            x22 = ff_fma(x22, c2, U2);
-          }
-        }
-      }
-      if (live) {
-        float2 fac = D.lmfacs[ilm];
-        if (Ma & 1) fac = make_float2(-fac.x, -fac.y);
-        const ffv z = {0.f, 0.f};
-        const float2 f00 = ff2(ff_fma(z, fac, ff2(x00))), f02 = ff2(ff_fma(z, fac, ff2(x02)));
-        const float2 f20 = ff2(ff_fma(z, fac, ff2(x20))), f22 = ff2(ff_fma(z, fac, ff2(x22)));
-        X[t] = f00;
-        X[n2 + t] = make_float2(-f02.x, -f02.y);
-        X[2 * n2 + t] = make_float2(-f20.x, -f20.y);
-        X[3 * n2 + t] = f22;
-        if (!diag) {
-          const size_t la = ((size_t)ilm * D.nel + a) * n2 + t, lb = ((size_t)ilm * D.nel + b) * n2 + t;
-          Im[t] = (a < b) ? D.p0s[la] : D.q0s[la];
-          Im[n2 + t] = (a < b) ? D.p2s[la] : D.q2s[la];
-          Jm[t] = (a < b) ? D.q0s[lb] : D.p0s[lb];
-          Jm[n2 + t] = (a < b) ? D.q2s[lb] : D.p2s[lb];
-        }
-      }
-      __syncthreads();
-      ffv acc = {0.f, 0.f};
-      if (diag) {
-        if (live) {
-          const float2* tx = D.txs + ((size_t)ilm * D.nel + a) * 4 * n2 * n2;
-          for (int ab = 0; ab < 4; ++ab) {
-            const float2* txb = tx + (size_t)ab * n2 * n2;
-            const float2* Xb = X + ab * n2;
-            for (int v0 = 0; v0 < n2; v0 += nn) {
-              if (NN > 0) {  // unrolled: the nn table loads are issued together
-#pragma unroll
-                for (int c = 0; c < (NN > 0 ? NN : 1); ++c)
-                  acc = ff_fma(acc, txb[t + (size_t)(v0 + c) * n2], Xb[v0 + c]);
-              } else {
-                for (int v = v0; v < v0 + nn; ++v) acc = ff_fma(acc, txb[t + (size_t)v * n2], Xb[v]);
-              }
-              acc = ff_norm(acc.hi, acc.lo);
-            }
-          }
-        }
-      } else {
-        if (live) {
-          ffv s0 = {0.f, 0.f}, s2 = {0.f, 0.f};
-#pragma unroll
-          for (int c = 0; c < (NN > 0 ? NN : 17); ++c) {
-            if (NN == 0 && c >= nn) break;
-            const float2 j0 = Jm[q + c * nn], j2 = Jm[n2 + q + c * nn];
-            s0 = ff_fma(s0, X[p + c * nn], j0);
-            s0 = ff_fma(s0, X[n2 + p + c * nn], j2);
-            s2 = ff_fma(s2, X[2 * n2 + p + c * nn], j0);
-            s2 = ff_fma(s2, X[3 * n2 + p + c * nn], j2);
-          }
-          T[t] = ff2(s0);
-          T[n2 + t] = ff2(s2);
-        }
-        __syncthreads();
-        if (live) {
-#pragma unroll
-          for (int c = 0; c < (NN > 0 ? NN : 17); ++c) {
-            if (NN == 0 && c >= nn) break;
-            acc = ff_fma(acc, Im[p + c * nn], T[c + q * nn]);
-            acc = ff_fma(acc, Im[n2 + p + c * nn], T[n2 + c + q * nn]);
-          }
-          // undo the tables' power-of-two scaling: 2^(k_inner - k_outer) <= 1
-          const int ka = D.kexp[(size_t)ilm * D.nel + a], kb = D.kexp[(size_t)ilm * D.nel + b];
-          const int dk = (a < b) ? ka - kb : kb - ka;
-          acc.hi = ldexpf(acc.hi, dk);
-          acc.lo = ldexpf(acc.lo, dk);
-        }
-      }
-      yacc = ff_add(yacc, ff_norm(acc.hi, acc.lo));
-      __syncthreads();
-    }
-    const double y = ff_to_d(yacc);
-    if (live) dk_store(D, S, Kd, a, b, jk, p, q, -y);
-    if (symmetric && (!diag || j != k)) {
-      if (live) Y[t] = -y;
-      __syncthreads();
-      if (live) dk_store(D, S, Kd, b, a, k + j * D.nang, p, q, Y[q + p * nn]);
-      __syncthreads();
-    }
-  }
-}
-
-// Diagonal element tiles of the split exchange, G output blocks per item.
-// Item w: element e = w / ngroups, the active output blocks
-// dlist[G*(w % ngroups) ...]. The members' entry lists (ascending multipole
-// index ilm) are merged: per multipole present in any member, the members
-// holding it recouple their density tiles into shared memory, then one pass
-// over the exchange-ordered kernel table of (ilm, e) feeds all of them, so
-// each table element is loaded once per item instead of once per member.
-// Per member the operations and their order are those of the item-by-item
-// schedule in dk_tiles_split, so K is bitwise the same.
-constexpr int DIAG_GROUP = 8;
-
-template <int NN, int G>
-__global__ void __launch_bounds__(NN == 15 ? 256 : 320, NN == 15 ? 3 : 1) dk_diag_split(DevDiatomic D, DevDiatomicScratch S, double* __restrict__ Kd,
-                                                         int symmetric) {
-  const int nn = NN > 0 ? NN : D.nn, n2 = nn * nn, nang2 = D.nang * D.nang;
-  const int n_dact = symmetric ? S.counts[1] : S.counts[0];
-  const int* dlist = symmetric ? S.jk_list + nang2 : S.jk_list;
-  const int ngrp = (n_dact + G - 1) / G;
-  const long total = (long)D.nel * ngrp;
-  extern __shared__ float2 sm2[];
-  float2* X = sm2;  // [G][4*n2]
-  double* Y = reinterpret_cast<double*>(X + (size_t)G * 4 * n2);
-  unsigned char* act = reinterpret_cast<unsigned char*>(Y + n2);
-  __shared__ int s_ptr[G], s_end[G], s_jk[G], s_has[G];
-  __shared__ int s_ilm;
-  for (int idx = threadIdx.x; idx < nang2; idx += blockDim.x) act[idx] = S.act[idx];
-  __syncthreads();
-  const int t = threadIdx.x;
-  const bool live = t < n2;
-  const int p = live ? t % nn : 0, q = live ? t / nn : 0;
-  for (long w = blockIdx.x; w < total; w += gridDim.x) {
-    const int e = (int)(w / ngrp), g0 = (int)(w % ngrp) * G;
-    const int ng = min(G, n_dact - g0);
-    if (t < G) {
-      if (t < ng) {
-        const int jk = dlist[g0 + t];
-        s_jk[t] = jk;
-        s_ptr[t] = D.kjk_ptr[jk];
-        s_end[t] = D.kjk_ptr[jk + 1];
-      } else {
-        s_jk[t] = -1;
-        s_ptr[t] = s_end[t] = 0;
-      }
-    }
-    __syncthreads();
-    const int gp = dgf(D, e, p), gq = dgf(D, e, q);
-    const bool vpq = live && gp < D.nrad && gq < D.nrad;
-    const float2* pbase = S.pd2 + (size_t)gq * D.nd + gp;
-    ffv yacc[G];
-#pragma unroll
-    for (int g = 0; g < G; ++g) yacc[g] = {0.f, 0.f};
-    for (;;) {
-      if (t < 32) {  // warp 0: skip inactive entries, smallest pending multipole
-        int pt = 0, me = 0x7fffffff;
-        if (t < G) {
-          pt = s_ptr[t];
-          while (pt < s_end[t] && !S.ent_act[pt]) ++pt;
-          s_ptr[t] = pt;
-          if (pt < s_end[t]) me = D.kent_ilm[pt];
-        }
-        int m = me;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (t < G) s_has[t] = (me == m && m != 0x7fffffff) ? 1 : 0;
-        if (t == 0) s_ilm = m;
-      }
-      __syncthreads();
-      const int ilm = s_ilm;
-      if (ilm == 0x7fffffff) break;
-#pragma unroll 1
-      for (int g = 0; g < G; ++g) {
-        float2* Xg = X + (size_t)g * 4 * n2;
-        if (!s_has[g]) {  // uniform over the CTA
-          if (live) Xg[t] = Xg[n2 + t] = Xg[2 * n2 + t] = Xg[3 * n2 + t] = make_float2(0.f, 0.f);
-          continue;
-        }
-        const int ent = s_ptr[g], jk = s_jk[g];
-        const int j = jk % D.nang, k = jk / D.nang;
-        const int L = D.kent_L[ent], Ma = D.kent_Ma[ent];
-        ffv x00 = {0.f, 0.f}, x02 = {0.f, 0.f}, x20 = {0.f, 0.f}, x22 = {0.f, 0.f};
-        if (vpq) {
-          for (int sgn = 0; sgn < (Ma ? 2 : 1); ++sgn) {
-            const int M = sgn ? -Ma : Ma;
-            const int xj = al_idx(D, j, L, M), xk = al_idx(D, k, L, M);
-            const int k0 = D.al_ptr[xk], k1 = D.al_ptr[xk + 1];
-            for (int uj = D.al_ptr[xj]; uj < D.al_ptr[xj + 1]; ++uj) {
-              const int i = D.al_b[uj];
-              ffv u0 = {0.f, 0.f}, u2 = {0.f, 0.f};
-              for (int uk = k0; uk < k1; ++uk) {
-                const int l = D.al_b[uk];
-                if (!act[i + l * D.nang]) continue;
-                const float2 v = pbase[(size_t)(l * D.nrad) * D.nd + (size_t)i * D.nrad];
-                u0 = ff_fma(u0, D.al_c0s[uk], v);
-                u2 = ff_fma(u2, D.al_c2s[uk], v);
-              }
-              const float2 U0 = ff2(u0), U2 = ff2(u2), c0 = D.al_c0s[uj], c2 = D.al_c2s[uj];
-              x00 = ff_fma(x00, c0, U0);
-              x02 = ff_fma(x02, c0, U2);
-              x20 = ff_fma(x20, c2, U0);
-              x22 = ff_fma(x22, c2, U2);
-            }
-          }
-        }
-        if (live) {
-          float2 fac = D.lmfacs[ilm];
-          if (Ma & 1) fac = make_float2(-fac.x, -fac.y);
-          const ffv z = {0.f, 0.f};
-          const float2 f00 = ff2(ff_fma(z, fac, ff2(x00))), f02 = ff2(ff_fma(z, fac, ff2(x02)));
-          const float2 f20 = ff2(ff_fma(z, fac, ff2(x20))), f22 = ff2(ff_fma(z, fac, ff2(x22)));
-          Xg[t] = f00;
-          Xg[n2 + t] = make_float2(-f02.x, -f02.y);
-          Xg[2 * n2 + t] = make_float2(-f20.x, -f20.y);
-          Xg[3 * n2 + t] = f22;
-        }
-      }
-      __syncthreads();
-      if (live) {
-        ffv acc[G];
-#pragma unroll
-        for (int g = 0; g < G; ++g) acc[g] = {0.f, 0.f};
-        const float2* tx = D.txs + ((size_t)ilm * D.nel + e) * 4 * n2 * n2;
-        for (int ab = 0; ab < 4; ++ab) {
-          const float2* txb = tx + (size_t)ab * n2 * n2;
-          for (int v0 = 0; v0 < n2; v0 += nn) {
-            if (NN > 0) {
-#pragma unroll
-              for (int c = 0; c < (NN > 0 ? NN : 1); ++c) {
-                const float2 tv = txb[t + (size_t)(v0 + c) * n2];
-#pragma unroll
-                for (int g = 0; g < G; ++g) acc[g] = ff_fma(acc[g], tv, X[(size_t)g * 4 * n2 + ab * n2 + v0 + c]);
-              }
-            } else {
-              for (int v = v0; v < v0 + nn; ++v) {
-                const float2 tv = txb[t + (size_t)v * n2];
-#pragma unroll
-                for (int g = 0; g < G; ++g) acc[g] = ff_fma(acc[g], tv, X[(size_t)g * 4 * n2 + ab * n2 + v]);
-              }
-            }
-#pragma unroll
-            for (int g = 0; g < G; ++g) acc[g] = ff_norm(acc[g].hi, acc[g].lo);
-          }
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g)
-          if (s_has[g]) yacc[g] = ff_add(yacc[g], ff_norm(acc[g].hi, acc[g].lo));
-      }
-      __syncthreads();
-      if (t < G && s_has[t]) ++s_ptr[t];
-    }
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      if (g >= ng) break;  // uniform over the CTA
-      const int jk = s_jk[g], j = jk % D.nang, k = jk / D.nang;
-      const double y = ff_to_d(yacc[g]);
-      if (live) dk_store(D, S, Kd, e, e, jk, p, q, -y);
-      if (symmetric && j != k) {
-        if (live) Y[t] = -y;
-        __syncthreads();
-        if (live) dk_store(D, S, Kd, e, e, k + j * D.nang, p, q, Y[q + p * nn]);
-      }
-      __syncthreads();
-    }
-  }
-}
-
-__global__ void d_split(const double* __restrict__ x, float2* __restrict__ y, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    y[i] = split_bits(x[i]);
 }
 
 // Shared-boundary fix-up: entry (p,q) of tile (a,b) in its first row or
@@ -861,64 +422,35 @@ cudaError_t launch_diatomic_coulomb(const DevDiatomic& D, const DevDiatomicScrat
   return cudaGetLastError();
 }
 
-cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScratch& S, const double* Pd, double* Kd,
-                                     bool symmetric, cudaStream_t st) {
-  const int n2 = D.nn * D.nn, th = dthreads(n2), nang2 = D.nang * D.nang;
+cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDia64& T,
+                                     const double* Pd, double* Kd, bool symmetric, cudaStream_t st) {
+  const int nang2 = D.nang * D.nang;
   cudaError_t e = cudaMemsetAsync(Kd, 0, sizeof(double) * (size_t)D.nd * D.nd, st);
   if (e != cudaSuccess) return e;
   dk_norms<<<dim3(nang2, DNORM_SPLIT), 256, 0, st>>>(D, Pd, S.bnorm, nullptr);
   dk_act<<<(nang2 + 255) / 256, 256, 0, st>>>(D, S);
-  dk_entry_act<<<(D.nent + 127) / 128 > 0 ? (D.nent + 127) / 128 : 1, 128, 0, st>>>(D, S);
-  dk_compact<<<1, 1024, 0, st>>>(D, S);
-  int dev = 0, nsm = 152, per = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const size_t smem = sizeof(double) * 10 * n2 + nang2;
-  e = smem_limit(dk_tiles, smem);
+  dk_entry_act<<<std::max(1, (D.nent + 127) / 128), 128, 0, st>>>(D, S);
+  dk_compact<<<1, 1024, 0, st>>>(D, S, symmetric ? 1 : 0);
+  e = launch_dk_share_diag(D, S, T, Pd, Kd, symmetric, st);
+  if (e == cudaSuccess) e = launch_dk_share_off(D, S, Pd, Kd, symmetric, false, st);
   if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dk_tiles, th, smem);
-  if (e != cudaSuccess) return e;
-  const int grid = nsm * std::max(per, 1);
-  dk_tiles<<<grid, th, smem, st>>>(D, S, Pd, Kd, symmetric ? 1 : 0);
   dk_fixup<<<D.nel * D.nel, 256, 0, st>>>(D, S, Kd);
   return cudaGetLastError();
 }
 
-cudaError_t launch_diatomic_split_tx(const double* tx, float2* txs, size_t n, cudaStream_t st) {
-  d_split<<<dgrid(n), 256, 0, st>>>(tx, txs, n);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_diatomic_exchange_split(const DevDiatomic& D, const DevDiatomicScratch& S, const double* Pd,
-                                           double* Kd, bool symmetric, cudaStream_t st, bool inline_diag) {
-  const int n2 = D.nn * D.nn, th = dthreads(n2), nang2 = D.nang * D.nang;
+cudaError_t launch_diatomic_exchange_split(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDiaTC& T,
+                                           const double* Pd, double* Kd, bool symmetric, cudaStream_t st,
+                                           bool itemwise) {
+  const int nang2 = D.nang * D.nang;
   cudaError_t e = cudaMemsetAsync(Kd, 0, sizeof(double) * (size_t)D.nd * D.nd, st);
   if (e != cudaSuccess) return e;
   dk_norms<<<dim3(nang2, DNORM_SPLIT), 256, 0, st>>>(D, Pd, S.bnorm, S.pd2);
   dk_act<<<(nang2 + 255) / 256, 256, 0, st>>>(D, S);
-  dk_entry_act<<<(D.nent + 127) / 128 > 0 ? (D.nent + 127) / 128 : 1, 128, 0, st>>>(D, S);
-  dk_compact<<<1, 1024, 0, st>>>(D, S);
-  int dev = 0, nsm = 152, per = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const size_t smem = sizeof(float2) * 10 * n2 + sizeof(double) * n2 + nang2;
-  auto kern = (D.nn == 15) ? dk_tiles_split<15> : dk_tiles_split<0>;
-  e = smem_limit(kern, smem);
+  dk_entry_act<<<std::max(1, (D.nent + 127) / 128), 128, 0, st>>>(D, S);
+  dk_compact<<<1, 1024, 0, st>>>(D, S, symmetric ? 1 : 0);
+  e = launch_dk_tc_diag(D, S, T, Kd, symmetric, itemwise, st);
+  if (e == cudaSuccess) e = launch_dk_share_off(D, S, Pd, Kd, symmetric, true, st);
   if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, th, smem);
-  if (e != cudaSuccess) return e;
-  kern<<<nsm * std::max(per, 1), th, smem, st>>>(D, S, Kd, symmetric ? 1 : 0, inline_diag ? 1 : 0);
-  if (!inline_diag) {
-    constexpr int G = DIAG_GROUP;
-    const size_t smd = sizeof(float2) * (size_t)G * 4 * n2 + sizeof(double) * n2 + nang2;
-    auto dkern = (D.nn == 15) ? dk_diag_split<15, G> : dk_diag_split<0, G>;
-    e = smem_limit(dkern, smd);
-    if (e != cudaSuccess) return e;
-    int dper = 1;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dper, dkern, th, smd);
-    if (e != cudaSuccess) return e;
-    dkern<<<nsm * std::max(dper, 1), th, smd, st>>>(D, S, Kd, symmetric ? 1 : 0);
-  }
   dk_fixup<<<D.nel * D.nel, 256, 0, st>>>(D, S, Kd);
   return cudaGetLastError();
 }

@@ -20,9 +20,15 @@ struct hfg_diatomic {
   hfg::DevDiatomicScratch scr{};
   DBuf d_p0, d_p2, d_q0, d_q2, d_cdB, d_cds, d_cdrank, d_tx, d_lmfac, d_al_ptr, d_al_b, d_al_c0, d_al_c2, d_chL,
       d_chM, d_chilm, d_chfac, d_jbra_ptr, d_jbra_chan, d_jbra_c0, d_jbra_c2, d_kjk_ptr, d_kentL, d_kentMa,
-      d_kentilm, d_kentjk, d_pairs_all, d_pairs_sym, d_pure, d_poff, d_pstart;
-  DBuf s_jin, s_jscal, s_khalo, s_bnorm, s_act, s_entact, s_jkact, s_jklist, s_counts, s_Pd, s_Fd;
-  DBuf d_p0s, d_p2s, d_q0s, d_q2s, d_txs, d_alc0s, d_alc2s, d_lmfacs, d_kexp, s_pd2;  // split-precision path
+      d_kentilm, d_kentjk, d_mval, d_msh, d_mshptr, d_grp, d_grp8, d_lmL, d_lmM, d_pairs_all, d_pairs_sym, d_pure, d_poff, d_pstart;
+  DBuf s_jin, s_jscal, s_khalo, s_bnorm, s_act, s_entact, s_jkact, s_jklist, s_jkpos, s_kglist, s_counts, s_Pd, s_Fd;
+  DBuf d_p0s, d_p2s, d_q0s, d_q2s, d_alc0s, d_alc2s, d_lmfacs, d_kexp, s_pd2;  // split-precision path
+  // its in-element tiles on the tensor cores
+  DBuf t_tx, t_txexp, t_cexp, t_x, t_xexp, t_part, t_err;
+  hfg::DevDiaTC tc{};
+  // scratch of the FP64 in-element tiles, part sums of the off-diagonal pairs
+  DBuf d_x64, d_xact, d_part64, s_offsum;
+  hfg::DevDia64 t64{};
   DBuf h_in, h_out;
   cudaEvent_t last_use = nullptr;
   std::vector<double> lmfac_host;
@@ -120,6 +126,34 @@ struct hfg_diatomic {
     for (int jk = 0; jk < H.nang * H.nang; ++jk)
       for (int e = H.kjk_ptr[jk]; e < H.kjk_ptr[jk + 1]; ++e) kjk[e] = jk;
     D.kent_jk = d_kentjk.upload(kjk);
+    {
+      // shells by m, and groups of at most 16 / 8 of one m (equal parts)
+      std::vector<int> msh, mptr(1, 0), grp(1, 0), grp8(1, 0);
+      D.gmax = 1;
+      for (int m = -H.mmax; m <= H.mmax; ++m) {
+        const int lo = (int)msh.size();
+        for (int s = 0; s < H.nang; ++s)
+          if (H.mval[s] == m) msh.push_back(s);
+        const int n = (int)msh.size() - lo;
+        mptr.push_back((int)msh.size());
+        for (auto x : {std::make_pair(16, &grp), std::make_pair(8, &grp8)}) {
+          const int parts = (n + x.first - 1) / x.first;
+          for (int i = 1; i <= parts; ++i) {
+            x.second->push_back(lo + n * i / parts);
+            if (x.first == 16) D.gmax = std::max(D.gmax, n * i / parts - n * (i - 1) / parts);
+          }
+        }
+      }
+      D.mval = d_mval.upload(H.mval);
+      D.msh = d_msh.upload(msh);
+      D.msh_ptr = d_mshptr.upload(mptr);
+      D.ngrp = (int)grp.size() - 1;
+      D.grp_ptr = d_grp.upload(grp);
+      D.ngrp8 = (int)grp8.size() - 1;
+      D.grp8_ptr = d_grp8.upload(grp8);
+      D.lmL = d_lmL.upload(H.lm_L);
+      D.lmM = d_lmM.upload(H.lm_M);
+    }
     std::vector<int2> pa, ps;
     for (int b = 0; b < H.nel; ++b)
       for (int a = 0; a < H.nel; ++a) {
@@ -145,7 +179,10 @@ struct hfg_diatomic {
     s_entact.alloc(std::max<size_t>(1, D.nent));
     s_jkact.alloc(nang2);
     s_jklist.alloc(sizeof(int) * 2 * nang2);
-    s_counts.alloc(sizeof(int) * 2);
+    s_jkpos.alloc(sizeof(int) * nang2);
+    scr.jk_pos = s_jkpos.as<int>();
+    s_kglist.alloc(sizeof(int) * (size_t)H.nang * (D.ngrp + D.ngrp8));
+    s_counts.alloc(sizeof(int) * 6);
     s_Pd.alloc(sizeof(double) * nd * nd);
     s_Fd.alloc(sizeof(double) * nd * nd);
     scr.jin = s_jin.as<double>();
@@ -156,6 +193,18 @@ struct hfg_diatomic {
     scr.ent_act = s_entact.as<unsigned char>();
     scr.jk_act = s_jkact.as<unsigned char>();
     scr.jk_list = s_jklist.as<int>();
+    scr.kg_list = s_kglist.as<int>();
+    // off-diagonal pairs: the multipole sum in parts where a density that does
+    // not mix m makes fewer than four items per SM
+    {
+      const long items = (long)D.npairs_sym * H.nang * std::max(1, D.ngrp / (2 * H.mmax + 1));
+      scr.offparts = (int)std::max<long>(1, std::min<long>(H.nlm, 608 / items));
+      scr.offsum = nullptr;
+      if (scr.offparts > 1) {
+        s_offsum.alloc(sizeof(double) * scr.offparts * (size_t)D.npairs_all * H.nang * D.ngrp * D.gmax * n2);
+        scr.offsum = s_offsum.as<double>();
+      }
+    }
     scr.counts = s_counts.as<int>();
     ck(cudaEventCreateWithFlags(&last_use, cudaEventDisableTiming), "cudaEventCreate");
     ck(cudaStreamSynchronize(own_stream), "sync after upload");
@@ -310,9 +359,63 @@ struct hfg_diatomic {
     ck(cudaStreamSynchronize(own_stream), "sync after the device tabulation");
   }
 
+  // a completion wait inside the tensor-core kernel ran out (checked by the
+  // host-pointer entry points after their synchronisation)
+  void tc_check() {
+    if (!tc.err) return;
+    int e = 0;
+    ck(cudaMemcpy(&e, tc.err, sizeof(int), cudaMemcpyDeviceToHost), "D2H");
+    if (e) throw std::runtime_error("tensor-core exchange: an MMA completion wait ran out");
+  }
+
+  // output blocks j <= k of one m: the active ones for a density that does
+  // not mix m
+  size_t same_m_pairs() const {
+    size_t n = 0;
+    for (int j = 0; j < host.nang; ++j)
+      for (int k = j; k < host.nang; ++k) n += host.mval[j] == host.mval[k];
+    return n;
+  }
+
+  // scratch of the FP64 in-element tiles, on the first FP64 exchange
+  void ensure_fp64() {
+    if (t64.x) return;
+    hfg_abi::AllocStream alloc_on(own_stream);
+    const hfg::DiatomicHost& H = host;
+    const size_t n2 = (size_t)H.nn * H.nn, nang = H.nang;
+    hfg::DevDia64 T;
+    const size_t unit = sizeof(double) * H.nlm * 4 * n2 * 8;
+    const size_t units = (size_t)H.nel * ((nang * nang + 7) / 8);
+    T.cap = (int)std::max<size_t>(1, std::min(units, ((size_t)2 << 30) / unit));
+    // Rows of a tile in rsplit parts, vsplit threads per row: the pair that
+    // leaves the fewest of the CTA's lanes idle (a partly filled warp costs the
+    // FP64 pipe as much as a full one; nn = 15: 45 rows x 7 threads, 315 of 320)
+    double best = 0.0;
+    for (int r = 1; r <= 8; ++r) {
+      const int rows = ((int)n2 + r - 1) / r, v = std::max(1, 320 / rows), th = (rows * v + 31) / 32 * 32;
+      const double eff = (double)n2 * v / ((double)r * th);
+      if (eff > best + 1e-9 && th <= 320) {
+        best = eff;
+        T.rsplit = r;
+        T.vsplit = v;
+      }
+    }
+    // parts of the multipole sum: ten CTAs per SM for a density that does not mix m
+    const size_t ctas = (size_t)H.nel * ((same_m_pairs() + 7) / 8) * T.rsplit;
+    T.lparts = (int)std::max<size_t>(1, std::min<size_t>(H.nlm, 1520 / ctas));
+    d_x64.alloc(unit * T.cap);
+    d_xact.alloc(sizeof(unsigned) * (size_t)T.cap * H.nlm);
+    d_part64.alloc(sizeof(double) * (size_t)T.lparts * T.cap * 8 * n2);
+    T.xact = d_xact.as<unsigned>();
+    T.part = d_part64.as<double>();
+    ck(cudaStreamSynchronize(own_stream), "sync after the exchange scratch");
+    T.x = d_x64.as<double>();
+    t64 = T;
+  }
+
   // split tables and the split density buffer, on the first split-precision call
   void ensure_split() {
-    if (dev.txs) return;
+    if (tc.err) return;
     hfg_abi::AllocStream alloc_on(own_stream);
     auto split = [](const std::vector<double>& v) {
       std::vector<float2> o(v.size());
@@ -348,21 +451,48 @@ struct hfg_diatomic {
     dev.al_c0s = d_alc0s.upload(split(H.al_c0));
     dev.al_c2s = d_alc2s.upload(split(H.al_c2));
     dev.lmfacs = d_lmfacs.upload(split(lmfac_host));
-    const size_t ntx = d_tx.n / sizeof(double);
-    d_txs.alloc(sizeof(float2) * ntx);
-    ck(hfg::launch_diatomic_split_tx(d_tx.as<double>(), d_txs.as<float2>(), ntx, own_stream), "split tables");
     s_pd2.alloc(sizeof(float2) * (size_t)H.ndummy * H.ndummy);
     scr.pd2 = s_pd2.as<float2>();
+    // in-element tiles: the kernel's digit planes, and scratch for the digits
+    // of as many (element, 128 output blocks) units as 4 GB hold (at least one)
+    hfg::DevDiaTC T;
+    T.ksteps = (int)((4 * n2 + 15) / 16);
+    T.ntt = (int)((n2 + DTC_TT - 1) / DTC_TT);
+    const size_t plane = 32;  // bytes of one row of a K step's plane
+    t_tx.alloc(ntile * T.ntt * T.ksteps * DTC_TDIGITS * DTC_TT * plane);
+    t_cexp.alloc(sizeof(int) * ntile * 4 * n2);
+    T.cexp = t_cexp.as<int>();
+    t_txexp.alloc(sizeof(int) * ntile * T.ntt * DTC_TT);
+    ck(hfg::launch_dk_tc_table(dev, T, t_tx.as<unsigned char>(), t_txexp.as<int>(), t_cexp.as<int>(), own_stream), "kernel digits");
+    T.tx = t_tx.as<unsigned char>();
+    T.txexp = t_txexp.as<int>();
+    const size_t unit = (size_t)H.nlm * T.ksteps * DTC_XDIGITS * 128 * plane, nang = H.nang;
+    const size_t units = (size_t)H.nel * ((nang * nang + 127) / 128);
+    T.cap = (int)std::max<size_t>(1, std::min(units, ((size_t)4 << 30) / unit));
+    // parts of the multipole sum where a density that does not mix m makes
+    // fewer units x tiles than there are SMs (one CTA per SM)
+    const size_t ctas = (size_t)H.nel * ((same_m_pairs() + 127) / 128) * T.ntt;
+    T.lparts = (int)std::max<size_t>(1, std::min<size_t>(H.nlm, 152 / ctas));
+    t_x.alloc(unit * T.cap);
+    t_xexp.alloc(sizeof(int) * (size_t)T.cap * H.nlm * 128);
+    t_part.alloc(sizeof(double) * (size_t)T.lparts * T.cap * T.ntt * DTC_TT * 128);
+    t_err.alloc(sizeof(int));
+    ck(cudaMemsetAsync(t_err.p, 0, sizeof(int), own_stream), "memset");
+    T.x = t_x.as<unsigned char>();
+    T.xexp = t_xexp.as<int>();
+    T.part = t_part.as<double>();
     ck(cudaStreamSynchronize(own_stream), "sync after split tables");
-    dev.txs = d_txs.as<float2>();
+    T.err = t_err.as<int>();
+    tc = T;
   }
 
   // J or K of a pure-basis density (device pointers) on stream st
   void build(const double* P, double* F, bool exchange, bool symmetric, cudaStream_t st, bool split = false,
-             bool inline_diag = false) {
+             bool itemwise = false) {
     check_device();
     const hfg::DiatomicHost& H = host;
     if (split) ensure_split();
+    else if (exchange) ensure_fp64();
     if (!exchange) {  // J reads the pure density and writes the pure J directly
       ck(hfg::launch_diatomic_coulomb(dev, scr, P, F, st), "coulomb");
       mark_use(st);
@@ -370,11 +500,11 @@ struct hfg_diatomic {
     }
     ck(hfg::launch_diatomic_expand(P, H.nbf, d_pure.as<int>(), s_Pd.as<double>(), H.ndummy, st), "expand");
     if (split)
-      ck(hfg::launch_diatomic_exchange_split(dev, scr, s_Pd.as<double>(), s_Fd.as<double>(), symmetric, st,
-                                             inline_diag),
+      ck(hfg::launch_diatomic_exchange_split(dev, scr, tc, s_Pd.as<double>(), s_Fd.as<double>(), symmetric, st,
+                                             itemwise),
          "exchange (split)");
     else
-      ck(hfg::launch_diatomic_exchange(dev, scr, s_Pd.as<double>(), s_Fd.as<double>(), symmetric, st), "exchange");
+      ck(hfg::launch_diatomic_exchange(dev, scr, t64, s_Pd.as<double>(), s_Fd.as<double>(), symmetric, st), "exchange");
     ck(hfg::launch_diatomic_gather(s_Fd.as<double>(), H.ndummy, d_pure.as<int>(), H.nbf, F, st), "gather");
     mark_use(st);
   }
@@ -436,6 +566,7 @@ struct hfg_diatomic {
     build(h_in.as<double>(), h_out.as<double>(), exchange, symmetric, own_stream, split);
     ck(cudaMemcpyAsync(F, h_out.p, bytes, cudaMemcpyDeviceToHost, own_stream), "copy out");
     ck(cudaStreamSynchronize(own_stream), "sync");
+    if (exchange && split) tc_check();
   }
 };
 

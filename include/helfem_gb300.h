@@ -554,12 +554,14 @@ hfg_status hfg_diatomic_coulomb(hfg_diatomic* d, const double* P, double* J, voi
 /* K(P) for a spin density, with the reference's sign (added to F): replaces
  * diatomic TwoDBasis::exchange (basis.cpp:1817-2061), including its
  * density-block screening. flags: HFG_EXCHANGE_SYMMETRIC (P = P^T),
- * HFG_EXCHANGE_SPLIT (split precision as for atoms; the first split call
- * allocates float-pair copies of the tables and an ndummy^2 density copy),
- * HFG_EXCHANGE_ITEMWISE (split form only: the diagonal element tiles one
- * output block per work item inside the tile kernel, instead of in groups of
- * output blocks sharing each in-element kernel-table pass; the same K bit
- * for bit, slower; kept for comparison). */
+ * HFG_EXCHANGE_SPLIT (split precision: element pairs in float pairs, the
+ * in-element tiles on the tensor cores; the first split call allocates
+ * float-pair copies of the tables, digit planes of the in-element kernel, an
+ * ndummy^2 density copy and up to 4 GB of scratch; the first plain call up to
+ * 2 GB), HFG_EXCHANGE_ITEMWISE (split form only: the density tiles of the
+ * in-element products are recoupled one output block per work item instead of
+ * in groups of output blocks that share the sums over l; the same K bit for
+ * bit, slower; kept for comparison). */
 #define HFG_EXCHANGE_ITEMWISE 4
 hfg_status hfg_diatomic_exchange(hfg_diatomic* d, const double* P, double* K, int flags, void* stream);
 /* host-pointer value-semantics variants */

@@ -1,0 +1,49 @@
+"""Diatomic exchange at the shapes where its tiles and groups can go wrong:
+the shortest and longest elements (partly filled row tiles, K steps and
+warps), more than 8 and more than 16 shells of one m (several groups of output
+rows per k), m up to 3 with few shells each, densities that mix m (every
+group active) and that do not, general and symmetric modes, against the
+oracle.
+
+Bars: the FP64 form 1e-10 of max|K| (the plain form's bar), the split form
+1e-11 (its bar on the other diatomic bases)."""
+import numpy as np
+import pytest
+
+import helfem_gb300 as hg
+from oracle import DiatomicOracle
+from oracle import diatomic as dia
+from gpu_util import from_dev, relerr, to_dev, torch_cuda
+from test_gpu_diatomic import bound_density
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # nnodes, nelem, lmax per |m|
+    (3, 2, [3, 2]),
+    (4, 3, [9]),
+    (5, 2, [17, 3]),
+    (8, 2, [3, 3, 3, 3]),
+    (16, 2, [2, 2]),
+    (17, 2, [3]),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: f"n{c[0]}_e{c[1]}_l{'-'.join(map(str, c[2]))}")
+def test_diatomic_exchange_shapes(case):
+    torch = torch_cuda()
+    nn, nelem, lm = case
+    d = hg.Diatomic.from_grid(3, 1, 3.0, nelem, lm, Rmax=12.0, nnodes=nn)
+    D = dia.build_diatomic(3, 1, 3.0, nn, nelem, lm, Rmax=12.0)
+    F = DiatomicOracle(D)
+    for blockdiag in (False, True):
+        P = bound_density(D, 1, seed=nn, blockdiag=blockdiag)
+        ref = F.exchange(P)
+        Pd = to_dev(torch, P)
+        for symmetric in (False, True):
+            for split, tol in ((False, 1e-10), (True, 1e-11)):
+                K = torch.full_like(Pd, np.nan)
+                d.exchange(Pd, K, symmetric=symmetric, split=split)
+                torch.cuda.synchronize()
+                err = relerr(from_dev(K), ref)
+                assert err < tol, (blockdiag, symmetric, split, err)
