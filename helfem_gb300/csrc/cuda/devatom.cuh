@@ -34,8 +34,14 @@ struct DevAtom {
   const int* kterm_blk;
   const int* kterm_off;  // density offset of the term's block: l*nrad*nbf + i*nrad
   const double* kterm_coef;
+  const int* kterm_L;    // multipole of the term's entry
+  const int* kterm_ent;  // the term's entry
   int nent;
   int max_terms_per_jk; // bound on terms of one output block
+  const int* kent_sig;  // the entry's output block jk | min(multipole, 7) << 24
+  // [nang*nang] output blocks, like multipole sets together: jk, first term,
+  // number of terms, j | k << 16
+  const int4* jk_order;
   // split-precision copies: every FP64 value v stored as float2 (hi, lo) with
   // hi = fl32(v), lo = fl32(v - hi)
   const float2* rs2 = nullptr;
@@ -54,14 +60,20 @@ struct DevScratch {
   double* jin;          // [nchan*nel*nn*nn]
   double* jscal;        // [nchan*nel*2]
   double* khalo;        // [nel*nel*nang*nang*(2nn-1)]
-  double* bnorm;        // [nang*nang*NORM_SPLIT] partial squared block norms
+  double* bnorm;        // [nang*nang][nel] squared norms of each block's columns of an element
+  unsigned int* count;  // norm-pass CTAs done (the last one sets the flags)
+  unsigned int* tmax;   // [nang*nang][nel][nel] largest |high word| of each density tile (split path)
   unsigned char* act;   // [nang*nang] density block above the screen
   unsigned char* ent_act;  // [nent] exchange entry with an active term
   float2* p2;           // [nbf*nbf] split copy of the density (split path)
+  // output blocks with an active entry, in jk_order (then those with j <= k),
+  // their counts, and per group of 8 of the first list the multipoles (bits)
+  // that some block of it has
+  int* olist;           // [2*nang*nang]
+  int4* oinfo;          // [nang*nang] of the first list: as jk_order
+  int* ocount;          // [2]
+  int* gmask;           // [ceil(nang*nang/8)]
 };
-
-// Column bands per angular block in the density-norm pass
-#define NORM_SPLIT 16
 
 // Exchange work units (int4: a, b, lo, hi), built once per atom on the host.
 // a != b: element pair, output blocks jk in [lo, hi) (natural order);
@@ -80,16 +92,16 @@ struct KUnits {
 __host__ __device__ inline int gfun(const DevAtom& A, int e, int p) { return e * (A.nn - 1) + p - 1; }
 
 // Tensor-core split-precision exchange (k_tc.cu): the radial tables as
-// balanced base-256 digit planes (bf16, 16 x 16 in the no-swizzle K-major
-// operand layout) with one power-of-two scale per row, the output blocks in
-// groups of up to 8, and the work units (a, b, range of groups).
-#define TC_NDIGITS 7
+// balanced base-1024 digit planes (f16, 16 x 16 in the no-swizzle K-major
+// operand layout) with one power-of-two scale per table and one per row
+// (shared by the multipoles), the output blocks in groups of up to 8, and the
+// work units (a, b, range of groups).
+#define TC_NDIGITS 6
 #define TC_TPLANE 512
 struct DevTC {
   const unsigned char* digits = nullptr;  // [kind (0 r_small, 1 r_big)][L][e][TC_NDIGITS][TC_TPLANE]
-  const int* rowexp = nullptr;            // [kind][L][e][16]
-  const int* group_jk = nullptr;          // [ngroups][8], -1: empty slot
-  const int* group_ent = nullptr;         // [ngroups][8][NL], -1: no entry with that L
+  const int* texp = nullptr;              // [kind][L][e] table exponent
+  const int* rowexp = nullptr;            // [kind][e][16] row exponents
   int ngroups = 0;
   const int4* units_sym = nullptr;        // (a, b, first group, end group), a < b
   int n_sym = 0;
@@ -97,19 +109,11 @@ struct DevTC {
   int n_all = 0;
   int* err = nullptr;                     // set when a completion wait ran out
   // diagonal element tiles: the exchange-ordered tensor as digit planes
-  // [L][e][row tile][K step][digit][128 x 16], per-row exponents, groups of
-  // up to 16 output blocks (j <= k in symmetric mode), units (a, group, row tile)
+  // [L][e][row tile][K step][digit][128 x 16] and per-row exponents
   const unsigned char* tk_digits = nullptr;
   const int* tk_rowexp = nullptr;         // [L][e][row tile][128]
   int dmtiles = 0, dksteps = 0;
-  const int* dgroup_jk_sym = nullptr;     // [groups][16]
-  const int* dgroup_ent_sym = nullptr;    // [groups][16][NL]
-  const int* dgroup_jk_all = nullptr;
-  const int* dgroup_ent_all = nullptr;
-  const int4* dunits_sym = nullptr;
-  int n_dsym = 0;
-  const int4* dunits_all = nullptr;
-  int n_dall = 0;
+  int dgroups = 0;                        // groups of 16 output blocks (at most), set per launch
 };
 
 #ifdef __CUDACC__

@@ -17,18 +17,22 @@ namespace hfg {
 // 2^-47 |v|. Values below 2^-126 and non-finite inputs map to (0, 0) and
 // (v, 0) respectively.
 static __device__ __forceinline__ float2 split_bits(double v) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-  const int e = (int)((b >> 52) & 0x7FF);
-  if (e == 0x7FF) return make_float2((float)v, 0.f);
-  const int E = e - 1023;
-  if (E < -126) return make_float2(0.f, 0.f);
-  const unsigned long long S = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-  const float sgn = (b >> 63) ? -1.f : 1.f;
-  const float hi = sgn * ldexpf(__uint2float_rn((unsigned)(S >> 29)), E - 23);
-  const float lo = sgn * ldexpf(__uint2float_rn((unsigned)(S & 0x1FFFFFFFull)), E - 52);
-  return make_float2(hi, lo);
+  const unsigned top = (unsigned)__double2hiint(v), low = (unsigned)__double2loint(v);
+  // hi: sign, exponent and the top 23 fraction bits as they are; lo: the
+  // remaining 29 bits, converted (rounded to 24) and scaled by 2^(E - 52) in
+  // two steps, E hi's exponent (the first exact, a subnormal result rounds once)
+  const unsigned h = (top & 0x80000000u) | ((__funnelshift_l(low, top, 3) - 0x40000000u) & 0x7FFFFFFFu);
+  const float l = __fmul_rn(__fmul_rn(__uint2float_rn(low & 0x1FFFFFFFu), 2.220446049250313e-16f),  // 2^-52
+                            __uint_as_float(h & 0x7F800000u));
+  float2 r = make_float2(__uint_as_float(h), __uint_as_float(__float_as_uint(l) | (top & 0x80000000u)));
+  if ((top & 0x7FFFFFFFu) - (897u << 20) >= (254u << 20)) {  // outside the normal floats
+    const unsigned e = (top >> 20) & 0x7FFu;
+    if (e == 0x7FFu) r = make_float2((float)v, 0.f);
+    else if (e < 897u) r = make_float2(0.f, 0.f);
+    else r = make_float2(__uint_as_float((top & 0x80000000u) | 0x7F800000u), 0.f);
+  }
+  return r;
 }
-
 
 struct ffv {
   float hi, lo;

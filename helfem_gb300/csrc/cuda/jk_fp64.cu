@@ -12,7 +12,8 @@
 //                loop) and the Gaunt-weighted bra scatter.
 // K restates TwoDBasisT::exchange (TwoDBasis.cpp:879-999) with
 // assemble_K_FE_one_multipole_cached_chol (CoulombExchangeFE.h:484-530):
-//   k_block_norms : density-block screening, ||P_il||_F < 10 eps skipped.
+//   k_block_norms : density-block screening, ||P_il||_F < 10 eps skipped, and
+//                   the split copy of the density.
 //   k_tiles       : work units of (element pair, range of output angular
 //                   blocks). Off-diagonal pairs: recouple the (a,b) tiles of
 //                   P, then A_L X B_L^T with A/B = r_small/r_big by element
@@ -303,73 +304,226 @@ __global__ void j_scatter(DevAtom A, DevScratch S, double* __restrict__ J, int a
 }
 
 // ----------------------------------------------------------------- exchange
-// Partial Frobenius norms of the angular blocks of P: grid (nang^2, NORM_SPLIT),
-// each CTA sums a band of columns; consumers add the partials in a fixed
-// order and apply the reference's 10*DBL_EPSILON screen.
-__global__ void k_block_norms(DevAtom A, const double* __restrict__ P, double* __restrict__ part,
-                              float2* __restrict__ p2) {
+// Density pass, grid (nang^2, nel), thread = row: the columns of one element of
+// one angular block. Squared norms of the columns that the element owns (the
+// shared last one is the next element's), and in the split form (p2) the
+// float-pair copy and the largest high word of every density tile of the
+// element's columns. The last CTA adds the norms up in a fixed order, applies
+// the reference's 10*DBL_EPSILON screen and marks the exchange entries that
+// see an active block (its own launch took 6 us for Kr and 30 us for l <= 3,
+// every entry summing its blocks' partial norms again).
+// Bound by HBM (202 MB read, 202 MB written for Kr in the split form, 320 and
+// 320 MB for the l <= 3 atom of 33 elements); up to eight loads in flight per
+// thread. With the flags 82 us (Kr) and 144 us; without the last CTA's part 75
+// and 117 us; the norms without the tiles' maxima plus the flags' own launch
+// took 90 and 137 us.
+template <bool SPLIT>
+__global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict__ P, float2* __restrict__ p2,
+                              int symmetric) {
   __shared__ double red[32];
-  const int blk = blockIdx.x, i = blk % A.nang, l = blk / A.nang;
-  const int c0 = (int)((long)A.nrad * blockIdx.y / NORM_SPLIT);
-  const int c1 = (int)((long)A.nrad * (blockIdx.y + 1) / NORM_SPLIT);
+  __shared__ bool last;
+  __shared__ int cnt[64];
+  extern __shared__ unsigned int emax[];  // [nel] (split form); flags of the last CTA
+  const int blk = blockIdx.x, i = blk % A.nang, l = blk / A.nang, b = blockIdx.y, nn = A.nn;
+  const int c0 = max(gfun(A, b, 0), 0), c1 = min(gfun(A, b, nn - 1), A.nrad - 1);
+  const int nc = c1 - c0 + 1, nown = b == A.nel - 1 ? nc : nc - 1;  // columns, those owned
+  if (SPLIT) {
+    for (int e = threadIdx.x; e < A.nel; e += blockDim.x) emax[e] = 0u;
+    __syncthreads();
+  }
   double s = 0.0;
   float sf = 0.f;
-  // the band's elements in column order (32-bit index arithmetic); four
-  // loads in flight per thread (one at a time left the pass latency-bound
-  // at half the HBM rate; eight measured the same as four), summed in the
-  // same order as one at a time
-  constexpr int NU = 4;
-  const int n = A.nrad * (c1 - c0), bd = blockDim.x;
-  for (int base = threadIdx.x; base < n; base += NU * bd) {
-    double v[NU];
-    size_t o[NU];
-#pragma unroll
-    for (int u = 0; u < NU; ++u) {
-      const int idx = base + u * bd;
-      const int r = idx % A.nrad, c = c0 + idx / A.nrad;
-      o[u] = (size_t)(l * A.nrad + c) * A.nbf + (size_t)i * A.nrad + r;
-      v[u] = idx < n ? P[o[u]] : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < NU; ++u) {
-      if (base + u * bd >= n) break;
-      if (p2) {
-        // split path: integer-only split (no FP64-pipe instructions) and an
-        // FP32 norm of the high words for the screen
-        const float2 h = split_bits(v[u]);
-        p2[o[u]] = h;
+  const size_t base = (size_t)l * A.nrad * A.nbf + (size_t)i * A.nrad + (size_t)c0 * A.nbf;
+  constexpr int NU = 8;  // loads in flight: the columns in equal passes of at most that many
+  const int nu = (nown + (nown + NU - 1) / NU - 1) / ((nown + NU - 1) / NU);
+  for (int r = threadIdx.x; r < A.nrad; r += blockDim.x) {
+    unsigned int mx = 0u;
+    const double* p = P + base + r;
+    float2* q = SPLIT ? p2 + base + r : nullptr;
+    auto add = [&](double v) {
+      if (SPLIT) {
+        // integer-only split (no FP64-pipe instructions) and an FP32 norm of
+        // the high words for the screen
+        const float2 h = split_bits(v);
+        mx = max(mx, __float_as_uint(h.x) & 0x7FFFFFFFu);
+        *q = h;
+        q += A.nbf;
         sf = fmaf(h.x, h.x, sf);
       } else {
-        s += v[u] * v[u];
+        s += v * v;
       }
+    };
+    const double vb = SPLIT && nown < nc ? p[(size_t)nown * A.nbf] : 0.0;  // the next element's first column
+    for (int c = 0; c < nown; c += nu) {
+      const int len = min(nu, nown - c);
+      double v[NU];
+#pragma unroll
+      for (int w = 0; w < NU; ++w)
+        if (w < len) v[w] = p[(size_t)w * A.nbf];
+#pragma unroll
+      for (int w = 0; w < NU; ++w)
+        if (w < len) add(v[w]);
+      p += (size_t)nu * A.nbf;
+    }
+    if (SPLIT) mx = max(mx, __float_as_uint(split_bits(vb).x) & 0x7FFFFFFFu);
+    if (SPLIT) {
+      // row r is function r + 1 - a (nn - 1) of element a, and the last of the one before
+      const int a = (r + 1) / (nn - 1), f = (r + 1) - a * (nn - 1);
+      if (a < A.nel) atomicMax(&emax[a], mx);
+      if (a > 0 && f == 0) atomicMax(&emax[a - 1], mx);
     }
   }
-  if (p2) s = (double)sf;
-  s = block_sum(s, red);
-  if (threadIdx.x == 0) part[blk * NORM_SPLIT + blockIdx.y] = s;
+  if (SPLIT) {  // float sums by warp, in a fixed order
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sf += __shfl_xor_sync(0xffffffffu, sf, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = (double)sf;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int v = 0; v < (int)blockDim.x >> 5; ++v) s += red[v];
+    for (int e = threadIdx.x; e < A.nel; e += blockDim.x) S.tmax[((size_t)blk * A.nel + e) * A.nel + b] = emax[e];
+  } else {
+    s = block_sum(s, red);
+  }
+  // ---- the last CTA: flags (bnorm alone is read here: the copy and the
+  // maxima are the next kernels' and need no fence) ----
+  const int nang2 = A.nang * A.nang;
+  if (threadIdx.x == 0) {
+    S.bnorm[(size_t)b * nang2 + blk] = s;
+    __threadfence();
+    last = atomicAdd(S.count, 1u) == gridDim.x * gridDim.y - 1;
+    if (last) __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  // (dynamic shared memory past emax: block, entry and output-block flags)
+  unsigned char* sact = reinterpret_cast<unsigned char*>(emax + (SPLIT ? A.nel + nang2 : 0));
+  unsigned char* sent = sact + nang2;
+  int* sout = reinterpret_cast<int*>(emax) + A.nel;  // multipoles of a block's active entries (bits)
+  for (int x = threadIdx.x; x < nang2; x += blockDim.x) {
+    double q = 0.0;
+#pragma unroll 16
+    for (int e = 0; e < A.nel; ++e) q += __ldcg(&S.bnorm[(size_t)e * nang2 + x]);
+    const unsigned char f = !(sqrt(q) < 10.0 * DBL_EPSILON);
+    sact[x] = f;
+    S.act[x] = f;
+  }
+  if (threadIdx.x == 0) *S.count = 0u;  // for the next call
+  __syncthreads();
+  // entries: every term marks its entry. (One CTA alone: each loop loads a
+  // batch before it stores, or the latencies of its loads add up.)
+  for (int ent = threadIdx.x; ent < A.nent; ent += blockDim.x) sent[ent] = 0;
+  __syncthreads();
+  constexpr int NB = 8;
+  const int nterm = A.kent_ptr[A.nent], step = blockDim.x;
+  for (int u0 = threadIdx.x; u0 < nterm; u0 += NB * step) {
+    int blk[NB], ent[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int u = min(u0 + i * step, nterm - 1);
+      blk[i] = A.kterm_blk[u];
+      ent[i] = A.kterm_ent[u];
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+      if (sact[blk[i]]) sent[ent[i]] = 1;
+  }
+  if (SPLIT)
+    for (int x = threadIdx.x; x < nang2; x += step) sout[x] = 0;
+  __syncthreads();
+  for (int e0 = threadIdx.x; e0 < A.nent; e0 += NB * step) {
+    int sig[NB];
+    if (SPLIT)
+#pragma unroll
+      for (int i = 0; i < NB; ++i) sig[i] = A.kent_sig[min(e0 + i * step, A.nent - 1)];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int e = e0 + i * step;
+      if (e >= A.nent) break;
+      S.ent_act[e] = sent[e];
+      if (SPLIT && sent[e]) atomicOr(&sout[sig[i] & 0xFFFFFF], 1 << (sig[i] >> 24));
+    }
+  }
+  if (!SPLIT) return;
+  // ---- split form: the active output blocks in jk_order. A symmetric
+  // density's transposed partner tile is written too: (j, k) counts as active
+  // where (k, j) is ----
+  for (int x = threadIdx.x; x < 64; x += blockDim.x) cnt[x] = 0;
+  __syncthreads();
+  // positions: warps count their parts of the order, then place them
+  const int part = ((nang2 + nw - 1) / nw + 31) / 32 * 32;
+  for (int pass = 0; pass < 2; ++pass) {
+    int n = 0, nh = 0;
+    if (pass) {
+      for (int v = 0; v < w; ++v) n += cnt[v], nh += cnt[32 + v];
+    }
+    for (int x0 = w * part; x0 < min((w + 1) * part, nang2); x0 += 32) {
+      const int x = x0 + lane;
+      const int4 info = x < nang2 ? A.jk_order[x] : make_int4(0, 0, 0, 0);
+      const int jk = info.x, j = info.w & 0xFFFF, k = info.w >> 16;
+      const bool on = x < nang2 && (sout[jk] || (symmetric && sout[k + j * A.nang])), half = on && j <= k;
+      const unsigned mo = __ballot_sync(0xffffffffu, on), mh = __ballot_sync(0xffffffffu, half);
+      const unsigned below = (1u << lane) - 1u;
+      if (pass && on) {
+        S.olist[n + __popc(mo & below)] = jk;
+        S.oinfo[n + __popc(mo & below)] = info;
+      }
+      if (pass && half) S.olist[nang2 + nh + __popc(mh & below)] = jk;
+      n += __popc(mo);
+      nh += __popc(mh);
+    }
+    if (!pass && lane == 0) {
+      cnt[w] = n;
+      cnt[32 + w] = nh;
+    }
+    __syncthreads();
+  }
+  int n = 0, nh = 0;
+  for (int v = 0; v < nw; ++v) n += cnt[v], nh += cnt[32 + v];
+  if (threadIdx.x == 0) {
+    S.ocount[0] = n;
+    S.ocount[1] = nh;
+  }
+  for (int g = threadIdx.x; g < (n + 7) / 8; g += blockDim.x) {
+    int m = 0;
+#pragma unroll
+    for (int x = 8 * g; x < 8 * g + 8; ++x)
+      if (x < n) m |= sout[S.olist[x]];
+    S.gmask[g] = m ? m : 1;
+  }
 }
 
-// density-block screen (10*DBL_EPSILON, the reference's threshold) and the
-// exchange entries that see an active block, once per build
-__global__ void k_flags(DevAtom A, DevScratch S) {
-  const int nang2 = A.nang * A.nang;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  for (int idx = tid; idx < nang2; idx += nth) {
-    double s = 0.0;
-    for (int c = 0; c < NORM_SPLIT; ++c) s += S.bnorm[idx * NORM_SPLIT + c];
-    S.act[idx] = !(sqrt(s) < 10.0 * DBL_EPSILON);
+// K of the output blocks without an active entry (the tensor-core tiles run
+// over the active ones alone); grid (nang^2, column bands)
+__global__ void k_zero_inactive(DevAtom A, DevScratch S, double* __restrict__ K, int symmetric) {
+  __shared__ int on;
+  const int jk = blockIdx.x, j = jk % A.nang, k = jk / A.nang, kj = k + j * A.nang;
+  if (threadIdx.x == 0) on = 0;
+  __syncthreads();
+  for (int e = A.kjk_ptr[jk] + threadIdx.x; e < A.kjk_ptr[jk + 1]; e += blockDim.x)
+    if (S.ent_act[e]) on = 1;
+  if (symmetric)
+    for (int e = A.kjk_ptr[kj] + threadIdx.x; e < A.kjk_ptr[kj + 1]; e += blockDim.x)
+      if (S.ent_act[e]) on = 1;
+  __syncthreads();
+  if (on) return;
+  for (int c = blockIdx.y * 8 + (threadIdx.x >> 5); c < A.nrad; c += 8 * gridDim.y) {
+    double* Kc = K + (size_t)(k * A.nrad + c) * A.nbf + (size_t)j * A.nrad;
+#pragma unroll 4
+    for (int r = threadIdx.x & 31; r < A.nrad; r += 32) Kc[r] = 0.0;
   }
-  // every thread recomputes the block flags its entries need (no grid sync)
-  for (int ent = tid; ent < A.nent; ent += nth) {
-    bool any = false;
-    for (int u = A.kent_ptr[ent]; u < A.kent_ptr[ent + 1] && !any; ++u) {
-      const int blk = A.kterm_blk[u];
-      double s = 0.0;
-      for (int c = 0; c < NORM_SPLIT; ++c) s += S.bnorm[blk * NORM_SPLIT + c];
-      any = !(sqrt(s) < 10.0 * DBL_EPSILON);
-    }
-    S.ent_act[ent] = any ? 1 : 0;
-  }
+}
+
+inline size_t norm_smem(const DevAtom& A, bool split) {
+  const size_t nang2 = (size_t)A.nang * A.nang;
+  return (split ? sizeof(int) * (A.nel + nang2) : 0) + nang2 + A.nent;
+}
+
+// threads of k_block_norms: the rows in equal passes of at most 224, so that
+// several CTAs share an SM and one's sums and count overlap another's loads
+inline int norm_threads(const DevAtom& A) {
+  const int passes = (A.nrad + 223) / 224;
+  return std::max(64, ((A.nrad + passes - 1) / passes + 31) / 32 * 32);
 }
 
 __device__ __forceinline__ void load_active(const DevAtom& A, const DevScratch& S, unsigned char* act) {
@@ -647,11 +801,11 @@ __global__ void __launch_bounds__(320) k_tiles_split(DevAtom A, DevScratch S, co
 
 // one CTA per element pair (a,b), all output blocks: the first row/column of
 // each tile receives its neighbours' halo entries in a fixed order
-__global__ void k_fixup(DevAtom A, DevScratch S, double* __restrict__ K) {
+__global__ void k_fixup(DevAtom A, DevScratch S, double* __restrict__ K, int active_only) {
   const int a = blockIdx.x % A.nel, b = blockIdx.x / A.nel;
-  const int nn = A.nn, per = 2 * nn - 3, nang2 = A.nang * A.nang;
-  for (int w = threadIdx.x; w < per * nang2; w += blockDim.x) {
-    const int idx = w % per, jk = w / per;
+  const int nn = A.nn, per = 2 * nn - 3, nblk = active_only ? S.ocount[0] : A.nang * A.nang;
+  for (int w = threadIdx.x; w < per * nblk; w += blockDim.x) {
+    const int idx = w % per, jk = active_only ? S.olist[w / per] : w / per;
     const int j = jk % A.nang, k = jk / A.nang;
     int p, q;
     double v;
@@ -743,8 +897,7 @@ cudaError_t launch_exchange_erfc(const DevAtom& A, const DevScratch& S, const do
   const int n2 = A.nn * A.nn, nang2 = A.nang * A.nang;
   {
     Mark m(prof, KC_K_NORMS, st);
-    k_block_norms<<<dim3(nang2, NORM_SPLIT), 256, 0, st>>>(A, P, S.bnorm, nullptr);
-    k_flags<<<std::max(1, std::min(152, (A.nent + 255) / 256)), 256, 0, st>>>(A, S);
+    k_block_norms<false><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, false), st>>>(A, S, P, nullptr, 0);
   }
   {
     Mark m(prof, KC_K_TILES, st);
@@ -755,7 +908,7 @@ cudaError_t launch_exchange_erfc(const DevAtom& A, const DevScratch& S, const do
   }
   {
     Mark m(prof, KC_K_FIXUP, st);
-    k_fixup<<<A.nel * A.nel, 256, 0, st>>>(A, S, K);
+    k_fixup<<<A.nel * A.nel, 256, 0, st>>>(A, S, K, 0);
   }
   return cudaGetLastError();
 }
@@ -765,8 +918,7 @@ cudaError_t launch_exchange_fp64(const DevAtom& A, const DevScratch& S, const KU
   const int n2 = A.nn * A.nn, th = threads_for(n2), nang2 = A.nang * A.nang;
   {
     Mark m(prof, KC_K_NORMS, st);
-    k_block_norms<<<dim3(nang2, NORM_SPLIT), 256, 0, st>>>(A, P, S.bnorm, nullptr);
-    k_flags<<<std::max(1, std::min(152, (A.nent + 255) / 256)), 256, 0, st>>>(A, S);
+    k_block_norms<false><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, false), st>>>(A, S, P, nullptr, 0);
   }
   {
     Mark m(prof, KC_K_TILES, st);
@@ -779,7 +931,7 @@ cudaError_t launch_exchange_fp64(const DevAtom& A, const DevScratch& S, const KU
   }
   {
     Mark m(prof, KC_K_FIXUP, st);
-    k_fixup<<<A.nel * A.nel, 256, 0, st>>>(A, S, K);
+    k_fixup<<<A.nel * A.nel, 256, 0, st>>>(A, S, K, 0);
   }
   return cudaGetLastError();
 }
@@ -790,8 +942,7 @@ cudaError_t launch_exchange_split(const DevAtom& A, const DevScratch& S, const K
   const int n2 = A.nn * A.nn, th = threads_for(n2), nang2 = A.nang * A.nang;
   {
     Mark m(prof, KC_K_NORMS, st);
-    k_block_norms<<<dim3(nang2, NORM_SPLIT), 256, 0, st>>>(A, P, S.bnorm, S.p2);
-    k_flags<<<std::max(1, std::min(152, (A.nent + 255) / 256)), 256, 0, st>>>(A, S);
+    k_block_norms<true><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, true), st>>>(A, S, P, S.p2, symmetric ? 1 : 0);
   }
   {
     Mark m(prof, KC_K_TILES, st);
@@ -808,12 +959,14 @@ cudaError_t launch_exchange_split(const DevAtom& A, const DevScratch& S, const K
         e = cudaEventRecord(side->fork, st);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(side->s, side->fork, 0);
         if (e == cudaSuccess) e = launch_k_diag_tc(A, S, *tc, symmetric, K, side->s);
+        k_zero_inactive<<<dim3(nang2, 8), 256, 0, side->s>>>(A, S, K, symmetric ? 1 : 0);
         if (e == cudaSuccess) e = cudaEventRecord(side->join, side->s);
         if (e == cudaSuccess) e = launch_k_tiles_tc(A, S, *tc, symmetric, K, st);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(st, side->join, 0);
       } else {
         e = launch_k_tiles_tc(A, S, *tc, symmetric, K, st);
         if (e == cudaSuccess) e = launch_k_diag_tc(A, S, *tc, symmetric, K, st);
+        k_zero_inactive<<<dim3(nang2, 8), 256, 0, st>>>(A, S, K, symmetric ? 1 : 0);
       }
       if (e != cudaSuccess) return e;
       nunits = 0;
@@ -828,7 +981,7 @@ cudaError_t launch_exchange_split(const DevAtom& A, const DevScratch& S, const K
   }
   {
     Mark m(prof, KC_K_FIXUP, st);
-    k_fixup<<<A.nel * A.nel, 256, 0, st>>>(A, S, K);
+    k_fixup<<<A.nel * A.nel, 256, 0, st>>>(A, S, K, tc ? 1 : 0);
   }
   return cudaGetLastError();
 }

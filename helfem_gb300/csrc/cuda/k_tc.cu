@@ -12,35 +12,53 @@
 //
 // Arithmetic (an Ozaki-style slicing with exact integer sums):
 //  * every operand is a fixed-point number below 1 written as balanced
-//    base-256 digits: x = sum_k d_k 256^-(k+1), |d_0| <= 256, |d_k| <= 128
-//    (k >= 1, the 4th digit of a density tile may reach 256); digits are
-//    integers, exact in bf16;
-//  * the radial tables and Tk are digitised once per atom with one
-//    power-of-two scale per row (row sum of |values| <= 1 after scaling); a
-//    density tile X (recoupled on the CUDA cores in float pairs) gets one
-//    scale per tile;
+//    digits, x = sum_k d_k b^-(k+1): integers, exact in the 16-bit operand
+//    type. Element pairs: base 1024 (|d_0| <= 1024, the others <= 512) in f16,
+//    six digits of the tables and of the intermediate, five of a density tile
+//    (50 bits: a float pair has 48). Diagonal elements: base 256 (|d_0| <= 256,
+//    |d_k| <= 128) in bf16, seven and six;
+//  * the radial tables are digitised once per atom: a power of two per table
+//    (L, element) brings its largest entry near 1, then one power of two per
+//    row, shared by all multipoles, its absolute row sums to at most 1; Tk one
+//    power of two per row;
+//  * a recoupled density tile X_L (float pairs on the CUDA cores) of an element
+//    pair is scaled by 2^(s_L - E), s_L the exponents of the pair's two tables
+//    of multipole L and E one exponent per output block, from the largest
+//    entries of the density tiles (taken in the norm pass): with tables of all
+//    multipoles near 1 and one scale for all X_L of a block, the products of
+//    all multipoles add up in tensor memory;
 //  * the tensor core forms the digit products level by level,
-//    acc_d = sum_{k+l=d} sum_p a_k b_l (d = 0..6), in FP32 in tensor memory;
-//    for the 16-term products of the off-diagonal tiles every acc_d is an
-//    integer below 2^23, so the FP32 sums are exact;
-//  * the levels are carried into balanced digits again on the CUDA cores:
-//    the first product (Y = A X, 128 rows = 8 output blocks x 16) becomes the
-//    digit operand of the second (Y B^T), whose levels are turned into a
-//    float pair, scaled, and accumulated over the multipoles of the output
-//    block; one FP64 conversion per output element at the end.
-// Truncation (levels above 6 dropped, 48-bit density tiles) leaves ~1e-14 of
-// max|K| against the FP64 result.
+//    acc_d = sum_{k+l=d} sum_p a_k b_l, in FP32 in tensor memory. The element
+//    pairs' sums run over 16 terms and up to 8 multipoles: leading digits obey
+//    the unit row sums and the others are spread over +-512, so that a level's
+//    spread stays below 2^21, far from the 2^24 where FP32 sums of integers
+//    would round;
+//  * the levels of the first product (Y = A X, 128 rows = 8 output blocks x 16)
+//    are carried into balanced digits on the CUDA cores and become the operand
+//    of the second, which accumulates over the multipoles; its levels are
+//    turned into a float pair, scaled, and converted to FP64 once per output
+//    element and group.
+// Truncation (48-bit density tiles, the levels dropped) leaves ~1e-14 of
+// max|K| against the FP64 result. A row scale shared by the multipoles without
+// the per-table power of two lost log2(1/r) L bits near the nucleus.
 //
 // Off-diagonal work unit = one element pair (a,b) and a range of groups of
-// up to 8 output angular blocks; per group and multipole L the group's
-// entries with that L form one batch of M = 128 rows. For density digit kx
-// the table planes kt = 0..6-kx are consecutive in shared memory and form one
-// operand of N = 16 (7 - kx) rows whose block kt lands on the tensor-memory
-// columns of level kx + kt, so a batch is 6 + 7 MMAs. 256 threads: 8 warps
-// recouple one block each (the next batch's while the tensor core works on
-// the current one); warps w and w+4 read the same tensor-memory lanes and
-// split the columns.
+// 8 active output angular blocks (listed by the density pass); per group and
+// multipole L the group's entries with that L form one batch of M = 128 rows.
+// For density digit kx the table planes kt = 0..5-kx are consecutive in shared
+// memory and form one operand of N = 16 (6 - kx) rows whose block kt lands on
+// the tensor-memory columns of level kx + kt, so a batch is 5 + 6 MMAs. The
+// CUDA-core work on the digits is the bound (370 M warp instructions for the Kr
+// basis at 58 % of the issue slots; the tensor pipe is some 6 % busy), so what
+// matters is few instructions, warps that rarely wait and a loop that fits the
+// instruction cache: one copy of every phase, nothing unrolled that need not
+// be. Element pairs of the Kr basis (l <= 2, 40 elements): warps in step with
+// their MMAs and the multipoles read back one by one 0.87 ms; multipoles summed
+// in tensor memory, base 1024 0.79 ms; one arrival count instead of a warp that
+// issues 0.68 ms; terms streamed through one register buffer by compact loops
+// 0.57 ms.
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cfloat>
@@ -54,8 +72,10 @@
 namespace hfg {
 namespace {
 
-constexpr int ND = TC_NDIGITS;  // digits per table / intermediate operand
-constexpr int NDX = 6;          // digits of a float-pair density tile (48 bits)
+constexpr int PD = TC_NDIGITS;  // element pairs: digits of the tables and the intermediate, levels
+constexpr int PX = 5;           // digits of a density tile
+constexpr int ND = 7;           // diagonal elements: digits of Tk, levels
+constexpr int NDX = 6;          // digits of a density tile (48 bits)
 constexpr int APLANE = 4096;    // bytes of one 128 x 16 bf16 operand plane
 constexpr int TPLANE = 512;     // bytes of one 16 x 16 bf16 table plane
 
@@ -189,345 +209,533 @@ __device__ __forceinline__ double pair_to_d(ffv a) {
   return f2d_bits(n.hi) + f2d_bits(n.lo);
 }
 
-// recoupled density tile of (slot = warp, entry ent) for this lane's 8
-// elements (rows p = 8 ph + j, column q), float pairs; the loads of two
-// terms are in flight together
-__device__ __forceinline__ void recouple(const DevAtom& A, const unsigned char* act, int ent, const float2* base,
-                                         const bool (&vp)[8], ffv (&x)[8]) {
+// ---- element pairs: base 1024 in f16 ----
+
+__device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
+  const __half2 v = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// all six levels (16 columns apart) of 8 consecutive columns, one wait
+__device__ __forceinline__ void tmem_ld_pairs(uint32_t taddr, float (&v)[PD][4]) {
+  static_assert(PD == 6, "level count of the load below");
+  uint32_t r[24];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%24];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4,%5,%6,%7}, [%25];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8,%9,%10,%11}, [%26];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%12,%13,%14,%15}, [%27];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%16,%17,%18,%19}, [%28];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%20,%21,%22,%23}, [%29];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23])
+      : "r"(taddr), "r"(taddr + 16), "r"(taddr + 32), "r"(taddr + 48), "r"(taddr + 64), "r"(taddr + 80)
+      : "memory");
 #pragma unroll
-  for (int j = 0; j < 8; ++j) x[j] = {0.f, 0.f};
-  const int u1 = A.kent_ptr[ent + 1];
-  for (int uu = A.kent_ptr[ent]; uu < u1; uu += 2) {
-    float2 c[2], pv[2][8];
+  for (int d = 0; d < PD; ++d)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[d][j] = __uint_as_float(r[4 * d + j]);
+}
+
+// carry the level sums (weights 1024^-(d+2)) so that every level but the
+// first is a balanced digit; y0, y1 the first level's two digits
+__device__ __forceinline__ void carry_pairs(float (&a)[PD], float& y0, float& y1) {
+#pragma unroll
+  for (int d = PD - 1; d >= 1; --d) {
+    const float c = rnd_mul(a[d], 1.0f / 1024.0f);
+    a[d] = __fmaf_rn(c, -1024.0f, a[d]);
+    a[d - 1] = __fadd_rn(a[d - 1], c);
+  }
+  y0 = rnd_mul(a[0], 1.0f / 1024.0f);
+  y1 = __fmaf_rn(y0, -1024.0f, a[0]);
+}
+
+// float -> double times 2^k through the bit pattern (no FP64-pipe
+// instructions); c = (896 + k) << 20, zero and subnormal floats give zero
+__device__ __forceinline__ double f2d_scaled(float f, int c) {
+  const uint32_t bits = __float_as_uint(f), t = bits & 0x7FFFFFFFu;
+  const uint32_t hi = t < 0x00800000u ? 0u : ((t >> 3) + (uint32_t)c) | (bits & 0x80000000u);
+  return __hiloint2double((int)hi, t < 0x00800000u ? 0 : (int)(bits << 29));
+}
+
+// the value of the level sums (integers below 2^24, weights 1024^-(d+2)) times
+// 2^k, c as above: the leading three with their rounding errors, the rest as
+// they come
+__device__ __forceinline__ double levels_to_d(const float (&a)[PD], int c) {
+  auto two_sum = [](float x, float y, float& e) {
+    const float s = __fadd_rn(x, y), bb = __fsub_rn(s, x);
+    e = __fadd_rn(__fsub_rn(x, __fsub_rn(s, bb)), __fsub_rn(y, bb));
+    return s;
+  };
+  float e1, e2;
+  const float s1 = two_sum(__fmul_rn(a[0], 1.0f / 1048576.0f), __fmul_rn(a[1], 1.0f / 1073741824.0f), e1);
+  const float s2 = two_sum(s1, __fmul_rn(a[2], 1.0f / 1099511627776.0f), e2);
+  float tail = __fmaf_rn(a[5], 1.0f / 1024.0f, a[4]);
+  tail = __fmaf_rn(tail, 1.0f / 1024.0f, a[3]);
+  tail = __fmaf_rn(tail, 8.8817841970012523e-16f, __fadd_rn(e1, e2));  // weight 2^-50
+  return f2d_scaled(s2, c) + f2d_scaled(tail, c);
+}
+
+// the 5 balanced base-1024 digits of 8 float pairs scaled by 2^-30 s to below
+// 1, packed in f16 pairs: pk[k][j/2] holds elements j, j+1 of digit plane k.
+// The high word (24 bits) ends inside the third digit for the tile's largest
+// entries, where the low word joins it exactly.
+__device__ __forceinline__ void digits_pairs(const ffv (&x)[8], float s, uint32_t (&pk)[PX][4]) {
+#pragma unroll
+  for (int jj = 0; jj < 8; jj += 2) {
+    float dg[PX][2];
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
-      const bool on = uu + w < u1 && act[A.kterm_blk[uu + w]];
-      c[w] = on ? A.kterm_coef2[uu + w] : make_float2(0.f, 0.f);
-      const float2* pb = base + (on ? A.kterm_off[uu + w] : 0);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) pv[w][j] = (on && vp[j]) ? pb[j] : make_float2(0.f, 0.f);
+      const float h = __fmul_rn(x[jj + w].hi, s), l = __fmul_rn(x[jj + w].lo, s);
+      const float d0 = rnd_mul(h, 1.0f / 1048576.0f);
+      const float t1 = __fmaf_rn(d0, -1048576.0f, h);
+      const float d1 = rnd_mul(t1, 1.0f / 1024.0f);
+      const float t2 = __fmaf_rn(d1, -1024.0f, t1);
+      const float d2 = rnd(__fadd_rn(t2, l));
+      float r = __fadd_rn(__fsub_rn(t2, d2), l);
+      const float d3 = rnd_mul(r, 1024.0f);
+      r = __fmaf_rn(r, 1024.0f, -d3);
+      dg[0][w] = d0;
+      dg[1][w] = d1;
+      dg[2][w] = d2;
+      dg[3][w] = d3;
+      dg[4][w] = rnd_mul(r, 1024.0f);
     }
 #pragma unroll
-    for (int w = 0; w < 2; ++w)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] = ff_fma(x[j], c[w], pv[w][j]);
+    for (int k = 0; k < PX; ++k) pk[k][jj / 2] = pack_f16(dg[k][0], dg[k][1]);
   }
 }
 
-// digits of the recoupled tile written as rows (slot, q), K = p of the first
-// product's operand; returns the tile exponent (warp-wide maximum)
-__device__ __forceinline__ int digitise(ffv (&x)[8], unsigned char* A1, int row, int k0) {
-  unsigned eb = 0;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    x[j] = ff_norm(x[j].hi, x[j].lo);
-    eb = max(eb, (__float_as_uint(x[j].hi) >> 23) & 0xFFu);
-  }
-  const int E = tile_exponent(__reduce_max_sync(0xffffffffu, eb));
-  uint32_t pk[NDX][4];
-  digits_of(x, E, pk);
-  const uint32_t off = tc::off_kmajor(row, k0);
-#pragma unroll
-  for (int k = 0; k < NDX; ++k)
-    *reinterpret_cast<uint4*>(A1 + k * APLANE + off) = make_uint4(pk[k][0], pk[k][1], pk[k][2], pk[k][3]);
-  return E;
-}
-
-// the 8 values y[j] of tile (a,b), block jk, at row p and columns q0 + j:
-// one pass over the columns with the block's base address computed once;
-// owned entries go to K, the shared last row / column to the halo buffer
-__device__ __forceinline__ void store_rows(const DevAtom& A, const DevScratch& S, double* K, int a, int b, int jk,
-                                           int p, int q0, const double (&y)[8]) {
+// the 8 values y[j] of tile (a,b), block jk (-1: none), at row p and columns
+// q0 + j: one pass over the columns with the block's base address computed
+// once; owned entries go to K, the shared last row / column to the halo buffer
+__device__ __forceinline__ void store_rows(const DevAtom& A, const DevScratch& S, double* K, int a, int b, int j,
+                                           int k, int p, int q0, const double (&y)[4]) {
   const int nn = A.nn;
-  const int gp = gfun(A, a, p);
+  const int gp = gfun(A, a, p), gq0 = gfun(A, b, q0);
   if (p >= nn || gp < 0 || gp >= A.nrad) return;
-  const int j = jk % A.nang, k = jk / A.nang;
-  double* base = K + (size_t)k * A.nrad * A.nbf + (size_t)j * A.nrad + gp;
-  double* halo = S.khalo + ((size_t)(a * A.nel + b) * (A.nang * A.nang) + jk) * (2 * nn - 1);
+  const int lo = max(0, -gq0), hi = min(min(4, nn - q0), A.nrad - gq0);
+  double* halo = S.khalo + ((size_t)(a * A.nel + b) * (A.nang * A.nang) + j + k * A.nang) * (2 * nn - 1);
+  // the last row goes to the halo whole, of the others the last column
+  const bool last = p == nn - 1;
+  double* d = last ? halo + q0 : K + ((ptrdiff_t)k * A.nrad + gq0) * A.nbf + j * A.nrad + gp;
+  const int step = last ? 1 : A.nbf, jl = last ? -1 : nn - 1 - q0;
+  halo += nn + p;
 #pragma unroll
-  for (int jj = 0; jj < 8; ++jj) {
-    const int q = q0 + jj, gq = gfun(A, b, q);
-    if (q >= nn || gq < 0 || gq >= A.nrad) continue;
-    if (p <= nn - 2 && q <= nn - 2)
-      base[(size_t)gq * A.nbf] = y[jj];
-    else if (p == nn - 1)
-      halo[q] = y[jj];
-    else
-      halo[nn + p] = y[jj];
-  }
+  for (int jj = 0; jj < 4; ++jj, d += step)
+    if (jj >= lo && jj < hi) *(jj == jl ? halo : d) = y[jj];
 }
 
-struct Smem {
-  unsigned char* A1;  // NDX planes: rows (slot, q), K = p (K-major)
-  unsigned char* A2;  // ND planes: rows (slot, i), K = q (MN-major)
-  unsigned char* T1;  // NL * ND planes of the left tables of element a
-  unsigned char* T2;  // NL * ND planes of the right tables of element b
-  int* alpha;         // [NL][16] row exponents of the left tables
-  int* beta;          // [NL][16] row exponents of the right tables
-  int* ex;            // [2][8] tile exponents, by batch parity
-  int* sact;          // [NL][8] slot active in the batch of multipole L
-  int* gent;          // [8][NL] entry of (slot, L) or -1
-  int* gjk;           // [8] output block of the slot or -1
-  unsigned char* act; // [nang^2] density block above the screen
-  uint64_t* mbar;
-  uint32_t* tslot;
-  int* fail;
-};
+constexpr int PW = 8;                 // working warps
+constexpr int PTHREADS = 32 * PW;
+constexpr uint32_t kWait = 1u << 17;  // limit of every wait
 
+// working warps q and q + 4 (named barriers 1-4)
+__device__ __forceinline__ void pair_sync(int q) {
+  if (q == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
+  else if (q == 1) asm volatile("bar.sync 2, 64;" ::: "memory");
+  else if (q == 2) asm volatile("bar.sync 3, 64;" ::: "memory");
+  else asm volatile("bar.sync 4, 64;" ::: "memory");
+}
+
+// shared-memory layout of k_tiles_tc past the operand planes
+struct PairMeta {
+  int alpha[16], beta[16];  // row exponents of the left and right tables
+  int sL[8];                // table exponents of the pair
+  // per group (four in flight), slot: exponent of the scaled density tiles,
+  // multipoles present (bits), output block or -1
+  int ex[4][8], mask[4][8], jk[4][8];  // jk: j | k << 16
+  int fail;
+  uint32_t tslot;
+  int arrived;            // warps past their part of a batch, all batches
+  uint64_t done;          // a batch's second and the next one's first product
+};
 }  // namespace
 
-__global__ void __launch_bounds__(256, 2) k_tiles_tc(DevAtom A, DevScratch S, DevTC T, const int4* __restrict__ units,
-                                                     int symmetric, double* __restrict__ K) {
+// Each of 8 warps, per batch: recouple and digitise slot w's density tile of
+// the next batch into the other stage of the first operand, then read this
+// batch's first product back (the lanes of slots 2 (w & 3) and the next one,
+// half of the columns) and write its digits as the second operand; at the end
+// of a group the second product into K. The last warp through issues the next
+// first and this second product, which run while the warps recouple. One
+// arrival count per batch is all the synchronisation between warps (a warp of
+// its own that issues, with a barrier per role, cost 32 registers a thread).
+__global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch S, DevTC T,
+                                                          const int4* __restrict__ units, int symmetric,
+                                                          double* __restrict__ K) {
   const int4 u = units[blockIdx.x];
   const int a = u.x, b = u.y;
   const int nn = A.nn, NL = A.NL, nang2 = A.nang * A.nang;
+  const int count = S.ocount[0], g0 = u.z, g1 = min(u.w, (count + 7) / 8);
+  if (g0 >= g1) return;  // uniform over the CTA
   extern __shared__ __align__(1024) unsigned char smraw[];
-  Smem sm;
-  {
-    unsigned char* p = smraw;
-    sm.A1 = p;
-    p += NDX * APLANE;
-    sm.A2 = p;
-    p += ND * APLANE;
-    sm.T1 = p;
-    p += NL * ND * TPLANE;
-    sm.T2 = p;
-    p += NL * ND * TPLANE;
-    int* ip = reinterpret_cast<int*>(p);
-    sm.alpha = ip;
-    ip += NL * 16;
-    sm.beta = ip;
-    ip += NL * 16;
-    sm.ex = ip;
-    ip += 16;
-    sm.sact = ip;
-    ip += 8 * NL;
-    sm.gent = ip;
-    ip += 8 * NL;
-    sm.gjk = ip;
-    ip += 8;
-    sm.fail = ip;
-    ip += 2;
-    sm.mbar = reinterpret_cast<uint64_t*>(ip);
-    sm.tslot = reinterpret_cast<uint32_t*>(sm.mbar + 1);
-    sm.act = reinterpret_cast<unsigned char*>(sm.tslot + 2);
-  }
+  unsigned char* A1 = smraw;                   // 2 stages x PX planes: rows (slot, q), K = p (MN-major)
+  unsigned char* A2 = A1 + 2 * PX * APLANE;    // PD planes: rows (slot, i), K = q (MN-major)
+  unsigned char* T1 = A2 + PD * APLANE;        // NL * PD planes of the left tables of element a
+  unsigned char* T2 = T1 + NL * PD * TPLANE;   // NL * PD planes of the right tables of element b
+  PairMeta& m = *reinterpret_cast<PairMeta*>(T2 + NL * PD * TPLANE);
+  unsigned char* act = reinterpret_cast<unsigned char*>(&m + 1);  // [nang^2] density block above the screen
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int qw = warp & 3, half = warp >> 2;
 
   // ---- set-up once per unit: tables of this element pair, block flags ----
+  const int kl = (a < b) ? 0 : 1, kr = (a < b) ? 1 : 0;  // left: r_small(a) if a < b
   {
-    const int kl = (a < b) ? 0 : 1, kr = (a < b) ? 1 : 0;  // left: r_small(a) if a < b
-    const uint4* s1 = reinterpret_cast<const uint4*>(T.digits) + (size_t)(kl * NL * A.nel) * (ND * TPLANE / 16);
-    const uint4* s2 = reinterpret_cast<const uint4*>(T.digits) + (size_t)(kr * NL * A.nel) * (ND * TPLANE / 16);
-    const int per = ND * TPLANE / 16;  // uint4 per (L, e)
+    const int per = PD * TPLANE / 16;  // uint4 per (L, e)
+    const uint4* s1 = reinterpret_cast<const uint4*>(T.digits) + (size_t)(kl * NL * A.nel) * per;
+    const uint4* s2 = reinterpret_cast<const uint4*>(T.digits) + (size_t)(kr * NL * A.nel) * per;
     for (int idx = t; idx < NL * per; idx += blockDim.x) {
       const int L = idx / per, o = idx % per;
-      reinterpret_cast<uint4*>(sm.T1)[idx] = s1[((size_t)L * A.nel + a) * per + o];
-      reinterpret_cast<uint4*>(sm.T2)[idx] = s2[((size_t)L * A.nel + b) * per + o];
+      reinterpret_cast<uint4*>(T1)[idx] = s1[((size_t)L * A.nel + a) * per + o];
+      reinterpret_cast<uint4*>(T2)[idx] = s2[((size_t)L * A.nel + b) * per + o];
     }
-    for (int idx = t; idx < NL * 16; idx += blockDim.x) {
-      const int L = idx / 16, r = idx % 16;
-      sm.alpha[idx] = T.rowexp[((size_t)(kl * NL + L) * A.nel + a) * 16 + r];
-      sm.beta[idx] = T.rowexp[((size_t)(kr * NL + L) * A.nel + b) * 16 + r];
+    if (t < 16) {
+      m.alpha[t] = T.rowexp[((size_t)kl * A.nel + a) * 16 + t];
+      m.beta[t] = T.rowexp[((size_t)kr * A.nel + b) * 16 + t];
     }
-    for (int idx = t; idx < nang2; idx += blockDim.x) sm.act[idx] = S.act[idx];
-    if (t == 0) sm.fail[0] = 0;
+    if (t < NL) m.sL[t] = T.texp[((size_t)kl * NL + t) * A.nel + a] + T.texp[((size_t)kr * NL + t) * A.nel + b];
+    for (int idx = t; idx < nang2; idx += blockDim.x) act[idx] = S.act[idx];
+    if (t == 0) {
+      m.fail = 0;
+      m.arrived = 0;
+      tc::mbar_init(&m.done, 1);
+    }
   }
-  // operand rows of an idle slot are never cleared: a tensor-core row only
-  // feeds the same row of the result, and idle rows are never read back
   if (warp == 0) {
-    tc::tmem_alloc(sm.tslot, 256);
+    tc::tmem_alloc(&m.tslot, 256);
     tc::tmem_relinquish();
   }
-  if (t == 0) tc::mbar_init(sm.mbar, 1);
+  tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tbase = *sm.tslot;
-  const uint32_t tD1 = tbase, tD2 = tbase + 128;
-  const uint32_t lane_off = (uint32_t)(32 * qw) << 16;
-  uint32_t phase = 0;
-  const uint64_t dA1 = tc::smem_desc(tc::smem_u32(sm.A1)), dA2 = tc::smem_desc(tc::smem_u32(sm.A2));
-  const uint64_t dT1 = tc::smem_desc(tc::smem_u32(sm.T1)), dT2 = tc::smem_desc(tc::smem_u32(sm.T2));
+  const uint32_t tD1 = m.tslot, tD2 = m.tslot + 128;
 
-  // this thread's tensor-memory lane (slot, row) and columns [8 half, 8 half + 8)
-  const int m_out = 32 * qw + lane;
-  const int oslot = m_out >> 4, oi = m_out & 15;
-  const int pslot = 2 * qw + ((lane >> 4) ^ 1);  // the other slot of this warp's lanes
-
-  // recoupling layout: warp = slot, lane = (q, p-half)
-  const int rq = lane & 15, rph = lane >> 4;
-  const int gq = gfun(A, b, rq);
-  const bool vq = rq < nn && gq >= 0 && gq < A.nrad;
-  const int gp0 = gfun(A, a, 8 * rph);
-  bool vp[8];
+  {
+    // ---- producing: warp = slot, lane = (p, q-half), element j: column q =
+    // 8 qh + j. Consecutive lanes load consecutive rows of a column (a lane
+    // holding 8 rows of one column cost 32 cache lines per load, and the loads
+    // bounded the kernel), and the lane's 8 columns are one 16-byte row of the
+    // MN-major operand. ----
+    int s_hi = m.sL[0];
+    for (int L = 1; L < NL; ++L) s_hi = max(s_hi, m.sL[L]);
+    const int rp = lane & 15, qh = lane >> 4;
+    // Rows and columns past the tile repeat its last ones: finite digits, which
+    // meet zero rows of the tables. Functions outside the basis (first and last
+    // element) have table entries: their elements are zeroed.
+    const int pa0 = max(gfun(A, a, 0), 0), pa1 = min(gfun(A, a, nn - 1), A.nrad - 1);
+    const int qb0 = max(gfun(A, b, 0), 0), qb1 = min(gfun(A, b, nn - 1), A.nrad - 1);
+    const bool edge = gfun(A, a, 0) < 0 || gfun(A, b, 0) < 0 || gfun(A, a, nn - 1) >= A.nrad || gfun(A, b, nn - 1) >= A.nrad;
+    unsigned vm = 0;  // elements inside the basis
+    int coff[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int p = 8 * rph + j, gp = gp0 + j;
-    vp[j] = vq && p < nn && gp >= 0 && gp < A.nrad;
-  }
-  const float2* pbase = S.p2 + (size_t)(vq ? gq : 0) * A.nbf + gp0;
-
-  auto next_active = [&](int L0) {
-    for (int L = L0; L < NL; ++L) {
-      int any = 0;
-#pragma unroll
-      for (int s = 0; s < 8; ++s) any |= sm.sact[L * 8 + s];
-      if (any) return L;
+    for (int j = 0; j < 8; ++j) {
+      const int gp = gfun(A, a, rp), gq = gfun(A, b, 8 * qh + j);
+      if (gp >= pa0 && gp <= pa1 && gq >= qb0 && gq <= qb1) vm |= 1u << j;
+      coff[j] = min(max(gq, qb0), qb1) * A.nbf + min(max(gp, pa0), pa1);
     }
-    return -1;
-  };
-
-  for (int g = u.z; g < u.w; ++g) {
-    // ---- the group's entries and their activity ----
-    for (int idx = t; idx < 8 * NL; idx += blockDim.x) {
-      const int e = T.group_ent[(size_t)g * 8 * NL + idx];  // idx = slot * NL + L
-      sm.gent[idx] = e;
-      sm.sact[(idx % NL) * 8 + idx / NL] = (e >= 0 && S.ent_act[e]) ? 1 : 0;
-    }
-    if (t < 8) sm.gjk[t] = T.group_jk[g * 8 + t];
-    __syncthreads();
-
-    ffv acc[8];
+    const uint32_t off1 = tc::off_mnmajor(warp * 16 + 8 * qh, rp);
+    // the slot's terms of the group being produced, two per lane, multipoles
+    // ascending: density offset, coefficient, multipole (-1: block below the
+    // screen). Their
+    // tiles stream through one register buffer: an element's next value is
+    // loaded, for the next batch too, as soon as the last one is added.
+    int toff[2], tL[2], E = 0, mask = 0;
+    float2 tc2[2];
+    unsigned r0 = 0, r1 = 0;  // terms not yet loaded
+    float2 c = make_float2(0.f, 0.f), pv[8];  // coefficient and tile of the term in flight
+    int off = 0;
+    auto next_term = [&]() {  // its offset and coefficient; false: none left in the group
+      if (!(r0 | r1)) return false;
+      const bool lo = r0 != 0;
+      const int src = __ffs(lo ? r0 : r1) - 1;
+      if (lo) r0 &= r0 - 1; else r1 &= r1 - 1;
+      off = __shfl_sync(0xffffffffu, lo ? toff[0] : toff[1], src);
+      c.x = __shfl_sync(0xffffffffu, lo ? tc2[0].x : tc2[1].x, src);
+      c.y = __shfl_sync(0xffffffffu, lo ? tc2[0].y : tc2[1].y, src);
+      return true;
+    };
+    // A group's terms come in three steps, each load's latency covered by a
+    // part of the batch before: the block's range, its terms, the tile maxima.
+    int4 next = 8 * g0 + warp < count ? S.oinfo[8 * g0 + warp] : make_int4(-1, 0, 0, -1);
+    int tblk[2], pairjk = -1;
+    float bd[2];
+    auto terms_of = [&](int g) {
+      const int4 info = next;  // block, first term, terms, j | k << 16
+      next = g + 1 < g1 && 8 * g + 8 + warp < count ? S.oinfo[8 * g + 8 + warp] : make_int4(-1, 0, 0, -1);
+      pairjk = info.w;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = {0.f, 0.f};
-
-    // prologue: the first active batch's density tiles
-    int L = next_active(0);
-    int par = 0;
-    if (L >= 0 && sm.sact[L * 8 + warp]) {
-      ffv x[8];
-      recouple(A, sm.act, sm.gent[warp * NL + L], pbase, vp, x);
-      const int E = digitise(x, sm.A1, warp * 16 + rq, 8 * rph);
-      if (lane == 0) sm.ex[par * 8 + warp] = E;
-    }
-
-    while (L >= 0) {
-      const int Ln = next_active(L + 1);
-      tc::fence_async_smem();
-      tc::fence_before_sync();
-      __syncthreads();
-      tc::fence_after_sync();
-      if (sm.fail[0]) break;  // read after the barrier: uniform over the CTA
-      // ---- first product: D1[(slot,q), 16 level + i] ----
-      if (t == 0) {
-#pragma unroll 1
-        for (int kx = 0; kx < NDX; ++kx)
-          tc::mma_bf16(tD1 + 16 * kx, dA1 + (uint64_t)(kx * APLANE >> 4), dT1 + (uint64_t)(L * ND * TPLANE >> 4),
-                       tc::idesc_bf16(128, 16 * (ND - kx), 0, 0), kx > 0 ? 1u : 0u);
-        tc::mma_commit(sm.mbar);
-      }
-      // the next batch's recoupling (global loads) overlaps the tensor core
-      ffv xn[8];
-      const bool nact = Ln >= 0 && sm.sact[Ln * 8 + warp];
-      if (nact) recouple(A, sm.act, sm.gent[warp * NL + Ln], pbase, vp, xn);
-      if (!__all_sync(0xffffffffu, tc::mbar_wait(sm.mbar, phase)) && lane == 0) atomicExch(sm.fail, 1);
-      phase ^= 1u;
-      tc::fence_after_sync();
-
-      // ---- levels -> balanced digits of Y = A X, the second product's
-      // MN-major operand: rows (slot, i), K = q (lane = (slot, q)) ----
-      if (sm.sact[L * 8 + oslot] | sm.sact[L * 8 + pslot]) {
-        float v[ND][8];
-        tmem_ld_levels(tD1 + lane_off + 8 * half, v);
-        uint32_t pk[ND][4];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          float lv[ND], y[ND];
-#pragma unroll
-          for (int d = 0; d < ND; ++d) lv[d] = v[d][j];
-          carry(lv, y);
-#pragma unroll
-          for (int k = 0; k < ND; ++k) v[k][j] = y[k];
+      for (int r = 0; r < 2; ++r) {
+        tblk[r] = -1;
+        if (lane + 32 * r < info.z) {
+          const int uu = info.y + lane + 32 * r;
+          tblk[r] = A.kterm_blk[uu];
+          tc2[r] = A.kterm_coef2[uu];
+          toff[r] = A.kterm_off[uu];
+          tL[r] = A.kterm_L[uu];
         }
-#pragma unroll
-        for (int k = 0; k < ND; ++k)
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) pk[k][jj] = pack_bf16(v[k][2 * jj], v[k][2 * jj + 1]);
-        const uint32_t off = tc::off_mnmajor(oslot * 16 + 8 * half, oi);
-#pragma unroll
-        for (int k = 0; k < ND; ++k)
-          *reinterpret_cast<uint4*>(sm.A2 + k * APLANE + off) = make_uint4(pk[k][0], pk[k][1], pk[k][2], pk[k][3]);
       }
-      tc::fence_async_smem();
-      tc::fence_before_sync();
-      __syncthreads();
-      tc::fence_after_sync();
-      if (sm.fail[0]) break;
-
-      // ---- second product: D2[(slot,i), 16 level + r], issued from another
-      // warp than the first product so that the issue cost is shared ----
-      if (t == 128) {
-#pragma unroll 1
-        for (int ky = 0; ky < ND; ++ky)
-          tc::mma_bf16(tD2 + 16 * ky, dA2 + (uint64_t)(ky * APLANE >> 4), dT2 + (uint64_t)(L * ND * TPLANE >> 4),
-                       tc::idesc_bf16(128, 16 * (ND - ky), 1, 0), ky > 0 ? 1u : 0u);
-        tc::mma_commit(sm.mbar);
+    };
+    auto bounds_of = [&]() {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        bd[r] = 0.f;
+        if (tblk[r] >= 0 && act[tblk[r]])
+          bd[r] = __uint_as_float(S.tmax[((size_t)tblk[r] * A.nel + a) * A.nel + b]);
+        else
+          tL[r] = -1;
       }
-      // the next batch's digits go to the first operand (its MMAs are done)
-      if (nact) {
-        const int E = digitise(xn, sm.A1, warp * 16 + rq, 8 * rph);
-        if (lane == 0) sm.ex[(par ^ 1) * 8 + warp] = E;
+    };
+    // the scan of group g, and one exponent for its scaled tiles from the
+    // largest entries of the density tiles
+    auto enter = [&](int g) {
+      unsigned any = 0;
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        if (tL[r] >= 0) any |= 1u << tL[r];
+      r0 = __ballot_sync(0xffffffffu, tL[0] >= 0);
+      r1 = __ballot_sync(0xffffffffu, tL[1] >= 0);
+      mask = (int)__reduce_or_sync(0xffffffffu, any);
+      if (next_term())
+#pragma unroll
+        for (int j = 0; j < 8; ++j) pv[j] = S.p2[off + coff[j]];
+      // |X_L| <= sum of |c| max|P| (high words and roundings: 2^-20), summed
+      // upwards in units of 2^(e0 - 24): the largest multipole's, scaled by its
+      // tables, gives E (s_hi - 96 at least: every scale stays a normal float)
+      unsigned mx = 0;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        if (tL[r] >= 0) bd[r] *= fabsf(tc2[r].x) * 1.000001f * exp2i(m.sL[tL[r]] - s_hi);
+        mx = max(mx, __float_as_uint(bd[r]));
       }
-      if (!__all_sync(0xffffffffu, tc::mbar_wait(sm.mbar, phase)) && lane == 0) atomicExch(sm.fail, 1);
-      phase ^= 1u;
-      tc::fence_after_sync();
-
-      // ---- levels -> float pairs, scaled, accumulated over the multipoles ----
-      if (sm.sact[L * 8 + oslot] | sm.sact[L * 8 + pslot]) {
-        float v[ND][8];
-        tmem_ld_levels(tD2 + lane_off + 8 * half, v);
-        if (sm.sact[L * 8 + oslot]) {
-          const int ea = sm.alpha[L * 16 + oi] + sm.ex[par * 8 + oslot];
+      const int e0 = max((int)(__reduce_max_sync(0xffffffffu, mx) >> 23) - 126, -96);
+      unsigned su[2], top = 0;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) su[r] = __float2uint_ru(bd[r] * exp2i(24 - e0));
+      for (int L = 0; L < NL; ++L)
+        top = max(top, __reduce_add_sync(0xffffffffu, (tL[0] == L ? su[0] : 0u) + (tL[1] == L ? su[1] : 0u)));
+      E = max(s_hi - 96, s_hi + e0 + 8 - __clz(top));
+      if (lane == 0) {
+        m.ex[g & 3][warp] = E;
+        m.mask[g & 3][warp] = mask;
+        m.jk[g & 3][warp] = pairjk;
+      }
+    };
+    // slot's tile of multipole L into stage st
+    auto produce = [&](int L, int st) {
+      if ((mask >> L) & 1) {
+        int left = __popc(__ballot_sync(0xffffffffu, tL[0] == L)) + __popc(__ballot_sync(0xffffffffu, tL[1] == L));
+        ffv x[8];
+        {  // an exact product: no sum to carry
+          const float2 cc = c;
+          const bool more = next_term();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            float lv[ND];
-#pragma unroll
-            for (int d = 0; d < ND; ++d) lv[d] = v[d][j];
-            acc[j] = ff_add(acc[j], levels_to_pair(lv, exp2i(ea + sm.beta[L * 16 + 8 * half + j])));
+            const float p = __fmul_rn(cc.x, pv[j].x);
+            float pe = fmaf(cc.x, pv[j].x, -p);
+            pe = fmaf(cc.x, pv[j].y, pe);
+            x[j] = {p, fmaf(cc.y, pv[j].x, pe)};
+            if (more) pv[j] = S.p2[off + coff[j]];
           }
         }
+#pragma unroll 1
+        while (--left > 0) {
+          const float2 cc = c;
+          const bool more = next_term();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            x[j] = ff_fma(x[j], cc, pv[j]);
+            if (more) pv[j] = S.p2[off + coff[j]];
+          }
+        }
+        if (edge)
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (!((vm >> j) & 1u)) x[j] = {0.f, 0.f};
+        uint32_t pk[PX][4];
+        digits_pairs(x, exp2i(30 + m.sL[L] - E), pk);
+        unsigned char* o = A1 + st * PX * APLANE + off1;
+#pragma unroll
+        for (int k = 0; k < PX; ++k)
+          *reinterpret_cast<uint4*>(o + k * APLANE) = make_uint4(pk[k][0], pk[k][1], pk[k][2], pk[k][3]);
       }
+      // (operand rows of an idle slot keep their old digits: a tensor-core row
+      // only feeds the same row of the result)
+    };
+
+    // the last warp through its part of batch n issues the second product of
+    // batch n (L2 >= 0; start: the first of its group) and the first product of
+    // batch n + 1 (L1 >= 0)
+    auto issue = [&](int st, int L1, int L2, bool start) {
       tc::fence_before_sync();
-      L = Ln;
-      par ^= 1;
-    }
-    __syncthreads();
+      tc::fence_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        uint32_t was;
+        asm volatile("atom.acq_rel.cta.shared.add.u32 %0, [%1], 1;"
+                     : "=r"(was)
+                     : "r"(tc::smem_u32(&m.arrived))
+                     : "memory");
+        if ((was & (PW - 1)) == PW - 1) {
+          tc::fence_after_sync();
+          if (L1 >= 0) {
+            const uint64_t dA = tc::smem_desc(tc::smem_u32(A1 + st * PX * APLANE));
+            const uint64_t dT = tc::smem_desc(tc::smem_u32(T1 + L1 * PD * TPLANE));
+#pragma unroll
+            for (int kx = 0; kx < PX; ++kx)
+              tc::mma_bf16(tD1 + 16 * kx, dA + (uint64_t)(kx * APLANE >> 4), dT, tc::idesc_f16(128, 16 * (PD - kx), 1, 0),
+                           kx > 0 ? 1u : 0u);
+          }
+          if (L2 >= 0) {
+            const uint64_t dA = tc::smem_desc(tc::smem_u32(A2)), dT = tc::smem_desc(tc::smem_u32(T2 + L2 * PD * TPLANE));
+#pragma unroll
+            for (int ky = 0; ky < PD; ++ky)
+              tc::mma_bf16(tD2 + 16 * ky, dA + (uint64_t)(ky * APLANE >> 4), dT, tc::idesc_f16(128, 16 * (PD - ky), 1, 0),
+                           (!start || ky > 0) ? 1u : 0u);
+          }
+          tc::mma_commit(&m.done);
+        }
+      }
+      __syncwarp();
+    };
 
-    // ---- store: K_jk(a,b) rows p = oi, columns q = 8 half + j; the
-    // transposed partner K_kj(b,a) through shared memory ----
-    const bool failed = sm.fail[0] != 0;
-    const int jk = sm.gjk[oslot];
-    double y[8];
+    // ---- read-back: tensor-memory lanes 32 (w & 3) .. (two slots), columns
+    // 8 half ..; lane = (slot, q) in the first product, (slot, i) in the second ----
+    const int qw = warp & 3, half = warp >> 2;
+    const uint32_t lane_off = (uint32_t)(32 * qw) << 16;
+    const int oslot = 2 * qw + (lane >> 4), oi = lane & 15;
+    const uint32_t off2 = tc::off_mnmajor(oslot * 16 + 8 * half, oi);
+    int E2 = 0, mask2 = 0, jk = -1;  // of the group being read back
+    // a group's sums -> FP64: rows p = oi, columns q = 8 half + j; staged in
+    // this warp's part of the (free) second operand for the transposed partner
+    auto store_group = [&]() {
+      // entry (slot, r, c): 1 KB of each of four planes per pair of slots
+      auto stage = [&](int r, int cc) {
+        const int idx = (lane >> 4) * 256 + r * 16 + (cc ^ r);  // ^ r: spread over the banks
+        return reinterpret_cast<double*>(A2 + (idx >> 7) * APLANE + qw * 1024) + (idx & 127);
+      };
+      const int ea = m.alpha[oi] + E2;
+#pragma unroll 1
+      for (int h = 8 * half; h < 8 * half + 8; h += 4) {
+        float v[PD][4];
+        tmem_ld_pairs(tD2 + lane_off + h, v);
+        double y[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) y[j] = failed ? __longlong_as_double(0x7ff8000000000000ll) : -pair_to_d(acc[j]);
-    if (jk >= 0) store_rows(A, S, K, a, b, jk, oi, 8 * half, y);
-    if (symmetric) {
-      double* stage = reinterpret_cast<double*>(sm.A1);  // 8 x 16 x 16 doubles; every MMA has completed
+        for (int j = 0; j < 4; ++j) {
+          float lv[PD];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) stage[(oslot * 16 + oi) * 16 + 8 * half + j] = y[j];
-      __syncthreads();
-      if (jk >= 0) {
-        // partner row p' = oi, columns q' = 8 half + j
+          for (int d = 0; d < PD; ++d) lv[d] = v[d][j];
+          y[j] = -levels_to_d(lv, (max(ea + m.beta[h + j], -800) + 896) << 20);
+          if (symmetric) *stage(oi, h + j) = y[j];
+        }
+        if (jk >= 0) store_rows(A, S, K, a, b, jk & 0xFFFF, jk >> 16, oi, h, y);
+      }
+      if (symmetric) {
+        // both column halves are staged: warps w and w + 4
+        pair_sync(qw);
+#pragma unroll 1
+        for (int h = 8 * half; h < 8 * half + 8; h += 4) {
+          double y[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) y[j] = stage[(oslot * 16 + 8 * half + j) * 16 + oi];
-        store_rows(A, S, K, b, a, (jk / A.nang) + (jk % A.nang) * A.nang, oi, 8 * half, y);
+          for (int j = 0; j < 4; ++j) y[j] = *stage(h + j, oi);
+          if (jk >= 0) store_rows(A, S, K, b, a, jk >> 16, jk & 0xFFFF, oi, h, y);
+        }
+        // read before the next batch's digits overwrite it
+        pair_sync(qw);
+      }
+    };
+    // iteration n produces batch n + 1 and reads batch n back
+    bool ok = true;
+    int g = g0 - 1, cur = 0;  // multipoles left of group g
+    bool start = false;       // the first of its group
+    terms_of(g0);
+    bounds_of();
+    for (int n = -1;; ++n) {
+      // ---- the batch after this one ----
+      int gn = g;
+      int nxt = cur & (cur - 1);
+      const bool begin = !nxt && ++gn < g1;
+      if (begin) {
+        nxt = S.gmask[gn];
+        enter(gn);
+      }
+      if (nxt) produce(__ffs(nxt) - 1, (n + 1) & 1);
+      const bool ahead = nxt && !(nxt & (nxt - 1)) && gn + 1 < g1;  // the one after that starts a group
+      if (ahead) terms_of(gn + 1);
+      const int L = __ffs(cur) - 1;
+      if (n >= 0) {
+        // this batch's first product, the last one's second
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&m.done, (uint32_t)(n & 1), kWait));
+        if (!ok) break;
+        tc::fence_after_sync();
+        if (start || !cur) {
+          if (n > 0) store_group();
+          if (!cur) break;
+          E2 = m.ex[g & 3][oslot];
+          mask2 = m.mask[g & 3][oslot];
+          jk = m.jk[g & 3][oslot];
+        }
+        // ---- levels -> balanced digits of Y = A X, the second product's
+        // MN-major operand: rows (slot, i), K = q ----
+        // the second product accumulates over the multipoles: a slot that is
+        // idle in this one adds zeros
+        const bool idle = !((mask2 >> L) & 1);
+        const bool none = __all_sync(0xffffffffu, idle);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {  // 4 columns at a time: registers
+          uint32_t pk[PD][2];
+          if (!none) {
+            float v[PD][4];
+            tmem_ld_pairs(tD1 + lane_off + 8 * half + 4 * h, v);
+#pragma unroll
+            for (int jj = 0; jj < 2; ++jj) {
+              float y[PD][2];
+#pragma unroll
+              for (int w = 0; w < 2; ++w) {
+                float lv[PD];
+#pragma unroll
+                for (int d = 0; d < PD; ++d) lv[d] = v[d][2 * jj + w];
+                carry_pairs(lv, y[0][w], y[1][w]);
+#pragma unroll
+                for (int k = 2; k < PD; ++k) y[k][w] = lv[k - 1];
+              }
+#pragma unroll
+              for (int k = 0; k < PD; ++k) pk[k][jj] = pack_f16(y[k][0], y[k][1]);
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < PD; ++k)
+            *reinterpret_cast<uint2*>(A2 + k * APLANE + off2 + 8 * h) =
+                idle ? make_uint2(0, 0) : make_uint2(pk[k][0], pk[k][1]);
+        }
+      }
+      if (ahead) bounds_of();
+      issue((n + 1) & 1, nxt ? __ffs(nxt) - 1 : -1, L, start);
+      g = gn;
+      cur = nxt;
+      start = begin;
+    }
+    if (!ok) {
+      if (lane == 0) atomicExch(&m.fail, 1);
+      // the results of this unit are marked
+      for (int g = g0; g < g1; ++g) {
+        if (8 * g + oslot >= count) break;
+        const int jkf = S.olist[8 * g + oslot];
+        double y[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j] = __longlong_as_double(0x7ff8000000000000ll);
+        for (int h = 0; h < 8; h += 4) store_rows(A, S, K, a, b, jkf % A.nang, jkf / A.nang, oi, 8 * half + h, y);
       }
     }
-    __syncthreads();  // the stage (first operand) and the group tables are reused
-    if (failed) break;
   }
-
-  if (sm.fail[0] && t == 0) {
+  __syncthreads();
+  if (m.fail && t == 0) {
     atomicExch(T.err, 1);
-    // the MMAs of the abandoned batch may still be running: give them one
-    // more bounded wait before the tensor memory is released
-    tc::mbar_wait(sm.mbar, phase ^ 1u);
+    // MMAs may still be running: give them time before the tensor memory is released
+    for (int i = 0; i < 100; ++i) __nanosleep(1000);
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tbase, 256);
+  if (warp == 0) tc::tmem_dealloc(tD1, 256);
 }
 
 // ------------------------------------------------------------------------
@@ -575,12 +783,15 @@ __global__ void tc_tk_digits_kernel(const double* __restrict__ tk, int NL, int n
 
 __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, DevTC T, int symmetric,
                                                     double* __restrict__ K) {
-  const int4 u = (symmetric ? T.dunits_sym : T.dunits_all)[blockIdx.x];
-  const int a = u.x, g = u.y, mt = u.z;
   const int nn = A.nn, n2 = nn * nn, NL = A.NL, nang2 = A.nang * A.nang;
   const int ksteps = T.dksteps, mtiles = T.dmtiles;
-  const int* gjk_all = symmetric ? T.dgroup_jk_sym : T.dgroup_jk_all;
-  const int* gent_all = symmetric ? T.dgroup_ent_sym : T.dgroup_ent_all;
+  // unit = (element, row tile, group of 16 active output blocks); the list is
+  // made by the density pass (j <= k only in symmetric mode)
+  const int count = symmetric ? S.ocount[1] : S.ocount[0];
+  const int* list = symmetric ? S.olist + nang2 : S.olist;
+  const int ngr = (count + DSLOT - 1) / DSLOT;
+  const int g = blockIdx.x % T.dgroups, mt = (blockIdx.x / T.dgroups) % mtiles, a = blockIdx.x / (T.dgroups * mtiles);
+  if (g >= ngr) return;  // uniform over the CTA
   extern __shared__ __align__(1024) unsigned char smraw[];
   unsigned char* Abuf = smraw;                                             // 2 x ND planes of 128 x 16
   unsigned char* Bx = Abuf + 2 * ND * APLANE;                              // ksteps x ND planes of 16 x 16
@@ -596,12 +807,19 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int qw = warp & 3, half = warp >> 2;
 
-  for (int idx = t; idx < DSLOT * NL; idx += blockDim.x) {
-    const int e = gent_all[(size_t)g * DSLOT * NL + idx];  // idx = slot * NL + L
-    gent[idx] = e;
-    sact[(idx % NL) * DSLOT + idx / NL] = (e >= 0 && S.ent_act[e]) ? 1 : 0;
+  if (t < DSLOT) {
+    const int jk = g * DSLOT + t < count ? list[g * DSLOT + t] : -1;
+    gjk[t] = jk;
+    for (int L = 0; L < NL; ++L) {
+      gent[t * NL + L] = -1;
+      sact[L * DSLOT + t] = 0;
+    }
+    if (jk >= 0)
+      for (int e = A.kjk_ptr[jk]; e < A.kjk_ptr[jk + 1]; ++e) {
+        gent[t * NL + A.kent_L[e]] = e;
+        sact[A.kent_L[e] * DSLOT + t] = S.ent_act[e] ? 1 : 0;
+      }
   }
-  if (t < DSLOT) gjk[t] = gjk_all[g * DSLOT + t];
   for (int idx = t; idx < nang2; idx += blockDim.x) act[idx] = S.act[idx];
   // the zero seventh density plane of every K step (operands of N = 112)
   for (int idx = t; idx < ksteps * (TPLANE / 16); idx += blockDim.x) {
@@ -789,8 +1007,7 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
 }
 
 size_t tc_smem_bytes(int NL, int nang) {
-  return (size_t)(NDX + ND) * APLANE + (size_t)2 * NL * ND * TPLANE +
-         sizeof(int) * (2 * NL * 16 + 16 + 8 * NL + 8 * NL + 8 + 2) + 16 + (size_t)nang * nang + 64;
+  return (size_t)(2 * PX + PD) * APLANE + (size_t)2 * NL * PD * TPLANE + sizeof(PairMeta) + (size_t)nang * nang + 16;
 }
 
 size_t tc_diag_smem_bytes(int NL, int ksteps, int nang) {
@@ -805,7 +1022,7 @@ cudaError_t launch_k_tiles_tc(const DevAtom& A, const DevScratch& S, const DevTC
   const size_t smem = tc_smem_bytes(A.NL, A.nang);
   const cudaError_t e = smem_limit(k_tiles_tc, smem);
   if (e != cudaSuccess) return e;
-  k_tiles_tc<<<n, 256, smem, st>>>(A, S, T, symmetric ? T.units_sym : T.units_all, symmetric ? 1 : 0, K);
+  k_tiles_tc<<<n, PTHREADS, smem, st>>>(A, S, T, symmetric ? T.units_sym : T.units_all, symmetric ? 1 : 0, K);
   return cudaGetLastError();
 }
 
@@ -820,12 +1037,14 @@ cudaError_t launch_tk_digits(const DevAtom& A, int mtiles, int ksteps, unsigned 
 
 cudaError_t launch_k_diag_tc(const DevAtom& A, const DevScratch& S, const DevTC& T, bool symmetric, double* K,
                              cudaStream_t st) {
-  const int n = symmetric ? T.n_dsym : T.n_dall;
-  if (n == 0) return cudaSuccess;
+  DevTC Td = T;
+  const int nblk = symmetric ? A.nang * (A.nang + 1) / 2 : A.nang * A.nang;
+  Td.dgroups = (nblk + DSLOT - 1) / DSLOT;
+  const int n = A.nel * T.dmtiles * Td.dgroups;
   const size_t smem = tc_diag_smem_bytes(A.NL, T.dksteps, A.nang);
   const cudaError_t e = smem_limit(k_diag_tc, smem);
   if (e != cudaSuccess) return e;
-  k_diag_tc<<<n, 256, smem, st>>>(A, S, T, symmetric ? 1 : 0, K);
+  k_diag_tc<<<n, 256, smem, st>>>(A, S, Td, symmetric ? 1 : 0, K);
   return cudaGetLastError();
 }
 

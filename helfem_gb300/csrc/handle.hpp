@@ -156,14 +156,15 @@ struct hfg_atom {
   // device copies of the tables
   DBuf d_rs, d_rb, d_cholp, d_rank, d_tk, d_chanL, d_jket_ptr, d_jket_blk, d_jket_coef, d_jbra_ptr,
       d_jbra_chan, d_jbra_coef, d_kjk_ptr, d_kent_L, d_kent_ptr, d_kterm_blk, d_kterm_off, d_kterm_coef;
-  DBuf s_jin, s_jscal, s_khalo, s_bnorm, s_p2, s_act, s_entact;
+  DBuf d_order, d_kterm_L, d_kterm_ent, d_kent_sig, s_olist, s_oinfo, s_ocount, s_gmask;
+  DBuf s_jin, s_jscal, s_khalo, s_bnorm, s_count, s_tmax, s_p2, s_act, s_entact;
   DBuf d_rs2, d_rb2, d_tk2, d_kcoef2, d_jkc2, d_jbc2, d_cholp2;
   DBuf d_units_all, d_units_sym, d_diag_all, d_diag_sym;
   hfg::KUnits units;
   // tensor-core split exchange: digit tables of the bare and of the
   // Yukawa-screened radial tables, shared groups and units, error flag
-  DBuf t_dig, t_exp, ty_dig, ty_exp, t_gjk, t_gent, t_usym, t_uall, t_err;
-  DBuf t_tkd, t_tke, ty_tkd, ty_tke, t_dgjk_s, t_dgent_s, t_dgjk_a, t_dgent_a, t_dus, t_dua;
+  DBuf t_dig, t_exp, t_texp, ty_dig, ty_exp, ty_texp, t_usym, t_uall, t_err;
+  DBuf t_tkd, t_tke, ty_tkd, ty_tke;
   hfg::DevTC tc{}, tc_rs{};
   bool tc_ok = false;
   // bf16 MMA FLOPs one tensor-core exchange issues with every entry active
@@ -181,44 +182,62 @@ struct hfg_atom {
     return screened ? (tc_rs.digits ? &tc_rs : nullptr) : &tc;
   }
   // digits of the radial tables (kind 0 r_small, 1 r_big; per (L, e) a
-  // 16 x 16 plane per digit, element (row n, column k) = table(n, k)) and the
-  // row exponents; see k_tc.cu for the arithmetic
-  void tc_tables(const std::vector<double>& rs, const std::vector<double>& rb, DBuf& dig, DBuf& rexp,
+  // 16 x 16 plane per digit, element (row n, column k) = table(n, k)), the
+  // exponents of the tables and of the rows; see k_tc.cu for the arithmetic
+  void tc_tables(const std::vector<double>& rs, const std::vector<double>& rb, DBuf& dig, DBuf& rexp, DBuf& texp,
                  hfg::DevTC& out) {
     const hfg::AtomHost& H = host;
     const int nn = H.rad.nn, nel = H.rad.nel, NL = H.NL, ND = TC_NDIGITS;
     const size_t n2 = (size_t)nn * nn;
     std::vector<uint16_t> d((size_t)2 * NL * nel * ND * (TC_TPLANE / 2), 0);
-    std::vector<int> ex((size_t)2 * NL * nel * 16, 0);
+    std::vector<int> ex((size_t)2 * nel * 16, 0), tx((size_t)2 * NL * nel, 0);
     auto off = [](int n, int k) { return ((n >> 3) * 256 + (k >> 3) * 128 + (n & 7) * 16 + (k & 7) * 2) / 2; };
+    auto half_bits = [](int v) {  // integer |v| <= 2048 as f16, exact
+      if (v == 0) return (uint16_t)0;
+      const int m = std::abs(v);
+      int e = 0;
+      while ((m >> (e + 1)) != 0) ++e;
+      return (uint16_t)((v < 0 ? 0x8000 : 0) | ((e + 15) << 10) | ((e <= 10 ? m << (10 - e) : m >> (e - 10)) & 0x3FF));
+    };
     for (int kind = 0; kind < 2; ++kind)
-      for (int L = 0; L < NL; ++L)
-        for (int e = 0; e < nel; ++e) {
-          const double* M = (kind == 0 ? rs : rb).data() + ((size_t)L * nel + e) * n2;
-          const size_t blk = ((size_t)kind * NL + L) * nel + e;
-          uint16_t* planes = d.data() + blk * ND * (TC_TPLANE / 2);
+      for (int e = 0; e < nel; ++e) {
+        auto table = [&](int L) { return (kind == 0 ? rs : rb).data() + ((size_t)L * nel + e) * n2; };
+        int* row = &ex[((size_t)kind * nel + e) * 16];
+        std::vector<double> rowmax(nn, 0.0);
+        for (int L = 0; L < NL; ++L) {
+          const double* M = table(L);
+          double mx = 0.0;
+          for (size_t i = 0; i < n2; ++i) mx = std::max(mx, std::fabs(M[i]));
+          int te = 0;
+          if (mx > 0.0) std::frexp(mx, &te);  // mx < 2^te
+          tx[((size_t)kind * NL + L) * nel + e] = te;
           for (int n = 0; n < nn; ++n) {
-            double rowsum = 0.0;
-            for (int k = 0; k < nn; ++k) rowsum += std::fabs(M[n + (size_t)k * nn]);
-            int a = 0;
-            if (rowsum > 0.0) std::frexp(rowsum, &a);  // rowsum <= 2^a
-            ex[blk * 16 + n] = a;
-            for (int k = 0; k < nn; ++k) {
-              double r = std::ldexp(M[n + (size_t)k * nn], -a);
-              for (int kd = 0; kd < ND; ++kd) {
-                r *= 256.0;
-                const double dg = std::nearbyint(r);
-                r -= dg;
-                const float f = (float)dg;  // integer |dg| <= 256: exact in bf16
-                uint32_t bits;
-                std::memcpy(&bits, &f, 4);
-                planes[(size_t)kd * (TC_TPLANE / 2) + off(n, k)] = (uint16_t)(bits >> 16);
-              }
-            }
+            double sum = 0.0;
+            for (int k = 0; k < nn; ++k) sum += std::fabs(M[n + (size_t)k * nn]);
+            rowmax[n] = std::max(rowmax[n], std::ldexp(sum, -te));
           }
         }
+        for (int n = 0; n < nn; ++n)
+          if (rowmax[n] > 0.0) std::frexp(rowmax[n], &row[n]);  // row sums <= 2^row
+        for (int L = 0; L < NL; ++L) {
+          const double* M = table(L);
+          const size_t blk = ((size_t)kind * NL + L) * nel + e;
+          uint16_t* planes = d.data() + blk * ND * (TC_TPLANE / 2);
+          for (int n = 0; n < nn; ++n)
+            for (int k = 0; k < nn; ++k) {
+              double r = std::ldexp(M[n + (size_t)k * nn], -row[n] - tx[blk]);
+              for (int kd = 0; kd < ND; ++kd) {
+                r *= 1024.0;
+                const double dg = std::nearbyint(r);
+                r -= dg;
+                planes[(size_t)kd * (TC_TPLANE / 2) + off(n, k)] = half_bits((int)dg);
+              }
+            }
+        }
+      }
     out.digits = reinterpret_cast<const unsigned char*>(dig.upload(d));
     out.rowexp = rexp.upload(ex);
+    out.texp = texp.upload(tx);
   }
   // digit planes of an exchange-ordered tensor (built on the device)
   void tc_tk_tables(const double* tk_dev, DBuf& dig, DBuf& rexp, hfg::DevTC& out) {
@@ -227,7 +246,7 @@ struct hfg_atom {
     out.dmtiles = (n2 + 127) / 128;
     out.dksteps = (n2 + 15) / 16;
     const size_t nslice = (size_t)H.NL * H.rad.nel * out.dmtiles;
-    dig.alloc(nslice * out.dksteps * TC_NDIGITS * 4096);
+    dig.alloc(nslice * out.dksteps * 7 * 4096);  // seven digit planes of 128 x 16
     rexp.alloc(sizeof(int) * nslice * 128);
     hfg::DevAtom A = dev;
     A.tk = tk_dev;
@@ -235,50 +254,6 @@ struct hfg_atom {
        "exchange tensor digits");
     out.tk_digits = dig.as<unsigned char>();
     out.tk_rowexp = rexp.as<int>();
-  }
-  // groups of up to 16 diagonal output blocks (sorted by multipole set) and
-  // the diagonal units (element, group, row tile)
-  void tc_diag_groups(bool sym, DBuf& djk, DBuf& dent, DBuf& du, const int*& gjk_out, const int*& gent_out,
-                      const int4*& u_out, int& n_out, int mtiles) {
-    const hfg::AtomHost& H = host;
-    const int NL = H.NL, nel = H.rad.nel;
-    std::vector<int> blocks;
-    for (int k = 0; k < H.nang; ++k)
-      for (int j = 0; j < H.nang; ++j)
-        if (!sym || j <= k) blocks.push_back(j + k * H.nang);
-    std::vector<int> sig(blocks.size(), 0);
-    for (size_t i = 0; i < blocks.size(); ++i)
-      for (int e = H.kjk_ptr[blocks[i]]; e < H.kjk_ptr[blocks[i] + 1]; ++e) sig[i] |= 1 << H.kent_L[e];
-    std::vector<int> order(blocks.size());
-    for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return sig[x] < sig[y]; });
-    const int G = ((int)blocks.size() + 15) / 16;
-    std::vector<int> gjk((size_t)G * 16, -1), gent((size_t)G * 16 * NL, -1);
-    for (size_t i = 0; i < order.size(); ++i) {
-      const int jk = blocks[order[i]], g = (int)i / 16, s2 = (int)i % 16;
-      gjk[(size_t)g * 16 + s2] = jk;
-      for (int e = H.kjk_ptr[jk]; e < H.kjk_ptr[jk + 1]; ++e) gent[((size_t)g * 16 + s2) * NL + H.kent_L[e]] = e;
-    }
-    std::vector<int4> u;
-    for (int a = 0; a < nel; ++a)
-      for (int mt = 0; mt < mtiles; ++mt)
-        for (int g = 0; g < G; ++g) u.push_back(make_int4(a, g, mt, 0));
-    {
-      long nb = 0;  // (group, L) batches with at least one entry
-      for (int g = 0; g < G; ++g)
-        for (int L = 0; L < NL; ++L) {
-          bool any = false;
-          for (int s2 = 0; s2 < 16; ++s2) any |= gent[((size_t)g * 16 + s2) * NL + L] >= 0;
-          nb += any ? 1 : 0;
-        }
-      // per batch and row tile: K steps x (N = 112 + 96 + ... + 16) x 128 x 16
-      const int ksteps = (H.rad.nn * H.rad.nn + 15) / 16;
-      tc_mma_flops[sym ? 0 : 1] += 2.0 * 128 * 16 * 448 * ksteps * (double)nb * nel * mtiles;
-    }
-    gjk_out = djk.upload(gjk);
-    gent_out = dent.upload(gent);
-    u_out = du.upload(u);
-    n_out = (int)u.size();
   }
   // off-diagonal tensor-core units: a unit is a range of groups of one
   // element pair (the pair's tables and the tensor memory are set up once per
@@ -312,54 +287,65 @@ struct hfg_atom {
       tc_rs.n_all = tc.n_all;
     }
   }
-  // output blocks in groups of 8 with similar multipole sets, and the units
+  // output blocks in an order that brings like multipole sets together (they
+  // share batches); false where some block has two entries of one multipole
+  bool block_order(std::vector<int>& order) const {
+    const hfg::AtomHost& H = host;
+    const int nang2 = H.nang * H.nang;
+    std::vector<int> sig(nang2, 0);
+    order.resize(nang2);
+    bool one = true;
+    for (int jk = 0; jk < nang2; ++jk) {
+      order[jk] = jk;
+      for (int e = H.kjk_ptr[jk]; e < H.kjk_ptr[jk + 1]; ++e) {
+        if (H.kent_L[e] < 31 && ((sig[jk] >> H.kent_L[e]) & 1)) one = false;
+        if (H.kent_L[e] < 31) sig[jk] |= 1 << H.kent_L[e];
+      }
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return sig[x] < sig[y]; });
+    return one;
+  }
+  // tensor-core tables and units, and the MMA work with every block active
   void tc_setup() {
     const hfg::AtomHost& H = host;
     const int nel = H.rad.nel, NL = H.NL, nang2 = H.nang * H.nang;
-    if (H.rad.nn > 16 || NL > 8 || nel < 2) return;
-    std::vector<int> sig(nang2, 0), order(nang2);
-    for (int jk = 0; jk < nang2; ++jk) {
-      order[jk] = jk;
-      for (int e = H.kjk_ptr[jk]; e < H.kjk_ptr[jk + 1]; ++e) sig[jk] |= 1 << H.kent_L[e];
+    std::vector<int> order;
+    const bool one = block_order(order);
+    std::vector<int4> info(order.size());
+    for (size_t x = 0; x < order.size(); ++x) {
+      const int jk = order[x], t0 = H.kent_ptr[H.kjk_ptr[jk]];
+      info[x] = make_int4(jk, t0, H.kent_ptr[H.kjk_ptr[jk + 1]] - t0, jk % H.nang | jk / H.nang << 16);
     }
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return sig[x] < sig[y]; });
-    const int G = (nang2 + 7) / 8;
-    std::vector<int> gjk((size_t)G * 8, -1), gent((size_t)G * 8 * NL, -1);
-    for (int i = 0; i < nang2; ++i) {
-      const int jk = order[i], g = i / 8, s = i % 8;
-      gjk[(size_t)g * 8 + s] = jk;
-      for (int e = H.kjk_ptr[jk]; e < H.kjk_ptr[jk + 1]; ++e) {
-        int& slot = gent[((size_t)g * 8 + s) * NL + H.kent_L[e]];
-        if (slot >= 0) return;  // two entries with one multipole: keep the float-pair form
-        slot = e;
+    dev.jk_order = d_order.upload(info);
+    // (a block's terms are held two per lane of a warp; the float-pair form otherwise)
+    if (H.rad.nn > 16 || NL > 8 || nel < 2 || !one || dev.max_terms_per_jk > 64) return;
+    tc.ngroups = (nang2 + 7) / 8;
+    // (group of n blocks, L) batches with at least one entry
+    auto batches = [&](const std::vector<int>& blocks, int n) {
+      long nb = 0;
+      for (size_t i = 0; i < blocks.size(); i += n) {
+        int m = 0;
+        for (size_t x = i; x < std::min(blocks.size(), i + n); ++x)
+          for (int e = H.kjk_ptr[blocks[x]]; e < H.kjk_ptr[blocks[x] + 1]; ++e) m |= 1 << H.kent_L[e];
+        for (; m; m &= m - 1) ++nb;
       }
-    }
-    tc.ngroups = G;
-    {
-      long nb = 0;  // (group, L) batches with at least one entry
-      for (int g = 0; g < G; ++g)
-        for (int L = 0; L < NL; ++L) {
-          bool any = false;
-          for (int s2 = 0; s2 < 8; ++s2) any |= gent[((size_t)g * 8 + s2) * NL + L] >= 0;
-          nb += any ? 1 : 0;
-        }
-      // per batch: 27 + 28 digit-plane products of 128 x 16 x 16
-      const double per = 2.0 * 128 * 16 * 16 * 55;
-      tc_mma_flops[0] += per * nb * ((double)nel * (nel - 1) / 2);
-      tc_mma_flops[1] += per * nb * ((double)nel * (nel - 1));
-    }
-    tc_tables(H.rs, H.rb, t_dig, t_exp, tc);
-    tc.group_jk = t_gjk.upload(gjk);
-    tc.group_ent = t_gent.upload(gent);
+      return nb;
+    };
+    std::vector<int> half;
+    for (int jk : order)
+      if (jk % H.nang <= jk / H.nang) half.push_back(jk);
+    // per batch: 20 + 21 digit-plane products of 128 x 16 x 16
+    const double per = 2.0 * 128 * 16 * 16 * 41 * (double)batches(order, 8);
+    tc_tables(H.rs, H.rb, t_dig, t_exp, t_texp, tc);
     tc_units();
     t_err.alloc(sizeof(int));
     ck(cudaMemsetAsync(t_err.p, 0, sizeof(int), own_stream), "memset");
     tc.err = t_err.as<int>();
     tc_tk_tables(dev.tk, t_tkd, t_tke, tc);
-    tc_diag_groups(true, t_dgjk_s, t_dgent_s, t_dus, tc.dgroup_jk_sym, tc.dgroup_ent_sym, tc.dunits_sym, tc.n_dsym,
-                   tc.dmtiles);
-    tc_diag_groups(false, t_dgjk_a, t_dgent_a, t_dua, tc.dgroup_jk_all, tc.dgroup_ent_all, tc.dunits_all, tc.n_dall,
-                   tc.dmtiles);
+    // diagonal, per batch of 16 blocks and row tile: K steps x (N = 112 + 96 + ... + 16) x 128 x 16
+    const double dper = 2.0 * 128 * 16 * 448 * tc.dksteps * (double)nel * tc.dmtiles;
+    tc_mma_flops[0] = per * ((double)nel * (nel - 1) / 2) + dper * (double)batches(half, 16);
+    tc_mma_flops[1] = per * ((double)nel * (nel - 1)) + dper * (double)batches(order, 16);
     tc_ok = true;
   }
   // a completion wait inside the tensor-core kernel ran out (checked by the
@@ -440,7 +426,7 @@ struct hfg_atom {
     dev_rs.tk2 = y_tk2.upload(split(host.y_tk));
     if (tc_ok) {
       tc_rs = tc;
-      tc_tables(host.y_rs, host.y_rb, ty_dig, ty_exp, tc_rs);
+      tc_tables(host.y_rs, host.y_rb, ty_dig, ty_exp, ty_texp, tc_rs);
       tc_tk_tables(dev_rs.tk, ty_tkd, ty_tke, tc_rs);
     }
     ck(cudaStreamSynchronize(own_stream), "sync after upload");
@@ -563,6 +549,20 @@ struct hfg_atom {
       }
       A.kterm_off = d_kterm_off.upload(off);
     }
+    {
+      std::vector<int> tL(H.kterm_blk.size()), te(H.kterm_blk.size());
+      for (size_t e = 0; e < H.kent_L.size(); ++e)
+        for (int u = H.kent_ptr[e]; u < H.kent_ptr[e + 1]; ++u) {
+          tL[u] = H.kent_L[e];
+          te[u] = (int)e;
+        }
+      A.kterm_L = d_kterm_L.upload(tL);
+      A.kterm_ent = d_kterm_ent.upload(te);
+      std::vector<int> sig(H.kent_L.size());
+      for (int jk = 0; jk < H.nang * H.nang; ++jk)
+        for (int e = H.kjk_ptr[jk]; e < H.kjk_ptr[jk + 1]; ++e) sig[e] = jk | std::min(H.kent_L[e], 7) << 24;
+      A.kent_sig = d_kent_sig.upload(sig);
+    }
     A.nent = (int)H.kent_L.size();
     A.kterm_coef = d_kterm_coef.upload(H.kterm_coef);
     int mx = 0;
@@ -578,16 +578,29 @@ struct hfg_atom {
     s_jin.alloc(sizeof(double) * A.nchan * A.nel * n2);
     s_jscal.alloc(sizeof(double) * A.nchan * A.nel * 2);
     s_khalo.alloc(sizeof(double) * (size_t)A.nel * A.nel * A.nang * A.nang * (2 * A.nn - 1));
-    s_bnorm.alloc(sizeof(double) * (size_t)A.nang * A.nang * NORM_SPLIT);
+    s_bnorm.alloc(sizeof(double) * (size_t)A.nang * A.nang * A.nel);
+    s_count.alloc(sizeof(unsigned));
+    ck(cudaMemsetAsync(s_count.p, 0, sizeof(unsigned), own_stream), "memset");
+    s_tmax.alloc(sizeof(unsigned) * (size_t)A.nang * A.nang * A.nel * A.nel);
     s_act.alloc((size_t)A.nang * A.nang);
     s_entact.alloc(std::max<size_t>(1, (size_t)A.nent));
     scr.jin = s_jin.as<double>();
     scr.jscal = s_jscal.as<double>();
     scr.khalo = s_khalo.as<double>();
     scr.bnorm = s_bnorm.as<double>();
+    scr.count = s_count.as<unsigned>();
+    scr.tmax = s_tmax.as<unsigned>();
     scr.act = s_act.as<unsigned char>();
     scr.ent_act = s_entact.as<unsigned char>();
     scr.p2 = nullptr;  // allocated on the first split-precision call
+    s_olist.alloc(sizeof(int) * 2 * (size_t)A.nang * A.nang);
+    s_oinfo.alloc(sizeof(int4) * (size_t)A.nang * A.nang);
+    scr.oinfo = s_oinfo.as<int4>();
+    s_ocount.alloc(sizeof(int) * 2);
+    s_gmask.alloc(sizeof(int) * (((size_t)A.nang * A.nang + 7) / 8));
+    scr.olist = s_olist.as<int>();
+    scr.ocount = s_ocount.as<int>();
+    scr.gmask = s_gmask.as<int>();
     ck(cudaEventCreateWithFlags(&last_use, cudaEventDisableTiming), "cudaEventCreate");
     auto split = [](const std::vector<double>& v) {
       std::vector<float2> o(v.size());
