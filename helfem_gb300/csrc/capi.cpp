@@ -208,7 +208,7 @@ static void sad_host(hfg_atom* a, const double* P, double* out, int kind, int fl
   need(a != nullptr, "null argument");
   sad_call(a, P, out, kind, flags, a->own_stream);
   ck(cudaStreamSynchronize(a->own_stream), "stream sync");
-  if (kind != 0 && (flags & HFG_EXCHANGE_SPLIT)) a->tc_check();
+  if (kind != 0 && ((flags & HFG_EXCHANGE_SPLIT) || a->tc64_for(false))) a->tc_check();
 }
 
 hfg_status hfg_sadatom_coulomb_host(hfg_atom* a, const double* P, double* J) {
@@ -411,7 +411,8 @@ hfg_status hfg_exchange_ex(hfg_atom* a, const double* P, double* K, int flags, v
                                     a->tc_for(false), a->side_stream()),
          "exchange kernels (split)");
     } else {
-      ck(hfg::launch_exchange_fp64(a->dev, a->scr, a->units, P, K, sym, (cudaStream_t)stream, &a->prof),
+      ck(hfg::launch_exchange_fp64(a->dev, a->scr, a->units, P, K, sym, (cudaStream_t)stream, &a->prof,
+                                   a->tc64_for(false), &a->k_side),
          "exchange kernels");
     }
     a->mark_use((cudaStream_t)stream);
@@ -474,13 +475,14 @@ static void host_call(hfg_atom* a, const double* P, double* out, bool coulomb, i
        "exchange (split)");
   } else {
     ck(hfg::launch_exchange_fp64(ctx, a->scr, a->units, a->h_in.as<double>(), a->h_out.as<double>(),
-                                 (flags & HFG_EXCHANGE_SYMMETRIC) != 0, st, &a->prof),
+                                 (flags & HFG_EXCHANGE_SYMMETRIC) != 0, st, &a->prof, a->tc64_for(screened),
+                                 &a->k_side),
        "exchange");
   }
   ck(cudaMemcpyAsync(out, a->h_out.p, bytes, cudaMemcpyDeviceToHost, st), "D2H copy");
   a->last_d2h = bytes;
   ck(cudaStreamSynchronize(st), "stream sync");
-  if (!coulomb && (flags & HFG_EXCHANGE_SPLIT)) a->tc_check();
+  if (!coulomb && ((flags & HFG_EXCHANGE_SPLIT) || a->tc64_for(screened))) a->tc_check();
 }
 
 // J(PJ) and K(PK) with one staging of the density when PK == PJ, the
@@ -535,14 +537,15 @@ static void jk_host(hfg_atom* a, const double* PJ, const double* PK, double* J, 
        "exchange (split)");
   } else {
     ck(hfg::launch_exchange_fp64(a->dev, a->scr, a->units, Pk, a->h_out2.as<double>(),
-                                 (flags & HFG_EXCHANGE_SYMMETRIC) != 0, st, &a->prof),
+                                 (flags & HFG_EXCHANGE_SYMMETRIC) != 0, st, &a->prof, a->tc64_for(false),
+                                 &a->k_side),
        "exchange");
   }
   ck(cudaMemcpyAsync(K, a->h_out2.p, bytes, cudaMemcpyDeviceToHost, st), "D2H copy");
   a->last_d2h = 2 * bytes;
   ck(cudaStreamSynchronize(st), "stream sync");
   ck(cudaStreamSynchronize(a->copy_stream), "stream sync");
-  if (flags & HFG_EXCHANGE_SPLIT) a->tc_check();
+  if ((flags & HFG_EXCHANGE_SPLIT) || a->tc64_for(false)) a->tc_check();
 }
 
 hfg_status hfg_jk(hfg_atom* a, const double* PJ, const double* PK, double* J, double* K, int flags, void* stream) {
@@ -581,7 +584,9 @@ hfg_status hfg_jk(hfg_atom* a, const double* PJ, const double* PK, double* J, do
                                     a->side_stream()),
          "exchange kernels (split)");
     else
-      ck(hfg::launch_exchange_fp64(a->dev, a->scr, a->units, PK, K, sym, st, &a->prof), "exchange kernels");
+      ck(hfg::launch_exchange_fp64(a->dev, a->scr, a->units, PK, K, sym, st, &a->prof, a->tc64_for(false),
+                                   &a->k_side),
+         "exchange kernels");
     ck(cudaStreamWaitEvent(st, a->ev_join, 0), "join");
     a->mark_use(st);
   });
@@ -628,14 +633,15 @@ hfg_status hfg_atom_autotune(hfg_atom* a, int flags, int* best_nsplit, double* b
                                       a->tc_for(false), a->side_stream()),
            "exchange");
       else
-        ck(hfg::launch_exchange_fp64(a->dev, a->scr, a->units, P.as<double>(), K.as<double>(), sym, st, nullptr),
+        ck(hfg::launch_exchange_fp64(a->dev, a->scr, a->units, P.as<double>(), K.as<double>(), sym, st, nullptr,
+                                     a->tc64_for(false), &a->k_side),
            "exchange");
     };
     double best = 1e300;
     int bestn = 0;
-    // the tensor-core split form: groups of 8 output blocks per element-pair
+    // the tensor-core forms: groups of 8 output blocks per element-pair
     // unit; otherwise output-block ranges per element pair
-    const bool tcform = (flags & HFG_EXCHANGE_SPLIT) && a->tc_for(false) != nullptr;
+    const bool tcform = ((flags & HFG_EXCHANGE_SPLIT) ? a->tc_for(false) : a->tc64_for(false)) != nullptr;
     const std::vector<int> cand = tcform ? std::vector<int>{0, 1, 2, 3, 4, 6, a->tc.ngroups}
                                          : std::vector<int>{0, 1, 2, 4, 8, 16};
     for (int ns : cand) {
@@ -761,7 +767,8 @@ hfg_status hfg_rs_exchange(hfg_atom* a, const double* P, double* K, int flags, v
                                     a->tc_for(true), a->side_stream()),
          "screened exchange (split)");
     } else {
-      ck(hfg::launch_exchange_fp64(a->dev_rs, a->scr, a->units, P, K, sym, (cudaStream_t)stream, &a->prof),
+      ck(hfg::launch_exchange_fp64(a->dev_rs, a->scr, a->units, P, K, sym, (cudaStream_t)stream, &a->prof,
+                                   a->tc64_for(true), &a->k_side),
          "screened exchange");
     }
     a->mark_use((cudaStream_t)stream);

@@ -62,7 +62,7 @@ struct DevScratch {
   double* khalo;        // [nel*nel*nang*nang*(2nn-1)]
   double* bnorm;        // [nang*nang][nel] squared norms of each block's columns of an element
   unsigned int* count;  // norm-pass CTAs done (the last one sets the flags)
-  unsigned int* tmax;   // [nang*nang][nel][nel] largest |high word| of each density tile (split path)
+  unsigned int* tmax;   // [nang*nang][nel][nel] largest |value| of each density tile: float bits of the high words (split), high words of the doubles (FP64)
   unsigned char* act;   // [nang*nang] density block above the screen
   unsigned char* ent_act;  // [nent] exchange entry with an active term
   float2* p2;           // [nbf*nbf] split copy of the density (split path)
@@ -191,10 +191,10 @@ cudaError_t launch_xc_fp64(const DevAtom& A, const DevXC& X, const XcScratch& S,
 // exceeds the capacity.
 cudaError_t noalloc_coulomb_scratch(size_t doubles_needed, double** out);
 // tensor-core exchange tiles (k_tc.cu): off-diagonal element pairs only
-cudaError_t launch_k_tiles_tc(const DevAtom& A, const DevScratch& S, const DevTC& T, bool symmetric, double* K,
-                              cudaStream_t st);
-cudaError_t launch_k_diag_tc(const DevAtom& A, const DevScratch& S, const DevTC& T, bool symmetric, double* K,
-                             cudaStream_t st);
+cudaError_t launch_k_tiles_tc(const DevAtom& A, const DevScratch& S, const DevTC& T, bool symmetric, const double* P,
+                              double* K, cudaStream_t st);
+cudaError_t launch_k_diag_tc(const DevAtom& A, const DevScratch& S, const DevTC& T, bool symmetric, const double* P,
+                             double* K, cudaStream_t st);
 cudaError_t launch_tk_digits(const DevAtom& A, int mtiles, int ksteps, unsigned char* out, int* rowexp,
                              cudaStream_t st);
 // tensor-core probe (tc_probe.cu)
@@ -215,17 +215,19 @@ cudaError_t launch_exchange_erfc(const DevAtom& A, const DevScratch& S, const do
 cudaError_t launch_mirror_blocks(double* P, int n, int bw, cudaStream_t st);
 cudaError_t launch_coulomb_split(const DevAtom& A, const DevScratch& S, const double* P, double* J,
                                 bool zero_output, cudaStream_t st, Profiler* prof = nullptr);
-cudaError_t launch_exchange_fp64(const DevAtom& A, const DevScratch& S, const KUnits& U, const double* P,
-                                 double* K, bool symmetric, cudaStream_t st, Profiler* prof = nullptr);
-// split-precision exchange (float-float on the FP32 pipe, FP64 recombination)
-// tc != nullptr: the off-diagonal element pairs run on the tensor cores (k_tc.cu)
 // a second stream with a fork and a join event (owned by the caller)
 struct SideStream {
   cudaStream_t s = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
 };
+// tc != nullptr: on the tensor cores (k_tc.cu), side: a second stream for the
+// diagonal elements or nullptr
+cudaError_t launch_exchange_fp64(const DevAtom& A, const DevScratch& S, const KUnits& U, const double* P,
+                                 double* K, bool symmetric, cudaStream_t st, Profiler* prof = nullptr,
+                                 const DevTC* tc = nullptr, const SideStream* side = nullptr);
 // side (tensor-core form only): the diagonal tiles run on side->s,
 // concurrently with the off-diagonal ones, joined back before the fix-up
+// split-precision exchange (float-float on the FP32 pipe, FP64 recombination)
 cudaError_t launch_exchange_split(const DevAtom& A, const DevScratch& S, const KUnits& U, const double* P,
                                   double* K, bool symmetric, cudaStream_t st, Profiler* prof = nullptr,
                                   const DevTC* tc = nullptr, const SideStream* side = nullptr);

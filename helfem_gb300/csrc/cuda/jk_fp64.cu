@@ -317,9 +317,14 @@ __global__ void j_scatter(DevAtom A, DevScratch S, double* __restrict__ J, int a
 // thread. With the flags 82 us (Kr) and 144 us; without the last CTA's part 75
 // and 117 us; the norms without the tiles' maxima plus the flags' own launch
 // took 90 and 137 us.
-template <bool SPLIT>
+// NORM_PLAIN: norms and flags; NORM_SPLIT: with the float-pair copy; NORM_LISTS:
+// with what the tensor-core form of an FP64 density needs (maxima as the high
+// words of the doubles, the lists)
+enum { NORM_PLAIN, NORM_SPLIT, NORM_LISTS };
+template <int MODE>
 __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict__ P, float2* __restrict__ p2,
                               int symmetric) {
+  constexpr bool SPLIT = MODE == NORM_SPLIT, LISTS = MODE != NORM_PLAIN;
   __shared__ double red[32];
   __shared__ bool last;
   __shared__ int cnt[64];
@@ -327,7 +332,7 @@ __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict_
   const int blk = blockIdx.x, i = blk % A.nang, l = blk / A.nang, b = blockIdx.y, nn = A.nn;
   const int c0 = max(gfun(A, b, 0), 0), c1 = min(gfun(A, b, nn - 1), A.nrad - 1);
   const int nc = c1 - c0 + 1, nown = b == A.nel - 1 ? nc : nc - 1;  // columns, those owned
-  if (SPLIT) {
+  if (LISTS) {
     for (int e = threadIdx.x; e < A.nel; e += blockDim.x) emax[e] = 0u;
     __syncthreads();
   }
@@ -350,10 +355,11 @@ __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict_
         q += A.nbf;
         sf = fmaf(h.x, h.x, sf);
       } else {
+        if (LISTS) mx = max(mx, (unsigned)__double2hiint(v) & 0x7FFFFFFFu);
         s += v * v;
       }
     };
-    const double vb = SPLIT && nown < nc ? p[(size_t)nown * A.nbf] : 0.0;  // the next element's first column
+    const double vb = LISTS && nown < nc ? p[(size_t)nown * A.nbf] : 0.0;  // the next element's first column
     for (int c = 0; c < nown; c += nu) {
       const int len = min(nu, nown - c);
       double v[NU];
@@ -365,8 +371,8 @@ __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict_
         if (w < len) add(v[w]);
       p += (size_t)nu * A.nbf;
     }
-    if (SPLIT) mx = max(mx, __float_as_uint(split_bits(vb).x) & 0x7FFFFFFFu);
-    if (SPLIT) {
+    if (LISTS) mx = max(mx, (SPLIT ? __float_as_uint(split_bits(vb).x) : (unsigned)__double2hiint(vb)) & 0x7FFFFFFFu);
+    if (LISTS) {
       // row r is function r + 1 - a (nn - 1) of element a, and the last of the one before
       const int a = (r + 1) / (nn - 1), f = (r + 1) - a * (nn - 1);
       if (a < A.nel) atomicMax(&emax[a], mx);
@@ -380,10 +386,11 @@ __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict_
     __syncthreads();
     if (threadIdx.x == 0)
       for (int v = 0; v < (int)blockDim.x >> 5; ++v) s += red[v];
-    for (int e = threadIdx.x; e < A.nel; e += blockDim.x) S.tmax[((size_t)blk * A.nel + e) * A.nel + b] = emax[e];
   } else {
     s = block_sum(s, red);
   }
+  if (LISTS)  // (both sums end after a barrier)
+    for (int e = threadIdx.x; e < A.nel; e += blockDim.x) S.tmax[((size_t)blk * A.nel + e) * A.nel + b] = emax[e];
   // ---- the last CTA: flags (bnorm alone is read here: the copy and the
   // maxima are the next kernels' and need no fence) ----
   const int nang2 = A.nang * A.nang;
@@ -397,7 +404,7 @@ __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict_
   if (!last) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   // (dynamic shared memory past emax: block, entry and output-block flags)
-  unsigned char* sact = reinterpret_cast<unsigned char*>(emax + (SPLIT ? A.nel + nang2 : 0));
+  unsigned char* sact = reinterpret_cast<unsigned char*>(emax + (LISTS ? A.nel + nang2 : 0));
   unsigned char* sent = sact + nang2;
   int* sout = reinterpret_cast<int*>(emax) + A.nel;  // multipoles of a block's active entries (bits)
   for (int x = threadIdx.x; x < nang2; x += blockDim.x) {
@@ -428,12 +435,12 @@ __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict_
     for (int i = 0; i < NB; ++i)
       if (sact[blk[i]]) sent[ent[i]] = 1;
   }
-  if (SPLIT)
+  if (LISTS)
     for (int x = threadIdx.x; x < nang2; x += step) sout[x] = 0;
   __syncthreads();
   for (int e0 = threadIdx.x; e0 < A.nent; e0 += NB * step) {
     int sig[NB];
-    if (SPLIT)
+    if (LISTS)
 #pragma unroll
       for (int i = 0; i < NB; ++i) sig[i] = A.kent_sig[min(e0 + i * step, A.nent - 1)];
 #pragma unroll
@@ -441,10 +448,10 @@ __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict_
       const int e = e0 + i * step;
       if (e >= A.nent) break;
       S.ent_act[e] = sent[e];
-      if (SPLIT && sent[e]) atomicOr(&sout[sig[i] & 0xFFFFFF], 1 << (sig[i] >> 24));
+      if (LISTS && sent[e]) atomicOr(&sout[sig[i] & 0xFFFFFF], 1 << (sig[i] >> 24));
     }
   }
-  if (!SPLIT) return;
+  if (!LISTS) return;
   // ---- split form: the active output blocks in jk_order. A symmetric
   // density's transposed partner tile is written too: (j, k) counts as active
   // where (k, j) is ----
@@ -514,9 +521,9 @@ __global__ void k_zero_inactive(DevAtom A, DevScratch S, double* __restrict__ K,
   }
 }
 
-inline size_t norm_smem(const DevAtom& A, bool split) {
+inline size_t norm_smem(const DevAtom& A, bool lists) {
   const size_t nang2 = (size_t)A.nang * A.nang;
-  return (split ? sizeof(int) * (A.nel + nang2) : 0) + nang2 + A.nent;
+  return (lists ? sizeof(int) * (A.nel + nang2) : 0) + nang2 + A.nent;
 }
 
 // threads of k_block_norms: the rows in equal passes of at most 224, so that
@@ -897,7 +904,7 @@ cudaError_t launch_exchange_erfc(const DevAtom& A, const DevScratch& S, const do
   const int n2 = A.nn * A.nn, nang2 = A.nang * A.nang;
   {
     Mark m(prof, KC_K_NORMS, st);
-    k_block_norms<false><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, false), st>>>(A, S, P, nullptr, 0);
+    k_block_norms<NORM_PLAIN><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, false), st>>>(A, S, P, nullptr, 0);
   }
   {
     Mark m(prof, KC_K_TILES, st);
@@ -913,12 +920,55 @@ cudaError_t launch_exchange_erfc(const DevAtom& A, const DevScratch& S, const do
   return cudaGetLastError();
 }
 
+// every element pair on the tensor cores, the off-diagonal tiles and the
+// diagonal ones through the exchange-ordered tensor (P: FP64 form); blocks
+// without an active entry are zeroed
+static cudaError_t launch_tiles_tc(const DevAtom& A, const DevScratch& S, const DevTC& tc, bool symmetric,
+                                   const double* P, double* K, cudaStream_t st, const SideStream* side) {
+  const int nang2 = A.nang * A.nang;
+  cudaError_t e = cudaSuccess;
+  if (side && side->s) {
+    // the diagonal stage (a chain of dependent steps in 0.8 of a wave)
+    // beside the issue-bound off-diagonal tiles, joined before the fix-up
+    e = cudaEventRecord(side->fork, st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(side->s, side->fork, 0);
+    if (e == cudaSuccess) e = launch_k_diag_tc(A, S, tc, symmetric, P, K, side->s);
+    k_zero_inactive<<<dim3(nang2, 8), 256, 0, side->s>>>(A, S, K, symmetric ? 1 : 0);
+    if (e == cudaSuccess) e = cudaEventRecord(side->join, side->s);
+    if (e == cudaSuccess) e = launch_k_tiles_tc(A, S, tc, symmetric, P, K, st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, side->join, 0);
+  } else {
+    e = launch_k_tiles_tc(A, S, tc, symmetric, P, K, st);
+    if (e == cudaSuccess) e = launch_k_diag_tc(A, S, tc, symmetric, P, K, st);
+    k_zero_inactive<<<dim3(nang2, 8), 256, 0, st>>>(A, S, K, symmetric ? 1 : 0);
+  }
+  return e;
+}
+
 cudaError_t launch_exchange_fp64(const DevAtom& A, const DevScratch& S, const KUnits& U, const double* P,
-                                 double* K, bool symmetric, cudaStream_t st, Profiler* prof) {
+                                 double* K, bool symmetric, cudaStream_t st, Profiler* prof, const DevTC* tc,
+                                 const SideStream* side) {
   const int n2 = A.nn * A.nn, th = threads_for(n2), nang2 = A.nang * A.nang;
+  if (tc) {
+    {
+      Mark m(prof, KC_K_NORMS, st);
+      k_block_norms<NORM_LISTS>
+          <<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, true), st>>>(A, S, P, nullptr, symmetric ? 1 : 0);
+    }
+    {
+      Mark m(prof, KC_K_TILES, st);
+      const cudaError_t e = launch_tiles_tc(A, S, *tc, symmetric, P, K, st, side);
+      if (e != cudaSuccess) return e;
+    }
+    {
+      Mark m(prof, KC_K_FIXUP, st);
+      k_fixup<<<A.nel * A.nel, 256, 0, st>>>(A, S, K, 1);
+    }
+    return cudaGetLastError();
+  }
   {
     Mark m(prof, KC_K_NORMS, st);
-    k_block_norms<false><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, false), st>>>(A, S, P, nullptr, 0);
+    k_block_norms<NORM_PLAIN><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, false), st>>>(A, S, P, nullptr, 0);
   }
   {
     Mark m(prof, KC_K_TILES, st);
@@ -942,7 +992,7 @@ cudaError_t launch_exchange_split(const DevAtom& A, const DevScratch& S, const K
   const int n2 = A.nn * A.nn, th = threads_for(n2), nang2 = A.nang * A.nang;
   {
     Mark m(prof, KC_K_NORMS, st);
-    k_block_norms<true><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, true), st>>>(A, S, P, S.p2, symmetric ? 1 : 0);
+    k_block_norms<NORM_SPLIT><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, true), st>>>(A, S, P, S.p2, symmetric ? 1 : 0);
   }
   {
     Mark m(prof, KC_K_TILES, st);
@@ -950,24 +1000,7 @@ cudaError_t launch_exchange_split(const DevAtom& A, const DevScratch& S, const K
     int nunits = symmetric ? U.n_sym : U.n_all;
     const int4* units = symmetric ? U.sym : U.all;
     if (tc) {
-      // every element pair on the tensor cores: the off-diagonal tiles and
-      // the diagonal ones through the exchange-ordered tensor
-      cudaError_t e = cudaSuccess;
-      if (side && side->s) {
-        // the diagonal stage (a chain of dependent steps in 0.8 of a wave)
-        // beside the issue-bound off-diagonal tiles, joined before the fix-up
-        e = cudaEventRecord(side->fork, st);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(side->s, side->fork, 0);
-        if (e == cudaSuccess) e = launch_k_diag_tc(A, S, *tc, symmetric, K, side->s);
-        k_zero_inactive<<<dim3(nang2, 8), 256, 0, side->s>>>(A, S, K, symmetric ? 1 : 0);
-        if (e == cudaSuccess) e = cudaEventRecord(side->join, side->s);
-        if (e == cudaSuccess) e = launch_k_tiles_tc(A, S, *tc, symmetric, K, st);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(st, side->join, 0);
-      } else {
-        e = launch_k_tiles_tc(A, S, *tc, symmetric, K, st);
-        if (e == cudaSuccess) e = launch_k_diag_tc(A, S, *tc, symmetric, K, st);
-        k_zero_inactive<<<dim3(nang2, 8), 256, 0, st>>>(A, S, K, symmetric ? 1 : 0);
-      }
+      const cudaError_t e = launch_tiles_tc(A, S, *tc, symmetric, nullptr, K, st, side);
       if (e != cudaSuccess) return e;
       nunits = 0;
     }

@@ -42,6 +42,17 @@
 // max|K| against the FP64 result. A row scale shared by the multipoles without
 // the per-table power of two lost log2(1/r) L bits near the nucleus.
 //
+//
+// FP64 form (F64): the same products from the FP64 density itself. The tiles
+// are recoupled with FP64 FMAs (a thirteenth of the FP64 contraction's) and cut
+// into fixed point by shifts of their significands, one digit more (58 bits
+// below the tile's bound, 56 in the diagonal elements); the sums, integers,
+// become FP64 numbers through exact integers. The contraction's own rounding is
+// then below that of the FP64 sums it replaces: the error against the exact K
+// is the tables' in both (4.120e-14 for Kr, l <= 3 dense 2.680e-14 and
+// 2.679e-14), at 1.04 instead of 4.52 ms for Kr. A tile with a value that is
+// not finite gives NaN throughout, as a product with FP64 NaNs does.
+//
 // Off-diagonal work unit = one element pair (a,b) and a range of groups of
 // 8 active output angular blocks (listed by the density pass); per group and
 // multipole L the group's entries with that L form one batch of M = 128 rows.
@@ -63,6 +74,7 @@
 
 #include <cfloat>
 #include <cstdint>
+#include <type_traits>
 
 #include "devatom.cuh"
 #include "smem_limit.hpp"
@@ -306,6 +318,96 @@ __device__ __forceinline__ void digits_pairs(const ffv (&x)[8], float s, uint32_
   }
 }
 
+// ---- FP64 density tiles ----
+
+// x 2^(bits - E) towards zero, two's complement, |x| < 2^E: by shifts of the
+// significand (no FP64-pipe instructions); exponents far below E give 0
+template <int BITS>
+__device__ __forceinline__ uint64_t fixed_point(double x, int E) {
+  const int h = __double2hiint(x);
+  const int sh = min(max(E + 1083 - BITS - ((h >> 20) & 0x7FF), 0), 63);  // from a 61-bit significand
+  const uint64_t m =
+      ((((uint64_t)(uint32_t)((h & 0xFFFFF) | 0x100000)) << 32 | (uint32_t)__double2loint(x)) << 8) >> sh;
+  const uint64_t sg = (uint64_t)(int64_t)(h >> 31);
+  return (m ^ sg) - sg;
+}
+
+// the 6 balanced base-1024 digits of 8 values against |X| < 2^(E + 2), packed
+// as in digits_pairs: with 512 added to every digit the digits are the 10-bit
+// fields of the fixed-point number, and 1024 + field an f16 bit pattern
+__device__ __forceinline__ void digits_fixed(const double (&x)[8], int E, uint32_t (&pk)[PD][4]) {
+  static_assert(PD == 6, "two words of three fields");
+#pragma unroll
+  for (int jj = 0; jj < 8; jj += 2) {
+    uint32_t hi[2], lo[2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const uint64_t f = fixed_point<58>(x[jj + w], E) + 0x0802008020080200ull;
+      lo[w] = (uint32_t)f & 0x3FFFFFFFu;
+      hi[w] = (uint32_t)(f >> 30);
+    }
+    auto digit = [](uint32_t fields) {
+      const uint32_t u = (fields & 0x03FF03FFu) | 0x64006400u;
+      const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&u), __floats2half2_rn(1536.f, 1536.f));
+      return *reinterpret_cast<const uint32_t*>(&d);
+    };
+    auto fields = [&](const uint32_t (&v)[2], int k) {
+      pk[k + 2][jj / 2] = digit(__byte_perm(v[0], v[1], 0x5410));
+      pk[k + 1][jj / 2] = digit(__byte_perm(v[0] << 6, v[1] << 6, 0x7632));
+      pk[k][jj / 2] = digit(__byte_perm(v[0], v[1], 0x7632) >> 4);
+    };
+    fields(hi, 0);
+    fields(lo, 3);
+  }
+}
+
+// the 7 balanced base-256 digits of 8 values against |X| < 2^E, packed as in
+// digits_of
+__device__ __forceinline__ void digits_fixed256(const double (&x)[8], int E, uint32_t (&pk)[ND][4]) {
+  static_assert(ND == 7, "a top digit and six bytes");
+#pragma unroll
+  for (int jj = 0; jj < 8; jj += 2) {
+    float dg[ND][2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const uint64_t f = fixed_point<56>(x[jj + w], E) + 0x0000808080808080ull;
+      const uint32_t hi = (uint32_t)(f >> 32), lo = (uint32_t)f;
+      auto byte = [](uint32_t v, int b) {  // 2^23 + byte, as a float
+        return __fsub_rn(__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440u | b)), 8388736.f);
+      };
+      dg[0][w] = (float)((int)hi >> 16);
+      dg[1][w] = byte(hi, 1);
+      dg[2][w] = byte(hi, 0);
+#pragma unroll
+      for (int k = 3; k < 7; ++k) dg[k][w] = byte(lo, 6 - k);
+    }
+#pragma unroll
+    for (int k = 0; k < ND; ++k) pk[k][jj / 2] = pack_bf16(dg[k][0], dg[k][1]);
+  }
+}
+
+__device__ __forceinline__ double exp2d(int k) {  // 2^k, k clamped to the normal range
+  return __hiloint2double((min(max(k, -1022), 1023) + 1023) << 20, 0);
+}
+// an integer below 2^51 in FP64
+__device__ __forceinline__ double i2d(int64_t i) {
+  return __longlong_as_double(0x4338000000000000ll + i) - 6755399441055744.0;
+}
+// level sums (integers) -> FP64 times 2^k: base 1024, weights 1024^-(d+2), and
+// base 256, weights 256^-(d+2)
+__device__ __forceinline__ double levels_to_f64(const float (&a)[PD], int k) {
+  const int64_t u = ((int64_t)__float2int_rn(a[0]) << 20) + ((int64_t)__float2int_rn(a[1]) << 10) + __float2int_rn(a[2]);
+  const int64_t v = ((int64_t)__float2int_rn(a[3]) << 20) + ((int64_t)__float2int_rn(a[4]) << 10) + __float2int_rn(a[5]);
+  return fma(i2d(v), 9.313225746154785e-10, i2d(u)) * exp2d(k - 40);
+}
+__device__ __forceinline__ double levels_to_f64(const float (&a)[ND], int k) {
+  const int64_t u = ((int64_t)__float2int_rn(a[0]) << 16) + ((int64_t)__float2int_rn(a[1]) << 8) + __float2int_rn(a[2]);
+  const int64_t v = ((int64_t)__float2int_rn(a[3]) << 24) + ((int64_t)__float2int_rn(a[4]) << 16) +
+                    ((int64_t)__float2int_rn(a[5]) << 8) + __float2int_rn(a[6]);
+  return fma(i2d(v), 2.3283064365386963e-10, i2d(u)) * exp2d(k - 32);
+}
+constexpr int kBadExp = 1 << 20;  // exponent of a tile with a value that is not finite
+
 // the 8 values y[j] of tile (a,b), block jk (-1: none), at row p and columns
 // q0 + j: one pass over the columns with the block's base address computed
 // once; owned entries go to K, the shared last row / column to the halo buffer
@@ -360,17 +462,22 @@ struct PairMeta {
 // first and this second product, which run while the warps recouple. One
 // arrival count per batch is all the synchronisation between warps (a warp of
 // its own that issues, with a barrier per role, cost 32 registers a thread).
+template <bool F64>
 __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch S, DevTC T,
                                                           const int4* __restrict__ units, int symmetric,
-                                                          double* __restrict__ K) {
+                                                          const double* __restrict__ P, double* __restrict__ K) {
+  using Val = std::conditional_t<F64, double, float2>;
+  constexpr int NX = F64 ? PD : PX;  // digits of a density tile
+  const Val* src;
+  if constexpr (F64) src = P; else src = S.p2;
   const int4 u = units[blockIdx.x];
   const int a = u.x, b = u.y;
   const int nn = A.nn, NL = A.NL, nang2 = A.nang * A.nang;
   const int count = S.ocount[0], g0 = u.z, g1 = min(u.w, (count + 7) / 8);
   if (g0 >= g1) return;  // uniform over the CTA
   extern __shared__ __align__(1024) unsigned char smraw[];
-  unsigned char* A1 = smraw;                   // 2 stages x PX planes: rows (slot, q), K = p (MN-major)
-  unsigned char* A2 = A1 + 2 * PX * APLANE;    // PD planes: rows (slot, i), K = q (MN-major)
+  unsigned char* A1 = smraw;                   // 2 stages x NX planes: rows (slot, q), K = p (MN-major)
+  unsigned char* A2 = A1 + 2 * NX * APLANE;    // PD planes: rows (slot, i), K = q (MN-major)
   unsigned char* T1 = A2 + PD * APLANE;        // NL * PD planes of the left tables of element a
   unsigned char* T2 = T1 + NL * PD * TPLANE;   // NL * PD planes of the right tables of element b
   PairMeta& m = *reinterpret_cast<PairMeta*>(T2 + NL * PD * TPLANE);
@@ -440,25 +547,29 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
     // tiles stream through one register buffer: an element's next value is
     // loaded, for the next batch too, as soon as the last one is added.
     int toff[2], tL[2], E = 0, mask = 0;
-    float2 tc2[2];
+    Val tc2[2];
     unsigned r0 = 0, r1 = 0;  // terms not yet loaded
-    float2 c = make_float2(0.f, 0.f), pv[8];  // coefficient and tile of the term in flight
+    Val c{}, pv[8];  // coefficient and tile of the term in flight
     int off = 0;
     auto next_term = [&]() {  // its offset and coefficient; false: none left in the group
       if (!(r0 | r1)) return false;
       const bool lo = r0 != 0;
-      const int src = __ffs(lo ? r0 : r1) - 1;
+      const int at = __ffs(lo ? r0 : r1) - 1;
       if (lo) r0 &= r0 - 1; else r1 &= r1 - 1;
-      off = __shfl_sync(0xffffffffu, lo ? toff[0] : toff[1], src);
-      c.x = __shfl_sync(0xffffffffu, lo ? tc2[0].x : tc2[1].x, src);
-      c.y = __shfl_sync(0xffffffffu, lo ? tc2[0].y : tc2[1].y, src);
+      off = __shfl_sync(0xffffffffu, lo ? toff[0] : toff[1], at);
+      if constexpr (F64) {
+        c = __shfl_sync(0xffffffffu, lo ? tc2[0] : tc2[1], at);
+      } else {
+        c.x = __shfl_sync(0xffffffffu, lo ? tc2[0].x : tc2[1].x, at);
+        c.y = __shfl_sync(0xffffffffu, lo ? tc2[0].y : tc2[1].y, at);
+      }
       return true;
     };
     // A group's terms come in three steps, each load's latency covered by a
     // part of the batch before: the block's range, its terms, the tile maxima.
     int4 next = 8 * g0 + warp < count ? S.oinfo[8 * g0 + warp] : make_int4(-1, 0, 0, -1);
     int tblk[2], pairjk = -1;
-    float bd[2];
+    unsigned bd[2];  // tile maxima: bits of a float, of a double's high word
     auto terms_of = [&](int g) {
       const int4 info = next;  // block, first term, terms, j | k << 16
       next = g + 1 < g1 && 8 * g + 8 + warp < count ? S.oinfo[8 * g + 8 + warp] : make_int4(-1, 0, 0, -1);
@@ -469,7 +580,7 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
         if (lane + 32 * r < info.z) {
           const int uu = info.y + lane + 32 * r;
           tblk[r] = A.kterm_blk[uu];
-          tc2[r] = A.kterm_coef2[uu];
+          if constexpr (F64) tc2[r] = A.kterm_coef[uu]; else tc2[r] = A.kterm_coef2[uu];
           toff[r] = A.kterm_off[uu];
           tL[r] = A.kterm_L[uu];
         }
@@ -478,9 +589,9 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
     auto bounds_of = [&]() {
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        bd[r] = 0.f;
+        bd[r] = 0u;
         if (tblk[r] >= 0 && act[tblk[r]])
-          bd[r] = __uint_as_float(S.tmax[((size_t)tblk[r] * A.nel + a) * A.nel + b]);
+          bd[r] = S.tmax[((size_t)tblk[r] * A.nel + a) * A.nel + b];
         else
           tL[r] = -1;
       }
@@ -497,23 +608,39 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
       mask = (int)__reduce_or_sync(0xffffffffu, any);
       if (next_term())
 #pragma unroll
-        for (int j = 0; j < 8; ++j) pv[j] = S.p2[off + coff[j]];
+        for (int j = 0; j < 8; ++j) pv[j] = src[off + coff[j]];
       // |X_L| <= sum of |c| max|P| (high words and roundings: 2^-20), summed
       // upwards in units of 2^(e0 - 24): the largest multipole's, scaled by its
       // tables, gives E (s_hi - 96 at least: every scale stays a normal float)
-      unsigned mx = 0;
+      unsigned mx = 0, su[2], top = 0;
+      int e0;
+      if constexpr (F64) {
+        double v[2];
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        if (tL[r] >= 0) bd[r] *= fabsf(tc2[r].x) * 1.000001f * exp2i(m.sL[tL[r]] - s_hi);
-        mx = max(mx, __float_as_uint(bd[r]));
+        for (int r = 0; r < 2; ++r) {
+          v[r] = tL[r] < 0 ? 0.0
+                           : __hiloint2double((int)bd[r], -1) * (fabs(tc2[r]) * 1.000001) * exp2d(m.sL[tL[r]] - s_hi);
+          mx = max(mx, (unsigned)__double2hiint(v[r]));
+        }
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        e0 = max((int)(mx >> 20) - 1022, -900);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) su[r] = __double2uint_ru(v[r] * exp2d(24 - e0));
+      } else {
+        float v[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          v[r] = tL[r] < 0 ? 0.f : __uint_as_float(bd[r]) * (fabsf(tc2[r].x) * 1.000001f * exp2i(m.sL[tL[r]] - s_hi));
+          mx = max(mx, __float_as_uint(v[r]));
+        }
+        e0 = max((int)(__reduce_max_sync(0xffffffffu, mx) >> 23) - 126, -96);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) su[r] = __float2uint_ru(v[r] * exp2i(24 - e0));
       }
-      const int e0 = max((int)(__reduce_max_sync(0xffffffffu, mx) >> 23) - 126, -96);
-      unsigned su[2], top = 0;
-#pragma unroll
-      for (int r = 0; r < 2; ++r) su[r] = __float2uint_ru(bd[r] * exp2i(24 - e0));
       for (int L = 0; L < NL; ++L)
         top = max(top, __reduce_add_sync(0xffffffffu, (tL[0] == L ? su[0] : 0u) + (tL[1] == L ? su[1] : 0u)));
-      E = max(s_hi - 96, s_hi + e0 + 8 - __clz(top));
+      E = max(s_hi + (F64 ? -900 : -96), s_hi + e0 + 8 - __clz(top));
+      if (F64 && mx >= 0x7FF00000u) E = kBadExp;
       if (lane == 0) {
         m.ex[g & 3][warp] = E;
         m.mask[g & 3][warp] = mask;
@@ -524,38 +651,42 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
     auto produce = [&](int L, int st) {
       if ((mask >> L) & 1) {
         int left = __popc(__ballot_sync(0xffffffffu, tL[0] == L)) + __popc(__ballot_sync(0xffffffffu, tL[1] == L));
-        ffv x[8];
+        std::conditional_t<F64, double, ffv> x[8];
         {  // an exact product: no sum to carry
-          const float2 cc = c;
+          const Val cc = c;
           const bool more = next_term();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float p = __fmul_rn(cc.x, pv[j].x);
-            float pe = fmaf(cc.x, pv[j].x, -p);
-            pe = fmaf(cc.x, pv[j].y, pe);
-            x[j] = {p, fmaf(cc.y, pv[j].x, pe)};
-            if (more) pv[j] = S.p2[off + coff[j]];
+            if constexpr (F64) {
+              x[j] = cc * pv[j];
+            } else {
+              const float p = __fmul_rn(cc.x, pv[j].x);
+              float pe = fmaf(cc.x, pv[j].x, -p);
+              pe = fmaf(cc.x, pv[j].y, pe);
+              x[j] = {p, fmaf(cc.y, pv[j].x, pe)};
+            }
+            if (more) pv[j] = src[off + coff[j]];
           }
         }
 #pragma unroll 1
         while (--left > 0) {
-          const float2 cc = c;
+          const Val cc = c;
           const bool more = next_term();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            x[j] = ff_fma(x[j], cc, pv[j]);
-            if (more) pv[j] = S.p2[off + coff[j]];
+            if constexpr (F64) x[j] = fma(cc, pv[j], x[j]); else x[j] = ff_fma(x[j], cc, pv[j]);
+            if (more) pv[j] = src[off + coff[j]];
           }
         }
         if (edge)
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            if (!((vm >> j) & 1u)) x[j] = {0.f, 0.f};
-        uint32_t pk[PX][4];
-        digits_pairs(x, exp2i(30 + m.sL[L] - E), pk);
-        unsigned char* o = A1 + st * PX * APLANE + off1;
+            if (!((vm >> j) & 1u)) x[j] = {};
+        uint32_t pk[NX][4];
+        if constexpr (F64) digits_fixed(x, E - m.sL[L], pk); else digits_pairs(x, exp2i(30 + m.sL[L] - E), pk);
+        unsigned char* o = A1 + st * NX * APLANE + off1;
 #pragma unroll
-        for (int k = 0; k < PX; ++k)
+        for (int k = 0; k < NX; ++k)
           *reinterpret_cast<uint4*>(o + k * APLANE) = make_uint4(pk[k][0], pk[k][1], pk[k][2], pk[k][3]);
       }
       // (operand rows of an idle slot keep their old digits: a tensor-core row
@@ -578,10 +709,10 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
         if ((was & (PW - 1)) == PW - 1) {
           tc::fence_after_sync();
           if (L1 >= 0) {
-            const uint64_t dA = tc::smem_desc(tc::smem_u32(A1 + st * PX * APLANE));
+            const uint64_t dA = tc::smem_desc(tc::smem_u32(A1 + st * NX * APLANE));
             const uint64_t dT = tc::smem_desc(tc::smem_u32(T1 + L1 * PD * TPLANE));
 #pragma unroll
-            for (int kx = 0; kx < PX; ++kx)
+            for (int kx = 0; kx < NX; ++kx)
               tc::mma_bf16(tD1 + 16 * kx, dA + (uint64_t)(kx * APLANE >> 4), dT, tc::idesc_f16(128, 16 * (PD - kx), 1, 0),
                            kx > 0 ? 1u : 0u);
           }
@@ -613,7 +744,7 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
         const int idx = (lane >> 4) * 256 + r * 16 + (cc ^ r);  // ^ r: spread over the banks
         return reinterpret_cast<double*>(A2 + (idx >> 7) * APLANE + qw * 1024) + (idx & 127);
       };
-      const int ea = m.alpha[oi] + E2;
+      const int ea = m.alpha[oi] + E2;  // (FP64 tiles are scaled to below 1/4)
 #pragma unroll 1
       for (int h = 8 * half; h < 8 * half + 8; h += 4) {
         float v[PD][4];
@@ -624,7 +755,10 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
           float lv[PD];
 #pragma unroll
           for (int d = 0; d < PD; ++d) lv[d] = v[d][j];
-          y[j] = -levels_to_d(lv, (max(ea + m.beta[h + j], -800) + 896) << 20);
+          if constexpr (F64)
+            y[j] = E2 == kBadExp ? __longlong_as_double(0x7ff8000000000000ll) : -levels_to_f64(lv, ea + m.beta[h + j] + 2);
+          else
+            y[j] = -levels_to_d(lv, (max(ea + m.beta[h + j], -800) + 896) << 20);
           if (symmetric) *stage(oi, h + j) = y[j];
         }
         if (jk >= 0) store_rows(A, S, K, a, b, jk & 0xFFFF, jk >> 16, oi, h, y);
@@ -781,8 +915,14 @@ __global__ void tc_tk_digits_kernel(const double* __restrict__ tk, int NL, int n
   }
 }
 
+template <bool F64>
 __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, DevTC T, int symmetric,
-                                                    double* __restrict__ K) {
+                                                    const double* __restrict__ P, double* __restrict__ K) {
+  using Val = std::conditional_t<F64, double, float2>;
+  using Sum = std::conditional_t<F64, double, ffv>;
+  constexpr int NX = F64 ? ND : NDX;  // digits of the density vectors
+  const Val* src;
+  if constexpr (F64) src = P; else src = S.p2;
   const int nn = A.nn, n2 = nn * nn, NL = A.NL, nang2 = A.nang * A.nang;
   const int ksteps = T.dksteps, mtiles = T.dmtiles;
   // unit = (element, row tile, group of 16 active output blocks); the list is
@@ -821,8 +961,8 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
       }
   }
   for (int idx = t; idx < nang2; idx += blockDim.x) act[idx] = S.act[idx];
-  // the zero seventh density plane of every K step (operands of N = 112)
-  for (int idx = t; idx < ksteps * (TPLANE / 16); idx += blockDim.x) {
+  // the zero seventh plane of float-pair densities in every K step (operands of N = 112)
+  for (int idx = t; NX < ND && idx < ksteps * (TPLANE / 16); idx += blockDim.x) {
     const int ks = idx / (TPLANE / 16), o = idx % (TPLANE / 16);
     reinterpret_cast<uint4*>(Bx + ((size_t)ks * ND + NDX) * TPLANE)[o] = make_uint4(0, 0, 0, 0);
   }
@@ -844,9 +984,9 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
   const uint64_t dA = tc::smem_desc(tc::smem_u32(Abuf)), dB = tc::smem_desc(tc::smem_u32(Bx));
   const int row = 32 * qw + lane, trow = 128 * mt + row;  // this thread's tensor-memory lane
   const int nchunk = DSLOT * 2 * ksteps;                  // chunks of 8 consecutive v per slot
-  ffv acc[8];
+  Sum acc[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j] = {0.f, 0.f};
+  for (int j = 0; j < 8; ++j) acc[j] = {};
 
   for (int L = 0; L < NL; ++L) {
     int any = 0;
@@ -862,15 +1002,15 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
       }
     }
     for (int idx = t; idx < 128; idx += blockDim.x) alpha[idx] = T.tk_rowexp[tslice * 128 + idx];
-    if (t < DSLOT) exs[t] = 0;
+    if (t < DSLOT) exs[t] = F64 ? 64 : 0;  // (FP64: so far above a zero that its significand is shifted out)
     __syncthreads();
     // ---- recouple the 16 density vectors and take each slot's exponent ----
-    ffv xs[2][8];
+    Sum xs[2][8];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const int ch = t + c * 256;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) xs[c][j] = {0.f, 0.f};
+      for (int j = 0; j < 8; ++j) xs[c][j] = {};
       if (ch >= nchunk) continue;
       const int s = ch / (2 * ksteps), v0 = 8 * (ch % (2 * ksteps));
       if (!sact[L * DSLOT + s]) continue;
@@ -885,25 +1025,39 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
       // two terms' loads in flight together
       const int u1 = A.kent_ptr[ent + 1];
       for (int uu = A.kent_ptr[ent]; uu < u1; uu += 2) {
-        float2 cf[2], pv[2][8];
+        Val cf[2], pv[2][8];
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
           const bool on = uu + w < u1 && act[A.kterm_blk[uu + w]];
-          cf[w] = on ? A.kterm_coef2[uu + w] : make_float2(0.f, 0.f);
-          const float2* pb = S.p2 + (on ? A.kterm_off[uu + w] : 0);
+          cf[w] = {};
+          if constexpr (F64) {
+            if (on) cf[w] = A.kterm_coef[uu + w];
+          } else {
+            if (on) cf[w] = A.kterm_coef2[uu + w];
+          }
+          const Val* pb = src + (on ? A.kterm_off[uu + w] : 0);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) pv[w][j] = (on && eo[j] >= 0) ? pb[eo[j]] : make_float2(0.f, 0.f);
+          for (int j = 0; j < 8; ++j) {
+            pv[w][j] = {};
+            if (on && eo[j] >= 0) pv[w][j] = pb[eo[j]];
+          }
         }
 #pragma unroll
         for (int w = 0; w < 2; ++w)
 #pragma unroll
-          for (int j = 0; j < 8; ++j) xs[c][j] = ff_fma(xs[c][j], cf[w], pv[w][j]);
+          for (int j = 0; j < 8; ++j) {
+            if constexpr (F64) xs[c][j] = fma(cf[w], pv[w][j], xs[c][j]); else xs[c][j] = ff_fma(xs[c][j], cf[w], pv[w][j]);
+          }
       }
       unsigned eb = 0;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        xs[c][j] = ff_norm(xs[c][j].hi, xs[c][j].lo);
-        eb = max(eb, (__float_as_uint(xs[c][j].hi) >> 23) & 0xFFu);
+        if constexpr (F64) {
+          eb = max(eb, ((unsigned)__double2hiint(xs[c][j]) >> 20) & 0x7FFu);
+        } else {
+          xs[c][j] = ff_norm(xs[c][j].hi, xs[c][j].lo);
+          eb = max(eb, (__float_as_uint(xs[c][j].hi) >> 23) & 0xFFu);
+        }
       }
       atomicMax(&exs[s], (int)eb);
     }
@@ -914,11 +1068,11 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
       const int ch = t + c * 256;
       if (ch >= nchunk) continue;
       const int s = ch / (2 * ksteps), kk = ch % (2 * ksteps), ks = kk >> 1, h = kk & 1;
-      uint32_t pk[NDX][4];
-      digits_of(xs[c], tile_exponent((unsigned)exs[s]), pk);
+      uint32_t pk[NX][4];
+      if constexpr (F64) digits_fixed256(xs[c], exs[s] - 1022, pk); else digits_of(xs[c], tile_exponent((unsigned)exs[s]), pk);
       const uint32_t off = tc::off_kmajor(s, 8 * h);
 #pragma unroll
-      for (int k = 0; k < NDX; ++k)
+      for (int k = 0; k < NX; ++k)
         *reinterpret_cast<uint4*>(Bx + ((size_t)ks * ND + k) * TPLANE + off) =
             make_uint4(pk[k][0], pk[k][1], pk[k][2], pk[k][3]);
     }
@@ -975,7 +1129,10 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
         float lv[ND];
 #pragma unroll
         for (int d = 0; d < ND; ++d) lv[d] = v[d][j];
-        acc[j] = ff_add(acc[j], levels_to_pair(lv, exp2i(ea + tile_exponent((unsigned)exs[s]))));
+        if constexpr (F64)
+          acc[j] += exs[s] == 0x7FF ? __longlong_as_double(0x7ff8000000000000ll) : levels_to_f64(lv, ea + exs[s] - 1022);
+        else
+          acc[j] = ff_add(acc[j], levels_to_pair(lv, exp2i(ea + tile_exponent((unsigned)exs[s]))));
       }
     }
     tc::fence_before_sync();
@@ -991,7 +1148,9 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
     for (int j = 0; j < 8; ++j) {
       const int jk = gjk[8 * half + j];
       if (jk < 0) continue;
-      const double y = failed ? __longlong_as_double(0x7ff8000000000000ll) : -pair_to_d(acc[j]);
+      double y;
+      if constexpr (F64) y = -acc[j]; else y = -pair_to_d(acc[j]);
+      if (failed) y = __longlong_as_double(0x7ff8000000000000ll);
       k_store_tile(A, S, K, a, a, jk, p, q, y);
       const int j0 = jk % A.nang, k0 = jk / A.nang;
       if (symmetric && j0 != k0) k_store_tile(A, S, K, a, a, k0 + j0 * A.nang, q, p, y);
@@ -1006,8 +1165,9 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
   if (warp == 0) tc::tmem_dealloc(tD, 128);
 }
 
-size_t tc_smem_bytes(int NL, int nang) {
-  return (size_t)(2 * PX + PD) * APLANE + (size_t)2 * NL * PD * TPLANE + sizeof(PairMeta) + (size_t)nang * nang + 16;
+size_t tc_smem_bytes(int NL, int nang, bool f64) {
+  return (size_t)(2 * (f64 ? PD : PX) + PD) * APLANE + (size_t)2 * NL * PD * TPLANE + sizeof(PairMeta) +
+         (size_t)nang * nang + 16;
 }
 
 size_t tc_diag_smem_bytes(int NL, int ksteps, int nang) {
@@ -1015,14 +1175,16 @@ size_t tc_diag_smem_bytes(int NL, int ksteps, int nang) {
          sizeof(int) * (128 + DSLOT + NL * DSLOT * 2 + DSLOT + 2) + 5 * 8 + 8 + (size_t)nang * nang + 64;
 }
 
-cudaError_t launch_k_tiles_tc(const DevAtom& A, const DevScratch& S, const DevTC& T, bool symmetric, double* K,
-                              cudaStream_t st) {
+// P: the FP64 form (from the density itself), nullptr: the split form (from S.p2)
+cudaError_t launch_k_tiles_tc(const DevAtom& A, const DevScratch& S, const DevTC& T, bool symmetric, const double* P,
+                              double* K, cudaStream_t st) {
   const int n = symmetric ? T.n_sym : T.n_all;
   if (n == 0) return cudaSuccess;
-  const size_t smem = tc_smem_bytes(A.NL, A.nang);
-  const cudaError_t e = smem_limit(k_tiles_tc, smem);
+  const size_t smem = tc_smem_bytes(A.NL, A.nang, P != nullptr);
+  auto kern = P ? k_tiles_tc<true> : k_tiles_tc<false>;
+  const cudaError_t e = smem_limit(kern, smem);
   if (e != cudaSuccess) return e;
-  k_tiles_tc<<<n, PTHREADS, smem, st>>>(A, S, T, symmetric ? T.units_sym : T.units_all, symmetric ? 1 : 0, K);
+  kern<<<n, PTHREADS, smem, st>>>(A, S, T, symmetric ? T.units_sym : T.units_all, symmetric ? 1 : 0, P, K);
   return cudaGetLastError();
 }
 
@@ -1035,16 +1197,17 @@ cudaError_t launch_tk_digits(const DevAtom& A, int mtiles, int ksteps, unsigned 
   return cudaGetLastError();
 }
 
-cudaError_t launch_k_diag_tc(const DevAtom& A, const DevScratch& S, const DevTC& T, bool symmetric, double* K,
-                             cudaStream_t st) {
+cudaError_t launch_k_diag_tc(const DevAtom& A, const DevScratch& S, const DevTC& T, bool symmetric, const double* P,
+                             double* K, cudaStream_t st) {
   DevTC Td = T;
   const int nblk = symmetric ? A.nang * (A.nang + 1) / 2 : A.nang * A.nang;
   Td.dgroups = (nblk + DSLOT - 1) / DSLOT;
   const int n = A.nel * T.dmtiles * Td.dgroups;
   const size_t smem = tc_diag_smem_bytes(A.NL, T.dksteps, A.nang);
-  const cudaError_t e = smem_limit(k_diag_tc, smem);
+  auto kern = P ? k_diag_tc<true> : k_diag_tc<false>;
+  const cudaError_t e = smem_limit(kern, smem);
   if (e != cudaSuccess) return e;
-  k_diag_tc<<<n, 256, smem, st>>>(A, S, Td, symmetric ? 1 : 0, K);
+  kern<<<n, 256, smem, st>>>(A, S, Td, symmetric ? 1 : 0, P, K);
   return cudaGetLastError();
 }
 

@@ -170,8 +170,9 @@ struct hfg_atom {
   // bf16 MMA FLOPs one tensor-core exchange issues with every entry active
   // (index 0: symmetric mode, 1: general)
   double tc_mma_flops[2] = {0.0, 0.0};
-  // the split exchange on the tensor cores (off-diagonal element pairs), or
-  // nullptr for the float-pair form everywhere (HFG_SPLIT_FORM=pairs)
+  // the split exchange on the tensor cores, or nullptr for the float-pair form
+  // everywhere (HFG_SPLIT_FORM=pairs, which keeps the FP64 form on its own
+  // kernel too)
   const hfg::DevTC* tc_for(bool screened) const {
     if (!tc_ok) return nullptr;
     static const bool pairs = [] {
@@ -180,6 +181,22 @@ struct hfg_atom {
     }();
     if (pairs) return nullptr;
     return screened ? (tc_rs.digits ? &tc_rs : nullptr) : &tc;
+  }
+  // The FP64 exchange on the tensor cores, or nullptr for the FP64 kernel
+  // (k_tiles). The line lies where the FP64 pipe's work per digit product (nn^3
+  // and, in the elements, nn^4 per entry) outweighs the digit work, which hardly
+  // depends on nn: below 13 nodes only with several m (entries share batches) and
+  // many element pairs, and never for a single shell, whose batches are seven
+  // eighths empty. Measured, FP64 kernel against this form, us: l <= 2, 20
+  // elements of 10 nodes 185 and 153 (m-diagonal density), 501 and 325 (dense),
+  // of 8 nodes 99 and 130, 226 and 294; l <= 1, 6 elements of 15 nodes 101 and
+  // 84, of 10 nodes 57 and 60; l = 0, 30 elements of 15 nodes 53 and 70; Kr
+  // (l <= 2, 40 elements of 15 nodes, dense) 4520 and 1040.
+  const hfg::DevTC* tc64_for(bool screened) const {
+    const int nn = host.rad.nn, nang = host.nang, nel = host.rad.nel;
+    const bool on = nn >= 13 ? nang >= 2 && (nel >= 6 || nang >= 9)
+                             : nn >= 10 && nang >= 4 && nel >= (nang >= 9 ? 12 : 16);
+    return on ? tc_for(screened) : nullptr;
   }
   // digits of the radial tables (kind 0 r_small, 1 r_big; per (L, e) a
   // 16 x 16 plane per digit, element (row n, column k) = table(n, k)), the
@@ -337,6 +354,7 @@ struct hfg_atom {
     // per batch: 20 + 21 digit-plane products of 128 x 16 x 16
     const double per = 2.0 * 128 * 16 * 16 * 41 * (double)batches(order, 8);
     tc_tables(H.rs, H.rb, t_dig, t_exp, t_texp, tc);
+    side_stream();
     tc_units();
     t_err.alloc(sizeof(int));
     ck(cudaMemsetAsync(t_err.p, 0, sizeof(int), own_stream), "memset");

@@ -746,7 +746,7 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
                "K (split)");
           else
             ck(hfg::launch_exchange_fp64(a->dev, a->scr, a->units, dPs[s].as<double>(), dK[s].as<double>(), true,
-                                         st, &a->prof),
+                                         st, &a->prof, a->tc64_for(false), &a->k_side),
                "K");
         }
       if (have_xc) run_xc();
