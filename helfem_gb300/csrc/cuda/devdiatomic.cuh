@@ -82,7 +82,7 @@ struct DevDiatomic {
 
 // In-element tiles of the split exchange on the tensor cores (dk_tc.cu): digit
 // planes of the exchange-ordered kernel, and the scratch of one call
-#define DTC_XDIGITS 6
+#define DTC_XDIGITS 6  // of a recoupled float-pair tile; one of FP64 has as many as the table
 #define DTC_TDIGITS 7
 #define DTC_TT 64
 struct DevDiaTC {
@@ -178,13 +178,14 @@ cudaError_t launch_diatomic_tx(const DevDiatomic& D, double* tx, cudaStream_t st
 // J of a pure-basis density, written to the pure-basis J (overwritten)
 cudaError_t launch_diatomic_coulomb(const DevDiatomic& D, const DevDiatomicScratch& S, const double* P, double* J,
                                     cudaStream_t st);
+// tc: the in-element tiles on the tensor cores, or nullptr for the FP64 kernels (T)
 cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDia64& T,
-                                     const double* Pd, double* Kd, bool symmetric, cudaStream_t st);
+                                     const DevDiaTC* tc, const double* Pd, double* Kd, bool symmetric, cudaStream_t st);
 cudaError_t launch_dk_tc_table(const DevDiatomic& D, const DevDiaTC& T, unsigned char* tx, int* txexp, int* cexp,
                                cudaStream_t st);
-size_t dtc_gemm_smem(const DevDiatomic& D);
-cudaError_t launch_dk_tc_diag(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDiaTC& T, double* Kd,
-                              bool symmetric, bool itemwise, cudaStream_t st);
+size_t dtc_gemm_smem(const DevDiatomic& D, bool f64);
+cudaError_t launch_dk_tc_diag(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDiaTC& T, const double* Pd,
+                              double* Kd, bool symmetric, bool itemwise, cudaStream_t st);
 // split-precision exchange: off-diagonal element pairs in float pairs, the
 // in-element tiles on the tensor cores; itemwise: their recoupled tiles one
 // output block at a time (bitwise the same K)

@@ -423,7 +423,8 @@ cudaError_t launch_diatomic_coulomb(const DevDiatomic& D, const DevDiatomicScrat
 }
 
 cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDia64& T,
-                                     const double* Pd, double* Kd, bool symmetric, cudaStream_t st) {
+                                     const DevDiaTC* tc, const double* Pd, double* Kd, bool symmetric,
+                                     cudaStream_t st) {
   const int nang2 = D.nang * D.nang;
   cudaError_t e = cudaMemsetAsync(Kd, 0, sizeof(double) * (size_t)D.nd * D.nd, st);
   if (e != cudaSuccess) return e;
@@ -431,7 +432,8 @@ cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScra
   dk_act<<<(nang2 + 255) / 256, 256, 0, st>>>(D, S);
   dk_entry_act<<<std::max(1, (D.nent + 127) / 128), 128, 0, st>>>(D, S);
   dk_compact<<<1, 1024, 0, st>>>(D, S, symmetric ? 1 : 0);
-  e = launch_dk_share_diag(D, S, T, Pd, Kd, symmetric, st);
+  e = tc ? launch_dk_tc_diag(D, S, *tc, Pd, Kd, symmetric, false, st)
+         : launch_dk_share_diag(D, S, T, Pd, Kd, symmetric, st);
   if (e == cudaSuccess) e = launch_dk_share_off(D, S, Pd, Kd, symmetric, false, st);
   if (e != cudaSuccess) return e;
   dk_fixup<<<D.nel * D.nel, 256, 0, st>>>(D, S, Kd);
@@ -448,7 +450,7 @@ cudaError_t launch_diatomic_exchange_split(const DevDiatomic& D, const DevDiatom
   dk_act<<<(nang2 + 255) / 256, 256, 0, st>>>(D, S);
   dk_entry_act<<<std::max(1, (D.nent + 127) / 128), 128, 0, st>>>(D, S);
   dk_compact<<<1, 1024, 0, st>>>(D, S, symmetric ? 1 : 0);
-  e = launch_dk_tc_diag(D, S, T, Kd, symmetric, itemwise, st);
+  e = launch_dk_tc_diag(D, S, T, nullptr, Kd, symmetric, itemwise, st);
   if (e == cudaSuccess) e = launch_dk_share_off(D, S, Pd, Kd, symmetric, true, st);
   if (e != cudaSuccess) return e;
   dk_fixup<<<D.nel * D.nel, 256, 0, st>>>(D, S, Kd);

@@ -7,7 +7,7 @@
 // t and K = 4 nn^2 per multipole and element.
 //
 // Arithmetic (as in k_tc.cu): fixed-point operands as balanced base-512 digits
-// (integers up to 512, exact in f16), six each; the kernel rows t are scaled
+// (integers up to 512, exact in f16), seven of the kernel, six of a tile; the kernel rows t are scaled
 // so that their absolute row sum (all channels, with the multipole's factor)
 // is at most 1, the recoupled tiles so that their largest entry is below 1.
 // The tensor core sums the digit products level by level (acc_d = sum over
@@ -16,6 +16,14 @@
 // unit row sum, and the others are spread over +-256, so that a level's sum of
 // 900 products has a spread below 2^21. The levels are carried into a float
 // pair, scaled and summed over the multipoles, one FP64 value per entry.
+//
+// FP64 form (F64): the tiles are recoupled in FP64 and cut into seven digits by
+// shifts of their significands (59 bits below the largest entry), the level
+// sums (integers) added up in FP64: the error against the exact K is that of the
+// FP64 kernels (H2 6.2e-15 and 6.4e-15, CO 1.005e-14 and 1.010e-14 of |K|). A
+// tile with a value that is not finite gives NaN in its rows. Whole K, FP64
+// kernels for these tiles and this form: H2 on 3 elements, l <= 4 0.55 and 0.29
+// ms; N2 on 9 elements, l <= 10, m <= 3 132 and 87 ms.
 //
 // Two passes: dk_tc_x recouples each (element, output block, multipole) once
 // (sharing the sums over l between the output rows of one k) and writes its
@@ -31,15 +39,17 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "dk_recouple.cuh"
+#include "fixed.cuh"
 #include "smem_limit.hpp"
 #include "tc.cuh"
 
 namespace hfg {
 namespace {
 
-constexpr int XD = DTC_XDIGITS;   // digits of a recoupled tile (54 bits: a float pair has 48)
+constexpr int XD = DTC_XDIGITS;   // digits of a float-pair tile (54 bits: a float pair has 48)
 constexpr int TD = DTC_TDIGITS;   // digits of the table, and levels kept
 constexpr int APL = 4096;             // bytes of a 128 x 16 f16 plane
 constexpr int TT = DTC_TT;            // tile entries t per CTA
@@ -70,6 +80,43 @@ __device__ __forceinline__ void digits512(float2 x, float s27, float (&d)[XD]) {
     d[k] = rnd_mul(r, 512.0f);
     r = __fmaf_rn(r, 512.0f, -d[k]);
   }
+}
+
+// seven balanced base-512 digits (weights 512^-(k+1)) of 8 values |x| < 2^(E+2):
+// with 256 added to every digit the digits are the 9-bit fields of the
+// fixed-point number, and 1024 + field an f16 bit pattern
+__device__ __forceinline__ void digits512_fixed(const double (&x)[8], int E, uint32_t (&pk)[TD][4]) {
+  static_assert(TD == 7, "three fields in each of two words and one on top");
+#pragma unroll
+  for (int jj = 0; jj < 8; jj += 2) {
+    uint32_t w[3][2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint64_t f = fixed_point<61>(x[jj + i], E) + 0x4020100804020100ull;
+      w[0][i] = (uint32_t)f & 0x7FFFFFFu;
+      w[1][i] = (uint32_t)(f >> 27) & 0x7FFFFFFu;
+      w[2][i] = (uint32_t)(f >> 54);
+    }
+    auto digit = [](uint32_t a, uint32_t b) {
+      const uint32_t u = (__byte_perm(a, b, 0x5410) & 0x01FF01FFu) | 0x64006400u;
+      const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&u), __floats2half2_rn(1280.f, 1280.f));
+      return *reinterpret_cast<const uint32_t*>(&d);
+    };
+    pk[0][jj / 2] = digit(w[2][0], w[2][1]);
+#pragma unroll
+    for (int k = 1; k < TD; ++k) {
+      const int v = k <= 3 ? 1 : 0, sh = 9 * ((6 - k) % 3);
+      pk[k][jj / 2] = digit(w[v][0] >> sh, w[v][1] >> sh);
+    }
+  }
+}
+
+// level sums (integers) -> FP64 times 2^k
+__device__ __forceinline__ double levels512_f64(const float (&a)[TD], int k) {
+  const int64_t u = ((int64_t)__float2int_rn(a[0]) << 18) + ((int64_t)__float2int_rn(a[1]) << 9) + __float2int_rn(a[2]);
+  const int64_t v = ((int64_t)__float2int_rn(a[3]) << 27) + ((int64_t)__float2int_rn(a[4]) << 18) +
+                    ((int64_t)__float2int_rn(a[5]) << 9) + __float2int_rn(a[6]);
+  return fma(i2d(v), 1.4551915228366852e-11, i2d(u)) * exp2d(k - 36);  // 2^-36
 }
 
 // the value of the level sums (weights 512^-(d+2)) as a float pair times sc
@@ -163,54 +210,52 @@ __global__ void __launch_bounds__(4 * TT) dk_tc_table(DevDiatomic D, DevDiaTC T,
   const int* ce = T.cexp + le * nv;
   double rs = 0.0;
   if (t < n2)
-    for (int v = c; v < nv; v += 4) rs += fabs(ldexp(fac * tx[t + (size_t)v * n2], -ce[v]));
+    for (int v = c; v < nv; v += 4) rs += fabs(fac * tx[t + (size_t)v * n2] * exp2d(-ce[v]));
   part[c][r] = rs;
   __syncthreads();
   rs = part[0][r] + part[1][r] + part[2][r] + part[3][r];
   int ex = 0;
   if (rs > 0.0) frexp(rs, &ex);  // rs < 2^ex
-  if (c == 0) rowexp[(le * T.ntt + tt) * TT + r] = ex;
+  ex = max(ex, -900);  // (a zero's significand is shifted out)
+  if (c == 0) rowexp[(le * T.ntt + tt) * TT + r] = ex + 2;  // the digits are of values below 1/4
   unsigned char* base = out + (le * T.ntt + tt) * T.ksteps * TD * BPL;
   for (int v8 = c; v8 < 2 * T.ksteps; v8 += 4) {
-    float d[TD][8];
+    double x[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int v = 8 * v8 + j;
-      double x = (t < n2 && v < nv) ? ldexp(fac * tx[t + (size_t)v * n2], -ex - ce[v]) : 0.0;
-#pragma unroll
-      for (int k = 0; k < TD; ++k) {
-        x *= 512.0;
-        const double g = rint(x);
-        x -= g;
-        d[k][j] = (float)g;
-      }
+      x[j] = (t < n2 && v < nv) ? fac * tx[t + (size_t)v * n2] * exp2d(-ce[v]) : 0.0;
     }
+    uint32_t pk[TD][4];
+    digits512_fixed(x, ex, pk);
     unsigned char* p = base + (size_t)(v8 >> 1) * TD * BPL + tc::off_kmajor(r, 8 * (v8 & 1));
 #pragma unroll
     for (int k = 0; k < TD; ++k)
-      *reinterpret_cast<uint4*>(p + k * BPL) = make_uint4(pack_f16(d[k][0], d[k][1]), pack_f16(d[k][2], d[k][3]),
-                                                          pack_f16(d[k][4], d[k][5]), pack_f16(d[k][6], d[k][7]));
+      *reinterpret_cast<uint4*>(p + k * BPL) = make_uint4(pk[k][0], pk[k][1], pk[k][2], pk[k][3]);
   }
 }
 
 // ---- recoupled tiles of the units [u0, u0 + cap) as digits: items (element,
 // active (k, group of rows), range of multipoles), or with `itemwise` one
 // output block per item (the same operations per block) ----
-template <int NN>
+template <int NN, bool F64>
 __global__ void __launch_bounds__(NN == 15 ? 256 : 320, 2) dk_tc_x(DevDiatomic D, DevDiatomicScratch S, DevDiaTC T,
-                                                                   int symmetric, int itemwise, int u0, int nchunk) {
-  using AR = ArF;
+                                                                   const double* __restrict__ Pd, int symmetric,
+                                                                   int itemwise, int u0, int nchunk) {
+  using AR = std::conditional_t<F64, ArD, ArF>;
+  using V = typename AR::V;
+  constexpr int NX = F64 ? TD : XD;  // digits of a tile
   const int nn = NN > 0 ? NN : D.nn, n2 = nn * nn;
   extern __shared__ __align__(16) unsigned char smraw[];
   Chunk<AR, JC_DIAG>& C = *reinterpret_cast<Chunk<AR, JC_DIAG>*>(smraw);
-  float2* Xs = reinterpret_cast<float2*>(smraw + sizeof(Chunk<AR, JC_DIAG>));  // [2][16 ksteps]
+  V* Xs = reinterpret_cast<V*>(smraw + sizeof(Chunk<AR, JC_DIAG>));  // [2][16 ksteps]
   __shared__ int s_js[JC_DIAG], s_row[JC_DIAG], s_unit[JC_DIAG], s_nj, s_use;
   __shared__ unsigned s_eb[JC_DIAG];
   const Blocks B = blocks_of(D, S, symmetric);
   if (B.count == 0) return;
   const int e_lo = u0 / B.ntile, e_hi = min(D.nel - 1, (u0 + T.cap - 1) / B.ntile);
   if (e_lo > e_hi) return;
-  const Src<AR> Sr = src_of<AR>(D, S, nullptr);
+  const Src<AR> Sr = src_of<AR>(D, S, Pd);
   const int nitem = itemwise ? B.count : S.counts[3];
   const int* kgl = S.kg_list + (size_t)D.nang * D.ngrp;
   const long total = (long)(e_hi - e_lo + 1) * nitem * nchunk;
@@ -255,16 +300,16 @@ __global__ void __launch_bounds__(NN == 15 ? 256 : 320, 2) dk_tc_x(DevDiatomic D
     const int mj = D.mval[s_js[0]];
     const int gp = sgf(D, e, p), gq = sgf(D, e, q);
     const bool vpq = live && gp < D.nrad && gq < D.nrad;
-    const float2* pb = S.pd2 + (size_t)gq * D.nd + gp;
+    const V* pb = Sr.P + (size_t)gq * D.nd + gp;
     const int l0 = (int)((long)D.nlm * c / nchunk), l1 = (int)((long)D.nlm * (c + 1) / nchunk);
     int par = 0;
     for (int ilm = l0; ilm < l1; ++ilm) {
       const int L = D.lmL[ilm], Ma = D.lmM[ilm];
-      ffv x[JC_DIAG][4];
+      typename AR::A x[JC_DIAG][4];
 #pragma unroll
       for (int jj = 0; jj < JC_DIAG; ++jj)
 #pragma unroll
-        for (int ab = 0; ab < 4; ++ab) x[jj][ab] = {0.f, 0.f};
+        for (int ab = 0; ab < 4; ++ab) x[jj][ab] = AR::zero();
       bool any = false;
       for (int sgn = 0; sgn < (Ma ? 2 : 1); ++sgn) {
         const int M = sgn ? -Ma : Ma, mi = mj - M;
@@ -281,25 +326,25 @@ __global__ void __launch_bounds__(NN == 15 ? 256 : 320, 2) dk_tc_x(DevDiatomic D
           first = false;
           if (nl == 0) continue;
           any = true;
-          ffv v0[IC], v2[IC];
+          typename AR::A v0[IC], v2[IC];
           recouple_k<AR, JC_DIAG>(D, C, pb, vpq, is + i0, ni, nl, par, v0, v2);
-          float2 a0[IC], a2[IC];
+          V a0[IC], a2[IC];
 #pragma unroll
           for (int ii = 0; ii < IC; ++ii) {
-            a0[ii] = ff2(v0[ii]);
-            a2[ii] = ff2(v2[ii]);
+            a0[ii] = AR::val(v0[ii]);
+            a2[ii] = AR::val(v2[ii]);
           }
 #pragma unroll
           for (int jj = 0; jj < JC_DIAG; ++jj) {
             if (jj >= nj) break;  // uniform
 #pragma unroll
             for (int ii = 0; ii < IC; ++ii) {
-              const float2 c0 = C.j0[par][jj][ii], c2 = C.j2[par][jj][ii];
-              if (c0.x != 0.f || c2.x != 0.f) {  // uniform
-                x[jj][0] = ff_fma(x[jj][0], c0, a0[ii]);
-                x[jj][1] = ff_fma(x[jj][1], c0, a2[ii]);
-                x[jj][2] = ff_fma(x[jj][2], c2, a0[ii]);
-                x[jj][3] = ff_fma(x[jj][3], c2, a2[ii]);
+              const V c0 = C.j0[par][jj][ii], c2 = C.j2[par][jj][ii];
+              if (AR::nz(c0) || AR::nz(c2)) {  // uniform
+                x[jj][0] = AR::fma(x[jj][0], c0, a0[ii]);
+                x[jj][1] = AR::fma(x[jj][1], c0, a2[ii]);
+                x[jj][2] = AR::fma(x[jj][2], c2, a0[ii]);
+                x[jj][3] = AR::fma(x[jj][3], c2, a2[ii]);
               }
             }
           }
@@ -309,10 +354,12 @@ __global__ void __launch_bounds__(NN == 15 ? 256 : 320, 2) dk_tc_x(DevDiatomic D
       if (!any) continue;  // uniform over the CTA
       if (t < JC_DIAG) s_eb[t] = 0;
       // the column scaling of the table, inverted
-      float cs[4];
+      std::conditional_t<F64, double, float> cs[4];
 #pragma unroll
-      for (int ab = 0; ab < 4; ++ab)
-        cs[ab] = live ? exp2i(T.cexp[((size_t)ilm * D.nel + e) * nv + ab * n2 + t]) : 0.f;
+      for (int ab = 0; ab < 4; ++ab) {
+        const int ce = live ? T.cexp[((size_t)ilm * D.nel + e) * nv + ab * n2 + t] : 0;
+        if constexpr (F64) cs[ab] = live ? exp2d(ce) : 0.0; else cs[ab] = live ? exp2i(ce) : 0.f;
+      }
       __syncthreads();
 #pragma unroll
       for (int jj = 0; jj < JC_DIAG; ++jj) {
@@ -320,8 +367,13 @@ __global__ void __launch_bounds__(NN == 15 ? 256 : 320, 2) dk_tc_x(DevDiatomic D
         unsigned eb = 0;
 #pragma unroll
         for (int ab = 0; ab < 4; ++ab) {
-          x[jj][ab] = ff_norm(x[jj][ab].hi * cs[ab], x[jj][ab].lo * cs[ab]);
-          if (live) eb = max(eb, (__float_as_uint(x[jj][ab].hi) >> 23) & 0xFFu);
+          if constexpr (F64) {
+            x[jj][ab] *= cs[ab];
+            if (live) eb = max(eb, ((unsigned)__double2hiint(x[jj][ab]) >> 20) & 0x7FFu);
+          } else {
+            x[jj][ab] = ff_norm(x[jj][ab].hi * cs[ab], x[jj][ab].lo * cs[ab]);
+            if (live) eb = max(eb, (__float_as_uint(x[jj][ab].hi) >> 23) & 0xFFu);
+          }
         }
         eb = __reduce_max_sync(0xffffffffu, eb);
         if (lane == 0) atomicMax(&s_eb[jj], eb);
@@ -336,35 +388,44 @@ __global__ void __launch_bounds__(NN == 15 ? 256 : 320, 2) dk_tc_x(DevDiatomic D
           for (int w2 = 0; w2 < 2; ++w2)
 #pragma unroll
             for (int ab = 0; ab < 4; ++ab) {
-              const ffv y = x[j2 + w2][ab];
-              const float sg = (ab == 1 || ab == 2) ? -1.f : 1.f;
-              Xs[w2 * 16 * T.ksteps + ab * n2 + t] = make_float2(sg * y.hi, sg * y.lo);
+              V y;
+              if constexpr (F64) y = x[j2 + w2][ab]; else y = make_float2(x[j2 + w2][ab].hi, x[j2 + w2][ab].lo);
+              Xs[w2 * 16 * T.ksteps + ab * n2 + t] = (ab == 1 || ab == 2) ? AR::neg(y) : y;
             }
         if (t < 2 * (16 * T.ksteps - nv)) {  // columns beyond 4 nn^2
           const int pad = 16 * T.ksteps - nv;
-          Xs[(t / pad) * 16 * T.ksteps + nv + t % pad] = make_float2(0.f, 0.f);
+          Xs[(t / pad) * 16 * T.ksteps + nv + t % pad] = V{};
         }
         __syncthreads();
         for (int ch = t; ch < 2 * nv8; ch += blockDim.x) {
           const int w2 = ch / nv8, v8 = ch % nv8, jj = j2 + w2;
           if (jj >= nj || s_unit[jj] < 0) continue;
-          const int E = max((int)max(s_eb[jj], 1u) - 126, -100);
-          const float s27 = exp2i(27 - E);
-          float d[XD][8];
+          uint32_t pk[NX][4];
+          int E;
+          if constexpr (F64) {
+            E = (int)max(s_eb[jj], 64u) - 1022;  // (64: a zero's significand is shifted out)
+            double xv[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float dj[XD];
-            digits512(Xs[w2 * 16 * T.ksteps + 8 * v8 + j], s27, dj);
+            for (int j = 0; j < 8; ++j) xv[j] = Xs[w2 * 16 * T.ksteps + 8 * v8 + j];
+            digits512_fixed(xv, E, pk);
+            E = s_eb[jj] == 0x7FFu ? kBadExp : E + 2;
+          } else {
+            E = max((int)max(s_eb[jj], 1u) - 126, -100);
+            const float s27 = exp2i(27 - E);
 #pragma unroll
-            for (int kk = 0; kk < XD; ++kk) d[kk][j] = dj[kk];
+            for (int j = 0; j < 8; j += 2) {
+              float d0[XD], d1[XD];
+              digits512(Xs[w2 * 16 * T.ksteps + 8 * v8 + j], s27, d0);
+              digits512(Xs[w2 * 16 * T.ksteps + 8 * v8 + j + 1], s27, d1);
+#pragma unroll
+              for (int kk = 0; kk < XD; ++kk) pk[kk][j / 2] = pack_f16(d0[kk], d1[kk]);
+            }
           }
-          unsigned char* o = T.x + (((size_t)s_unit[jj] * D.nlm + ilm) * T.ksteps + (v8 >> 1)) * XD * APL +
+          unsigned char* o = T.x + (((size_t)s_unit[jj] * D.nlm + ilm) * T.ksteps + (v8 >> 1)) * NX * APL +
                              tc::off_kmajor(s_row[jj], 8 * (v8 & 1));
 #pragma unroll
-          for (int kk = 0; kk < XD; ++kk)
-            *reinterpret_cast<uint4*>(o + kk * APL) =
-                make_uint4(pack_f16(d[kk][0], d[kk][1]), pack_f16(d[kk][2], d[kk][3]), pack_f16(d[kk][4], d[kk][5]),
-                           pack_f16(d[kk][6], d[kk][7]));
+          for (int kk = 0; kk < NX; ++kk)
+            *reinterpret_cast<uint4*>(o + kk * APL) = make_uint4(pk[kk][0], pk[kk][1], pk[kk][2], pk[kk][3]);
           if (v8 == 0) T.xexp[((size_t)s_unit[jj] * D.nlm + ilm) * 128 + s_row[jj]] = E;
         }
       }
@@ -374,16 +435,19 @@ __global__ void __launch_bounds__(NN == 15 ? 256 : 320, 2) dk_tc_x(DevDiatomic D
 
 // ---- the products: CTA = (unit, tile of TT entries t, part of the
 // multipoles); warps 0-7 read back, warp 8 copies, warp 9 issues ----
+template <bool F64>
 __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicScratch S, DevDiaTC T, int symmetric,
                                                      int u0) {
+  constexpr int NX = F64 ? TD : XD;
+  using Sum = std::conditional_t<F64, double, ffv>;
   const Blocks B = blocks_of(D, S, symmetric);
   const int tt = blockIdx.x % T.ntt, lp = (blockIdx.x / T.ntt) % T.lparts, lu = blockIdx.x / (T.ntt * T.lparts);
   const int u = u0 + lu;
   if (u >= D.nel * B.ntile) return;  // uniform over the CTA
   const int e = u / B.ntile;
   extern __shared__ __align__(1024) unsigned char smg[];
-  unsigned char* Abuf = smg;                                        // NSTAGE x XD planes of 128 x 16
-  unsigned char* Bbuf = Abuf + NSTAGE * XD * APL;                     // NSTAGE x TD planes of TT x 16
+  unsigned char* Abuf = smg;                                        // NSTAGE x NX planes of 128 x 16
+  unsigned char* Bbuf = Abuf + NSTAGE * NX * APL;                     // NSTAGE x TD planes of TT x 16
   uint64_t* full = reinterpret_cast<uint64_t*>(Bbuf + NSTAGE * TD * BPL);
   uint64_t* empty = full + NSTAGE;
   uint64_t* done = empty + NSTAGE;
@@ -426,16 +490,16 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
   tc::fence_after_sync();
   const uint32_t tD = *tslot;
   const int na = nact[0];
-  ffv acc[32];
+  Sum acc[32];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) acc[j] = {0.f, 0.f};
+  for (int j = 0; j < 32; ++j) acc[j] = {};
 
   if (warp == 8) {
     if (lane == 0) {
       bool ok = true;
       int it = 0;
       for (int a = 0; a < na && ok; ++a) {
-        const unsigned char* xs = T.x + ((size_t)lu * D.nlm + act[a]) * T.ksteps * XD * APL;
+        const unsigned char* xs = T.x + ((size_t)lu * D.nlm + act[a]) * T.ksteps * NX * APL;
         const unsigned char* ts = T.tx + (((size_t)act[a] * D.nel + e) * T.ntt + tt) * T.ksteps * TD * BPL;
         for (int ks = 0; ks < T.ksteps; ++ks, ++it) {
           const int s = it % NSTAGE;
@@ -443,8 +507,8 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
             ok = false;
             break;
           }
-          tc::mbar_expect_tx(&full[s], XD * APL + TD * BPL);
-          tc::bulk_g2s(Abuf + s * XD * APL, xs + (size_t)ks * XD * APL, XD * APL, &full[s]);
+          tc::mbar_expect_tx(&full[s], NX * APL + TD * BPL);
+          tc::bulk_g2s(Abuf + s * NX * APL, xs + (size_t)ks * NX * APL, NX * APL, &full[s]);
           tc::bulk_g2s(Bbuf + s * TD * BPL, ts + (size_t)ks * TD * BPL, TD * BPL, &full[s]);
         }
       }
@@ -467,12 +531,12 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
           const int s = it % NSTAGE;
           if (!tc::mbar_wait(&full[s], (uint32_t)((it / NSTAGE) & 1), kWait)) { ok = false; break; }
           tc::fence_after_sync();
-          const uint64_t da = tc::smem_desc(tc::smem_u32(Abuf + s * XD * APL));
+          const uint64_t da = tc::smem_desc(tc::smem_u32(Abuf + s * NX * APL));
           const uint64_t db = tc::smem_desc(tc::smem_u32(Bbuf + s * TD * BPL));
           // digit kx of the tiles against the table digits 0..6-kx, which are
           // consecutive: levels kx.. at columns TT kx.. (at most 256 per MMA)
 #pragma unroll 1
-          for (int kx = 0; kx < XD; ++kx) {
+          for (int kx = 0; kx < NX; ++kx) {
             const int n = TT * (TD - kx);
             const uint64_t ad = da + (uint64_t)(kx * APL >> 4);
             const uint32_t on = (ks > 0 || kx > 0) ? 1u : 0u;
@@ -511,7 +575,11 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
             float lv[TD];
 #pragma unroll
             for (int d = 0; d < TD; ++d) lv[d] = v[d][j];
-            acc[8 * g + j] = ff_add(acc[8 * g + j], levels512(lv, exp2i(te[8 * g + j] + E)));
+            if constexpr (F64)
+              acc[8 * g + j] += E == kBadExp ? __longlong_as_double(0x7ff8000000000000ll)
+                                             : levels512_f64(lv, te[8 * g + j] + E);
+            else
+              acc[8 * g + j] = ff_add(acc[8 * g + j], levels512(lv, exp2i(te[8 * g + j] + E)));
           }
         }
       }
@@ -526,9 +594,11 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
     const bool bad = fail[0] != 0;
     double* o = T.part + ((((size_t)lp * T.cap + lu) * T.ntt + tt) * TT + 32 * half) * 128 + row;
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      o[(size_t)j * 128] =
-          bad ? __longlong_as_double(0x7ff8000000000000ll) : (double)acc[j].hi + (double)acc[j].lo;
+    for (int j = 0; j < 32; ++j) {
+      double y;
+      if constexpr (F64) y = acc[j]; else y = (double)acc[j].hi + (double)acc[j].lo;
+      o[(size_t)j * 128] = bad ? __longlong_as_double(0x7ff8000000000000ll) : y;
+    }
   }
   if (t == 0 && fail[0]) atomicExch(T.err, 1);
   tc::fence_before_sync();
@@ -563,24 +633,27 @@ cudaError_t launch_dk_tc_table(const DevDiatomic& D, const DevDiaTC& T, unsigned
   return cudaGetLastError();
 }
 
-size_t dtc_gemm_smem(const DevDiatomic& D) {
-  return (size_t)NSTAGE * (XD * APL + TD * BPL) + 8 * (2 * NSTAGE + 2) + 4 * (4 + (size_t)D.nlm);
+size_t dtc_gemm_smem(const DevDiatomic& D, bool f64) {
+  return (size_t)NSTAGE * ((f64 ? TD : XD) * APL + TD * BPL) + 8 * (2 * NSTAGE + 2) + 4 * (4 + (size_t)D.nlm);
 }
 
-cudaError_t launch_dk_tc_diag(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDiaTC& T, double* Kd,
-                              bool symmetric, bool itemwise, cudaStream_t st) {
+// Pd: the FP64 form (from the density itself), nullptr: the split form (S.pd2)
+cudaError_t launch_dk_tc_diag(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDiaTC& T, const double* Pd,
+                              double* Kd, bool symmetric, bool itemwise, cudaStream_t st) {
   const int n2 = D.nn * D.nn, th = ((n2 + 31) / 32) * 32;
   int dev = 0, nsm = 152, per = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  auto xk = D.nn == 15 ? dk_tc_x<15> : dk_tc_x<0>;
+  auto xk = Pd ? (D.nn == 15 ? dk_tc_x<15, true> : dk_tc_x<0, true>)
+               : (D.nn == 15 ? dk_tc_x<15, false> : dk_tc_x<0, false>);
+  auto gk = Pd ? dk_tc_gemm<true> : dk_tc_gemm<false>;
   const size_t xsm = sizeof(Chunk<ArF, JC_DIAG>) + sizeof(float2) * 2 * 16 * (size_t)T.ksteps;
   cudaError_t e = smem_limit(xk, xsm);
   if (e != cudaSuccess) return e;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, xk, th, xsm);
   if (e != cudaSuccess) return e;
-  const size_t gsm = dtc_gemm_smem(D);
-  if ((e = smem_limit(dk_tc_gemm, gsm)) != cudaSuccess) return e;
+  const size_t gsm = dtc_gemm_smem(D, Pd != nullptr);
+  if ((e = smem_limit(gk, gsm)) != cudaSuccess) return e;
   const int slots = nsm * std::max(per, 1);
   const long nblk = symmetric ? (long)D.nang * (D.nang + 1) / 2 : (long)D.nang * D.nang;
   const int units = (int)(D.nel * ((nblk + 127) / 128));
@@ -591,9 +664,9 @@ cudaError_t launch_dk_tc_diag(const DevDiatomic& D, const DevDiatomicScratch& S,
   for (int u0 = 0; u0 < units; u0 += T.cap) {
     e = cudaMemsetAsync(T.xexp, 0x80, sizeof(int) * (size_t)T.cap * D.nlm * 128, st);
     if (e != cudaSuccess) return e;
-    xk<<<slots, th, xsm, st>>>(D, S, T, symmetric ? 1 : 0, itemwise ? 1 : 0, u0, nchunk);
+    xk<<<slots, th, xsm, st>>>(D, S, T, Pd, symmetric ? 1 : 0, itemwise ? 1 : 0, u0, nchunk);
     const int nu = std::min(T.cap, units - u0);
-    dk_tc_gemm<<<nu * T.ntt * T.lparts, 320, gsm, st>>>(D, S, T, symmetric ? 1 : 0, u0);
+    gk<<<nu * T.ntt * T.lparts, 320, gsm, st>>>(D, S, T, symmetric ? 1 : 0, u0);
     dk_tc_store<<<dim3(nu, 32), 256, 0, st>>>(D, S, T, symmetric ? 1 : 0, u0, Kd);
   }
   return cudaGetLastError();

@@ -1,0 +1,32 @@
+// FP64 values as fixed-point integers and back, for the digit planes of the
+// tensor-core kernels.
+#pragma once
+
+#include <cstdint>
+
+namespace hfg {
+namespace {
+
+// x 2^(bits - E) towards zero, two's complement, |x| < 2^E: by shifts of the
+// significand (no FP64-pipe instructions); exponents far below E give 0
+template <int BITS>
+__device__ __forceinline__ uint64_t fixed_point(double x, int E) {
+  const int h = __double2hiint(x);
+  const int sh = min(max(E + 1083 - BITS - ((h >> 20) & 0x7FF), 0), 63);  // from a 61-bit significand
+  const uint64_t m =
+      ((((uint64_t)(uint32_t)((h & 0xFFFFF) | 0x100000)) << 32 | (uint32_t)__double2loint(x)) << 8) >> sh;
+  const uint64_t sg = (uint64_t)(int64_t)(h >> 31);
+  return (m ^ sg) - sg;
+}
+
+__device__ __forceinline__ double exp2d(int k) {  // 2^k, k clamped to the normal range
+  return __hiloint2double((min(max(k, -1022), 1023) + 1023) << 20, 0);
+}
+// an integer below 2^51 in FP64
+__device__ __forceinline__ double i2d(int64_t i) {
+  return __longlong_as_double(0x4338000000000000ll + i) - 6755399441055744.0;
+}
+constexpr int kBadExp = 1 << 20;  // exponent of a tile with a value that is not finite
+
+}  // namespace
+}  // namespace hfg

@@ -79,6 +79,7 @@
 #include "devatom.cuh"
 #include "smem_limit.hpp"
 #include "ff.cuh"
+#include "fixed.cuh"
 #include "tc.cuh"
 
 namespace hfg {
@@ -320,18 +321,6 @@ __device__ __forceinline__ void digits_pairs(const ffv (&x)[8], float s, uint32_
 
 // ---- FP64 density tiles ----
 
-// x 2^(bits - E) towards zero, two's complement, |x| < 2^E: by shifts of the
-// significand (no FP64-pipe instructions); exponents far below E give 0
-template <int BITS>
-__device__ __forceinline__ uint64_t fixed_point(double x, int E) {
-  const int h = __double2hiint(x);
-  const int sh = min(max(E + 1083 - BITS - ((h >> 20) & 0x7FF), 0), 63);  // from a 61-bit significand
-  const uint64_t m =
-      ((((uint64_t)(uint32_t)((h & 0xFFFFF) | 0x100000)) << 32 | (uint32_t)__double2loint(x)) << 8) >> sh;
-  const uint64_t sg = (uint64_t)(int64_t)(h >> 31);
-  return (m ^ sg) - sg;
-}
-
 // the 6 balanced base-1024 digits of 8 values against |X| < 2^(E + 2), packed
 // as in digits_pairs: with 512 added to every digit the digits are the 10-bit
 // fields of the fixed-point number, and 1024 + field an f16 bit pattern
@@ -386,13 +375,6 @@ __device__ __forceinline__ void digits_fixed256(const double (&x)[8], int E, uin
   }
 }
 
-__device__ __forceinline__ double exp2d(int k) {  // 2^k, k clamped to the normal range
-  return __hiloint2double((min(max(k, -1022), 1023) + 1023) << 20, 0);
-}
-// an integer below 2^51 in FP64
-__device__ __forceinline__ double i2d(int64_t i) {
-  return __longlong_as_double(0x4338000000000000ll + i) - 6755399441055744.0;
-}
 // level sums (integers) -> FP64 times 2^k: base 1024, weights 1024^-(d+2), and
 // base 256, weights 256^-(d+2)
 __device__ __forceinline__ double levels_to_f64(const float (&a)[PD], int k) {
@@ -406,8 +388,6 @@ __device__ __forceinline__ double levels_to_f64(const float (&a)[ND], int k) {
                     ((int64_t)__float2int_rn(a[5]) << 8) + __float2int_rn(a[6]);
   return fma(i2d(v), 2.3283064365386963e-10, i2d(u)) * exp2d(k - 32);
 }
-constexpr int kBadExp = 1 << 20;  // exponent of a tile with a value that is not finite
-
 // the 8 values y[j] of tile (a,b), block jk (-1: none), at row p and columns
 // q0 + j: one pass over the columns with the block's base address computed
 // once; owned entries go to K, the shared last row / column to the halo buffer

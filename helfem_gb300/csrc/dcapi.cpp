@@ -378,6 +378,12 @@ struct hfg_diatomic {
   }
 
   // scratch of the FP64 in-element tiles, on the first FP64 exchange
+  // The FP64 in-element tiles on the tensor cores. Their K steps and tiles are
+  // padded, which short elements do not pay back: K of l = 0..3 on three
+  // elements of 6 nodes 110 us on the FP64 kernels and 115 us here, of 8 nodes
+  // 131 and 121, of 15 nodes 302 and 185; l <= 5, m <= 1 on six elements of 8
+  // nodes 1711 and 1353, of 15 nodes 10.9 and 6.3 ms.
+  bool use_tc64() const { return host.nn >= 8; }
   void ensure_fp64() {
     if (t64.x) return;
     hfg_abi::AllocStream alloc_on(own_stream);
@@ -415,7 +421,8 @@ struct hfg_diatomic {
 
   // split tables and the split density buffer, on the first split-precision call
   void ensure_split() {
-    if (tc.err) return;
+    if (scr.pd2) return;
+    ensure_tc(true);
     hfg_abi::AllocStream alloc_on(own_stream);
     auto split = [](const std::vector<double>& v) {
       std::vector<float2> o(v.size());
@@ -452,23 +459,39 @@ struct hfg_diatomic {
     dev.al_c2s = d_alc2s.upload(split(H.al_c2));
     dev.lmfacs = d_lmfacs.upload(split(lmfac_host));
     s_pd2.alloc(sizeof(float2) * (size_t)H.ndummy * H.ndummy);
+    ck(cudaStreamSynchronize(own_stream), "sync after split tables");
     scr.pd2 = s_pd2.as<float2>();
-    // in-element tiles: the kernel's digit planes, and scratch for the digits
-    // of as many (element, 128 output blocks) units as 4 GB hold (at least one)
+  }
+
+  // in-element tiles on the tensor cores: the kernel's digit planes, and scratch
+  // for the digits of as many (element, 128 output blocks) units as 4 GB hold
+  // of float pairs (at least one; seven sixths of it for FP64), on the first exchange that uses them. false (unless the
+  // caller must have them): the device has no room, the FP64 kernels stay.
+  bool ensure_tc(bool must) {
+    if (tc.err) return true;
+    hfg_abi::AllocStream alloc_on(own_stream);
+    const hfg::DiatomicHost& H = host;
+    const size_t n2 = (size_t)H.nn * H.nn, ntile = (size_t)H.nlm * H.nel;
     hfg::DevDiaTC T;
     T.ksteps = (int)((4 * n2 + 15) / 16);
     T.ntt = (int)((n2 + DTC_TT - 1) / DTC_TT);
     const size_t plane = 32;  // bytes of one row of a K step's plane
-    t_tx.alloc(ntile * T.ntt * T.ksteps * DTC_TDIGITS * DTC_TT * plane);
+    const size_t tx_bytes = ntile * T.ntt * T.ksteps * DTC_TDIGITS * DTC_TT * plane;
+    if (!must) {
+      size_t avail = 0, total = 0;
+      ck(cudaMemGetInfo(&avail, &total), "memory");
+      if (avail < tx_bytes + ((size_t)8 << 30)) return false;
+    }
+    t_tx.alloc(tx_bytes);
     t_cexp.alloc(sizeof(int) * ntile * 4 * n2);
     T.cexp = t_cexp.as<int>();
     t_txexp.alloc(sizeof(int) * ntile * T.ntt * DTC_TT);
     ck(hfg::launch_dk_tc_table(dev, T, t_tx.as<unsigned char>(), t_txexp.as<int>(), t_cexp.as<int>(), own_stream), "kernel digits");
     T.tx = t_tx.as<unsigned char>();
     T.txexp = t_txexp.as<int>();
-    const size_t unit = (size_t)H.nlm * T.ksteps * DTC_XDIGITS * 128 * plane, nang = H.nang;
+    const size_t digit = (size_t)H.nlm * T.ksteps * 128 * plane, unit = DTC_TDIGITS * digit, nang = H.nang;
     const size_t units = (size_t)H.nel * ((nang * nang + 127) / 128);
-    T.cap = (int)std::max<size_t>(1, std::min(units, ((size_t)4 << 30) / unit));
+    T.cap = (int)std::max<size_t>(1, std::min(units, ((size_t)4 << 30) / (DTC_XDIGITS * digit)));
     // parts of the multipole sum where a density that does not mix m makes
     // fewer units x tiles than there are SMs (one CTA per SM)
     const size_t ctas = (size_t)H.nel * ((same_m_pairs() + 127) / 128) * T.ntt;
@@ -481,9 +504,10 @@ struct hfg_diatomic {
     T.x = t_x.as<unsigned char>();
     T.xexp = t_xexp.as<int>();
     T.part = t_part.as<double>();
-    ck(cudaStreamSynchronize(own_stream), "sync after split tables");
+    ck(cudaStreamSynchronize(own_stream), "sync after the kernel's digits");
     T.err = t_err.as<int>();
     tc = T;
+    return true;
   }
 
   // J or K of a pure-basis density (device pointers) on stream st
@@ -492,7 +516,8 @@ struct hfg_diatomic {
     check_device();
     const hfg::DiatomicHost& H = host;
     if (split) ensure_split();
-    else if (exchange) ensure_fp64();
+    const bool tc64 = !split && exchange && use_tc64() && ensure_tc(false);
+    if (!split && exchange && !tc64) ensure_fp64();
     if (!exchange) {  // J reads the pure density and writes the pure J directly
       ck(hfg::launch_diatomic_coulomb(dev, scr, P, F, st), "coulomb");
       mark_use(st);
@@ -504,7 +529,7 @@ struct hfg_diatomic {
                                              itemwise),
          "exchange (split)");
     else
-      ck(hfg::launch_diatomic_exchange(dev, scr, t64, s_Pd.as<double>(), s_Fd.as<double>(), symmetric, st), "exchange");
+      ck(hfg::launch_diatomic_exchange(dev, scr, t64, tc64 ? &tc : nullptr, s_Pd.as<double>(), s_Fd.as<double>(), symmetric, st), "exchange");
     ck(hfg::launch_diatomic_gather(s_Fd.as<double>(), H.ndummy, d_pure.as<int>(), H.nbf, F, st), "gather");
     mark_use(st);
   }
@@ -566,7 +591,7 @@ struct hfg_diatomic {
     build(h_in.as<double>(), h_out.as<double>(), exchange, symmetric, own_stream, split);
     ck(cudaMemcpyAsync(F, h_out.p, bytes, cudaMemcpyDeviceToHost, own_stream), "copy out");
     ck(cudaStreamSynchronize(own_stream), "sync");
-    if (exchange && split) tc_check();
+    if (exchange) tc_check();
   }
 };
 

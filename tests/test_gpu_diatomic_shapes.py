@@ -47,3 +47,32 @@ def test_diatomic_exchange_shapes(case):
                 torch.cuda.synchronize()
                 err = relerr(from_dev(K), ref)
                 assert err < tol, (blockdiag, symmetric, split, err)
+
+
+@pytest.mark.parametrize("nn", [7, 8, 15])
+def test_diatomic_fp64_scales(nn):
+    """FP64 form on either side of the line between its in-element kernels, at
+    a scale far outside the float range (1e-12 of max|K|: 53-bit sums), and a
+    NaN of one element's density that leaves the other elements' tiles alone."""
+    torch = torch_cuda()
+    nelem, lm = 3, [4, 2]
+    d = hg.Diatomic.from_grid(3, 1, 3.0, nelem, lm, Rmax=12.0, nnodes=nn)
+    D = dia.build_diatomic(3, 1, 3.0, nn, nelem, lm, Rmax=12.0)
+    P = bound_density(D, 1, seed=nn, blockdiag=False)
+    ref = DiatomicOracle(D).exchange(P)
+    for scale in (1.0, 2.0**600):
+        Pd = to_dev(torch, P * scale)
+        for symmetric in (False, True):
+            K = torch.full_like(Pd, np.nan)
+            d.exchange(Pd, K, symmetric=symmetric)
+            torch.cuda.synchronize()
+            assert relerr(from_dev(K) / scale, ref) < 1e-12, (scale, symmetric)
+    Pd = to_dev(torch, P)
+    Pd[0, 0] = np.nan  # first element, first shell
+    K = torch.empty_like(Pd)
+    d.exchange(Pd, K)
+    k = from_dev(K)
+    hit = np.isnan(k)
+    n = nelem * (nn - 1)  # functions of an m = 0 shell
+    assert hit.any() and not hit[:n, :n][2 * (nn - 1):, 2 * (nn - 1):].any()
+    assert np.allclose(k[~hit], ref[~hit], rtol=0, atol=1e-10 * np.abs(ref).max())
