@@ -14,8 +14,8 @@
 // digit pairs with k + l = d) in FP32 tensor memory. The 4 nn^2-term sums of
 // digit products stay far below 2^24: the leading digits of a row obey its
 // unit row sum, and the others are spread over +-256, so that a level's sum of
-// 900 products has a spread below 2^21. The levels are carried into a float
-// pair, scaled and summed over the multipoles, one FP64 value per entry.
+// 900 products has a spread below 2^21. The levels are carried into three
+// floats and summed in FP64 over the multipoles.
 //
 // FP64 form (F64): the tiles are recoupled in FP64 and cut into seven digits by
 // shifts of their significands (59 bits below the largest entry), the level
@@ -119,8 +119,11 @@ __device__ __forceinline__ double levels512_f64(const float (&a)[TD], int k) {
   return fma(i2d(v), 1.4551915228366852e-11, i2d(u)) * exp2d(k - 36);  // 2^-36
 }
 
-// the value of the level sums (weights 512^-(d+2)) as a float pair times sc
-__device__ __forceinline__ ffv levels512(float (&a)[TD], float sc) {
+// the value of the level sums (weights 512^-(d+2)) as three floats. The first
+// two are exact where the value is far below the bound that scales it: with one
+// float for the tail its rounding, 2^-51 of the bound, was the form's error
+// (3.0e-14 of |K| for H2, 1.0e-14 now).
+__device__ __forceinline__ void levels512(float (&a)[TD], float& head, float& mid, float& tail) {
 #pragma unroll
   for (int d = TD - 1; d >= 1; --d) {
     const float c = rnd_mul(a[d], 1.0f / 512.0f);
@@ -132,11 +135,9 @@ __device__ __forceinline__ ffv levels512(float (&a)[TD], float sc) {
   const float m2 = __fmul_rn(a[1], 1.0f / 134217728.0f);
   const float sh = __fadd_rn(h, m2), bb = __fsub_rn(sh, h);
   const float e = __fadd_rn(__fsub_rn(h, __fsub_rn(sh, bb)), __fsub_rn(m2, bb));
-  float tail = 0.f;
-#pragma unroll
-  for (int k = TD - 1; k >= 2; --k) tail = __fmaf_rn(tail, 1.0f / 512.0f, a[k]);
-  tail = __fmul_rn(tail, 1.0f / 68719476736.0f);  // weight 2^-36 of a[2]
-  return {__fmul_rn(sh, sc), __fmul_rn(__fadd_rn(e, tail), sc)};
+  head = sh;
+  mid = __fmaf_rn(__fmaf_rn(a[3], 1.0f / 512.0f, a[2]), 1.0f / 68719476736.0f, e);  // weight 2^-36 of a[2]
+  tail = __fmul_rn(__fmaf_rn(__fmaf_rn(a[6], 1.0f / 512.0f, a[5]), 1.0f / 512.0f, a[4]), 5.551115123125783e-17f);
 }
 
 // all seven levels (TT columns apart) of 8 consecutive columns, one wait
@@ -439,7 +440,6 @@ template <bool F64>
 __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicScratch S, DevDiaTC T, int symmetric,
                                                      int u0) {
   constexpr int NX = F64 ? TD : XD;
-  using Sum = std::conditional_t<F64, double, ffv>;
   const Blocks B = blocks_of(D, S, symmetric);
   const int tt = blockIdx.x % T.ntt, lp = (blockIdx.x / T.ntt) % T.lparts, lu = blockIdx.x / (T.ntt * T.lparts);
   const int u = u0 + lu;
@@ -490,9 +490,9 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
   tc::fence_after_sync();
   const uint32_t tD = *tslot;
   const int na = nact[0];
-  Sum acc[32];
+  double acc[32];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) acc[j] = {};
+  for (int j = 0; j < 32; ++j) acc[j] = 0.0;
 
   if (warp == 8) {
     if (lane == 0) {
@@ -575,11 +575,17 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
             float lv[TD];
 #pragma unroll
             for (int d = 0; d < TD; ++d) lv[d] = v[d][j];
-            if constexpr (F64)
+            if constexpr (F64) {
               acc[8 * g + j] += E == kBadExp ? __longlong_as_double(0x7ff8000000000000ll)
                                              : levels512_f64(lv, te[8 * g + j] + E);
-            else
-              acc[8 * g + j] = ff_add(acc[8 * g + j], levels512(lv, exp2i(te[8 * g + j] + E)));
+            } else {
+              float z0, z1, z2;
+              levels512(lv, z0, z1, z2);
+              const int c = (max(te[8 * g + j] + E, -800) + 896) << 20;
+              acc[8 * g + j] += f2d_scaled(z0, c);
+              acc[8 * g + j] += f2d_scaled(z1, c);
+              acc[8 * g + j] += f2d_scaled(z2, c);
+            }
           }
         }
       }
@@ -594,11 +600,8 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
     const bool bad = fail[0] != 0;
     double* o = T.part + ((((size_t)lp * T.cap + lu) * T.ntt + tt) * TT + 32 * half) * 128 + row;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      double y;
-      if constexpr (F64) y = acc[j]; else y = (double)acc[j].hi + (double)acc[j].lo;
-      o[(size_t)j * 128] = bad ? __longlong_as_double(0x7ff8000000000000ll) : y;
-    }
+    for (int j = 0; j < 32; ++j)
+      o[(size_t)j * 128] = bad ? __longlong_as_double(0x7ff8000000000000ll) : acc[j];
   }
   if (t == 0 && fail[0]) atomicExch(T.err, 1);
   tc::fence_before_sync();

@@ -26,6 +26,15 @@ __device__ __forceinline__ double exp2d(int k) {  // 2^k, k clamped to the norma
 __device__ __forceinline__ double i2d(int64_t i) {
   return __longlong_as_double(0x4338000000000000ll + i) - 6755399441055744.0;
 }
+
+// float -> double times 2^k through the bit pattern (no FP64-pipe
+// instructions); c = (896 + k) << 20, zero and subnormal floats give zero
+__device__ __forceinline__ double f2d_scaled(float f, int c) {
+  const uint32_t bits = __float_as_uint(f), t = bits & 0x7FFFFFFFu;
+  const uint32_t hi = t < 0x00800000u ? 0u : ((t >> 3) + (uint32_t)c) | (bits & 0x80000000u);
+  return __hiloint2double((int)hi, t < 0x00800000u ? 0 : (int)(bits << 29));
+}
+
 constexpr int kBadExp = 1 << 20;  // exponent of a tile with a value that is not finite
 
 }  // namespace

@@ -263,14 +263,6 @@ __device__ __forceinline__ void carry_pairs(float (&a)[PD], float& y0, float& y1
   y1 = __fmaf_rn(y0, -1024.0f, a[0]);
 }
 
-// float -> double times 2^k through the bit pattern (no FP64-pipe
-// instructions); c = (896 + k) << 20, zero and subnormal floats give zero
-__device__ __forceinline__ double f2d_scaled(float f, int c) {
-  const uint32_t bits = __float_as_uint(f), t = bits & 0x7FFFFFFFu;
-  const uint32_t hi = t < 0x00800000u ? 0u : ((t >> 3) + (uint32_t)c) | (bits & 0x80000000u);
-  return __hiloint2double((int)hi, t < 0x00800000u ? 0 : (int)(bits << 29));
-}
-
 // the value of the level sums (integers below 2^24, weights 1024^-(d+2)) times
 // 2^k, c as above: the leading three with their rounding errors, the rest as
 // they come
