@@ -50,7 +50,7 @@
 // become FP64 numbers through exact integers. The contraction's own rounding is
 // then below that of the FP64 sums it replaces: the error against the exact K
 // is the tables' in both (4.120e-14 for Kr, l <= 3 dense 2.680e-14 and
-// 2.679e-14), at 1.04 instead of 4.52 ms for Kr. A tile with a value that is
+// 2.679e-14), at 1.00 instead of 4.52 ms for Kr. A tile with a value that is
 // not finite gives NaN throughout, as a product with FP64 NaNs does.
 //
 // Off-diagonal work unit = one element pair (a,b) and a range of groups of
@@ -849,12 +849,16 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
 // and row tile of 128 rows t of Tk, one batch per multipole L:
 //     D[t, 16 level + slot] = sum_{kt+kx=level} sum_v Tk_kt[t, v] X_kx[slot, v],
 // v = p + q nn. Tk's digit planes are streamed through shared memory one K
-// step (16 columns v) at a time by bulk asynchronous copies,
-// double-buffered; the density digits of all 16 slots are resident. For
-// table digit kt the density planes kx = 0..6-kt are consecutive and form
-// one operand of N = 16 (7 - kt). The level sums here run over up to nn^2
-// products: the leading levels stay exact, and a rounding in the deepest
-// ones is below 2^-60 of max|K|.
+// step (16 columns v) at a time by bulk asynchronous copies, four steps in
+// flight; the density digits of all 16 slots are resident, those of the next
+// multipole beside those in use. For table digit kt the density planes kx =
+// 0..6-kt are consecutive and form one operand of N = 16 (7 - kt). The level
+// sums here run over up to nn^2 products: the leading levels stay exact, and a
+// rounding in the deepest ones is below 2^-60 of max|K|.
+// A chain of short steps, so bound by latency: copies, products and the digit
+// work each have their own warps and run a multipole ahead of one another. Two
+// CTAs per SM with one thread that copied, issued and waited in turn took 148
+// us for Kr and 61 us for Ne (FP64 form, cold), this 115 and 29.
 
 namespace {
 constexpr int DSLOT = 16;  // output blocks per diagonal group
@@ -887,9 +891,16 @@ __global__ void tc_tk_digits_kernel(const double* __restrict__ tk, int NL, int n
   }
 }
 
+constexpr int DST = 4;                   // stages of the table stream
+constexpr int DW = 8;                    // working warps
+constexpr int DTHREADS = 32 * (DW + 2);  // a copying and an issuing one
+
+// warps 0-7: recouple and digitise the density vectors of one multipole while
+// the products of the one before run, then read those back; warp 8 streams the
+// tables' digits, warp 9 issues
 template <bool F64>
-__global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, DevTC T, int symmetric,
-                                                    const double* __restrict__ P, double* __restrict__ K) {
+__global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S, DevTC T, int symmetric,
+                                                         const double* __restrict__ P, double* __restrict__ K) {
   using Val = std::conditional_t<F64, double, float2>;
   using Sum = std::conditional_t<F64, double, ffv>;
   constexpr int NX = F64 ? ND : NDX;  // digits of the density vectors
@@ -905,16 +916,20 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
   const int g = blockIdx.x % T.dgroups, mt = (blockIdx.x / T.dgroups) % mtiles, a = blockIdx.x / (T.dgroups * mtiles);
   if (g >= ngr) return;  // uniform over the CTA
   extern __shared__ __align__(1024) unsigned char smraw[];
-  unsigned char* Abuf = smraw;                                             // 2 x ND planes of 128 x 16
-  unsigned char* Bx = Abuf + 2 * ND * APLANE;                              // ksteps x ND planes of 16 x 16
-  int* alpha = reinterpret_cast<int*>(Bx + (size_t)ksteps * ND * TPLANE);  // [128]
-  int* exs = alpha + 128;                                                  // [16] slot exponents (float bits)
-  int* sact = exs + DSLOT;                                                 // [NL][16]
-  int* gent = sact + NL * DSLOT;                                           // [16][NL]
-  int* gjk = gent + NL * DSLOT;                                            // [16]
-  int* fail = gjk + DSLOT;                                                 // [2]
-  uint64_t* mb = reinterpret_cast<uint64_t*>(fail + 2);                    // full[2], empty[2], done
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(mb + 5);
+  unsigned char* Abuf = smraw;                  // DST x ND planes of 128 x 16
+  unsigned char* Bx = Abuf + DST * ND * APLANE;  // 2 x ksteps x ND planes of 16 x 16
+  const size_t bsize = (size_t)ksteps * ND * TPLANE;
+  int* exs = reinterpret_cast<int*>(Bx + 2 * bsize);  // [4][16] slot exponents (bits) of four multipoles
+  int* sact = exs + 4 * DSLOT;                        // [NL][16]
+  int* gent = sact + NL * DSLOT;                      // [16][NL]
+  int* gjk = gent + NL * DSLOT;                       // [16]
+  int* fail = gjk + DSLOT;                            // [2]: flag, number of multipoles
+  int* actL = fail + 2;                               // [NL] the multipoles of the group's entries
+  uint64_t* full = reinterpret_cast<uint64_t*>(actL + NL + (NL & 1));
+  uint64_t* empty = full + DST;
+  uint64_t* bfull = empty + DST;  // [2] density digits there
+  uint64_t* done = bfull + 2;     // [2] products finished
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 2);
   unsigned char* act = reinterpret_cast<unsigned char*>(tslot + 2);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int qw = warp & 3, half = warp >> 2;
@@ -934,166 +949,198 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
   }
   for (int idx = t; idx < nang2; idx += blockDim.x) act[idx] = S.act[idx];
   // the zero seventh plane of float-pair densities in every K step (operands of N = 112)
-  for (int idx = t; NX < ND && idx < ksteps * (TPLANE / 16); idx += blockDim.x) {
+  for (int idx = t; NX < ND && idx < 2 * ksteps * (TPLANE / 16); idx += blockDim.x) {
     const int ks = idx / (TPLANE / 16), o = idx % (TPLANE / 16);
     reinterpret_cast<uint4*>(Bx + ((size_t)ks * ND + NDX) * TPLANE)[o] = make_uint4(0, 0, 0, 0);
   }
+  if (t < 4 * DSLOT) exs[t] = F64 ? 64 : 0;  // (FP64: so far above a zero that its significand is shifted out)
   if (t == 0) {
     fail[0] = 0;
-    for (int i = 0; i < 5; ++i) tc::mbar_init(&mb[i], 1);
+    for (int i = 0; i < DST; ++i) {
+      tc::mbar_init(&full[i], 1);
+      tc::mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&bfull[i], DW);
+      tc::mbar_init(&done[i], 1);
+    }
   }
-  if (warp == 0) {
-    tc::tmem_alloc(tslot, 128);
+  if (warp == DW + 1) {
+    tc::tmem_alloc(tslot, 256);
     tc::tmem_relinquish();
+  }
+  __syncthreads();
+  if (t == 0) {
+    int n = 0;
+    for (int L = 0; L < NL; ++L) {
+      int any = 0;
+      for (int s = 0; s < DSLOT; ++s) any |= sact[L * DSLOT + s];
+      if (any) actL[n++] = L;
+    }
+    fail[1] = n;
   }
   tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tD = *tslot;
-  const uint32_t lane_off = (uint32_t)(32 * qw) << 16;
-  uint32_t nfull[2] = {0, 0}, nempty[2] = {0, 0}, ndone = 0;
-  const uint64_t dA = tc::smem_desc(tc::smem_u32(Abuf)), dB = tc::smem_desc(tc::smem_u32(Bx));
-  const int row = 32 * qw + lane, trow = 128 * mt + row;  // this thread's tensor-memory lane
-  const int nchunk = DSLOT * 2 * ksteps;                  // chunks of 8 consecutive v per slot
+  const int na = fail[1];
+  const int row = 32 * qw + lane, trow = 128 * mt + row;  // a working thread's tensor-memory lane
   Sum acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = {};
 
-  for (int L = 0; L < NL; ++L) {
-    int any = 0;
-    for (int s = 0; s < DSLOT; ++s) any |= sact[L * DSLOT + s];
-    if (!any) continue;  // uniform: sact is written before the first barrier
-    const size_t tslice = ((size_t)L * A.nel + a) * mtiles + mt;
-    const unsigned char* Ag = T.tk_digits + tslice * ksteps * ND * APLANE;
-    // the producer starts streaming the first two K steps of the table
-    if (t == 0) {
-      for (int ks = 0; ks < 2 && ks < ksteps; ++ks) {
-        tc::mbar_expect_tx(&mb[ks], ND * APLANE);
-        tc::bulk_g2s(Abuf + ks * ND * APLANE, Ag + (size_t)ks * ND * APLANE, ND * APLANE, &mb[ks]);
-      }
-    }
-    for (int idx = t; idx < 128; idx += blockDim.x) alpha[idx] = T.tk_rowexp[tslice * 128 + idx];
-    if (t < DSLOT) exs[t] = F64 ? 64 : 0;  // (FP64: so far above a zero that its significand is shifted out)
-    __syncthreads();
-    // ---- recouple the 16 density vectors and take each slot's exponent ----
-    Sum xs[2][8];
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int ch = t + c * 256;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) xs[c][j] = {};
-      if (ch >= nchunk) continue;
-      const int s = ch / (2 * ksteps), v0 = 8 * (ch % (2 * ksteps));
-      if (!sact[L * DSLOT + s]) continue;
-      const int ent = gent[s * NL + L];
-      int eo[8];  // density offsets of the 8 elements (nbf^2 < 2^31), -1: outside the basis
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int v = v0 + j, p = v % nn, q = v / nn;
-        const int gp = gfun(A, a, p), gq = gfun(A, a, q);
-        eo[j] = (v < n2 && gp >= 0 && gp < A.nrad && gq >= 0 && gq < A.nrad) ? gq * A.nbf + gp : -1;
-      }
-      // two terms' loads in flight together
-      const int u1 = A.kent_ptr[ent + 1];
-      for (int uu = A.kent_ptr[ent]; uu < u1; uu += 2) {
-        Val cf[2], pv[2][8];
-#pragma unroll
-        for (int w = 0; w < 2; ++w) {
-          const bool on = uu + w < u1 && act[A.kterm_blk[uu + w]];
-          cf[w] = {};
-          if constexpr (F64) {
-            if (on) cf[w] = A.kterm_coef[uu + w];
-          } else {
-            if (on) cf[w] = A.kterm_coef2[uu + w];
-          }
-          const Val* pb = src + (on ? A.kterm_off[uu + w] : 0);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            pv[w][j] = {};
-            if (on && eo[j] >= 0) pv[w][j] = pb[eo[j]];
-          }
-        }
-#pragma unroll
-        for (int w = 0; w < 2; ++w)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            if constexpr (F64) xs[c][j] = fma(cf[w], pv[w][j], xs[c][j]); else xs[c][j] = ff_fma(xs[c][j], cf[w], pv[w][j]);
-          }
-      }
-      unsigned eb = 0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if constexpr (F64) {
-          eb = max(eb, ((unsigned)__double2hiint(xs[c][j]) >> 20) & 0x7FFu);
-        } else {
-          xs[c][j] = ff_norm(xs[c][j].hi, xs[c][j].lo);
-          eb = max(eb, (__float_as_uint(xs[c][j].hi) >> 23) & 0xFFu);
-        }
-      }
-      atomicMax(&exs[s], (int)eb);
-    }
-    __syncthreads();
-    // ---- digits: B[ks][kx][row slot, k = v mod 16] ----
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int ch = t + c * 256;
-      if (ch >= nchunk) continue;
-      const int s = ch / (2 * ksteps), kk = ch % (2 * ksteps), ks = kk >> 1, h = kk & 1;
-      uint32_t pk[NX][4];
-      if constexpr (F64) digits_fixed256(xs[c], exs[s] - 1022, pk); else digits_of(xs[c], tile_exponent((unsigned)exs[s]), pk);
-      const uint32_t off = tc::off_kmajor(s, 8 * h);
-#pragma unroll
-      for (int k = 0; k < NX; ++k)
-        *reinterpret_cast<uint4*>(Bx + ((size_t)ks * ND + k) * TPLANE + off) =
-            make_uint4(pk[k][0], pk[k][1], pk[k][2], pk[k][3]);
-    }
-    tc::fence_async_smem();
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-
-    // ---- the K loop (one thread): MMAs of step ks from buffer ks & 1; the
-    // buffer is refilled with step ks + 2 once those MMAs have finished ----
-    if (t == 0) {
+  if (warp == DW) {
+    if (lane == 0) {
       bool ok = true;
-      for (int ks = 0; ks < ksteps && ok; ++ks) {
-        const int bf = ks & 1;
-        ok = tc::mbar_wait(&mb[bf], nfull[bf] & 1u);
-        ++nfull[bf];
-        if (!ok) break;
-        tc::fence_after_sync();
-#pragma unroll 1
-        for (int kt = 0; kt < ND; ++kt)
-          tc::mma_bf16(tD + 16 * kt, dA + (uint64_t)((bf * ND + kt) * APLANE >> 4),
-                       dB + (uint64_t)((size_t)ks * ND * TPLANE >> 4), tc::idesc_bf16(128, 16 * (ND - kt), 0, 0),
-                       (ks > 0 || kt > 0) ? 1u : 0u);
-        tc::mma_commit(&mb[2 + bf]);
-        if (ks + 2 < ksteps) {
-          ok = tc::mbar_wait(&mb[2 + bf], nempty[bf] & 1u);
-          ++nempty[bf];
-          if (!ok) break;
-          tc::mbar_expect_tx(&mb[bf], ND * APLANE);
-          tc::bulk_g2s(Abuf + bf * ND * APLANE, Ag + (size_t)(ks + 2) * ND * APLANE, ND * APLANE, &mb[bf]);
-        } else {
-          ++nempty[bf];  // that phase completes without a wait
+      int it = 0;
+      for (int n = 0; n < na && ok; ++n) {
+        const unsigned char* Ag =
+            T.tk_digits + (((size_t)actL[n] * A.nel + a) * mtiles + mt) * ksteps * ND * APLANE;
+        for (int ks = 0; ks < ksteps; ++ks, ++it) {
+          const int s = it % DST;
+          if (it >= DST && !tc::mbar_wait(&empty[s], (uint32_t)((it / DST - 1) & 1), kWait)) {
+            ok = false;
+            break;
+          }
+          tc::mbar_expect_tx(&full[s], ND * APLANE);
+          tc::bulk_g2s(Abuf + s * ND * APLANE, Ag + (size_t)ks * ND * APLANE, ND * APLANE, &full[s]);
         }
       }
-      tc::mma_commit(&mb[4]);
+      if (!ok) {
+        atomicExch(fail, 1);
+        // the copies in flight must land before the CTA leaves
+        for (int i = max(0, it - DST); i < it; ++i) tc::mbar_wait(&full[i % DST], (uint32_t)((i / DST) & 1), kWait);
+      }
+    }
+  } else if (warp == DW + 1) {
+    if (lane == 0) {
+      bool ok = true;
+      int it = 0;
+      for (int n = 0; n < na && ok; ++n) {
+        const int bf = n & 1;
+        // (the working warps arrive after reading batch n - 2 back)
+        if (!(ok = tc::mbar_wait(&bfull[bf], (uint32_t)((n >> 1) & 1), kWait))) break;
+        tc::fence_after_sync();
+        const uint64_t dB = tc::smem_desc(tc::smem_u32(Bx + bf * bsize));
+        for (int ks = 0; ks < ksteps; ++ks, ++it) {
+          const int s = it % DST;
+          if (!(ok = tc::mbar_wait(&full[s], (uint32_t)((it / DST) & 1), kWait))) break;
+          tc::fence_after_sync();
+          const uint64_t dA = tc::smem_desc(tc::smem_u32(Abuf + s * ND * APLANE));
+#pragma unroll
+          for (int kt = 0; kt < ND; ++kt)
+            tc::mma_bf16(tD + 128 * bf + 16 * kt, dA + (uint64_t)(kt * APLANE >> 4),
+                         dB + (uint64_t)((size_t)ks * ND * TPLANE >> 4), tc::idesc_bf16(128, 16 * (ND - kt), 0, 0),
+                         (ks > 0 || kt > 0) ? 1u : 0u);
+          tc::mma_commit(&empty[s]);
+        }
+        if (ok) tc::mma_commit(&done[bf]);
+      }
       if (!ok) atomicExch(fail, 1);
     }
-    if (!__all_sync(0xffffffffu, tc::mbar_wait(&mb[4], ndone & 1u)) && lane == 0) atomicExch(fail, 1);
-    ++ndone;
-    tc::fence_after_sync();
-    __syncthreads();
-    if (fail[0]) break;
-
-    // ---- levels -> float pairs, scaled by 2^(alpha_t + E_slot), accumulated
-    // over the multipoles; columns [8 half, 8 half + 8) = slots ----
-    {
+  } else {
+    const int nchunk = DSLOT * 2 * ksteps;  // chunks of 8 consecutive v per slot
+    for (int n = 0; n <= na; ++n) {
+      if (n < na) {
+        const int L = actL[n];
+        int* ex = exs + (n & 3) * DSLOT;
+        // ---- recouple the 16 density vectors and take each slot's exponent ----
+        Sum xs[2][8];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int ch = t + c * 256;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) xs[c][j] = {};
+          if (ch >= nchunk) continue;
+          const int s = ch / (2 * ksteps), v0 = 8 * (ch % (2 * ksteps));
+          if (!sact[L * DSLOT + s]) continue;
+          const int ent = gent[s * NL + L];
+          int eo[8];  // density offsets of the 8 elements (nbf^2 < 2^31), -1: outside the basis
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int v = v0 + j, p = v % nn, q = v / nn;
+            const int gp = gfun(A, a, p), gq = gfun(A, a, q);
+            eo[j] = (v < n2 && gp >= 0 && gp < A.nrad && gq >= 0 && gq < A.nrad) ? gq * A.nbf + gp : -1;
+          }
+          // two terms' loads in flight together
+          const int u1 = A.kent_ptr[ent + 1];
+          for (int uu = A.kent_ptr[ent]; uu < u1; uu += 2) {
+            Val cf[2], pv[2][8];
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+              const bool on = uu + w < u1 && act[A.kterm_blk[uu + w]];
+              cf[w] = {};
+              if constexpr (F64) {
+                if (on) cf[w] = A.kterm_coef[uu + w];
+              } else {
+                if (on) cf[w] = A.kterm_coef2[uu + w];
+              }
+              const Val* pb = src + (on ? A.kterm_off[uu + w] : 0);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                pv[w][j] = {};
+                if (on && eo[j] >= 0) pv[w][j] = pb[eo[j]];
+              }
+            }
+#pragma unroll
+            for (int w = 0; w < 2; ++w)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                if constexpr (F64) xs[c][j] = fma(cf[w], pv[w][j], xs[c][j]); else xs[c][j] = ff_fma(xs[c][j], cf[w], pv[w][j]);
+              }
+          }
+          unsigned eb = 0;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if constexpr (F64) {
+              eb = max(eb, ((unsigned)__double2hiint(xs[c][j]) >> 20) & 0x7FFu);
+            } else {
+              xs[c][j] = ff_norm(xs[c][j].hi, xs[c][j].lo);
+              eb = max(eb, (__float_as_uint(xs[c][j].hi) >> 23) & 0xFFu);
+            }
+          }
+          atomicMax(&ex[s], (int)eb);
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (t < DSLOT) exs[((n + 2) & 3) * DSLOT + t] = F64 ? 64 : 0;  // last read for batch n - 2
+        // ---- digits: B[ks][kx][row slot, k = v mod 16]; batch n - 2 has been
+        // read back, its products are over ----
+        unsigned char* Bn = Bx + (n & 1) * bsize;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int ch = t + c * 256;
+          if (ch >= nchunk) continue;
+          const int s = ch / (2 * ksteps), kk = ch % (2 * ksteps), ks = kk >> 1, h = kk & 1;
+          uint32_t pk[NX][4];
+          if constexpr (F64) digits_fixed256(xs[c], ex[s] - 1022, pk); else digits_of(xs[c], tile_exponent((unsigned)ex[s]), pk);
+          const uint32_t off = tc::off_kmajor(s, 8 * h);
+#pragma unroll
+          for (int k = 0; k < NX; ++k)
+            *reinterpret_cast<uint4*>(Bn + ((size_t)ks * ND + k) * TPLANE + off) =
+                make_uint4(pk[k][0], pk[k][1], pk[k][2], pk[k][3]);
+        }
+        tc::fence_before_sync();
+        tc::fence_async_smem();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&bfull[n & 1]);
+      }
+      if (n == 0) continue;
+      // ---- the batch before: levels scaled by 2^(alpha_t + E_slot), summed
+      // over the multipoles; columns [8 half, 8 half + 8) = slots ----
+      const int m = n - 1, L = actL[m];
+      const int* ex = exs + (m & 3) * DSLOT;
+      const int ea = T.tk_rowexp[(((size_t)L * A.nel + a) * mtiles + mt) * 128 + row];
+      const bool ok = tc::mbar_wait(&done[m & 1], (uint32_t)((m >> 1) & 1), kWait);
+      if (!__all_sync(0xffffffffu, ok)) {
+        // (the other working warps meet at barrier 1: all give up in turn)
+        if (lane == 0) atomicExch(fail, 1);
+        if (n < na) continue;
+        break;
+      }
+      tc::fence_after_sync();
       float v[ND][8];
-      tmem_ld_levels(tD + lane_off + 8 * half, v);
-      const int ea = alpha[row];
+      tmem_ld_levels(tD + 128 * (m & 1) + ((uint32_t)(32 * qw) << 16) + 8 * half, v);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int s = 8 * half + j;
@@ -1102,19 +1149,19 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
 #pragma unroll
         for (int d = 0; d < ND; ++d) lv[d] = v[d][j];
         if constexpr (F64)
-          acc[j] += exs[s] == 0x7FF ? __longlong_as_double(0x7ff8000000000000ll) : levels_to_f64(lv, ea + exs[s] - 1022);
+          acc[j] += ex[s] == 0x7FF ? __longlong_as_double(0x7ff8000000000000ll) : levels_to_f64(lv, ea + ex[s] - 1022);
         else
-          acc[j] = ff_add(acc[j], levels_to_pair(lv, exp2i(ea + tile_exponent((unsigned)exs[s]))));
+          acc[j] = ff_add(acc[j], levels_to_pair(lv, exp2i(ea + tile_exponent((unsigned)ex[s]))));
       }
     }
-    tc::fence_before_sync();
-    __syncthreads();
   }
+  tc::fence_before_sync();
+  __syncthreads();
 
   // ---- store K_jk(a,a)[p, q], t = p + q nn; with a symmetric density also
   // the transposed partner K_kj(a,a)[q, p] (j != k) ----
   const bool failed = fail[0] != 0;
-  if (trow < n2) {
+  if (warp < DW && trow < n2) {
     const int p = trow % nn, q = trow / nn;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -1130,11 +1177,11 @@ __global__ void __launch_bounds__(256, 2) k_diag_tc(DevAtom A, DevScratch S, Dev
   }
   if (failed && t == 0) {
     atomicExch(T.err, 1);
-    tc::mbar_wait(&mb[4], ndone & 1u);
+    // MMAs may still be running: give them time before the tensor memory is released
+    for (int i = 0; i < 100; ++i) __nanosleep(1000);
   }
-  tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tD, 128);
+  if (warp == DW + 1) tc::tmem_dealloc(tD, 256);
 }
 
 size_t tc_smem_bytes(int NL, int nang, bool f64) {
@@ -1143,8 +1190,8 @@ size_t tc_smem_bytes(int NL, int nang, bool f64) {
 }
 
 size_t tc_diag_smem_bytes(int NL, int ksteps, int nang) {
-  return (size_t)2 * ND * APLANE + (size_t)ksteps * ND * TPLANE +
-         sizeof(int) * (128 + DSLOT + NL * DSLOT * 2 + DSLOT + 2) + 5 * 8 + 8 + (size_t)nang * nang + 64;
+  return (size_t)DST * ND * APLANE + (size_t)2 * ksteps * ND * TPLANE +
+         sizeof(int) * (4 * DSLOT + NL * DSLOT * 2 + DSLOT + 2 + NL + 1) + 8 * (2 * DST + 4) + 8 + (size_t)nang * nang + 64;
 }
 
 // P: the FP64 form (from the density itself), nullptr: the split form (from S.p2)
@@ -1179,7 +1226,7 @@ cudaError_t launch_k_diag_tc(const DevAtom& A, const DevScratch& S, const DevTC&
   auto kern = P ? k_diag_tc<true> : k_diag_tc<false>;
   const cudaError_t e = smem_limit(kern, smem);
   if (e != cudaSuccess) return e;
-  kern<<<n, 256, smem, st>>>(A, S, Td, symmetric ? 1 : 0, P, K);
+  kern<<<n, DTHREADS, smem, st>>>(A, S, Td, symmetric ? 1 : 0, P, K);
   return cudaGetLastError();
 }
 

@@ -70,9 +70,12 @@ CASES64 = [
     (36, 3, 3, 2, 16),
     (36, 2, 2, 12, 10),
     (10, 1, 1, 16, 12),
-    (10, 1, 1, 5, 13),
-    (36, 2, 2, 11, 10),
-    (10, 0, 0, 6, 15),
+    (6, 1, 0, 3, 10),
+    (6, 1, 0, 3, 9),
+    (36, 2, 2, 11, 9),
+    (10, 0, 0, 10, 15),
+    (10, 0, 0, 11, 15),
+    (4, 0, 0, 6, 14),
     (18, 1, 1, 6, 17),
 ]
 
