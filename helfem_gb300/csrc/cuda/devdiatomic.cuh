@@ -130,33 +130,31 @@ struct DevDiatomicScratch {
 
 #define DNORM_SPLIT 8
 
-// pure-m DFT grid: nq mu points per element, na nu points, npair same-m
-// unordered angular pairs (s <= t)
+// pure-m DFT grid: nq mu points per element, na nu points, npair unordered
+// pairs of shells (s <= t) of one m, those of m < 0 with their m > 0 mirrors
 struct DevDiatomicXC {
   int nq = 0, na = 0, npair = 0;
-  const int* ps = nullptr;     // [npair]
-  const int* pt = nullptr;
+  const int4* pair = nullptr;    // [npair] s, t and the mirror shells of -m (or -1)
   const double* mult = nullptr;  // 2 (s != t) or 1
-  const double* W = nullptr;   // [k*na + a]: Y_s Y_t
-  const double* Wt = nullptr;  //             Y_s' Y_t + Y_s Y_t'
-  const double* R = nullptr;   // [(e*nq + q)*nn + p]
+  const double* W = nullptr;     // [k*na + a]: Y_s Y_t
+  const double* Wt = nullptr;    //             Y_s' Y_t + Y_s Y_t'
+  const double* WT = nullptr;    // [a*npair + k]: the same, transposed
+  const double* WtT = nullptr;
+  const double* R = nullptr;     // [(e*nq + q)*nn + p]
   const double* dR = nullptr;
-  const double* w = nullptr;   // [(e*nq + q)*na + a]
+  const double* w = nullptr;     // [(e*nq + q)*na + a]
   const double* hinv = nullptr;
-  // Fock-side pairs: tiles built for pairs fk[0..nfock), each also written to
-  // the mirror shells (fms, fmt) of opposite m when fms >= 0
-  int nfock = 0;
-  const int* fk = nullptr;
-  const int* fms = nullptr;
-  const int* fmt = nullptr;
 };
 struct DiatomicXcScratch {
-  double* D;      // [nsd][nel][nq][npair]  mult * B^T P_st B
+  double* D;      // [nsd][nel][npair][nq]  mult * B^T P_st B (and the mirror's)
   double* Dr;     // same                   mult/2 * (dB^T P_st B + B^T P_st dB)
   double* F;      // [nout][3][nel][nq][na]
   double* U;      // [nout][3][nel][npair][nq]
-  double* epart;  // [nel*nq][2]
+  double* epart;  // [nel*blocks of points][2]
 };
+// blocks of grid points of one element
+constexpr int DXC_POINTS = 32;  // one warp: the functional is a long serial chain, few points still fill the SMs
+inline int dxc_blocks(int nq, int na) { return (nq * na + DXC_POINTS - 1) / DXC_POINTS; }
 // Pb == nullptr: restricted (Pa is the total density, Ha the potential).
 // Densities and potentials are in the pure basis (nbf x nbf, column-major);
 // H is overwritten. energies (device, may be null) receives {Exc, Nel}.

@@ -36,7 +36,7 @@ struct hfg_diatomic {
   hfg::DevDiatomicXC xc{};
   hfg::DiatomicXcScratch xs{};
   bool xc_ready = false;
-  DBuf x_ps, x_pt, x_mult, x_W, x_Wt, x_R, x_dR, x_w, x_hinv, x_fk, x_fms, x_fmt, xs_D, xs_Dr, xs_F, xs_U, xs_ep,
+  DBuf x_pair, x_mult, x_W, x_Wt, x_WT, x_WtT, x_R, x_dR, x_w, x_hinv, xs_D, xs_Dr, xs_F, xs_U, xs_ep,
       h_in2, h_out2, h_e;
 
   ~hfg_diatomic() {
@@ -542,26 +542,36 @@ struct hfg_diatomic {
     need(H.xc_lang <= 1024, "hfg_diatomic_dft_grid: at most 1024 nu points");
     xc.nq = H.xc_nq;
     xc.na = H.xc_lang;
-    xc.npair = H.xc_npair;
-    xc.ps = x_ps.upload(H.xc_ps);
-    xc.pt = x_pt.upload(H.xc_pt);
-    xc.mult = x_mult.upload(H.xc_mult);
-    xc.nfock = (int)H.xc_fk.size();
-    xc.fk = x_fk.upload(H.xc_fk);
-    xc.fms = x_fms.upload(H.xc_fms);
-    xc.fmt = x_fmt.upload(H.xc_fmt);
-    xc.W = x_W.upload(H.xc_W);
-    xc.Wt = x_Wt.upload(H.xc_Wt);
+    // the pairs whose tiles are built, each with its mirror
+    const size_t nf = H.xc_fk.size(), nla = H.xc_lang;
+    xc.npair = (int)nf;
+    std::vector<int4> pair(nf);
+    std::vector<double> mult(nf), W(nf * nla), Wt(nf * nla), WT(nf * nla), WtT(nf * nla);
+    for (size_t f = 0; f < nf; ++f) {
+      const int k = H.xc_fk[f];
+      pair[f] = make_int4(H.xc_ps[k], H.xc_pt[k], H.xc_fms[f], H.xc_fmt[f]);
+      mult[f] = H.xc_mult[k];
+      for (size_t i = 0; i < nla; ++i) {
+        W[f * nla + i] = WT[i * nf + f] = H.xc_W[k * nla + i];
+        Wt[f * nla + i] = WtT[i * nf + f] = H.xc_Wt[k * nla + i];
+      }
+    }
+    xc.pair = x_pair.upload(pair);
+    xc.mult = x_mult.upload(mult);
+    xc.W = x_W.upload(W);
+    xc.Wt = x_Wt.upload(Wt);
+    xc.WT = x_WT.upload(WT);
+    xc.WtT = x_WtT.upload(WtT);
     xc.R = x_R.upload(H.xc_R);
     xc.dR = x_dR.upload(H.xc_dR);
     xc.w = x_w.upload(H.xc_w);
     xc.hinv = x_hinv.upload(H.xc_hinv);
-    const size_t nel = H.nel, nq = H.xc_nq, np = H.xc_npair, na = H.xc_lang;
+    const size_t nel = H.nel, nq = H.xc_nq, np = nf, na = H.xc_lang;
     xs_D.alloc(sizeof(double) * 2 * nel * nq * np);
     xs_Dr.alloc(sizeof(double) * 2 * nel * nq * np);
     xs_F.alloc(sizeof(double) * 6 * nel * nq * na);
     xs_U.alloc(sizeof(double) * 6 * nel * np * nq);
-    xs_ep.alloc(sizeof(double) * 2 * nel * nq);
+    xs_ep.alloc(sizeof(double) * 2 * nel * hfg::dxc_blocks((int)nq, (int)na));
     xs.D = xs_D.as<double>();
     xs.Dr = xs_Dr.as<double>();
     xs.F = xs_F.as<double>();
