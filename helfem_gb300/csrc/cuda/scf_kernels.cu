@@ -145,6 +145,73 @@ __global__ void dav_olsen(const double* __restrict__ Zr, const double* __restric
 
 inline int grid_for(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 152 * 16); }
 
+// Products with few columns (the Ritz vectors of a refinement, occupied
+// orbitals): cuBLAS gives them to a handful of CTAs with tiles of 32 columns, 80
+// us for 279 x 9 x 279, where the FP64 work and the bytes are a microsecond's.
+// N: lane = row, the 8 warps of a CTA share the sum over k (added in order);
+// T: a warp per row of op(A), its lanes along k. NC columns at a time: one
+// while CTAs are few, more where A would be read too often.
+template <int NC>
+__global__ void __launch_bounds__(256) thin_n(int m, int n, int k, double alpha, const double* __restrict__ A, int lda,
+                                              size_t sa, const double* __restrict__ B, int ldb, size_t sb, double beta,
+                                              double* __restrict__ C, int ldc, size_t sc) {
+  __shared__ double part[8][NC][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, row = blockIdx.x * 32 + lane, c0 = blockIdx.y * NC;
+  A += blockIdx.z * sa;
+  B += blockIdx.z * sb;
+  C += blockIdx.z * sc;
+  const int k0 = (int)((long)k * w / 8), k1 = (int)((long)k * (w + 1) / 8);
+  double acc[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+  const int r = min(row, m - 1);
+#pragma unroll 8
+  for (int i = k0; i < k1; ++i) {
+    const double a = A[(size_t)i * lda + r];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] += a * B[(size_t)min(c0 + c, n - 1) * ldb + i];
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) part[w][c][lane] = acc[c];
+  __syncthreads();
+  for (int c = w; c < NC; c += 8) {
+    if (row >= m || c0 + c >= n) continue;
+    double s = 0.0;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) s += part[v][c][lane];
+    double* o = C + (size_t)(c0 + c) * ldc + row;
+    *o = beta == 0.0 ? alpha * s : alpha * s + beta * *o;
+  }
+}
+template <int NC>
+__global__ void __launch_bounds__(256) thin_t(int m, int n, int k, double alpha, const double* __restrict__ A, int lda,
+                                              size_t sa, const double* __restrict__ B, int ldb, size_t sb, double beta,
+                                              double* __restrict__ C, int ldc, size_t sc) {
+  const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5), c0 = blockIdx.y * NC;
+  if (row >= m) return;  // whole warps
+  A += blockIdx.z * sa + (size_t)row * lda;
+  B += blockIdx.z * sb;
+  C += blockIdx.z * sc;
+  double acc[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+#pragma unroll 4
+  for (int i = lane; i < k; i += 32) {
+    const double a = A[i];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] += a * B[(size_t)min(c0 + c, n - 1) * ldb + i];
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    if (lane == 0 && c0 + c < n) {
+      double* d = C + (size_t)(c0 + c) * ldc + row;
+      *d = beta == 0.0 ? alpha * acc[c] : alpha * acc[c] + beta * *d;
+    }
+  }
+}
+
 }  // namespace
 
 void k_gather_block(const double* M, int nbf, int nrad, const int* ang, int nk, double* Mk, cudaStream_t st) {
@@ -215,6 +282,20 @@ void k_add4(double* out, const double* a, const double* b, const double* c, cons
             cudaStream_t st) {
   add4<<<grid_for(n), 256, 0, st>>>(out, a, b, c, d, n);
 }
+bool thin_gemm_ok(int m, int n, int k) { return n <= 64 && (long)m * k <= (1l << 24); }
+
+void k_thin_gemm(bool transa, int m, int n, int k, double alpha, const double* A, int lda, size_t sa, const double* B,
+                 int ldb, size_t sb, double beta, double* C, int ldc, size_t sc, int batch, cudaStream_t st) {
+  if (m <= 0 || n <= 0 || batch <= 0) return;
+  const long rows = transa ? (m + 7) / 8 : (m + 31) / 32;
+  // columns at a time: the most that leave every SM a CTA
+  const int nc = rows * ((n + 7) / 8) * batch >= 152 ? 8 : rows * ((n + 3) / 4) * batch >= 152 ? 4 : transa ? 2 : 1;
+  const dim3 grid((unsigned)rows, (n + nc - 1) / nc, batch);
+  auto kern = transa ? (nc == 8 ? thin_t<8> : nc == 4 ? thin_t<4> : thin_t<2>)
+                     : (nc == 8 ? thin_n<8> : nc == 4 ? thin_n<4> : thin_n<1>);
+  kern<<<grid, 256, 0, st>>>(m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc);
+}
+
 void k_scale_cols(const double* X, int n, int m, const double* s, double* Y, cudaStream_t st) {
   scale_cols<<<grid_for((size_t)n * m), 256, 0, st>>>(X, n, m, s, Y);
 }

@@ -37,6 +37,12 @@ void k_lerp(double* out, const double* a, double lam, size_t n, cudaStream_t st)
 void fill_test_density(double* P, int n, cudaStream_t st);
 // A[i,i] += v, A n x n column-major
 void k_add_diag(double* A, int n, double v, cudaStream_t st);
+// C = alpha op(A) B + beta C, op(A) m x k, B k x n, column-major, batch of them
+// at the given strides; for few columns n (beta = 0: C is not read)
+void k_thin_gemm(bool transa, int m, int n, int k, double alpha, const double* A, int lda, size_t sa, const double* B,
+                 int ldb, size_t sb, double beta, double* C, int ldc, size_t sc, int batch, cudaStream_t st);
+// whether k_thin_gemm is the one to call (else cuBLAS)
+bool thin_gemm_ok(int m, int n, int k);
 // Davidson steps (n x k column blocks): residuals R = AX - X diag(theta) with
 // column norms; reference-preconditioned Olsen corrections in the reference
 // eigenbasis (Zr = Vr^T R, Zx = Vr^T X -> Zt)

@@ -73,6 +73,16 @@ void jacobi_eigh(int m, std::vector<double> A, std::vector<double>& w, std::vect
 
 namespace {
 
+// C = alpha op(A) B + beta C
+void gemm(cublasHandle_t bl, cudaStream_t st, bool transa, int m, int n, int k, double alpha, const double* A, int lda,
+          const double* B, int ldb, double beta, double* C, int ldc, const char* what) {
+  if (thin_gemm_ok(m, n, k))
+    k_thin_gemm(transa, m, n, k, alpha, A, lda, 0, B, ldb, 0, beta, C, ldc, 0, 1, st);
+  else
+    cbl(cublasDgemm(bl, transa ? CUBLAS_OP_T : CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, &alpha, A, lda, B, ldb, &beta, C, ldc),
+        what);
+}
+
 // Orthogonalise the u columns of T (device, n x u) against Q[:, :m] (two
 // classical Gram-Schmidt passes) and append an orthonormal basis of what is
 // left to Q (canonical orthonormalisation: directions with a Gram eigenvalue
@@ -82,10 +92,10 @@ int append_orthonormal(cublasHandle_t bl, cudaStream_t st, int n, double* Q, int
   const double one = 1.0, zero = 0.0, mone = -1.0;
   double* C = w.sm2.as<double>();
   for (int pass = 0; pass < 2 && m > 0; ++pass) {
-    cbl(cublasDgemm(bl, CUBLAS_OP_T, CUBLAS_OP_N, m, u, n, &one, Q, n, T, n, &zero, C, m), "Q^T T");
-    cbl(cublasDgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, n, u, m, &mone, Q, n, C, m, &one, T, n), "T -= Q C");
+    gemm(bl, st, true, m, u, n, one, Q, n, T, n, zero, C, m, "Q^T T");
+    gemm(bl, st, false, n, u, m, mone, Q, n, C, m, one, T, n, "T -= Q C");
   }
-  cbl(cublasDgemm(bl, CUBLAS_OP_T, CUBLAS_OP_N, u, u, n, &one, T, n, T, n, &zero, C, u), "T^T T");
+  gemm(bl, st, true, u, u, n, one, T, n, T, n, zero, C, u, "T^T T");
   w.h1.resize((size_t)u * u);
   ck(cudaMemcpyAsync(w.h1.data(), C, sizeof(double) * u * u, cudaMemcpyDeviceToHost, st), "D2H gram");
   ck(cudaStreamSynchronize(st), "sync");
@@ -108,11 +118,11 @@ int append_orthonormal(cublasHandle_t bl, cudaStream_t st, int n, double* Q, int
   if (kept == 0) return m;
   ck(cudaMemcpyAsync(C, M.data(), sizeof(double) * M.size(), cudaMemcpyHostToDevice, st), "H2D transform");
   double* Qn = Q + (size_t)m * n;
-  cbl(cublasDgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, n, kept, u, &one, T, n, C, u, &zero, Qn, n), "T M");
+  gemm(bl, st, false, n, kept, u, one, T, n, C, u, zero, Qn, n, "T M");
   if (m > 0) {  // one more pass against the old columns
     double* C2 = w.sm.as<double>();
-    cbl(cublasDgemm(bl, CUBLAS_OP_T, CUBLAS_OP_N, m, kept, n, &one, Q, n, Qn, n, &zero, C2, m), "Q^T Qn");
-    cbl(cublasDgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, n, kept, m, &mone, Q, n, C2, m, &one, Qn, n), "Qn -= Q C");
+    gemm(bl, st, true, m, kept, n, one, Q, n, Qn, n, zero, C2, m, "Q^T Qn");
+    gemm(bl, st, false, n, kept, m, mone, Q, n, C2, m, one, Qn, n, "Qn -= Q C");
   }
   return m + kept;
 }
@@ -143,7 +153,7 @@ int davidson_lowest(cublasHandle_t bl, cudaStream_t st, const BlockOperator& app
   for (int it = 0; it < maxit; ++it) {
     apply(Q + (size_t)mo * n, m - mo, AQ + (size_t)mo * n);
     double* Hd = w.sm.as<double>();
-    cbl(cublasDgemm(bl, CUBLAS_OP_T, CUBLAS_OP_N, m, m, n, &one, Q, n, AQ, n, &zero, Hd, m), "Q^T F Q");
+    gemm(bl, st, true, m, m, n, one, Q, n, AQ, n, zero, Hd, m, "Q^T F Q");
     Hh.resize((size_t)m * m);
     ck(cudaMemcpyAsync(Hh.data(), Hd, sizeof(double) * m * m, cudaMemcpyDeviceToHost, st), "D2H H");
     ck(cudaStreamSynchronize(st), "sync");
@@ -157,8 +167,8 @@ int davidson_lowest(cublasHandle_t bl, cudaStream_t st, const BlockOperator& app
     double* Yd = w.sm2.as<double>();
     ck(cudaMemcpyAsync(Yd, Y.data(), sizeof(double) * m * k, cudaMemcpyHostToDevice, st), "H2D Y");
     ck(cudaMemcpyAsync(w.th.p, th.data(), sizeof(double) * k, cudaMemcpyHostToDevice, st), "H2D theta");
-    cbl(cublasDgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, n, k, m, &one, Q, n, Yd, m, &zero, X, n), "Q Y");
-    cbl(cublasDgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, n, k, m, &one, AQ, n, Yd, m, &zero, AX, n), "AQ Y");
+    gemm(bl, st, false, n, k, m, one, Q, n, Yd, m, zero, X, n, "Q Y");
+    gemm(bl, st, false, n, k, m, one, AQ, n, Yd, m, zero, AX, n, "AQ Y");
     k_dav_residual(AX, X, w.th.as<double>(), n, k, R, w.nrm.as<double>(), st);
     ck(cudaMemcpyAsync(nrm.data(), w.nrm.p, sizeof(double) * k, cudaMemcpyDeviceToHost, st), "D2H norms");
     ck(cudaStreamSynchronize(st), "sync");
@@ -197,13 +207,11 @@ int davidson_lowest(cublasHandle_t bl, cudaStream_t st, const BlockOperator& app
       (*pc)(Rg, Xg, thd, u, T);
     } else {
       // corrections in the reference eigenbasis, then back: T = Vr Zt
-      cbl(cublasDgemm(bl, CUBLAS_OP_T, CUBLAS_OP_N, n, u, n, &one, Vr, n, Rg, n, &zero, w.Zr.as<double>(), n),
-          "Vr^T R");
-      cbl(cublasDgemm(bl, CUBLAS_OP_T, CUBLAS_OP_N, n, u, n, &one, Vr, n, Xg, n, &zero, w.Zx.as<double>(), n),
-          "Vr^T X");
+      gemm(bl, st, true, n, u, n, one, Vr, n, Rg, n, zero, w.Zr.as<double>(), n, "Vr^T R");
+      gemm(bl, st, true, n, u, n, one, Vr, n, Xg, n, zero, w.Zx.as<double>(), n, "Vr^T X");
       const double floor_ = 1e-8 * std::max(1.0, std::fabs(thU.empty() ? 0.0 : thU[0]));
       k_dav_olsen(w.Zr.as<double>(), w.Zx.as<double>(), lam, thd, n, u, floor_, Rg, st);
-      cbl(cublasDgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, n, u, n, &one, Vr, n, Rg, n, &zero, T, n), "Vr Zt");
+      gemm(bl, st, false, n, u, n, one, Vr, n, Rg, n, zero, T, n, "Vr Zt");
     }
     mo = m;
     m = append_orthonormal(bl, st, n, Q, m, T, u, w);

@@ -270,9 +270,23 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
     // out = (I x X) V or (I x X)^T V for an nk x cols block V
     auto x_cols = [&](const Block& b, const double* Vin, int cols, double* out, bool trans) {
       const int p = (int)b.ang.size(), nk = b.nk;
-      cb(cublasDgemmStridedBatched(hd.bl, trans ? CUBLAS_OP_T : CUBLAS_OP_N, CUBLAS_OP_N, nrad, cols, nrad, &one,
-                                   dX.as<double>(), nrad, 0, Vin, nk, nrad, &zero, out, nk, nrad, p),
-         "X V");
+      if (hfg::thin_gemm_ok(nrad, cols, nrad))
+        hfg::k_thin_gemm(trans, nrad, cols, nrad, 1.0, dX.as<double>(), nrad, 0, Vin, nk, nrad, 0.0, out, nk, nrad, p, st);
+      else
+        cb(cublasDgemmStridedBatched(hd.bl, trans ? CUBLAS_OP_T : CUBLAS_OP_N, CUBLAS_OP_N, nrad, cols, nrad, &one,
+                                     dX.as<double>(), nrad, 0, Vin, nk, nrad, &zero, out, nk, nrad, p),
+           "X V");
+    };
+
+    // C = op(A) B for a few columns
+    auto thin = [&](bool trans, int m, int n, int k, double alpha, const double* A, int lda, const double* B, int ldb,
+                    double beta, double* C, int ldc, const char* what) {
+      if (hfg::thin_gemm_ok(m, n, k))
+        hfg::k_thin_gemm(trans, m, n, k, alpha, A, lda, 0, B, ldb, 0, beta, C, ldc, 0, 1, st);
+      else
+        cb(cublasDgemm(hd.bl, trans ? CUBLAS_OP_T : CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, &alpha, A, lda, B, ldb, &beta, C,
+                       ldc),
+           what);
     };
 
     // orbitals: eps (all blocks, per spin), occupations
@@ -307,8 +321,10 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
     size_t work_bytes = 0;
 
     // full eigensolves of the representative blocks selected by `full`
-    // (all when empty); results copied to every block they represent
-    auto diagonalise = [&](const double* Fo_all, int s, const std::vector<char>& full = {}) {
+    // (all when empty); results copied to every block they represent, without
+    // vectors the eigenvalues alone
+    auto diagonalise = [&](const double* Fo_all, int s, const std::vector<char>& full = {}, bool vectors = true) {
+      const cusolverEigMode_t mode = vectors ? CUSOLVER_EIG_MODE_VECTOR : CUSOLVER_EIG_MODE_NOVECTOR;
       double* Vs = dVec.as<double>() + Lblk * s;
       double* Ws = deps.as<double>() + (size_t)nbf * s;
       for (auto& grp0 : by_size) {
@@ -326,7 +342,7 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
                              sizeof(double) * n2, cudaMemcpyDeviceToDevice, st),
              "gather blocks");
         size_t wd = 0, wh = 0;
-        cs(cusolverDnXsyevBatched_bufferSize(hd.so, sparams, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, n,
+        cs(cusolverDnXsyevBatched_bufferSize(hd.so, sparams, mode, CUBLAS_FILL_MODE_LOWER, n,
                                              CUDA_R_64F, dBatch.p, n, CUDA_R_64F, dBatchW.p, CUDA_R_64F, &wd, &wh, nb),
            "syevBatched buffer size");
         if (wd > work_bytes) {
@@ -334,7 +350,7 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
           work_bytes = wd;
         }
         if (hwork.size() < wh) hwork.resize(wh);
-        cs(cusolverDnXsyevBatched(hd.so, sparams, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, n, CUDA_R_64F,
+        cs(cusolverDnXsyevBatched(hd.so, sparams, mode, CUBLAS_FILL_MODE_LOWER, n, CUDA_R_64F,
                                   dBatch.p, n, CUDA_R_64F, dBatchW.p, CUDA_R_64F, dWork.p, wd,
                                   hwork.empty() ? nullptr : hwork.data(), wh, dInfo.as<int>(), nb),
            "syevBatched");
@@ -343,9 +359,10 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
           const auto it = std::find(grp.second.begin(), grp.second.end(), r);
           if (it == grp.second.end()) continue;
           const int q = (int)(it - grp.second.begin());
-          ck(cudaMemcpyAsync(Vs + blocks[k].off, dBatch.as<double>() + n2 * q, sizeof(double) * n2,
-                             cudaMemcpyDeviceToDevice, st),
-             "scatter vectors");
+          if (vectors)
+            ck(cudaMemcpyAsync(Vs + blocks[k].off, dBatch.as<double>() + n2 * q, sizeof(double) * n2,
+                               cudaMemcpyDeviceToDevice, st),
+               "scatter vectors");
           ck(cudaMemcpyAsync(Ws + eoff[k], dBatchW.as<double>() + (size_t)n * q, sizeof(double) * n,
                              cudaMemcpyDeviceToDevice, st),
              "scatter values");
@@ -420,9 +437,7 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
           const double* Vk = dVec.as<double>() + Lblk * s + b.off;
           const int p = (int)b.ang.size(), nk = b.nk;
           // C_occ = (I x X) V_occ : nk x nocc
-          cb(cublasDgemmStridedBatched(hd.bl, CUBLAS_OP_N, CUBLAS_OP_N, nrad, nocc, nrad, &one, dX.as<double>(), nrad,
-                                       0, Vk, nk, nrad, &zero, dCo.as<double>(), nk, nrad, p),
-             "X V");
+          x_cols(b, Vk, nocc, dCo.as<double>(), false);
           hfg::k_scale_cols(dCo.as<double>(), nk, nocc, dOcc.as<double>() + (size_t)nbf * s + eoff[k], dW.as<double>(),
                             st);
           cb(cublasDgemm(hd.bl, CUBLAS_OP_N, CUBLAS_OP_T, nk, nk, nocc, &one, dW.as<double>(), nk, dCo.as<double>(),
@@ -442,8 +457,10 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
       }
     };
 
-    // Eigensolver policy: full batched solves for the first three
-    // diagonalisations (and whenever a block has no reference yet), then
+    // Eigensolver policy: full batched solves for the first two
+    // diagonalisations (a third costs 25 ms of Ar's 116, the refinement in its
+    // place 4: 101 ms; with one full solve the second refinement falls back, 107
+    // ms) and whenever a block has no reference yet, then
     // Davidson refinement of the previous orbitals of each representative
     // block, preconditioned by that block's last full eigendecomposition, to
     // residuals |F'x - theta x| <= dav_tol = 1e-2 x the current orbital
@@ -467,8 +484,8 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
     bool all_single = true;
     for (const Block& b : blocks) all_single = all_single && b.ang.size() == 1;
     const bool banded = band_ok && all_single;
-    const char* nenv = std::getenv("HFG_SCF_NFULL");  // full solves before refinement (default 3; 1 when banded)
-    const int n_full_first = (nenv && std::atoi(nenv) > 0) ? std::atoi(nenv) : (banded ? 1 : 3);
+    const char* nenv = std::getenv("HFG_SCF_NFULL");  // full solves before refinement (default 2; 1 when banded)
+    const int n_full_first = (nenv && std::atoi(nenv) > 0) ? std::atoi(nenv) : (banded ? 1 : 2);
     DBuf dSrad, dSX, dZr, dZx, dYt, dBandWork;
     if (banded) {
       dSrad.upload(H.Srad);
@@ -545,21 +562,15 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
             if (dOpA.n < need) dOpA.alloc(need);
             if (dOpB.n < need) dOpB.alloc(need);
             x_cols(b, Q, c, dOpA.as<double>(), false);
-            cb(cublasDgemm(hd.bl, CUBLAS_OP_N, CUBLAS_OP_N, b.nk, c, b.nk, &one, Fk, b.nk, dOpA.as<double>(), b.nk,
-                           &zero, dOpB.as<double>(), b.nk),
-               "F (X Q)");
+            thin(false, b.nk, c, b.nk, one, Fk, b.nk, dOpA.as<double>(), b.nk, zero, dOpB.as<double>(), b.nk, "F (X Q)");
             x_cols(b, dOpB.as<double>(), c, AQ, true);
             if (shift > 0.0) {
               cb(cublasDaxpy(hd.bl, b.nk * c, &shift, Q, 1, AQ, 1), "shift Q");
               if (nocc > 0) {
                 if (dOpC.n < sizeof(double) * (size_t)nocc * c) dOpC.alloc(sizeof(double) * (size_t)nocc * c);
                 const double mshift = -shift;
-                cb(cublasDgemm(hd.bl, CUBLAS_OP_T, CUBLAS_OP_N, nocc, c, b.nk, &one, V, b.nk, Q, b.nk, &zero,
-                               dOpC.as<double>(), nocc),
-                   "V^T Q");
-                cb(cublasDgemm(hd.bl, CUBLAS_OP_N, CUBLAS_OP_N, b.nk, c, nocc, &mshift, V, b.nk, dOpC.as<double>(),
-                               nocc, &one, AQ, b.nk),
-                   "shift projector");
+                thin(true, nocc, c, b.nk, one, V, b.nk, Q, b.nk, zero, dOpC.as<double>(), nocc, "V^T Q");
+                thin(false, b.nk, c, nocc, mshift, V, b.nk, dOpC.as<double>(), nocc, one, AQ, b.nk, "shift projector");
               }
             }
           };
@@ -844,9 +855,7 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
           const double* Vk = dVec.as<double>() + Lblk * s + b.off;
           // W = F' V_occ = X^T F_k (X V_occ);  G = W diag(occ) V_occ^T;  E = G - G^T
           x_cols(b, Vk, nocc, dCo.as<double>(), false);
-          cb(cublasDgemm(hd.bl, CUBLAS_OP_N, CUBLAS_OP_N, b.nk, nocc, b.nk, &one, Fo, b.nk, dCo.as<double>(), b.nk,
-                         &zero, dT1.as<double>(), b.nk),
-             "F (X V)");
+          thin(false, b.nk, nocc, b.nk, one, Fo, b.nk, dCo.as<double>(), b.nk, zero, dT1.as<double>(), b.nk, "F (X V)");
           x_cols(b, dT1.as<double>(), nocc, dW.as<double>(), true);
           hfg::k_scale_cols(dW.as<double>(), b.nk, nocc, dOcc.as<double>() + (size_t)nbf * s + eoff[k],
                             dCo.as<double>(), st);
@@ -1031,7 +1040,7 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
       for (int s = 0; s < nspin; ++s) {
         for (int k = 0; k < nblk; ++k)
           if (rep[k] == k) form_ortho(dFx.as<double>(), s, k);
-        diagonalise(dFp.as<double>(), s);
+        diagonalise(dFp.as<double>(), s, {}, false);
       }
       ck(cudaMemcpyAsync(eps.data(), deps.p, sizeof(double) * eps.size(), cudaMemcpyDeviceToHost, st), "D2H eps");
     }
