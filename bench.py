@@ -35,18 +35,22 @@ UNIT = "builds/s"
 WORKLOAD = ("Kr (Z=36) J+K Fock build: 40 elements r_i=61^(i/40)-1, 15-node LIP, l<=2, m<=2, "
             "Nbf=5031, L<=4, P=CC^T (18 cols, N(0,1), seed 12345, Loewdin in S)")
 KERNELS_PER_STEP = 5  # profiler marks per step: J contract, J scatter, K norms, K tiles, K fix-up
-# kernel launches per step: j_contract, j_scatter, k_block_norms, k_flags, then
-# k_tiles_tc + k_diag_tc (split form) or k_tiles (plain form), k_fixup
-LAUNCHES_PER_STEP = {"split": 7, "plain": 6}
+# kernel launches per step: j_contract, j_scatter, k_block_norms, k_tiles_tc,
+# k_diag_tc, k_zero_inactive, k_fixup
+LAUNCHES_PER_STEP = {"split": 7, "plain": 7}
 # what the timed K form computes in (the dtype key names the arithmetic, the
 # form key the scheme)
 FORMS = {
-    "plain": {"dtype": "f64", "form": "plain FP64"},
-    "split": {"dtype": "bf16 digits (7 x 8-bit slices, exact FP32 level sums on the tensor cores, FP64 recombination)",
+    "plain": {"dtype": "f64 (contractions as exact sums of f16 and bf16 digits, 56 bits and more)",
+              "form": "FP64: density tiles recoupled in FP64, cut into fixed-point digit planes, tcgen05 MMAs form "
+                      "exact FP32 level sums in tensor memory, recombined to FP64; J in FP64"},
+    "split": {"dtype": "f16 and bf16 digits (50-bit density tiles, exact FP32 level sums on the tensor cores, FP64 "
+                       "recombination)",
               "form": "split precision on the tensor cores: density tiles recoupled in float pairs, radial tables "
-                      "and density as balanced base-256 digit planes (bf16), tcgen05 MMAs form exact FP32 level "
-                      "sums in tensor memory, carried and recombined to FP64 once per output element; J in float "
-                      "pairs (hi + lo, error-free products) with one FP64 conversion per output element"},
+                      "and density as balanced digit planes (element pairs base 1024 in f16, diagonal elements base "
+                      "256 in bf16), tcgen05 MMAs form exact FP32 level sums in tensor memory, recombined to FP64 "
+                      "once per output element; J in float pairs (hi + lo, error-free products) with one FP64 "
+                      "conversion per output element"},
 }
 
 
@@ -325,8 +329,8 @@ def n2_summary(hg, torch, builds=2):
            "builds_per_s_split": 1e3 / (j_ms + k_ms), "builds_per_s_plain": 1e3 / (j_ms + p0.elapsed_time(p1)),
            "split_error_vs_fp64": {"k_max_rel": float(dK.abs().max() / Kd.abs().max()),
                                    "exchange_energy_abs_eh": abs(float((Pa * dK).sum()))},
-           "form": "split: float-pair diatomic tiles (the atomic tensor-core path does not cover the "
-                   "diatomic four-channel kernel)", "builds": builds}
+           "form": "split: element pairs in float pairs, in-element tiles as digit planes on the tensor cores; plain: "
+                   "element pairs in FP64, in-element tiles as digit planes of the FP64 tiles", "builds": builds}
     del Pd, Pa, Jd, Kd, K32, dK
     d.close()
     torch.cuda.empty_cache()
@@ -464,31 +468,26 @@ def run_ours(args):
     fp32 = fp32_peak_tflops(torch)
     hbm_peak = measured_peaks().get("hbm_gbs")
     kernel_ms = {k: (v[1] / max(v[0], 1)) for k, v in prof_all.items()}
-    if split:
-        # executed tensor work: the bf16 digit-plane MMAs of one exchange
-        mma = atom.tc_work(symmetric=True)
-        tc_rate = mma / (off_ms * 1e-3) / 1e12
-        mp = measured_peaks()
-        if mp.get("bf16_tflops"):
-            tpeak, tsrc = float(mp["bf16_tflops"]), "MEASURED_PEAKS.json bf16_tflops (cuBLAS bf16 GEMM, burst)"
-        else:
-            tpeak = hg.tc_peak(2, 4096)["tflops"]
-            tsrc = "measured in this run: this library's tcgen05 bf16 MMA loop (hfg_tc_peak)"
-        roofline = {
-            "bound": "tensor", "kernel": "k_tiles_tc + k_diag_tc (the exchange tile stage)", "achieved": tc_rate,
-            "peak": tpeak, "unit": "TFLOP/s", "frac": tc_rate / tpeak if tpeak else None,
-            "peak_source": tsrc,
-            "mma_flops_per_launch": mma,
-            "achieved_fp64_equivalent_tflops": achieved,
-            "fp64_peak_tflops": peak, "fp32_peak_tflops": fp32,
-            "achieved_note": "tensor FLOPs actually issued (digit-plane products, 55 per batch of 8 output blocks) "
-                             "over the tile stage's time; the stage is bound by the digit conversions on the CUDA "
-                             "cores (about half of the issue slots busy in ncu), not by the tensor pipe",
-        }
+    # executed tensor work: the bf16 digit-plane MMAs of one exchange
+    mma = atom.tc_work(symmetric=True)
+    tc_rate = mma / (off_ms * 1e-3) / 1e12
+    mp = measured_peaks()
+    if mp.get("bf16_tflops"):
+        tpeak, tsrc = float(mp["bf16_tflops"]), "MEASURED_PEAKS.json bf16_tflops (cuBLAS bf16 GEMM, burst)"
     else:
-        roofline = {"bound": "fp64", "kernel": "k_tiles", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                    "frac": achieved / peak if peak else None,
-                    "peak_source": "measured in this run: cuBLAS DGEMM 4096^3 (no FP64 figure in MEASURED_PEAKS.json)"}
+        tpeak = hg.tc_peak(2, 4096)["tflops"]
+        tsrc = "measured in this run: this library's tcgen05 bf16 MMA loop (hfg_tc_peak)"
+    roofline = {
+        "bound": "tensor", "kernel": "k_tiles_tc + k_diag_tc (the exchange tile stage)", "achieved": tc_rate,
+        "peak": tpeak, "unit": "TFLOP/s", "frac": tc_rate / tpeak if tpeak else None,
+        "peak_source": tsrc,
+        "mma_flops_per_launch": mma,
+        "achieved_fp64_equivalent_tflops": achieved,
+        "fp64_peak_tflops": peak, "fp32_peak_tflops": fp32,
+        "achieved_note": "tensor FLOPs actually issued (digit-plane products, 41 per batch of 8 output blocks, 42 in the "
+                         "plain form) over the tile stage's time; the stage is bound by the digit conversions on the CUDA "
+                         "cores (58 % of the issue slots busy in ncu), not by the tensor pipe",
+    }
     roofline.update({
         "flops_per_launch": kflops, "ms_per_launch": off_ms,
         "traffic": None,
@@ -997,22 +996,28 @@ def run_n2(args):
         "config": {"workload": N2_WORKLOAD if (args.n2_elements, args.n2_lmax) == (30, 12) else
                    f"reduced N2 case: {args.n2_elements} mu-elements, l<={args.n2_lmax} (profiling)", "nbf": nbf, "ndummy": d.ndummy, "parallelism": f"replicas x{ws}",
                    "inputs_vs_l2": "P is 8.8 GB > 129 MB L2: no flush needed"},
-        "form": ("split precision (FP32-pair contraction, FP64 recombination)" if split else "plain FP64")
+        "form": ("split precision (element pairs in float pairs, in-element tiles as digit planes on the tensor cores)"
+                 if split else "FP64 (element pairs on the FP64 pipe, in-element tiles as digit planes of FP64 tiles)")
                 + ", symmetric exchange mode",
         "kernel_ms": {"coulomb": j_ms, "exchange": k_ms},
         "plain_fp64": plain,
         "dft": dft,
         "energies_eh": {"coulomb": Ecoul, "exchange": Exx},
-        "roofline": ({"bound": "fp32", "kernel": "dk_tiles_split (whole exchange call)",
+        "roofline": ({"bound": "fp32", "kernel": "dk_share_off + dk_tc_x + dk_tc_gemm (whole exchange call)",
                       "achieved": achieved * 12.0, "peak": fp32_peak_tflops(torch), "unit": "TFLOP/s",
                       "frac": achieved * 12.0 / fp32_peak_tflops(torch),
                       "achieved_fp64_equivalent_tflops": achieved, "fp64_peak_tflops": peak,
                       "achieved_note": "FP32 rate = FP64-equivalent algorithmic FLOP rate x 12 FP32 instructions "
-                                       "per emulated multiply-add",
+                                       "per emulated multiply-add; the FLOPs are the unshared sums', one output block "
+                                       "at a time, of which the kernels execute a part (shared recoupling), the "
+                                       "in-element products on the tensor cores",
                       "flops_per_launch": kflops, "ms_per_launch": k_ms,
                       "peak_source": "measured in this run: cuBLAS SGEMM 8192^3 with TF32 off", "traffic": None}
                      if split else
-                     {"bound": "fp64", "kernel": "dk_tiles (whole exchange call)", "achieved": achieved,
+                     {"bound": "fp64", "kernel": "dk_share_off + dk_tc_x + dk_tc_gemm (whole exchange call)",
+                      "achieved": achieved,
+                      "achieved_note": "FLOPs of the unshared sums; the kernels execute a part of them, the in-element "
+                                       "products on the tensor cores",
                       "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
                       "flops_per_launch": kflops, "ms_per_launch": k_ms,
                       "peak_source": "measured in this run: cuBLAS DGEMM 4096^3", "traffic": None}),
@@ -1021,8 +1026,8 @@ def run_n2(args):
                 "d2h_bytes_per_step": 2 * 8 * nbf * nbf, "steps": ne,
                 "path": "hfg_diatomic_coulomb_host + hfg_diatomic_exchange_host (pinned host P, J, K)"},
         "clocks": clk.summary(),
-        "gpu_launches": args.steps * 11,  # J: contract, tiles, scatter; K: expand, norms, act,
-                                           # entry_act, compact, tiles, fixup, gather
+        "gpu_launches": args.steps * 14,  # J: contract, tiles, scatter; K: expand, norms, act, entry_act, compact,
+                                           # one pass at least of x, gemm, store; pairs, fixup, gather
     }
     print(json.dumps(out), flush=True)
     if dist is not None:

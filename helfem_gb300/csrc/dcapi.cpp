@@ -515,9 +515,20 @@ struct hfg_diatomic {
              bool itemwise = false) {
     check_device();
     const hfg::DiatomicHost& H = host;
-    if (split) ensure_split();
-    const bool tc64 = !split && exchange && use_tc64() && ensure_tc(false);
-    if (!split && exchange && !tc64) ensure_fp64();
+    // (first-call tables and scratch are made on the handle's own stream, also
+    // while the caller captures st)
+    struct Relaxed {
+      cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
+      Relaxed() { cudaThreadExchangeStreamCaptureMode(&m); }
+      ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&m); }
+    };
+    bool tc64 = false;
+    {
+      Relaxed relaxed;
+      if (split) ensure_split();
+      tc64 = !split && exchange && use_tc64() && ensure_tc(false);
+      if (!split && exchange && !tc64) ensure_fp64();
+    }
     if (!exchange) {  // J reads the pure density and writes the pure J directly
       ck(hfg::launch_diatomic_coulomb(dev, scr, P, F, st), "coulomb");
       mark_use(st);

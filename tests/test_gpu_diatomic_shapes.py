@@ -76,3 +76,29 @@ def test_diatomic_fp64_scales(nn):
     n = nelem * (nn - 1)  # functions of an m = 0 shell
     assert hit.any() and not hit[:n, :n][2 * (nn - 1):, 2 * (nn - 1):].any()
     assert np.allclose(k[~hit], ref[~hit], rtol=0, atol=1e-10 * np.abs(ref).max())
+
+
+def test_plain_exchange_under_capture():
+    """A handle's first plain exchange may be captured: what it makes on its
+    first call is made outside the capture, and the replay repeats the eager
+    result bit for bit (atomic form with its side stream too)."""
+    torch = torch_cuda()
+    lv, mv = hg.angular_basis(1, 1)
+    for make in (lambda: hg.Diatomic.from_grid(3, 1, 3.0, 3, [3, 2], Rmax=12.0, nnodes=10),
+                 lambda: hg.Atom(10, hg.get_grid(30.0, 6, 4, 2.0), lv, mv, nnodes=15)):
+        d = make()
+        rng = np.random.default_rng(3)
+        C = rng.standard_normal((d.nbf, 4))
+        P = to_dev(torch, C @ C.T)
+        K = torch.zeros_like(P)
+        st = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            d.exchange(P, K, stream=st, symmetric=True)
+        g.replay()
+        torch.cuda.synchronize()
+        K2 = torch.zeros_like(P)
+        d.exchange(P, K2, symmetric=True)
+        torch.cuda.synchronize()
+        assert bool((K2 != 0).any()) and torch.equal(K, K2)
