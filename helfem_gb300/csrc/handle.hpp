@@ -209,13 +209,15 @@ struct hfg_atom {
     std::vector<uint16_t> d((size_t)2 * NL * nel * ND * (TC_TPLANE / 2), 0);
     std::vector<int> ex((size_t)2 * nel * 16, 0), tx((size_t)2 * NL * nel, 0);
     auto off = [](int n, int k) { return ((n >> 3) * 256 + (k >> 3) * 128 + (n & 7) * 16 + (k & 7) * 2) / 2; };
-    auto half_bits = [](int v) {  // integer |v| <= 2048 as f16, exact
-      if (v == 0) return (uint16_t)0;
+    std::vector<uint16_t> half_bits(4097, 0);  // integers |v| <= 2048 as f16, exact
+    for (int v = -2048; v <= 2048; ++v) {
+      if (v == 0) continue;
       const int m = std::abs(v);
       int e = 0;
       while ((m >> (e + 1)) != 0) ++e;
-      return (uint16_t)((v < 0 ? 0x8000 : 0) | ((e + 15) << 10) | ((e <= 10 ? m << (10 - e) : m >> (e - 10)) & 0x3FF));
-    };
+      half_bits[v + 2048] =
+          (uint16_t)((v < 0 ? 0x8000 : 0) | ((e + 15) << 10) | ((e <= 10 ? m << (10 - e) : m >> (e - 10)) & 0x3FF));
+    }
     for (int kind = 0; kind < 2; ++kind)
       for (int e = 0; e < nel; ++e) {
         auto table = [&](int L) { return (kind == 0 ? rs : rb).data() + ((size_t)L * nel + e) * n2; };
@@ -240,16 +242,20 @@ struct hfg_atom {
           const double* M = table(L);
           const size_t blk = ((size_t)kind * NL + L) * nel + e;
           uint16_t* planes = d.data() + blk * ND * (TC_TPLANE / 2);
-          for (int n = 0; n < nn; ++n)
+          for (int n = 0; n < nn; ++n) {
+            const int sh = -row[n] - tx[blk];
+            const double sc = std::ldexp(1.0, sh);  // (exact unless it leaves the range)
             for (int k = 0; k < nn; ++k) {
-              double r = std::ldexp(M[n + (size_t)k * nn], -row[n] - tx[blk]);
+              const double m = M[n + (size_t)k * nn];
+              double r = std::abs(sh) < 1000 ? m * sc : std::ldexp(m, sh);
               for (int kd = 0; kd < ND; ++kd) {
                 r *= 1024.0;
-                const double dg = std::nearbyint(r);
-                r -= dg;
-                planes[(size_t)kd * (TC_TPLANE / 2) + off(n, k)] = half_bits((int)dg);
+                const long dg = std::lrint(r);
+                r -= (double)dg;
+                planes[(size_t)kd * (TC_TPLANE / 2) + off(n, k)] = half_bits[std::clamp(dg, -2048l, 2048l) + 2048];
               }
             }
+          }
         }
       }
     out.digits = reinterpret_cast<const unsigned char*>(dig.upload(d));
