@@ -5,6 +5,8 @@
 // AO index = iang*nrad + irad; matrices are column-major FP64 (nbf x nbf).
 #pragma once
 
+#include "side_stream.hpp"
+
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -215,11 +217,6 @@ cudaError_t launch_exchange_erfc(const DevAtom& A, const DevScratch& S, const do
 cudaError_t launch_mirror_blocks(double* P, int n, int bw, cudaStream_t st);
 cudaError_t launch_coulomb_split(const DevAtom& A, const DevScratch& S, const double* P, double* J,
                                 bool zero_output, cudaStream_t st, Profiler* prof = nullptr);
-// a second stream with a fork and a join event (owned by the caller)
-struct SideStream {
-  cudaStream_t s = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
-};
 // tc != nullptr: on the tensor cores (k_tc.cu), side: a second stream for the
 // diagonal elements or nullptr
 cudaError_t launch_exchange_fp64(const DevAtom& A, const DevScratch& S, const KUnits& U, const double* P,

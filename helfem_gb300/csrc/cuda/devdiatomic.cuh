@@ -7,6 +7,8 @@
 // Matrices are column-major FP64.
 #pragma once
 
+#include "side_stream.hpp"
+
 #include <cuda_runtime.h>
 
 namespace hfg {
@@ -178,7 +180,8 @@ cudaError_t launch_diatomic_coulomb(const DevDiatomic& D, const DevDiatomicScrat
                                     cudaStream_t st);
 // tc: the in-element tiles on the tensor cores, or nullptr for the FP64 kernels (T)
 cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDia64& T,
-                                     const DevDiaTC* tc, const double* Pd, double* Kd, bool symmetric, cudaStream_t st);
+                                     const DevDiaTC* tc, const double* Pd, double* Kd, bool symmetric, cudaStream_t st,
+                                     const SideStream& side);
 cudaError_t launch_dk_tc_table(const DevDiatomic& D, const DevDiaTC& T, unsigned char* tx, int* txexp, int* cexp,
                                cudaStream_t st);
 size_t dtc_gemm_smem(const DevDiatomic& D, bool f64);
@@ -189,6 +192,6 @@ cudaError_t launch_dk_tc_diag(const DevDiatomic& D, const DevDiatomicScratch& S,
 // output block at a time (bitwise the same K)
 cudaError_t launch_diatomic_exchange_split(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDiaTC& T,
                                            const double* Pd, double* Kd, bool symmetric, cudaStream_t st,
-                                           bool itemwise = false);
+                                           const SideStream& side, bool itemwise = false);
 
 }  // namespace hfg

@@ -422,39 +422,47 @@ cudaError_t launch_diatomic_coulomb(const DevDiatomic& D, const DevDiatomicScrat
   return cudaGetLastError();
 }
 
-cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDia64& T,
-                                     const DevDiaTC* tc, const double* Pd, double* Kd, bool symmetric,
-                                     cudaStream_t st) {
+// Screening, then the in-element tiles on the side stream beside the element
+// pairs: neither needs the other, and on small bases neither fills the GPU (H2
+// on 3 elements: 130 and 107 us of a K of 282; 244 side by side).
+template <class Diag>
+static cudaError_t exchange_stages(const DevDiatomic& D, const DevDiatomicScratch& S, const double* Pd, float2* pd2,
+                                   double* Kd, bool symmetric, cudaStream_t st, const SideStream& side, Diag&& diag) {
   const int nang2 = D.nang * D.nang;
   cudaError_t e = cudaMemsetAsync(Kd, 0, sizeof(double) * (size_t)D.nd * D.nd, st);
   if (e != cudaSuccess) return e;
-  dk_norms<<<dim3(nang2, DNORM_SPLIT), 256, 0, st>>>(D, Pd, S.bnorm, nullptr);
+  dk_norms<<<dim3(nang2, DNORM_SPLIT), 256, 0, st>>>(D, Pd, S.bnorm, pd2);
   dk_act<<<(nang2 + 255) / 256, 256, 0, st>>>(D, S);
   dk_entry_act<<<std::max(1, (D.nent + 127) / 128), 128, 0, st>>>(D, S);
   dk_compact<<<1, 1024, 0, st>>>(D, S, symmetric ? 1 : 0);
-  e = tc ? launch_dk_tc_diag(D, S, *tc, Pd, Kd, symmetric, false, st)
-         : launch_dk_share_diag(D, S, T, Pd, Kd, symmetric, st);
-  if (e == cudaSuccess) e = launch_dk_share_off(D, S, Pd, Kd, symmetric, false, st);
+  if ((e = cudaEventRecord(side.fork, st)) != cudaSuccess) return e;
+  if ((e = cudaStreamWaitEvent(side.s, side.fork, 0)) != cudaSuccess) return e;
+  e = diag(side.s);
+  const cudaError_t j = cudaEventRecord(side.join, side.s);
+  if (e == cudaSuccess) e = j;
+  if (e == cudaSuccess) e = launch_dk_share_off(D, S, Pd, Kd, symmetric, pd2 != nullptr, st);
+  const cudaError_t w = cudaStreamWaitEvent(st, side.join, 0);  // (joined whatever failed)
+  if (e == cudaSuccess) e = w;
   if (e != cudaSuccess) return e;
   dk_fixup<<<D.nel * D.nel, 256, 0, st>>>(D, S, Kd);
   return cudaGetLastError();
 }
 
+cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDia64& T,
+                                     const DevDiaTC* tc, const double* Pd, double* Kd, bool symmetric,
+                                     cudaStream_t st, const SideStream& side) {
+  return exchange_stages(D, S, Pd, nullptr, Kd, symmetric, st, side, [&](cudaStream_t s) {
+    return tc ? launch_dk_tc_diag(D, S, *tc, Pd, Kd, symmetric, false, s)
+              : launch_dk_share_diag(D, S, T, Pd, Kd, symmetric, s);
+  });
+}
+
 cudaError_t launch_diatomic_exchange_split(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDiaTC& T,
                                            const double* Pd, double* Kd, bool symmetric, cudaStream_t st,
-                                           bool itemwise) {
-  const int nang2 = D.nang * D.nang;
-  cudaError_t e = cudaMemsetAsync(Kd, 0, sizeof(double) * (size_t)D.nd * D.nd, st);
-  if (e != cudaSuccess) return e;
-  dk_norms<<<dim3(nang2, DNORM_SPLIT), 256, 0, st>>>(D, Pd, S.bnorm, S.pd2);
-  dk_act<<<(nang2 + 255) / 256, 256, 0, st>>>(D, S);
-  dk_entry_act<<<std::max(1, (D.nent + 127) / 128), 128, 0, st>>>(D, S);
-  dk_compact<<<1, 1024, 0, st>>>(D, S, symmetric ? 1 : 0);
-  e = launch_dk_tc_diag(D, S, T, nullptr, Kd, symmetric, itemwise, st);
-  if (e == cudaSuccess) e = launch_dk_share_off(D, S, Pd, Kd, symmetric, true, st);
-  if (e != cudaSuccess) return e;
-  dk_fixup<<<D.nel * D.nel, 256, 0, st>>>(D, S, Kd);
-  return cudaGetLastError();
+                                           const SideStream& side, bool itemwise) {
+  return exchange_stages(D, S, Pd, S.pd2, Kd, symmetric, st, side, [&](cudaStream_t s) {
+    return launch_dk_tc_diag(D, S, T, nullptr, Kd, symmetric, itemwise, s);
+  });
 }
 
 }  // namespace hfg

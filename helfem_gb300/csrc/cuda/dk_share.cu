@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(NN == 15 ? 256 : 320, 2) dk_share_off(DevDiato
 }
 
 // The off-diagonal items' parts summed in order and stored; grid (items' upper
-// bound), one CTA per item
+// bound, parts of their entries)
 __global__ void dk_share_sum(DevDiatomic D, DevDiatomicScratch S, double* __restrict__ Kd, int symmetric) {
   const int2* pairs = symmetric ? D.pairs_sym : D.pairs_all;
   const int nkg = S.counts[2], nitem = (symmetric ? D.npairs_sym : D.npairs_all) * nkg, nn = D.nn, n2 = nn * nn;
@@ -232,10 +232,10 @@ __global__ void dk_share_sum(DevDiatomic D, DevDiatomicScratch S, double* __rest
   const int kg = S.kg_list[it % nkg], k = kg / D.ngrp, g = kg % D.ngrp;
   const int* js = D.msh + D.grp_ptr[g];
   const int nj = D.grp_ptr[g + 1] - D.grp_ptr[g];
-  for (int x = threadIdx.x; x < nj * n2; x += blockDim.x) {
+  for (int x = blockIdx.y * blockDim.x + threadIdx.x; x < nj * n2; x += gridDim.y * blockDim.x) {
     const int jj = x / n2, t = x % n2, p = t % nn, q = t / nn;
     double s = 0.0;
-#pragma unroll 4
+#pragma unroll 8
     for (int lp = 0; lp < S.offparts; ++lp) s += S.offsum[(((size_t)lp * nitem + it) * D.gmax + jj) * n2 + t];
     share_store(D, S, Kd, pr.x, pr.y, js[jj] + k * D.nang, p, q, -s);
     if (symmetric) share_store(D, S, Kd, pr.y, pr.x, k + js[jj] * D.nang, q, p, -s);
@@ -463,7 +463,7 @@ cudaError_t launch_off(const DevDiatomic& D, const DevDiatomicScratch& S, const 
   const long items = (long)(symmetric ? D.npairs_sym : D.npairs_all) * D.nang * D.ngrp;
   const int grid = (int)std::min<long>(items * S.offparts, (long)sm_count() * std::max(per, 1));
   kern<<<grid, th, smem, st>>>(D, S, Pd, Kd, symmetric ? 1 : 0);
-  if (S.offparts > 1) dk_share_sum<<<(int)items, 256, 0, st>>>(D, S, Kd, symmetric ? 1 : 0);
+  if (S.offparts > 1) dk_share_sum<<<dim3((int)items, (D.gmax * n2 + 255) / 256), 256, 0, st>>>(D, S, Kd, symmetric ? 1 : 0);
   return cudaGetLastError();
 }
 

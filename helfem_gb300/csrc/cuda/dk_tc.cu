@@ -621,7 +621,7 @@ __global__ void dk_tc_store(DevDiatomic D, DevDiatomicScratch S, DevDiaTC T, int
     const int row = idx % 128, t = idx / 128, pos = tile * 128 + row;
     if (pos >= B.count) continue;
     double s = 0.0;
-#pragma unroll 4
+#pragma unroll 8
     for (int lp = 0; lp < T.lparts; ++lp) s += T.part[((((size_t)lp * T.cap + lu) * T.ntt) * TT + t) * 128 + row];
     const int jk = B.list[pos], j = jk % D.nang, k = jk / D.nang, p = t % D.nn, q = t / D.nn;
     share_store(D, S, Kd, e, e, jk, p, q, -s);
@@ -670,7 +670,7 @@ cudaError_t launch_dk_tc_diag(const DevDiatomic& D, const DevDiatomicScratch& S,
     xk<<<slots, th, xsm, st>>>(D, S, T, Pd, symmetric ? 1 : 0, itemwise ? 1 : 0, u0, nchunk);
     const int nu = std::min(T.cap, units - u0);
     gk<<<nu * T.ntt * T.lparts, 320, gsm, st>>>(D, S, T, symmetric ? 1 : 0, u0);
-    dk_tc_store<<<dim3(nu, 32), 256, 0, st>>>(D, S, T, symmetric ? 1 : 0, u0, Kd);
+    dk_tc_store<<<dim3(nu, 64), 256, 0, st>>>(D, S, T, symmetric ? 1 : 0, u0, Kd);
   }
   return cudaGetLastError();
 }

@@ -44,6 +44,10 @@ struct hfg_diatomic {
       if (own_stream) cudaStreamWaitEvent(own_stream, last_use, 0);
       cudaEventDestroy(last_use);
     }
+    // (its work is joined into the streams that last_use stands for)
+    if (k_side.s) cudaStreamDestroy(k_side.s);
+    if (k_side.fork) cudaEventDestroy(k_side.fork);
+    if (k_side.join) cudaEventDestroy(k_side.join);
   }
   void mark_use(cudaStream_t st) {
     if (last_use) cudaEventRecord(last_use, st);
@@ -419,6 +423,15 @@ struct hfg_diatomic {
     t64 = T;
   }
 
+  // second stream of the exchange (in-element tiles)
+  hfg::SideStream k_side{};
+  void ensure_side() {
+    if (k_side.s) return;
+    ck(cudaEventCreateWithFlags(&k_side.fork, cudaEventDisableTiming), "cudaEventCreate");
+    ck(cudaEventCreateWithFlags(&k_side.join, cudaEventDisableTiming), "cudaEventCreate");
+    ck(cudaStreamCreateWithFlags(&k_side.s, cudaStreamNonBlocking), "cudaStreamCreate");
+  }
+
   // split tables and the split density buffer, on the first split-precision call
   void ensure_split() {
     if (scr.pd2) return;
@@ -525,6 +538,7 @@ struct hfg_diatomic {
     bool tc64 = false;
     {
       Relaxed relaxed;
+      if (exchange) ensure_side();
       if (split) ensure_split();
       tc64 = !split && exchange && use_tc64() && ensure_tc(false);
       if (!split && exchange && !tc64) ensure_fp64();
@@ -537,10 +551,12 @@ struct hfg_diatomic {
     ck(hfg::launch_diatomic_expand(P, H.nbf, d_pure.as<int>(), s_Pd.as<double>(), H.ndummy, st), "expand");
     if (split)
       ck(hfg::launch_diatomic_exchange_split(dev, scr, tc, s_Pd.as<double>(), s_Fd.as<double>(), symmetric, st,
-                                             itemwise),
+                                             k_side, itemwise),
          "exchange (split)");
     else
-      ck(hfg::launch_diatomic_exchange(dev, scr, t64, tc64 ? &tc : nullptr, s_Pd.as<double>(), s_Fd.as<double>(), symmetric, st), "exchange");
+      ck(hfg::launch_diatomic_exchange(dev, scr, t64, tc64 ? &tc : nullptr, s_Pd.as<double>(), s_Fd.as<double>(),
+                                       symmetric, st, k_side),
+         "exchange");
     ck(hfg::launch_diatomic_gather(s_Fd.as<double>(), H.ndummy, d_pure.as<int>(), H.nbf, F, st), "gather");
     mark_use(st);
   }
