@@ -341,19 +341,29 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
           ck(cudaMemcpyAsync(dBatch.as<double>() + n2 * q, Fo_all + Lblk * s + blocks[grp.second[q]].off,
                              sizeof(double) * n2, cudaMemcpyDeviceToDevice, st),
              "gather blocks");
-        size_t wd = 0, wh = 0;
-        cs(cusolverDnXsyevBatched_bufferSize(hd.so, sparams, mode, CUBLAS_FILL_MODE_LOWER, n,
-                                             CUDA_R_64F, dBatch.p, n, CUDA_R_64F, dBatchW.p, CUDA_R_64F, &wd, &wh, nb),
-           "syevBatched buffer size");
-        if (wd > work_bytes) {
-          dWork.alloc(wd);
-          work_bytes = wd;
+        // two blocks of more than 256 rows are solved one by one: a batch of two
+        // costs more than twice one (Ar, whole solve: 559 rows 215 and 171 ms, 335
+        // rows 116 and 106, but 237 rows 75 and 78); three are faster batched (Kr,
+        // 279 rows: 144 and 160 ms)
+        const int chunk = nb == 2 && n > 256 ? 1 : nb;
+        for (int q0 = 0; q0 < nb; q0 += chunk) {
+          const int nq = std::min(chunk, nb - q0);
+          double* Aq = dBatch.as<double>() + n2 * q0;
+          double* wq = dBatchW.as<double>() + (size_t)n * q0;
+          size_t wd = 0, wh = 0;
+          cs(cusolverDnXsyevBatched_bufferSize(hd.so, sparams, mode, CUBLAS_FILL_MODE_LOWER, n, CUDA_R_64F, Aq, n,
+                                               CUDA_R_64F, wq, CUDA_R_64F, &wd, &wh, nq),
+             "syevBatched buffer size");
+          if (wd > work_bytes) {
+            dWork.alloc(wd);
+            work_bytes = wd;
+          }
+          if (hwork.size() < wh) hwork.resize(wh);
+          cs(cusolverDnXsyevBatched(hd.so, sparams, mode, CUBLAS_FILL_MODE_LOWER, n, CUDA_R_64F, Aq, n, CUDA_R_64F, wq,
+                                    CUDA_R_64F, dWork.p, wd, hwork.empty() ? nullptr : hwork.data(), wh,
+                                    dInfo.as<int>() + q0, nq),
+             "syevBatched");
         }
-        if (hwork.size() < wh) hwork.resize(wh);
-        cs(cusolverDnXsyevBatched(hd.so, sparams, mode, CUBLAS_FILL_MODE_LOWER, n, CUDA_R_64F,
-                                  dBatch.p, n, CUDA_R_64F, dBatchW.p, CUDA_R_64F, dWork.p, wd,
-                                  hwork.empty() ? nullptr : hwork.data(), wh, dInfo.as<int>(), nb),
-           "syevBatched");
         for (int k = 0; k < nblk; ++k) {
           const int r = rep[k];
           const auto it = std::find(grp.second.begin(), grp.second.end(), r);
