@@ -641,7 +641,7 @@ hfg_status hfg_atom_autotune(hfg_atom* a, int flags, int* best_nsplit, double* b
     int bestn = 0;
     // the tensor-core forms: groups of 8 output blocks per element-pair
     // unit; otherwise output-block ranges per element pair
-    const bool tcform = ((flags & HFG_EXCHANGE_SPLIT) ? a->tc_for(false) : a->tc64_for(false)) != nullptr;
+    const bool tcform = a->tc_ok && ((flags & HFG_EXCHANGE_SPLIT) ? a->tc_for(false) : a->tc64_for(false)) != nullptr;
     const std::vector<int> cand = tcform ? std::vector<int>{0, 1, 2, 3, 4, 6, a->tc.ngroups}
                                          : std::vector<int>{0, 1, 2, 4, 8, 16};
     for (int ns : cand) {

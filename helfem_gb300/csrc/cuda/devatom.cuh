@@ -114,7 +114,7 @@ struct DevTC {
   // [L][e][row tile][K step][digit][128 x 16] and per-row exponents
   const unsigned char* tk_digits = nullptr;
   const int* tk_rowexp = nullptr;         // [L][e][row tile][128]
-  int dmtiles = 0, dksteps = 0;
+  int dmtiles = 0, dksteps = 0, dstages = 0;
   int dgroups = 0;                        // groups of 16 output blocks (at most), set per launch
 };
 

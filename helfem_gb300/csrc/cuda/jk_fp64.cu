@@ -920,11 +920,13 @@ cudaError_t launch_exchange_erfc(const DevAtom& A, const DevScratch& S, const do
   return cudaGetLastError();
 }
 
-// every element pair on the tensor cores, the off-diagonal tiles and the
-// diagonal ones through the exchange-ordered tensor (P: FP64 form); blocks
-// without an active entry are zeroed
+// The diagonal elements on the tensor cores, through the exchange-ordered
+// tensor, and the element pairs by pairs(st): on the tensor cores too, or, for
+// elements they do not take (17 nodes), by the FP64 or float-pair kernel. Blocks
+// without an active entry are zeroed. P: FP64 form.
+template <class Pairs>
 static cudaError_t launch_tiles_tc(const DevAtom& A, const DevScratch& S, const DevTC& tc, bool symmetric,
-                                   const double* P, double* K, cudaStream_t st, const SideStream* side) {
+                                   const double* P, double* K, cudaStream_t st, const SideStream* side, Pairs&& pairs) {
   const int nang2 = A.nang * A.nang;
   cudaError_t e = cudaSuccess;
   if (side && side->s) {
@@ -932,13 +934,15 @@ static cudaError_t launch_tiles_tc(const DevAtom& A, const DevScratch& S, const 
     // beside the issue-bound off-diagonal tiles, joined before the fix-up
     e = cudaEventRecord(side->fork, st);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(side->s, side->fork, 0);
+    // (the FP64 and float-pair kernels first: a diagonal CTA takes an SM whole)
+    if (e == cudaSuccess && !tc.digits) e = pairs();
     if (e == cudaSuccess) e = launch_k_diag_tc(A, S, tc, symmetric, P, K, side->s);
     k_zero_inactive<<<dim3(nang2, 8), 256, 0, side->s>>>(A, S, K, symmetric ? 1 : 0);
     if (e == cudaSuccess) e = cudaEventRecord(side->join, side->s);
-    if (e == cudaSuccess) e = launch_k_tiles_tc(A, S, tc, symmetric, P, K, st);
+    if (e == cudaSuccess && tc.digits) e = pairs();
     if (e == cudaSuccess) e = cudaStreamWaitEvent(st, side->join, 0);
   } else {
-    e = launch_k_tiles_tc(A, S, tc, symmetric, P, K, st);
+    e = pairs();
     if (e == cudaSuccess) e = launch_k_diag_tc(A, S, tc, symmetric, P, K, st);
     k_zero_inactive<<<dim3(nang2, 8), 256, 0, st>>>(A, S, K, symmetric ? 1 : 0);
   }
@@ -957,7 +961,17 @@ cudaError_t launch_exchange_fp64(const DevAtom& A, const DevScratch& S, const KU
     }
     {
       Mark m(prof, KC_K_TILES, st);
-      const cudaError_t e = launch_tiles_tc(A, S, *tc, symmetric, P, K, st, side);
+      const cudaError_t e = launch_tiles_tc(A, S, *tc, symmetric, P, K, st, side, [&]() -> cudaError_t {
+        if (tc->digits) return launch_k_tiles_tc(A, S, *tc, symmetric, P, K, st);
+        const size_t smem = sizeof(double) * (2 * n2 + 2 * A.NL * n2) + nang2;
+        const int nunits = symmetric ? U.n_off_sym : U.n_off_all;
+        const cudaError_t l = smem_limit(k_tiles, smem);
+        if (l != cudaSuccess) return l;
+        if (nunits > 0)
+          k_tiles<<<nunits, th, smem, st>>>(A, S, symmetric ? U.sym : U.all, U.diag_jk_src(symmetric), symmetric ? 1 : 0, P,
+                                            K);
+        return cudaGetLastError();
+      });
       if (e != cudaSuccess) return e;
     }
     {
@@ -997,20 +1011,23 @@ cudaError_t launch_exchange_split(const DevAtom& A, const DevScratch& S, const K
   {
     Mark m(prof, KC_K_TILES, st);
     const size_t smem = sizeof(float2) * (2 * n2 + 2 * A.NL * n2) + sizeof(double) * n2 + nang2;
-    int nunits = symmetric ? U.n_sym : U.n_all;
     const int4* units = symmetric ? U.sym : U.all;
-    if (tc) {
-      const cudaError_t e = launch_tiles_tc(A, S, *tc, symmetric, nullptr, K, st, side);
-      if (e != cudaSuccess) return e;
-      nunits = 0;
-    }
     auto kern = (A.nn == 15) ? k_tiles_split<15> : k_tiles_split<0>;
-    if (nunits > 0) {
-      const cudaError_t e = smem_limit(kern, smem);
-      if (e != cudaSuccess) return e;
-    }
-    if (nunits > 0)
-      kern<<<nunits, th, smem, st>>>(A, S, units, U.diag_jk_src(symmetric), symmetric ? 1 : 0, K);
+    auto pairs = [&](int nunits) -> cudaError_t {
+      const cudaError_t l = smem_limit(kern, smem);
+      if (l != cudaSuccess) return l;
+      if (nunits > 0)
+        kern<<<nunits, th, smem, st>>>(A, S, units, U.diag_jk_src(symmetric), symmetric ? 1 : 0, K);
+      return cudaGetLastError();
+    };
+    const cudaError_t e =
+        tc ? launch_tiles_tc(A, S, *tc, symmetric, nullptr, K, st, side,
+                             [&]() {
+                               return tc->digits ? launch_k_tiles_tc(A, S, *tc, symmetric, nullptr, K, st)
+                                                 : pairs(symmetric ? U.n_off_sym : U.n_off_all);
+                             })
+           : pairs(symmetric ? U.n_sym : U.n_all);
+    if (e != cudaSuccess) return e;
   }
   {
     Mark m(prof, KC_K_FIXUP, st);

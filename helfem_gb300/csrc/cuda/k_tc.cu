@@ -891,14 +891,15 @@ __global__ void tc_tk_digits_kernel(const double* __restrict__ tk, int NL, int n
   }
 }
 
-constexpr int DST = 4;                   // stages of the table stream
+constexpr int DST = 4;                   // stages of the table stream (at most)
 constexpr int DW = 8;                    // working warps
 constexpr int DTHREADS = 32 * (DW + 2);  // a copying and an issuing one
 
 // warps 0-7: recouple and digitise the density vectors of one multipole while
 // the products of the one before run, then read those back; warp 8 streams the
 // tables' digits, warp 9 issues
-template <bool F64>
+// NC: chunks of eight density entries per thread (2: up to 16 nodes, 3: 17)
+template <bool F64, int NC>
 __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S, DevTC T, int symmetric,
                                                          const double* __restrict__ P, double* __restrict__ K) {
   using Val = std::conditional_t<F64, double, float2>;
@@ -907,7 +908,7 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
   const Val* src;
   if constexpr (F64) src = P; else src = S.p2;
   const int nn = A.nn, n2 = nn * nn, NL = A.NL, nang2 = A.nang * A.nang;
-  const int ksteps = T.dksteps, mtiles = T.dmtiles;
+  const int ksteps = T.dksteps, mtiles = T.dmtiles, nst = T.dstages;
   // unit = (element, row tile, group of 16 active output blocks); the list is
   // made by the density pass (j <= k only in symmetric mode)
   const int count = symmetric ? S.ocount[1] : S.ocount[0];
@@ -916,8 +917,8 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
   const int g = blockIdx.x % T.dgroups, mt = (blockIdx.x / T.dgroups) % mtiles, a = blockIdx.x / (T.dgroups * mtiles);
   if (g >= ngr) return;  // uniform over the CTA
   extern __shared__ __align__(1024) unsigned char smraw[];
-  unsigned char* Abuf = smraw;                  // DST x ND planes of 128 x 16
-  unsigned char* Bx = Abuf + DST * ND * APLANE;  // 2 x ksteps x ND planes of 16 x 16
+  unsigned char* Abuf = smraw;                  // nst x ND planes of 128 x 16
+  unsigned char* Bx = Abuf + nst * ND * APLANE;  // 2 x ksteps x ND planes of 16 x 16
   const size_t bsize = (size_t)ksteps * ND * TPLANE;
   int* exs = reinterpret_cast<int*>(Bx + 2 * bsize);  // [4][16] slot exponents (bits) of four multipoles
   int* sact = exs + 4 * DSLOT;                        // [NL][16]
@@ -998,8 +999,8 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
         const unsigned char* Ag =
             T.tk_digits + (((size_t)actL[n] * A.nel + a) * mtiles + mt) * ksteps * ND * APLANE;
         for (int ks = 0; ks < ksteps; ++ks, ++it) {
-          const int s = it % DST;
-          if (it >= DST && !tc::mbar_wait(&empty[s], (uint32_t)((it / DST - 1) & 1), kWait)) {
+          const int s = it % nst;
+          if (it >= nst && !tc::mbar_wait(&empty[s], (uint32_t)((it / nst - 1) & 1), kWait)) {
             ok = false;
             break;
           }
@@ -1010,7 +1011,7 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
       if (!ok) {
         atomicExch(fail, 1);
         // the copies in flight must land before the CTA leaves
-        for (int i = max(0, it - DST); i < it; ++i) tc::mbar_wait(&full[i % DST], (uint32_t)((i / DST) & 1), kWait);
+        for (int i = max(0, it - nst); i < it; ++i) tc::mbar_wait(&full[i % nst], (uint32_t)((i / nst) & 1), kWait);
       }
     }
   } else if (warp == DW + 1) {
@@ -1024,8 +1025,8 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
         tc::fence_after_sync();
         const uint64_t dB = tc::smem_desc(tc::smem_u32(Bx + bf * bsize));
         for (int ks = 0; ks < ksteps; ++ks, ++it) {
-          const int s = it % DST;
-          if (!(ok = tc::mbar_wait(&full[s], (uint32_t)((it / DST) & 1), kWait))) break;
+          const int s = it % nst;
+          if (!(ok = tc::mbar_wait(&full[s], (uint32_t)((it / nst) & 1), kWait))) break;
           tc::fence_after_sync();
           const uint64_t dA = tc::smem_desc(tc::smem_u32(Abuf + s * ND * APLANE));
 #pragma unroll
@@ -1046,9 +1047,9 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
         const int L = actL[n];
         int* ex = exs + (n & 3) * DSLOT;
         // ---- recouple the 16 density vectors and take each slot's exponent ----
-        Sum xs[2][8];
+        Sum xs[NC][8];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < NC; ++c) {
           const int ch = t + c * 256;
 #pragma unroll
           for (int j = 0; j < 8; ++j) xs[c][j] = {};
@@ -1108,7 +1109,7 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
         // read back, its products are over ----
         unsigned char* Bn = Bx + (n & 1) * bsize;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < NC; ++c) {
           const int ch = t + c * 256;
           if (ch >= nchunk) continue;
           const int s = ch / (2 * ksteps), kk = ch % (2 * ksteps), ks = kk >> 1, h = kk & 1;
@@ -1189,8 +1190,8 @@ size_t tc_smem_bytes(int NL, int nang, bool f64) {
          (size_t)nang * nang + 16;
 }
 
-size_t tc_diag_smem_bytes(int NL, int ksteps, int nang) {
-  return (size_t)DST * ND * APLANE + (size_t)2 * ksteps * ND * TPLANE +
+size_t tc_diag_smem_bytes(int NL, int ksteps, int nang, int stages) {
+  return (size_t)stages * ND * APLANE + (size_t)2 * ksteps * ND * TPLANE +
          sizeof(int) * (4 * DSLOT + NL * DSLOT * 2 + DSLOT + 2 + NL + 1) + 8 * (2 * DST + 4) + 8 + (size_t)nang * nang + 64;
 }
 
@@ -1222,8 +1223,16 @@ cudaError_t launch_k_diag_tc(const DevAtom& A, const DevScratch& S, const DevTC&
   const int nblk = symmetric ? A.nang * (A.nang + 1) / 2 : A.nang * A.nang;
   Td.dgroups = (nblk + DSLOT - 1) / DSLOT;
   const int n = A.nel * T.dmtiles * Td.dgroups;
-  const size_t smem = tc_diag_smem_bytes(A.NL, T.dksteps, A.nang);
-  auto kern = P ? k_diag_tc<true> : k_diag_tc<false>;
+  // as many stages as fit (four up to 16 nodes, three for 17)
+  int dev = 0, most = 0;
+  cudaError_t e0 = cudaGetDevice(&dev);
+  if (e0 == cudaSuccess) e0 = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e0 != cudaSuccess) return e0;
+  Td.dstages = DST;
+  while (Td.dstages > 2 && tc_diag_smem_bytes(A.NL, T.dksteps, A.nang, Td.dstages) > (size_t)most) --Td.dstages;
+  const size_t smem = tc_diag_smem_bytes(A.NL, T.dksteps, A.nang, Td.dstages);
+  const bool wide = DSLOT * 2 * T.dksteps > 512;
+  auto kern = P ? (wide ? k_diag_tc<true, 3> : k_diag_tc<true, 2>) : (wide ? k_diag_tc<false, 3> : k_diag_tc<false, 2>);
   const cudaError_t e = smem_limit(kern, smem);
   if (e != cudaSuccess) return e;
   kern<<<n, DTHREADS, smem, st>>>(A, S, Td, symmetric ? 1 : 0, P, K);

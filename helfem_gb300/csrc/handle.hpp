@@ -167,6 +167,7 @@ struct hfg_atom {
   DBuf t_tkd, t_tke, ty_tkd, ty_tke;
   hfg::DevTC tc{}, tc_rs{};
   bool tc_ok = false;
+  bool tc_diag_only = false;  // 17 nodes: tc without the element pairs' tables
   // bf16 MMA FLOPs one tensor-core exchange issues with every entry active
   // (index 0: symmetric mode, 1: general)
   double tc_mma_flops[2] = {0.0, 0.0};
@@ -174,7 +175,7 @@ struct hfg_atom {
   // everywhere (HFG_SPLIT_FORM=pairs, which keeps the FP64 form on its own
   // kernel too)
   const hfg::DevTC* tc_for(bool screened) const {
-    if (!tc_ok) return nullptr;
+    if (!tc_ok && !(tc_diag_only && !screened)) return nullptr;
     static const bool pairs = [] {
       const char* v = std::getenv("HFG_SPLIT_FORM");
       return v && std::string(v) == "pairs";
@@ -341,7 +342,21 @@ struct hfg_atom {
     }
     dev.jk_order = d_order.upload(info);
     // (a block's terms are held two per lane of a warp; the float-pair form otherwise)
-    if (H.rad.nn > 16 || NL > 8 || nel < 2 || !one || dev.max_terms_per_jk > 64) return;
+    if (NL > 8 || nel < 2 || !one || dev.max_terms_per_jk > 64) return;
+    if (H.rad.nn > 16) {
+      // element pairs take 16 local rows; the diagonal elements, half of the work
+      // of 17 nodes and a chain of 289 terms each, any number whose digits fit a
+      // block's shared memory (l <= 1, 10 elements, us: split 176 and 69, plain 245
+      // and 72; l <= 3, 12 elements, dense, plain 6865 and 4690)
+      if (H.rad.nn > 17) return;
+      side_stream();
+      t_err.alloc(sizeof(int));
+      ck(cudaMemsetAsync(t_err.p, 0, sizeof(int), own_stream), "memset");
+      tc.err = t_err.as<int>();
+      tc_tk_tables(dev.tk, t_tkd, t_tke, tc);
+      tc_diag_only = true;
+      return;
+    }
     tc.ngroups = (nang2 + 7) / 8;
     // (group of n blocks, L) batches with at least one entry
     auto batches = [&](const std::vector<int>& blocks, int n) {
@@ -375,7 +390,7 @@ struct hfg_atom {
   // a completion wait inside the tensor-core kernel ran out (checked by the
   // host-pointer entry points after their synchronisation)
   void tc_check() {
-    if (!tc_ok) return;
+    if (!tc.err) return;
     int e = 0;
     ck(cudaMemcpy(&e, tc.err, sizeof(int), cudaMemcpyDeviceToHost), "D2H");
     if (e) throw std::runtime_error("tensor-core exchange: an MMA completion wait ran out");
@@ -776,7 +791,9 @@ struct hfg_atom {
     auto make = [&](bool sym, std::vector<int>& dj, int& noff) {
       std::vector<int4> u;
       const long npairs = sym ? (long)nel * (nel - 1) / 2 : (long)nel * (nel - 1);
-      int nsplit = (int)std::min<long>(std::max<long>(1, (2432 + npairs - 1) / std::max<long>(npairs, 1)), 8);
+      // (no diagonal units to fill the tail where those elements are on the tensor cores)
+      const long most = host.rad.nn > 16 ? 32 : 8;
+      int nsplit = (int)std::min<long>(std::max<long>(1, (2432 + npairs - 1) / std::max<long>(npairs, 1)), most);
       if (nsplit_fixed > 0) nsplit = nsplit_fixed;
       nsplit = std::min(nsplit, nang2);
       const std::vector<int> cut = ranges(nsplit);
