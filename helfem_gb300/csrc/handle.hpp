@@ -186,17 +186,18 @@ struct hfg_atom {
   // The FP64 exchange on the tensor cores, or nullptr for the FP64 kernel
   // (k_tiles). The line lies where the FP64 pipe's work per digit product (nn^3
   // and, in the elements, nn^4 per entry) outweighs the digit work, which hardly
-  // depends on nn: from 10 nodes on, for a single shell, whose batches are seven
-  // eighths empty, only for few long elements. Measured, FP64 kernel against this
-  // form, us: l <= 1, 20 elements of 9 nodes 63 and 59 (m-diagonal density), 95
-  // and 98 (general mode), of 10 nodes 79 and 62, 130 and 101; l <= 1, m = 0, 20
-  // elements of 9 nodes 48 and 53, of 10 nodes 57 and 56; l <= 3, 20 elements of
-  // 8 nodes 255 and 266, dense 1016 and 1517; l = 0, 6 elements of 15 nodes 44
-  // and 38, 20 elements 46 and 50; Kr (l <= 2, 40 elements of 15 nodes, dense)
-  // 4520 and 1004.
+  // depends on nn: from 10 nodes on; for one shell, whose batches are seven
+  // eighths empty, only for few long elements, for two not for many short ones.
+  // Measured, FP64 kernel against this form, us: l <= 1, 20 elements of 9 nodes
+  // 63 and 59 (m-diagonal density), 95 and 98 (general mode), of 10 nodes 79 and
+  // 62, 130 and 101; l <= 3, 20 elements of 8 nodes 255 and 266, dense 1016 and
+  // 1517; two shells, 20 elements of 9 nodes 48 and 53, of 10 nodes 57 and 56, 60
+  // elements of 10 nodes 125 and 152, of 13 nodes 274 and 185; l = 0, 6 elements
+  // of 15 nodes 44 and 38, 20 elements 46 and 50; Kr (l <= 2, 40 elements of 15
+  // nodes, dense) 4520 and 1004.
   const hfg::DevTC* tc64_for(bool screened) const {
-    const int nn = host.rad.nn;
-    const bool on = host.nang >= 2 ? nn >= 10 : nn >= 15 && host.rad.nel <= 10;
+    const int nn = host.rad.nn, nang = host.nang, nel = host.rad.nel;
+    const bool on = nang >= 3 ? nn >= 10 : nang == 2 ? nn >= (nel <= 24 ? 10 : 12) : nn >= 15 && nel <= 10;
     return on ? tc_for(screened) : nullptr;
   }
   // digits of the radial tables (kind 0 r_small, 1 r_big; per (L, e) a

@@ -72,6 +72,7 @@ CASES64 = [
     (10, 1, 1, 16, 12),
     (6, 1, 0, 3, 10),
     (6, 1, 0, 3, 9),
+    (6, 1, 0, 25, 10),
     (36, 2, 2, 11, 9),
     (10, 0, 0, 10, 15),
     (10, 0, 0, 11, 15),
