@@ -20,10 +20,11 @@
 // FP64 form (F64): the tiles are recoupled in FP64 and cut into seven digits by
 // shifts of their significands (59 bits below the largest entry), the level
 // sums (integers) added up in FP64: the error against the exact K is that of the
-// FP64 kernels (H2 6.2e-15 and 6.4e-15, CO 1.005e-14 and 1.010e-14 of |K|). A
-// tile with a value that is not finite gives NaN in its rows. Whole K, FP64
-// kernels for these tiles and this form: H2 on 3 elements, l <= 4 0.55 and 0.29
+// FP64 kernels (H2 6.2e-15 and 6.4e-15, CO 1.005e-14 and 1.010e-14 of |K|). Whole
+// K, FP64 kernels for these tiles and this form: H2 on 3 elements, l <= 4 0.55 and 0.29
 // ms; N2 on 9 elements, l <= 10, m <= 3 132 and 87 ms.
+//
+// In both forms a tile with a value that is not finite gives NaN in its rows.
 //
 // Two passes: dk_tc_x recouples each (element, output block, multipole) once
 // (sharing the sums over l between the output rows of one k) and writes its
@@ -413,6 +414,7 @@ __global__ void __launch_bounds__(NN == 15 ? 256 : 320, 2) dk_tc_x(DevDiatomic D
           } else {
             E = max((int)max(s_eb[jj], 1u) - 126, -100);
             const float s27 = exp2i(27 - E);
+            if (s_eb[jj] == 0xFFu) E = kBadExp;
 #pragma unroll
             for (int j = 0; j < 8; j += 2) {
               float d0[XD], d1[XD];
@@ -575,9 +577,10 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
             float lv[TD];
 #pragma unroll
             for (int d = 0; d < TD; ++d) lv[d] = v[d][j];
-            if constexpr (F64) {
-              acc[8 * g + j] += E == kBadExp ? __longlong_as_double(0x7ff8000000000000ll)
-                                             : levels512_f64(lv, te[8 * g + j] + E);
+            if (E == kBadExp) {
+              acc[8 * g + j] = __longlong_as_double(0x7ff8000000000000ll);
+            } else if constexpr (F64) {
+              acc[8 * g + j] += levels512_f64(lv, te[8 * g + j] + E);
             } else {
               float z0, z1, z2;
               levels512(lv, z0, z1, z2);
