@@ -208,12 +208,13 @@ __device__ __forceinline__ void digits_of(const ffv (&x)[8], int E, uint32_t (&p
 __device__ __forceinline__ int tile_exponent(unsigned eb) { return max((int)max(eb, 1u) - 126, -100); }
 
 // exact float -> double through the bit pattern (no FP64-pipe conversion);
-// zero and subnormal floats map to zero
+// zero and subnormal floats map to zero, infinities and NaN to themselves
 __device__ __forceinline__ double f2d_bits(float f) {
   const uint32_t bits = __float_as_uint(f);
   const uint32_t e = (bits >> 23) & 0xFFu;
   if (e == 0) return 0.0;
-  const unsigned long long r = ((unsigned long long)(bits >> 31) << 63) | ((unsigned long long)(e + 896u) << 52) |
+  const uint32_t e64 = e == 0xFFu ? 0x7FFu : e + 896u;
+  const unsigned long long r = ((unsigned long long)(bits >> 31) << 63) | ((unsigned long long)e64 << 52) |
                                ((unsigned long long)(bits & 0x7FFFFFu) << 29);
   return __longlong_as_double((long long)r);
 }
@@ -605,14 +606,15 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
           v[r] = tL[r] < 0 ? 0.f : __uint_as_float(bd[r]) * (fabsf(tc2[r].x) * 1.000001f * exp2i(m.sL[tL[r]] - s_hi));
           mx = max(mx, __float_as_uint(v[r]));
         }
-        e0 = max((int)(__reduce_max_sync(0xffffffffu, mx) >> 23) - 126, -96);
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        e0 = max((int)(mx >> 23) - 126, -96);
 #pragma unroll
         for (int r = 0; r < 2; ++r) su[r] = __float2uint_ru(v[r] * exp2i(24 - e0));
       }
       for (int L = 0; L < NL; ++L)
         top = max(top, __reduce_add_sync(0xffffffffu, (tL[0] == L ? su[0] : 0u) + (tL[1] == L ? su[1] : 0u)));
       E = max(s_hi + (F64 ? -900 : -96), s_hi + e0 + 8 - __clz(top));
-      if (F64 && mx >= 0x7FF00000u) E = kBadExp;
+      if (mx >= (F64 ? 0x7FF00000u : 0x7F800000u)) E = kBadExp;  // a value that is not finite
       if (lane == 0) {
         m.ex[g & 3][warp] = E;
         m.mask[g & 3][warp] = mask;
@@ -728,9 +730,10 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
 #pragma unroll
           for (int d = 0; d < PD; ++d) lv[d] = v[d][j];
           if constexpr (F64)
-            y[j] = E2 == kBadExp ? __longlong_as_double(0x7ff8000000000000ll) : -levels_to_f64(lv, ea + m.beta[h + j] + 2);
+            y[j] = -levels_to_f64(lv, ea + m.beta[h + j] + 2);
           else
             y[j] = -levels_to_d(lv, (max(ea + m.beta[h + j], -800) + 896) << 20);
+          if (E2 == kBadExp) y[j] = __longlong_as_double(0x7ff8000000000000ll);
           if (symmetric) *stage(oi, h + j) = y[j];
         }
         if (jk >= 0) store_rows(A, S, K, a, b, jk & 0xFFFF, jk >> 16, oi, h, y);
