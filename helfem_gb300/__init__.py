@@ -60,6 +60,7 @@ _SIGS = {
     "hfg_tc_selftest": ([ctypes.POINTER(ctypes.c_float), ctypes.POINTER(ctypes.c_float),
                          ctypes.POINTER(ctypes.c_float), ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                          ctypes.c_int], ctypes.c_int),
+    "hfg_atom_tc_wait_limit": ([_P, ctypes.c_uint], ctypes.c_int),
     "hfg_tc_peak": ([ctypes.c_int, ctypes.c_int, _D, _D], ctypes.c_int),
     "hfg_atom_tc_work": ([_P, ctypes.c_int, _D], ctypes.c_int),
     "hfg_atom_get_dims": ([_P, ctypes.POINTER(_Dims)], ctypes.c_int),
@@ -365,6 +366,10 @@ class Atom:
             _check(_lib.hfg_exchange_ex(self._h, _ptr(P), _ptr(K), flags, _stream(stream)))
         else:
             _check(_lib.hfg_exchange(self._h, _ptr(P), _ptr(K), _stream(stream)))
+
+    def tc_wait_limit(self, polls: int):
+        """Polls after which a completion wait of the tensor-core exchange gives up (K is NaN then)."""
+        _check(_lib.hfg_atom_tc_wait_limit(self._h, polls))
 
     def tc_work(self, symmetric: bool = True) -> float:
         """bf16 MMA FLOPs of one split-precision exchange (all entries active)."""

@@ -380,6 +380,13 @@ hfg_status hfg_tc_selftest(const float* A, const float* B, float* D, int N, int 
   });
 }
 
+hfg_status hfg_atom_tc_wait_limit(hfg_atom* a, unsigned polls) {
+  return guard([&] {
+    need(a != nullptr, "hfg_atom_tc_wait_limit: null argument");
+    a->tc_wait_limit(polls);
+  });
+}
+
 hfg_status hfg_tc_peak(int ctas_per_sm, int iters, double* tflops, double* ms) {
   return guard([&] {
     need(tflops && ms && ctas_per_sm >= 1 && ctas_per_sm <= 2 && iters >= 1, "hfg_tc_peak: bad arguments");

@@ -100,6 +100,7 @@ __host__ __device__ inline int gfun(const DevAtom& A, int e, int p) { return e *
 // work units (a, b, range of groups).
 #define TC_NDIGITS 6
 #define TC_TPLANE 512
+#define TC_WAIT (1u << 17)  // polls of a completion wait before it gives up
 struct DevTC {
   const unsigned char* digits = nullptr;  // [kind (0 r_small, 1 r_big)][L][e][TC_NDIGITS][TC_TPLANE]
   const int* texp = nullptr;              // [kind][L][e] table exponent
@@ -110,6 +111,7 @@ struct DevTC {
   const int4* units_all = nullptr;        // (a, b, first group, end group), a != b
   int n_all = 0;
   int* err = nullptr;                     // set when a completion wait ran out
+  unsigned wait = TC_WAIT;
   // diagonal element tiles: the exchange-ordered tensor as digit planes
   // [L][e][row tile][K step][digit][128 x 16] and per-row exponents
   const unsigned char* tk_digits = nullptr;

@@ -403,7 +403,9 @@ __device__ __forceinline__ void store_rows(const DevAtom& A, const DevScratch& S
 
 constexpr int PW = 8;                 // working warps
 constexpr int PTHREADS = 32 * PW;
-constexpr uint32_t kWait = 1u << 17;  // limit of every wait
+constexpr uint32_t kWait = TC_WAIT;  // limit of the waits of a CTA that gives up
+constexpr int kNoFail = 0x7FFFFFFF;
+constexpr int kGaveUp = 1 << 24;       // a warp's mark in the count of arrivals
 
 // working warps q and q + 4 (named barriers 1-4)
 __device__ __forceinline__ void pair_sync(int q) {
@@ -420,12 +422,28 @@ struct PairMeta {
   // per group (four in flight), slot: exponent of the scaled density tiles,
   // multipoles present (bits), output block or -1
   int ex[4][8], mask[4][8], jk[4][8];  // jk: j | k << 16
-  int fail;
+  int fail;               // the first batch whose wait ran out, or kNoFail
   uint32_t tslot;
-  int arrived;            // warps past their part of a batch, all batches
+  int arrived;            // warps past their part of a batch, all batches (and kGaveUp)
   uint64_t done;          // a batch's second and the next one's first product
 };
 }  // namespace
+
+// NaN in every result of a unit whose CTA gave up, the transposed partners' too
+// (out of line: inside k_tiles_tc it cost 1 % of Kr's K)
+__device__ __noinline__ void mark_unit(const DevAtom& A, const DevScratch& S, const int4* __restrict__ units,
+                                       int symmetric, double* K) {
+  const int4 u = units[blockIdx.x];
+  const int nn = A.nn, end = min(8 * u.w, S.ocount[0]);
+  for (int x = 8 * u.z + (int)(threadIdx.x >> 5); x < end; x += PW) {
+    const int jk = S.olist[x], kj = jk / A.nang + jk % A.nang * A.nang;
+    for (int i = threadIdx.x & 31; i < nn * nn; i += 32) {
+      const double bad = __longlong_as_double(0x7ff8000000000000ll);
+      k_store_tile(A, S, K, u.x, u.y, jk, i % nn, i / nn, bad);
+      if (symmetric) k_store_tile(A, S, K, u.y, u.x, kj, i / nn, i % nn, bad);
+    }
+  }
+}
 
 // Each of 8 warps, per batch: recouple and digitise slot w's density tile of
 // the next batch into the other stage of the first operand, then read this
@@ -475,7 +493,7 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
     if (t < NL) m.sL[t] = T.texp[((size_t)kl * NL + t) * A.nel + a] + T.texp[((size_t)kr * NL + t) * A.nel + b];
     for (int idx = t; idx < nang2; idx += blockDim.x) act[idx] = S.act[idx];
     if (t == 0) {
-      m.fail = 0;
+      m.fail = kNoFail;
       m.arrived = 0;
       tc::mbar_init(&m.done, 1);
     }
@@ -680,7 +698,8 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
                      : "=r"(was)
                      : "r"(tc::smem_u32(&m.arrived))
                      : "memory");
-        if ((was & (PW - 1)) == PW - 1) {
+        // (not after a warp gave up, which it says before it arrives)
+        if ((was & (PW - 1)) == PW - 1 && was < kGaveUp) {
           tc::fence_after_sync();
           if (L1 >= 0) {
             const uint64_t dA = tc::smem_desc(tc::smem_u32(A1 + st * NX * APLANE));
@@ -753,7 +772,7 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
       }
     };
     // iteration n produces batch n + 1 and reads batch n back
-    bool ok = true;
+    uint32_t limit = T.wait;  // of this warp's next wait
     int g = g0 - 1, cur = 0;  // multipoles left of group g
     bool start = false;       // the first of its group
     terms_of(g0);
@@ -772,9 +791,16 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
       if (ahead) terms_of(gn + 1);
       const int L = __ffs(cur) - 1;
       if (n >= 0) {
-        // this batch's first product, the last one's second
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(&m.done, (uint32_t)(n & 1), kWait));
-        if (!ok) break;
+        // this batch's first product, the last one's second. Where a wait runs
+        // out nothing more is issued and the unit is marked below, but the warp
+        // stays in the loop: its partner meets it at barriers without a limit.
+        if (!__all_sync(0xffffffffu, tc::mbar_wait(&m.done, (uint32_t)(n & 1), limit))) {
+          if (lane == 0) {
+            atomicMin(&m.fail, n);
+            atomicOr(&m.arrived, kGaveUp);
+          }
+          limit = 0;
+        }
         tc::fence_after_sync();
         if (start || !cur) {
           if (n > 0) store_group();
@@ -823,24 +849,17 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
       cur = nxt;
       start = begin;
     }
-    if (!ok) {
-      if (lane == 0) atomicExch(&m.fail, 1);
-      // the results of this unit are marked
-      for (int g = g0; g < g1; ++g) {
-        if (8 * g + oslot >= count) break;
-        const int jkf = S.olist[8 * g + oslot];
-        double y[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) y[j] = __longlong_as_double(0x7ff8000000000000ll);
-        for (int h = 0; h < 8; h += 4) store_rows(A, S, K, a, b, jkf % A.nang, jkf / A.nang, oi, 8 * half + h, y);
-      }
-    }
   }
   __syncthreads();
-  if (m.fail && t == 0) {
-    atomicExch(T.err, 1);
-    // MMAs may still be running: give them time before the tensor memory is released
-    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  if (m.fail != kNoFail) {  // uniform over the CTA
+    if (t == 0) {
+      atomicExch(T.err, 1);
+      // the products of that batch may still be running (none came after them):
+      // the tensor memory is released after them
+      if (!tc::mbar_wait(&m.done, (uint32_t)(m.fail & 1), kWait))
+        for (int i = 0; i < 100; ++i) __nanosleep(1000);
+    }
+    mark_unit(A, S, units, symmetric, K);
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -1003,7 +1022,7 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
             T.tk_digits + (((size_t)actL[n] * A.nel + a) * mtiles + mt) * ksteps * ND * APLANE;
         for (int ks = 0; ks < ksteps; ++ks, ++it) {
           const int s = it % nst;
-          if (it >= nst && !tc::mbar_wait(&empty[s], (uint32_t)((it / nst - 1) & 1), kWait)) {
+          if (it >= nst && !tc::mbar_wait(&empty[s], (uint32_t)((it / nst - 1) & 1), T.wait)) {
             ok = false;
             break;
           }
@@ -1024,12 +1043,12 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
       for (int n = 0; n < na && ok; ++n) {
         const int bf = n & 1;
         // (the working warps arrive after reading batch n - 2 back)
-        if (!(ok = tc::mbar_wait(&bfull[bf], (uint32_t)((n >> 1) & 1), kWait))) break;
+        if (!(ok = tc::mbar_wait(&bfull[bf], (uint32_t)((n >> 1) & 1), T.wait))) break;
         tc::fence_after_sync();
         const uint64_t dB = tc::smem_desc(tc::smem_u32(Bx + bf * bsize));
         for (int ks = 0; ks < ksteps; ++ks, ++it) {
           const int s = it % nst;
-          if (!(ok = tc::mbar_wait(&full[s], (uint32_t)((it / nst) & 1), kWait))) break;
+          if (!(ok = tc::mbar_wait(&full[s], (uint32_t)((it / nst) & 1), T.wait))) break;
           tc::fence_after_sync();
           const uint64_t dA = tc::smem_desc(tc::smem_u32(Abuf + s * ND * APLANE));
 #pragma unroll
@@ -1135,7 +1154,7 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
       const int m = n - 1, L = actL[m];
       const int* ex = exs + (m & 3) * DSLOT;
       const int ea = T.tk_rowexp[(((size_t)L * A.nel + a) * mtiles + mt) * 128 + row];
-      const bool ok = tc::mbar_wait(&done[m & 1], (uint32_t)((m >> 1) & 1), kWait);
+      const bool ok = tc::mbar_wait(&done[m & 1], (uint32_t)((m >> 1) & 1), T.wait);
       if (!__all_sync(0xffffffffu, ok)) {
         // (the other working warps meet at barrier 1: all give up in turn)
         if (lane == 0) atomicExch(fail, 1);

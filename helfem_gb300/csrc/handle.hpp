@@ -388,6 +388,7 @@ struct hfg_atom {
     tc_mma_flops[1] = per * ((double)nel * (nel - 1)) + dper * (double)batches(order, 16);
     tc_ok = true;
   }
+  void tc_wait_limit(unsigned polls) { tc.wait = tc_rs.wait = polls; }
   // a completion wait inside the tensor-core kernel ran out (checked by the
   // host-pointer entry points after their synchronisation)
   void tc_check() {

@@ -294,6 +294,14 @@ hfg_status hfg_tc_selftest(const float* A, const float* B, float* D, int N, int 
                            int b_mn_major, int swap_offsets);
 hfg_status hfg_tc_peak(int ctas_per_sm, int iters, double* tflops, double* ms);
 
+/* ---- bounded waits of the tensor-core exchange ----
+ * Every wait inside the tensor-core exchange kernels is bounded. Where one runs
+ * out (a GPU in trouble) the kernels still end, and the part of K that they did
+ * not finish is NaN. hfg_atom_tc_wait_limit sets the polls after which a wait
+ * gives up, for builds queued later (2^17 by default; 0: every wait gives up at
+ * once, which is how that path is tested). */
+hfg_status hfg_atom_tc_wait_limit(hfg_atom* atom, unsigned polls);
+
 /* ---- XC potential on the atomic DFT grid ----
  * Replaces DFTGrid::eval_Fxc (src/atomic/dftgrid.h:156-159,
  * src/atomic/dftgrid.cpp:591-712) with functionals restated from the papers

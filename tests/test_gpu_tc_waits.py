@@ -1,0 +1,37 @@
+"""Completion waits of the tensor-core exchange kernels that run out (a limit of
+no polls): the kernels end, K is NaN wherever the build was not finished, and
+the handle's next build with the usual limit is what it was before."""
+import pytest
+
+from gpu_util import make_pair, random_density, to_dev, torch_cuda
+
+pytestmark = pytest.mark.gpu
+DEFAULT = 1 << 17
+
+
+# two groups of output blocks per element pair, many, diagonal tiles alone
+@pytest.mark.parametrize("case", [(10, 1, 1, 6, 13), (36, 3, 3, 3, 13), (18, 1, 1, 4, 17)],
+                         ids=lambda c: f"l{c[1]}_e{c[3]}_n{c[4]}")
+@pytest.mark.parametrize("split", [False, True], ids=["plain", "split"])
+def test_atomic_wait_runs_out(case, split):
+    torch = torch_cuda()
+    A, O = make_pair(*case)
+    nn, n = case[4], O.nbf // len(A.lval)
+    P = to_dev(torch, random_density(O.nbf, 5, seed=1))
+    g = torch.arange(n, device="cuda")
+    inner = (g + 1) % (nn - 1) != 0  # not on a boundary between elements
+    el = (g + 1) // (nn - 1)
+    tiles = (inner[:, None] & inner[None, :]) & ((el[:, None] == el[None, :]) | (nn <= 16))
+    tiles = tiles.repeat(len(A.lval), len(A.lval))
+    for symmetric in (False, True):
+        K0, K = torch.empty_like(P), torch.zeros_like(P)
+        A.exchange(P, K0, symmetric=symmetric, split=split)
+        A.tc_wait_limit(0)
+        A.exchange(P, K, symmetric=symmetric, split=split)
+        torch.cuda.synchronize()
+        A.tc_wait_limit(DEFAULT)
+        assert torch.isnan(K[tiles]).all()
+        assert torch.equal(K[~torch.isnan(K)], K0[~torch.isnan(K)])
+        A.exchange(P, K, symmetric=symmetric, split=split)
+        torch.cuda.synchronize()
+        assert torch.isfinite(K0).all() and torch.equal(K, K0)
