@@ -61,6 +61,7 @@ _SIGS = {
                          ctypes.POINTER(ctypes.c_float), ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                          ctypes.c_int], ctypes.c_int),
     "hfg_atom_tc_wait_limit": ([_P, ctypes.c_uint], ctypes.c_int),
+    "hfg_diatomic_tc_wait_limit": ([_P, ctypes.c_uint], ctypes.c_int),
     "hfg_tc_peak": ([ctypes.c_int, ctypes.c_int, _D, _D], ctypes.c_int),
     "hfg_atom_tc_work": ([_P, ctypes.c_int, _D], ctypes.c_int),
     "hfg_atom_get_dims": ([_P, ctypes.POINTER(_Dims)], ctypes.c_int),
@@ -862,6 +863,10 @@ class Diatomic:
         return L.value, M.value, out, sg
 
     # ---- hot path: device pointers ----
+    def tc_wait_limit(self, polls: int):
+        """Polls after which a completion wait of the tensor-core exchange gives up (K is NaN then)."""
+        _check(_lib.hfg_diatomic_tc_wait_limit(self._h, polls))
+
     def coulomb(self, P, J, stream=None):
         _check(_lib.hfg_diatomic_coulomb(self._h, _ptr(P), _ptr(J), _stream(stream)))
 

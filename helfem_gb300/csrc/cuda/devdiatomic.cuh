@@ -87,6 +87,7 @@ struct DevDiatomic {
 #define DTC_XDIGITS 6  // of a recoupled float-pair tile; one of FP64 has as many as the table
 #define DTC_TDIGITS 7
 #define DTC_TT 64
+#define DTC_WAIT (1u << 20)  // polls of a completion wait before it gives up
 struct DevDiaTC {
   int ksteps = 0, ntt = 0;            // K steps of 16 over 4 nn^2 columns, tiles of DTC_TT rows
   const unsigned char* tx = nullptr;  // [ilm][e][tile][K step][digit][DTC_TT x 16]
@@ -97,6 +98,7 @@ struct DevDiaTC {
   int* xexp = nullptr;                // [unit][ilm][128]
   double* part = nullptr;             // [part][unit][tile][DTC_TT][128]
   int* err = nullptr;                 // set when a completion wait ran out
+  unsigned wait = DTC_WAIT;
 };
 
 // Scratch of the in-element tiles of the FP64 exchange (dk_share.cu): units

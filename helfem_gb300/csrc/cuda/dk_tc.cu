@@ -57,7 +57,7 @@ constexpr int TT = DTC_TT;            // tile entries t per CTA
 constexpr int BPL = TT * 32;          // bytes of a TT x 16 f16 plane
 constexpr int NSTAGE = 5;
 constexpr int kNoRow = (int)0x80808080;
-constexpr uint32_t kWait = 1u << 20;  // limit of every wait
+constexpr uint32_t kWait = DTC_WAIT;  // limit of the waits of a CTA that gives up
 
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: x + M - M rounds |x| < 2^22 to an integer
 __device__ __forceinline__ float rnd(float x) { return __fsub_rn(__fadd_rn(x, kMagic), kMagic); }
@@ -454,7 +454,8 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
   uint64_t* empty = full + NSTAGE;
   uint64_t* done = empty + NSTAGE;
   uint64_t* fre = done + 1;
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(fre + 1);
+  uint64_t* drain = fre + 1;  // every product finished (of a CTA that gives up)
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(drain + 1);
   int* fail = reinterpret_cast<int*>(tslot + 1);
   int* nact = fail + 1;
   int* act = nact + 1;  // [nlm] multipoles with a row in this tile
@@ -478,6 +479,7 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
     }
     tc::mbar_init(done, 1);
     tc::mbar_init(fre, 8);
+    tc::mbar_init(drain, 1);
     fail[0] = 0;
   }
   tc::fence_before_sync();
@@ -505,7 +507,7 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
         const unsigned char* ts = T.tx + (((size_t)act[a] * D.nel + e) * T.ntt + tt) * T.ksteps * TD * BPL;
         for (int ks = 0; ks < T.ksteps; ++ks, ++it) {
           const int s = it % NSTAGE;
-          if (it >= NSTAGE && !tc::mbar_wait(&empty[s], (uint32_t)((it / NSTAGE - 1) & 1), kWait)) {
+          if (it >= NSTAGE && !tc::mbar_wait(&empty[s], (uint32_t)((it / NSTAGE - 1) & 1), T.wait)) {
             ok = false;
             break;
           }
@@ -527,11 +529,11 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
       int it = 0;
       for (int a = 0; a < na && ok; ++a) {
         // the sums of the previous multipole have been read back
-        if (a > 0 && !tc::mbar_wait(fre, (uint32_t)((a - 1) & 1), kWait)) { ok = false; break; }
+        if (a > 0 && !tc::mbar_wait(fre, (uint32_t)((a - 1) & 1), T.wait)) { ok = false; break; }
         tc::fence_after_sync();
         for (int ks = 0; ks < T.ksteps; ++ks, ++it) {
           const int s = it % NSTAGE;
-          if (!tc::mbar_wait(&full[s], (uint32_t)((it / NSTAGE) & 1), kWait)) { ok = false; break; }
+          if (!tc::mbar_wait(&full[s], (uint32_t)((it / NSTAGE) & 1), T.wait)) { ok = false; break; }
           tc::fence_after_sync();
           const uint64_t da = tc::smem_desc(tc::smem_u32(Abuf + s * NX * APL));
           const uint64_t db = tc::smem_desc(tc::smem_u32(Bbuf + s * TD * BPL));
@@ -561,7 +563,7 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
       const int ilm = act[a];
       const int E = T.xexp[((size_t)lu * D.nlm + ilm) * 128 + row];
       const int* te = T.txexp + (((size_t)ilm * D.nel + e) * T.ntt + tt) * TT + 32 * half;
-      const bool ok = tc::mbar_wait(done, (uint32_t)(a & 1), kWait);
+      const bool ok = tc::mbar_wait(done, (uint32_t)(a & 1), T.wait);
       if (!__all_sync(0xffffffffu, ok)) {
         if (lane == 0) atomicExch(fail, 1);
         break;
@@ -606,7 +608,12 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
     for (int j = 0; j < 32; ++j)
       o[(size_t)j * 128] = bad ? __longlong_as_double(0x7ff8000000000000ll) : acc[j];
   }
-  if (t == 0 && fail[0]) atomicExch(T.err, 1);
+  if (warp == 9 && lane == 0 && fail[0]) {
+    atomicExch(T.err, 1);
+    // products may still be running: the tensor memory is released after them
+    tc::mma_commit(drain);
+    tc::mbar_wait(drain, 0, kWait);
+  }
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 9) tc::tmem_dealloc(tD, 512);
@@ -640,7 +647,7 @@ cudaError_t launch_dk_tc_table(const DevDiatomic& D, const DevDiaTC& T, unsigned
 }
 
 size_t dtc_gemm_smem(const DevDiatomic& D, bool f64) {
-  return (size_t)NSTAGE * ((f64 ? TD : XD) * APL + TD * BPL) + 8 * (2 * NSTAGE + 2) + 4 * (4 + (size_t)D.nlm);
+  return (size_t)NSTAGE * ((f64 ? TD : XD) * APL + TD * BPL) + 8 * (2 * NSTAGE + 3) + 4 * (4 + (size_t)D.nlm);
 }
 
 // Pd: the FP64 form (from the density itself), nullptr: the split form (S.pd2)

@@ -952,7 +952,8 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
   uint64_t* empty = full + DST;
   uint64_t* bfull = empty + DST;  // [2] density digits there
   uint64_t* done = bfull + 2;     // [2] products finished
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 2);
+  uint64_t* drain = done + 2;     // every product finished (of a CTA that gives up)
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(drain + 1);
   unsigned char* act = reinterpret_cast<unsigned char*>(tslot + 2);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int qw = warp & 3, half = warp >> 2;
@@ -987,6 +988,7 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
       tc::mbar_init(&bfull[i], DW);
       tc::mbar_init(&done[i], 1);
     }
+    tc::mbar_init(drain, 1);
   }
   if (warp == DW + 1) {
     tc::tmem_alloc(tslot, 256);
@@ -1198,10 +1200,11 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
       if (symmetric && j0 != k0) k_store_tile(A, S, K, a, a, k0 + j0 * A.nang, q, p, y);
     }
   }
-  if (failed && t == 0) {
+  if (failed && warp == DW + 1 && lane == 0) {
     atomicExch(T.err, 1);
-    // MMAs may still be running: give them time before the tensor memory is released
-    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+    // products may still be running: the tensor memory is released after them
+    tc::mma_commit(drain);
+    tc::mbar_wait(drain, 0, kWait);
   }
   __syncthreads();
   if (warp == DW + 1) tc::tmem_dealloc(tD, 256);
@@ -1214,7 +1217,7 @@ size_t tc_smem_bytes(int NL, int nang, bool f64) {
 
 size_t tc_diag_smem_bytes(int NL, int ksteps, int nang, int stages) {
   return (size_t)stages * ND * APLANE + (size_t)2 * ksteps * ND * TPLANE +
-         sizeof(int) * (4 * DSLOT + NL * DSLOT * 2 + DSLOT + 2 + NL + 1) + 8 * (2 * DST + 4) + 8 + (size_t)nang * nang + 64;
+         sizeof(int) * (4 * DSLOT + NL * DSLOT * 2 + DSLOT + 2 + NL + 1) + 8 * (2 * DST + 5) + 8 + (size_t)nang * nang + 64;
 }
 
 // P: the FP64 form (from the density itself), nullptr: the split form (from S.p2)

@@ -519,6 +519,7 @@ struct hfg_diatomic {
     T.part = t_part.as<double>();
     ck(cudaStreamSynchronize(own_stream), "sync after the kernel's digits");
     T.err = t_err.as<int>();
+    T.wait = tc.wait;
     tc = T;
     return true;
   }
@@ -764,6 +765,13 @@ hfg_status hfg_diatomic_coulomb(hfg_diatomic* d, const double* P, double* J, voi
   return guard([&] {
     need(d && P && J, "hfg_diatomic_coulomb: null argument");
     d->build(P, J, false, false, to_stream(stream));
+  });
+}
+
+hfg_status hfg_diatomic_tc_wait_limit(hfg_diatomic* d, unsigned polls) {
+  return guard([&] {
+    need(d != nullptr, "hfg_diatomic_tc_wait_limit: null argument");
+    d->tc.wait = polls;
   });
 }
 

@@ -3,6 +3,7 @@ no polls): the kernels end, K is NaN wherever the build was not finished, and
 the handle's next build with the usual limit is what it was before."""
 import pytest
 
+import helfem_gb300 as hg
 from gpu_util import make_pair, random_density, to_dev, torch_cuda
 
 pytestmark = pytest.mark.gpu
@@ -33,5 +34,29 @@ def test_atomic_wait_runs_out(case, split):
         assert torch.isnan(K[tiles]).all()
         assert torch.equal(K[~torch.isnan(K)], K0[~torch.isnan(K)])
         A.exchange(P, K, symmetric=symmetric, split=split)
+        torch.cuda.synchronize()
+        assert torch.isfinite(K0).all() and torch.equal(K, K0)
+
+
+@pytest.mark.parametrize("split", [False, True], ids=["plain", "split"])
+def test_diatomic_wait_runs_out(split):
+    torch = torch_cuda()
+    nn, nel = 10, 3
+    d = hg.Diatomic.from_grid(3, 1, 3.0, nel, [4, 2], Rmax=12.0, nnodes=nn)
+    P = to_dev(torch, random_density(d.nbf, 5, seed=1))
+    n = nel * (nn - 1)  # functions of an m = 0 shell, the first of the basis
+    g = torch.arange(n, device="cuda")
+    el = g // (nn - 1)
+    tiles = (el[:, None] == el[None, :]) & (g % (nn - 1) != 0)[:, None] & (g % (nn - 1) != 0)[None, :]
+    for symmetric in (False, True):
+        K0, K = torch.empty_like(P), torch.zeros_like(P)
+        d.exchange(P, K0, symmetric=symmetric, split=split)
+        d.tc_wait_limit(0)
+        d.exchange(P, K, symmetric=symmetric, split=split)
+        torch.cuda.synchronize()
+        d.tc_wait_limit(1 << 20)
+        assert torch.isnan(K[:n, :n][tiles]).all()
+        assert torch.equal(K[~torch.isnan(K)], K0[~torch.isnan(K)])
+        d.exchange(P, K, symmetric=symmetric, split=split)
         torch.cuda.synchronize()
         assert torch.isfinite(K0).all() and torch.equal(K, K0)
