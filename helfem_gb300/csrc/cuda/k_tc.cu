@@ -800,6 +800,7 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
             atomicOr(&m.arrived, kGaveUp);
           }
           limit = 0;
+          jk = -1;
         }
         tc::fence_after_sync();
         if (start || !cur) {
@@ -807,7 +808,9 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
           if (!cur) break;
           E2 = m.ex[g & 3][oslot];
           mask2 = m.mask[g & 3][oslot];
-          jk = m.jk[g & 3][oslot];
+          // (the warps that gave up no longer meet the others at every batch: what
+          // those say of a group may not be there yet, so nothing is stored)
+          jk = limit ? m.jk[g & 3][oslot] : -1;
         }
         // ---- levels -> balanced digits of Y = A X, the second product's
         // MN-major operand: rows (slot, i), K = q ----

@@ -14,11 +14,15 @@ DEFAULT = 1 << 17
 @pytest.mark.parametrize("case", [(10, 1, 1, 6, 13), (36, 3, 3, 3, 13), (18, 1, 1, 4, 17)],
                          ids=lambda c: f"l{c[1]}_e{c[3]}_n{c[4]}")
 @pytest.mark.parametrize("split", [False, True], ids=["plain", "split"])
-def test_atomic_wait_runs_out(case, split):
+@pytest.mark.parametrize("mix", [True, False], ids=["dense", "same_m"])
+def test_atomic_wait_runs_out(case, split, mix):
     torch = torch_cuda()
     A, O = make_pair(*case)
     nn, n = case[4], O.nbf // len(A.lval)
     P = to_dev(torch, random_density(O.nbf, 5, seed=1))
+    if not mix:  # the output blocks of different m are inactive, and zero
+        m = torch.as_tensor(A.mval, device="cuda").repeat_interleave(n)
+        P *= m[:, None] == m[None, :]
     g = torch.arange(n, device="cuda")
     inner = (g + 1) % (nn - 1) != 0  # not on a boundary between elements
     el = (g + 1) // (nn - 1)
@@ -31,7 +35,7 @@ def test_atomic_wait_runs_out(case, split):
         A.exchange(P, K, symmetric=symmetric, split=split)
         torch.cuda.synchronize()
         A.tc_wait_limit(DEFAULT)
-        assert torch.isnan(K[tiles]).all()
+        assert torch.isnan(K[tiles & (K0 != 0)]).all()
         assert torch.equal(K[~torch.isnan(K)], K0[~torch.isnan(K)])
         A.exchange(P, K, symmetric=symmetric, split=split)
         torch.cuda.synchronize()
