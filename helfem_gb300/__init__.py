@@ -61,6 +61,8 @@ _SIGS = {
                          ctypes.POINTER(ctypes.c_float), ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                          ctypes.c_int], ctypes.c_int),
     "hfg_atom_tc_wait_limit": ([_P, ctypes.c_uint], ctypes.c_int),
+    "hfg_atom_tc_status": ([_P, _P], ctypes.c_int),
+    "hfg_diatomic_tc_status": ([_P, _P], ctypes.c_int),
     "hfg_diatomic_tc_wait_limit": ([_P, ctypes.c_uint], ctypes.c_int),
     "hfg_tc_peak": ([ctypes.c_int, ctypes.c_int, _D, _D], ctypes.c_int),
     "hfg_atom_tc_work": ([_P, ctypes.c_int, _D], ctypes.c_int),
@@ -371,6 +373,10 @@ class Atom:
     def tc_wait_limit(self, polls: int):
         """Polls after which a completion wait of the tensor-core exchange gives up (K is NaN then)."""
         _check(_lib.hfg_atom_tc_wait_limit(self._h, polls))
+
+    def tc_status(self, stream=None):
+        """Waits for `stream`; raises HfgError if a wait ran out since the last report."""
+        _check(_lib.hfg_atom_tc_status(self._h, _stream(stream)))
 
     def tc_work(self, symmetric: bool = True) -> float:
         """bf16 MMA FLOPs of one split-precision exchange (all entries active)."""
@@ -866,6 +872,10 @@ class Diatomic:
     def tc_wait_limit(self, polls: int):
         """Polls after which a completion wait of the tensor-core exchange gives up (K is NaN then)."""
         _check(_lib.hfg_diatomic_tc_wait_limit(self._h, polls))
+
+    def tc_status(self, stream=None):
+        """Waits for `stream`; raises HfgError if a wait ran out since the last report."""
+        _check(_lib.hfg_diatomic_tc_status(self._h, _stream(stream)))
 
     def coulomb(self, P, J, stream=None):
         _check(_lib.hfg_diatomic_coulomb(self._h, _ptr(P), _ptr(J), _stream(stream)))

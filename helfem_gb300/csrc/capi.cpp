@@ -208,7 +208,7 @@ static void sad_host(hfg_atom* a, const double* P, double* out, int kind, int fl
   need(a != nullptr, "null argument");
   sad_call(a, P, out, kind, flags, a->own_stream);
   ck(cudaStreamSynchronize(a->own_stream), "stream sync");
-  if (kind != 0 && ((flags & HFG_EXCHANGE_SPLIT) || a->tc64_for(false))) a->tc_check();
+  if (kind != 0) a->tc_check(a->own_stream, (flags & HFG_EXCHANGE_SPLIT) != 0, kind == 2);
 }
 
 hfg_status hfg_sadatom_coulomb_host(hfg_atom* a, const double* P, double* J) {
@@ -387,6 +387,14 @@ hfg_status hfg_atom_tc_wait_limit(hfg_atom* a, unsigned polls) {
   });
 }
 
+hfg_status hfg_atom_tc_status(hfg_atom* a, void* stream) {
+  return guard([&] {
+    need(a != nullptr, "hfg_atom_tc_status: null argument");
+    a->check_device();
+    a->tc_check((cudaStream_t)stream);
+  });
+}
+
 hfg_status hfg_tc_peak(int ctas_per_sm, int iters, double* tflops, double* ms) {
   return guard([&] {
     need(tflops && ms && ctas_per_sm >= 1 && ctas_per_sm <= 2 && iters >= 1, "hfg_tc_peak: bad arguments");
@@ -489,7 +497,7 @@ static void host_call(hfg_atom* a, const double* P, double* out, bool coulomb, i
   ck(cudaMemcpyAsync(out, a->h_out.p, bytes, cudaMemcpyDeviceToHost, st), "D2H copy");
   a->last_d2h = bytes;
   ck(cudaStreamSynchronize(st), "stream sync");
-  if (!coulomb && ((flags & HFG_EXCHANGE_SPLIT) || a->tc64_for(screened))) a->tc_check();
+  if (!coulomb) a->tc_check(st, (flags & HFG_EXCHANGE_SPLIT) != 0, screened);
 }
 
 // J(PJ) and K(PK) with one staging of the density when PK == PJ, the
@@ -552,7 +560,7 @@ static void jk_host(hfg_atom* a, const double* PJ, const double* PK, double* J, 
   a->last_d2h = 2 * bytes;
   ck(cudaStreamSynchronize(st), "stream sync");
   ck(cudaStreamSynchronize(a->copy_stream), "stream sync");
-  if ((flags & HFG_EXCHANGE_SPLIT) || a->tc64_for(false)) a->tc_check();
+  a->tc_check(st, (flags & HFG_EXCHANGE_SPLIT) != 0, false);
 }
 
 hfg_status hfg_jk(hfg_atom* a, const double* PJ, const double* PK, double* J, double* K, int flags, void* stream) {

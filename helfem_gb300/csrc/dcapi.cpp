@@ -363,14 +363,8 @@ struct hfg_diatomic {
     ck(cudaStreamSynchronize(own_stream), "sync after the device tabulation");
   }
 
-  // a completion wait inside the tensor-core kernel ran out (checked by the
-  // host-pointer entry points after their synchronisation)
-  void tc_check() {
-    if (!tc.err) return;
-    int e = 0;
-    ck(cudaMemcpy(&e, tc.err, sizeof(int), cudaMemcpyDeviceToHost), "D2H");
-    if (e) throw std::runtime_error("tensor-core exchange: an MMA completion wait ran out");
-  }
+  // as hfg_atom::tc_check
+  void tc_check(cudaStream_t st) { hfg_abi::tc_report(tc.err, st); }
 
   // output blocks j <= k of one m: the active ones for a density that does
   // not mix m
@@ -629,7 +623,7 @@ struct hfg_diatomic {
     build(h_in.as<double>(), h_out.as<double>(), exchange, symmetric, own_stream, split);
     ck(cudaMemcpyAsync(F, h_out.p, bytes, cudaMemcpyDeviceToHost, own_stream), "copy out");
     ck(cudaStreamSynchronize(own_stream), "sync");
-    if (exchange) tc_check();
+    if (exchange) tc_check(own_stream);
   }
 };
 
@@ -772,6 +766,14 @@ hfg_status hfg_diatomic_tc_wait_limit(hfg_diatomic* d, unsigned polls) {
   return guard([&] {
     need(d != nullptr, "hfg_diatomic_tc_wait_limit: null argument");
     d->tc.wait = polls;
+  });
+}
+
+hfg_status hfg_diatomic_tc_status(hfg_diatomic* d, void* stream) {
+  return guard([&] {
+    need(d != nullptr, "hfg_diatomic_tc_status: null argument");
+    d->check_device();
+    d->tc_check((cudaStream_t)stream);
   });
 }
 

@@ -82,6 +82,19 @@ struct AllocStream {
   ~AllocStream() { t_alloc_stream = prev; }
 };
 
+// Waits for st; throws where a tensor-core kernel set the flag err (device
+// memory, or null) since the last report, and clears it.
+inline void tc_report(int* err, cudaStream_t st) {
+  if (!err) return;
+  int e = 0;
+  ck(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
+  ck(cudaStreamSynchronize(st), "stream sync");
+  if (!e) return;
+  ck(cudaMemsetAsync(err, 0, sizeof(int), st), "memset");
+  ck(cudaStreamSynchronize(st), "stream sync");
+  throw std::runtime_error("tensor-core exchange: an MMA completion wait ran out (K is NaN where it did)");
+}
+
 // RAII device allocation
 struct DBuf {
   void* p = nullptr;
@@ -389,13 +402,13 @@ struct hfg_atom {
     tc_ok = true;
   }
   void tc_wait_limit(unsigned polls) { tc.wait = tc_rs.wait = polls; }
-  // a completion wait inside the tensor-core kernel ran out (checked by the
-  // host-pointer entry points after their synchronisation)
-  void tc_check() {
-    if (!tc.err) return;
-    int e = 0;
-    ck(cudaMemcpy(&e, tc.err, sizeof(int), cudaMemcpyDeviceToHost), "D2H");
-    if (e) throw std::runtime_error("tensor-core exchange: an MMA completion wait ran out");
+  // Waits for st; throws where a completion wait of a tensor-core kernel ran out
+  // in the work queued there (once: the flag is cleared). The synchronous entry
+  // points and the SCF driver call it, hfg_atom_tc_status for the others.
+  void tc_check(cudaStream_t st) { hfg_abi::tc_report(tc.err, st); }
+  // the same after an exchange of the given form, if it ran on the tensor cores
+  void tc_check(cudaStream_t st, bool split, bool screened) {
+    if (split ? tc_for(screened) : tc64_for(screened)) tc_check(st);
   }
   // staging for the host-pointer entry points (allocated on first use)
   DBuf h_in, h_out, h_in2, h_out2, h_e;

@@ -827,6 +827,7 @@ void hfg_scf_impl(hfg_atom* a, const hfg_scf_desc* d, hfg_scf_result* res, doubl
         }
         oda_have = true;
       }
+      if (kfrac != 0.0) a->tc_check(st, d->split_exchange != 0, false);  // (st is waited for next in any case)
       Ekin = dot(dP.as<double>(), T);
       pt.lap(0);  // Fock build (J, K, XC, assembly) + first blocking dot
       Enuc = dot(dP.as<double>(), V);

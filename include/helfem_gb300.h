@@ -297,10 +297,14 @@ hfg_status hfg_tc_peak(int ctas_per_sm, int iters, double* tflops, double* ms);
 /* ---- bounded waits of the tensor-core exchange ----
  * Every wait inside the tensor-core exchange kernels is bounded. Where one runs
  * out (a GPU in trouble) the kernels still end, and the part of K that they did
- * not finish is NaN. hfg_atom_tc_wait_limit (hfg_diatomic_tc_wait_limit, below)
+ * not finish is NaN, in the plain and in the split form. The host-pointer entries
+ * and hfg_scf_run (and so the engine) report it as an error; the entries that
+ * return without synchronising cannot: hfg_atom_tc_status waits for the work
+ * queued on `stream` and reports a wait that ran out since the last report. hfg_atom_tc_wait_limit (hfg_diatomic_tc_*, below)
  * sets the polls after which a wait gives up, for builds queued later (2^17 and
  * 2^20 by default; 0: every wait gives up at once, which is how that path is
  * tested). */
+hfg_status hfg_atom_tc_status(hfg_atom* atom, void* stream);
 hfg_status hfg_atom_tc_wait_limit(hfg_atom* atom, unsigned polls);
 
 /* ---- XC potential on the atomic DFT grid ----
@@ -573,6 +577,7 @@ hfg_status hfg_diatomic_coulomb(hfg_diatomic* d, const double* P, double* J, voi
  * bit, slower; kept for comparison). */
 #define HFG_EXCHANGE_ITEMWISE 4
 hfg_status hfg_diatomic_exchange(hfg_diatomic* d, const double* P, double* K, int flags, void* stream);
+hfg_status hfg_diatomic_tc_status(hfg_diatomic* d, void* stream);
 hfg_status hfg_diatomic_tc_wait_limit(hfg_diatomic* d, unsigned polls);
 /* host-pointer value-semantics variants */
 hfg_status hfg_diatomic_coulomb_host(hfg_diatomic* d, const double* P, double* J);

@@ -64,3 +64,32 @@ def test_diatomic_wait_runs_out(split):
         d.exchange(P, K, symmetric=symmetric, split=split)
         torch.cuda.synchronize()
         assert torch.isfinite(K0).all() and torch.equal(K, K0)
+
+
+@pytest.mark.parametrize("split", [False, True], ids=["plain", "split"])
+def test_wait_that_ran_out_is_reported_once(split):
+    """By the host-pointer entries and the SCF driver themselves, after a
+    device-pointer entry by the status query; then the handle works as before."""
+    torch = torch_cuda()
+    A, O = make_pair(10, 1, 1, 6, 13)
+    d = hg.Diatomic.from_grid(3, 1, 3.0, 3, [4, 2], Rmax=12.0, nnodes=10)
+    for h in (A, d):
+        P = random_density(h.nbf, 4, seed=2)
+        K0 = h.exchange_host(P, split=split)
+        h.tc_wait_limit(0)
+        with pytest.raises(hg.HfgError, match="ran out"):
+            h.exchange_host(P, split=split)
+        Pd = to_dev(torch, P)
+        K = torch.zeros_like(Pd)
+        h.exchange(Pd, K, split=split)
+        with pytest.raises(hg.HfgError, match="ran out"):
+            h.tc_status()
+        h.tc_status()
+        h.tc_wait_limit(DEFAULT if h is A else 1 << 20)
+        assert (h.exchange_host(P, split=split) == K0).all()
+    E = A.scf(5, 5, split=split)["Etot"]
+    A.tc_wait_limit(0)
+    with pytest.raises(hg.HfgError, match="ran out"):
+        A.scf(5, 5, split=split)
+    A.tc_wait_limit(DEFAULT)
+    assert A.scf(5, 5, split=split)["Etot"] == pytest.approx(E, abs=1e-9)
