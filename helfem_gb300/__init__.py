@@ -63,6 +63,7 @@ _SIGS = {
     "hfg_atom_tc_wait_limit": ([_P, ctypes.c_uint], ctypes.c_int),
     "hfg_atom_tc_status": ([_P, _P], ctypes.c_int),
     "hfg_diatomic_tc_status": ([_P, _P], ctypes.c_int),
+    "hfg_diatomic_scratch_limit": ([_P, ctypes.c_size_t], ctypes.c_int),
     "hfg_diatomic_tc_wait_limit": ([_P, ctypes.c_uint], ctypes.c_int),
     "hfg_tc_peak": ([ctypes.c_int, ctypes.c_int, _D, _D], ctypes.c_int),
     "hfg_atom_tc_work": ([_P, ctypes.c_int, _D], ctypes.c_int),
@@ -872,6 +873,10 @@ class Diatomic:
     def tc_wait_limit(self, polls: int):
         """Polls after which a completion wait of the tensor-core exchange gives up (K is NaN then)."""
         _check(_lib.hfg_diatomic_tc_wait_limit(self._h, polls))
+
+    def scratch_limit(self, nbytes: int):
+        """Device bytes that the handle's first exchanges may take (0: what is free)."""
+        _check(_lib.hfg_diatomic_scratch_limit(self._h, nbytes))
 
     def tc_status(self, stream=None):
         """Waits for `stream`; raises HfgError if a wait ran out since the last report."""

@@ -382,6 +382,25 @@ struct hfg_diatomic {
   // 131 and 121, of 15 nodes 302 and 185; l <= 5, m <= 1 on six elements of 8
   // nodes 1711 and 1353, of 15 nodes 10.9 and 6.3 ms.
   bool use_tc64() const { return host.nn >= 8; }
+  // The plain form's in-element kernels, decided by the handle's first plain
+  // exchange (they differ in the last bits of K): 1 tensor cores, 2 FP64
+  int plain_form = 0;
+  // device bytes that first calls may take, 0: what is free
+  size_t scratch_limit = 0;
+  size_t room() const {
+    size_t avail = 0, total = 0;
+    ck(cudaMemGetInfo(&avail, &total), "memory");
+    // what the stream-ordered pool holds unused is free too
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    uint64_t held = 0, used = 0;
+    ck(cudaGetDevice(&dev), "device");
+    ck(cudaDeviceGetDefaultMemPool(&pool, dev), "pool");
+    ck(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held), "pool size");
+    ck(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used), "pool use");
+    avail += held > used ? held - used : 0;
+    return scratch_limit ? std::min(avail, scratch_limit) : avail;
+  }
   void ensure_fp64() {
     if (t64.x) return;
     hfg_abi::AllocStream alloc_on(own_stream);
@@ -390,7 +409,7 @@ struct hfg_diatomic {
     hfg::DevDia64 T;
     const size_t unit = sizeof(double) * H.nlm * 4 * n2 * 8;
     const size_t units = (size_t)H.nel * ((nang * nang + 7) / 8);
-    T.cap = (int)std::max<size_t>(1, std::min(units, ((size_t)2 << 30) / unit));
+    T.cap = (int)std::max<size_t>(1, std::min(units, std::min((size_t)2 << 30, room() / 2) / unit));
     // Rows of a tile in rsplit parts, vsplit threads per row: the pair that
     // leaves the fewest of the CTA's lanes idle (a partly filled warp costs the
     // FP64 pipe as much as a full one; nn = 15: 45 rows x 7 threads, 315 of 320)
@@ -470,10 +489,11 @@ struct hfg_diatomic {
     scr.pd2 = s_pd2.as<float2>();
   }
 
-  // in-element tiles on the tensor cores: the kernel's digit planes, and scratch
-  // for the digits of as many (element, 128 output blocks) units as 4 GB hold
-  // of float pairs (at least one; seven sixths of it for FP64), on the first exchange that uses them. false (unless the
-  // caller must have them): the device has no room, the FP64 kernels stay.
+  // in-element tiles on the tensor cores, on the first exchange that uses them:
+  // the kernel's digit planes, and scratch for the seven digits of as many
+  // (element, 128 output blocks) units as 4.7 GB, or half of the room that the
+  // planes leave, hold (at least one). false (unless the caller must have them):
+  // the device has no room, the FP64 kernels stay.
   bool ensure_tc(bool must) {
     if (tc.err) return true;
     hfg_abi::AllocStream alloc_on(own_stream);
@@ -484,11 +504,8 @@ struct hfg_diatomic {
     T.ntt = (int)((n2 + DTC_TT - 1) / DTC_TT);
     const size_t plane = 32;  // bytes of one row of a K step's plane
     const size_t tx_bytes = ntile * T.ntt * T.ksteps * DTC_TDIGITS * DTC_TT * plane;
-    if (!must) {
-      size_t avail = 0, total = 0;
-      ck(cudaMemGetInfo(&avail, &total), "memory");
-      if (avail < tx_bytes + ((size_t)8 << 30)) return false;
-    }
+    const size_t avail = room();
+    if (!must && avail < tx_bytes + ((size_t)8 << 30)) return false;
     t_tx.alloc(tx_bytes);
     t_cexp.alloc(sizeof(int) * ntile * 4 * n2);
     T.cexp = t_cexp.as<int>();
@@ -498,7 +515,8 @@ struct hfg_diatomic {
     T.txexp = t_txexp.as<int>();
     const size_t digit = (size_t)H.nlm * T.ksteps * 128 * plane, unit = DTC_TDIGITS * digit, nang = H.nang;
     const size_t units = (size_t)H.nel * ((nang * nang + 127) / 128);
-    T.cap = (int)std::max<size_t>(1, std::min(units, ((size_t)4 << 30) / (DTC_XDIGITS * digit)));
+    const size_t left = avail > tx_bytes ? (avail - tx_bytes) / 2 : 0;
+    T.cap = (int)std::max<size_t>(1, std::min(units, std::min(((size_t)4 << 30) / 6 * 7, left) / unit));
     // parts of the multipole sum where a density that does not mix m makes
     // fewer units x tiles than there are SMs (one CTA per SM)
     const size_t ctas = (size_t)H.nel * ((same_m_pairs() + 127) / 128) * T.ntt;
@@ -535,8 +553,11 @@ struct hfg_diatomic {
       Relaxed relaxed;
       if (exchange) ensure_side();
       if (split) ensure_split();
-      tc64 = !split && exchange && use_tc64() && ensure_tc(false);
-      if (!split && exchange && !tc64) ensure_fp64();
+      if (!split && exchange) {
+        if (!plain_form) plain_form = use_tc64() && ensure_tc(false) ? 1 : 2;
+        if (plain_form == 2) ensure_fp64();
+        tc64 = plain_form == 1;
+      }
     }
     if (!exchange) {  // J reads the pure density and writes the pure J directly
       ck(hfg::launch_diatomic_coulomb(dev, scr, P, F, st), "coulomb");
@@ -759,6 +780,13 @@ hfg_status hfg_diatomic_coulomb(hfg_diatomic* d, const double* P, double* J, voi
   return guard([&] {
     need(d && P && J, "hfg_diatomic_coulomb: null argument");
     d->build(P, J, false, false, to_stream(stream));
+  });
+}
+
+hfg_status hfg_diatomic_scratch_limit(hfg_diatomic* d, size_t bytes) {
+  return guard([&] {
+    need(d != nullptr, "hfg_diatomic_scratch_limit: null argument");
+    d->scratch_limit = bytes;
   });
 }
 

@@ -568,15 +568,22 @@ hfg_status hfg_diatomic_coulomb(hfg_diatomic* d, const double* P, double* J, voi
  * diatomic TwoDBasis::exchange (basis.cpp:1817-2061), including its
  * density-block screening. flags: HFG_EXCHANGE_SYMMETRIC (P = P^T),
  * HFG_EXCHANGE_SPLIT (split precision: element pairs in float pairs, the
- * in-element tiles on the tensor cores; the first split call allocates
- * float-pair copies of the tables, digit planes of the in-element kernel, an
- * ndummy^2 density copy and up to 4 GB of scratch; the first plain call up to
- * 2 GB), HFG_EXCHANGE_ITEMWISE (split form only: the density tiles of the
- * in-element products are recoupled one output block per work item instead of
- * in groups of output blocks that share the sums over l; the same K bit for
- * bit, slower; kept for comparison). */
+ * in-element tiles on the tensor cores), HFG_EXCHANGE_ITEMWISE (split form only:
+ * the density tiles of the in-element products are recoupled one output block
+ * per work item instead of in groups of output blocks that share the sums over
+ * l; the same K bit for bit, slower; kept for comparison).
+ * Memory: the first split call makes float-pair copies of the tables, an
+ * ndummy^2 float-pair density, the digit planes of the in-element kernel (14
+ * bytes for each of its entries, rows padded to 64 and columns to 16) and digit
+ * scratch of at most 4.7 GB. The first plain call makes the planes and that
+ * scratch too or, where it uses the FP64 kernels for these tiles (elements of
+ * few nodes, or less than the planes and 8 GB free), at most 2 GB. Less is taken
+ * where less is free; the handle keeps the kernels of its first plain call.
+ * hfg_diatomic_scratch_limit: device bytes that first calls made after it may
+ * take (0: what is free). */
 #define HFG_EXCHANGE_ITEMWISE 4
 hfg_status hfg_diatomic_exchange(hfg_diatomic* d, const double* P, double* K, int flags, void* stream);
+hfg_status hfg_diatomic_scratch_limit(hfg_diatomic* d, size_t bytes);
 hfg_status hfg_diatomic_tc_status(hfg_diatomic* d, void* stream);
 hfg_status hfg_diatomic_tc_wait_limit(hfg_diatomic* d, unsigned polls);
 /* host-pointer value-semantics variants */
