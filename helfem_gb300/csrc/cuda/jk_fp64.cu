@@ -317,18 +317,21 @@ __global__ void j_scatter(DevAtom A, DevScratch S, double* __restrict__ J, int a
 // thread. With the flags 82 us (Kr) and 144 us; without the last CTA's part 75
 // and 117 us; the norms without the tiles' maxima plus the flags' own launch
 // took 90 and 137 us.
-// NORM_PLAIN: norms and flags; NORM_SPLIT: with the float-pair copy; NORM_LISTS:
-// with what the tensor-core form of an FP64 density needs (maxima as the high
-// words of the doubles, the lists)
-enum { NORM_PLAIN, NORM_SPLIT, NORM_LISTS };
+// NORM_PLAIN: norms and flags; NORM_COPY: with the float-pair copy; NORM_SPLIT:
+// with the copy and what the tensor-core form needs (the tiles' maxima, the
+// lists); NORM_LISTS: the latter for an FP64 density (maxima as the high words of
+// the doubles)
+// entries: the last CTA marks the exchange entries too; otherwise (their flags
+// do not fit its shared memory) k_flags does.
+enum { NORM_PLAIN, NORM_COPY, NORM_SPLIT, NORM_LISTS };
 template <int MODE>
 __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict__ P, float2* __restrict__ p2,
-                              int symmetric) {
-  constexpr bool SPLIT = MODE == NORM_SPLIT, LISTS = MODE != NORM_PLAIN;
+                              int symmetric, int entries) {
+  constexpr bool SPLIT = MODE == NORM_COPY || MODE == NORM_SPLIT, LISTS = MODE == NORM_SPLIT || MODE == NORM_LISTS;
   __shared__ double red[32];
   __shared__ bool last;
   __shared__ int cnt[64];
-  extern __shared__ unsigned int emax[];  // [nel] (split form); flags of the last CTA
+  extern __shared__ unsigned int emax[];  // [nel] (list forms); flags of the last CTA
   const int blk = blockIdx.x, i = blk % A.nang, l = blk / A.nang, b = blockIdx.y, nn = A.nn;
   const int c0 = max(gfun(A, b, 0), 0), c1 = min(gfun(A, b, nn - 1), A.nrad - 1);
   const int nc = c1 - c0 + 1, nown = b == A.nel - 1 ? nc : nc - 1;  // columns, those owned
@@ -412,10 +415,11 @@ __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict_
 #pragma unroll 16
     for (int e = 0; e < A.nel; ++e) q += __ldcg(&S.bnorm[(size_t)e * nang2 + x]);
     const unsigned char f = !(sqrt(q) < 10.0 * DBL_EPSILON);
-    sact[x] = f;
+    if (entries) sact[x] = f;
     S.act[x] = f;
   }
   if (threadIdx.x == 0) *S.count = 0u;  // for the next call
+  if (!entries) return;
   __syncthreads();
   // entries: every term marks its entry. (One CTA alone: each loop loads a
   // batch before it stores, or the latencies of its loads add up.)
@@ -452,7 +456,7 @@ __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict_
     }
   }
   if (!LISTS) return;
-  // ---- split form: the active output blocks in jk_order. A symmetric
+  // ---- list forms: the active output blocks in jk_order. A symmetric
   // density's transposed partner tile is written too: (j, k) counts as active
   // where (k, j) is ----
   for (int x = threadIdx.x; x < 64; x += blockDim.x) cnt[x] = 0;
@@ -521,9 +525,13 @@ __global__ void k_zero_inactive(DevAtom A, DevScratch S, double* __restrict__ K,
   }
 }
 
-inline size_t norm_smem(const DevAtom& A, bool lists) {
-  const size_t nang2 = (size_t)A.nang * A.nang;
-  return (lists ? sizeof(int) * (A.nel + nang2) : 0) + nang2 + A.nent;
+// the entries that see an active block, where the density pass leaves them out
+__global__ void k_flags(DevAtom A, DevScratch S) {
+  for (int ent = blockIdx.x * blockDim.x + threadIdx.x; ent < A.nent; ent += gridDim.x * blockDim.x) {
+    bool any = false;
+    for (int u = A.kent_ptr[ent]; u < A.kent_ptr[ent + 1] && !any; ++u) any = S.act[A.kterm_blk[u]];
+    S.ent_act[ent] = any ? 1 : 0;
+  }
 }
 
 // threads of k_block_norms: the rows in equal passes of at most 224, so that
@@ -531,6 +539,25 @@ inline size_t norm_smem(const DevAtom& A, bool lists) {
 inline int norm_threads(const DevAtom& A) {
   const int passes = (A.nrad + 223) / 224;
   return std::max(64, ((A.nrad + passes - 1) / passes + 31) / 32 * 32);
+}
+
+// The density pass. Its last CTA keeps a flag per block and entry in shared
+// memory where that fits the default limit, as for every basis of distinct (l, m)
+// functions (at most 1.7 KB); a basis that repeats them often has more entries,
+// and a CTA would take long over them.
+template <int MODE>
+cudaError_t launch_norms(const DevAtom& A, const DevScratch& S, const double* P, float2* p2, bool symmetric,
+                         cudaStream_t st) {
+  constexpr bool lists = MODE == NORM_SPLIT || MODE == NORM_LISTS;
+  const size_t nang2 = (size_t)A.nang * A.nang, flags = nang2 + A.nent;
+  const bool entries = lists || flags <= 48 * 1024;
+  const size_t smem = (lists ? sizeof(int) * (A.nel + nang2) : 0) + (entries ? flags : 0);
+  const cudaError_t e = smem_limit(k_block_norms<MODE>, smem);
+  if (e != cudaSuccess) return e;
+  k_block_norms<MODE><<<dim3((int)nang2, A.nel), norm_threads(A), smem, st>>>(A, S, P, p2, symmetric ? 1 : 0,
+                                                                            entries ? 1 : 0);
+  if (!entries) k_flags<<<std::min(152 * 4, (A.nent + 255) / 256), 256, 0, st>>>(A, S);
+  return cudaGetLastError();
 }
 
 __device__ __forceinline__ void load_active(const DevAtom& A, const DevScratch& S, unsigned char* act) {
@@ -904,7 +931,8 @@ cudaError_t launch_exchange_erfc(const DevAtom& A, const DevScratch& S, const do
   const int n2 = A.nn * A.nn, nang2 = A.nang * A.nang;
   {
     Mark m(prof, KC_K_NORMS, st);
-    k_block_norms<NORM_PLAIN><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, false), st>>>(A, S, P, nullptr, 0);
+    const cudaError_t e = launch_norms<NORM_PLAIN>(A, S, P, nullptr, false, st);
+    if (e != cudaSuccess) return e;
   }
   {
     Mark m(prof, KC_K_TILES, st);
@@ -956,8 +984,8 @@ cudaError_t launch_exchange_fp64(const DevAtom& A, const DevScratch& S, const KU
   if (tc) {
     {
       Mark m(prof, KC_K_NORMS, st);
-      k_block_norms<NORM_LISTS>
-          <<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, true), st>>>(A, S, P, nullptr, symmetric ? 1 : 0);
+      const cudaError_t e = launch_norms<NORM_LISTS>(A, S, P, nullptr, symmetric, st);
+      if (e != cudaSuccess) return e;
     }
     {
       Mark m(prof, KC_K_TILES, st);
@@ -982,7 +1010,8 @@ cudaError_t launch_exchange_fp64(const DevAtom& A, const DevScratch& S, const KU
   }
   {
     Mark m(prof, KC_K_NORMS, st);
-    k_block_norms<NORM_PLAIN><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, false), st>>>(A, S, P, nullptr, 0);
+    const cudaError_t e = launch_norms<NORM_PLAIN>(A, S, P, nullptr, symmetric, st);
+    if (e != cudaSuccess) return e;
   }
   {
     Mark m(prof, KC_K_TILES, st);
@@ -1006,7 +1035,9 @@ cudaError_t launch_exchange_split(const DevAtom& A, const DevScratch& S, const K
   const int n2 = A.nn * A.nn, th = threads_for(n2), nang2 = A.nang * A.nang;
   {
     Mark m(prof, KC_K_NORMS, st);
-    k_block_norms<NORM_SPLIT><<<dim3(nang2, A.nel), norm_threads(A), norm_smem(A, true), st>>>(A, S, P, S.p2, symmetric ? 1 : 0);
+    const cudaError_t e = tc ? launch_norms<NORM_SPLIT>(A, S, P, S.p2, symmetric, st)
+                             : launch_norms<NORM_COPY>(A, S, P, S.p2, symmetric, st);
+    if (e != cudaSuccess) return e;
   }
   {
     Mark m(prof, KC_K_TILES, st);
