@@ -22,6 +22,7 @@
 
 #include <atomic>
 #include <chrono>
+#include <cmath>
 #include <condition_variable>
 #include <deque>
 #include <map>
@@ -61,15 +62,15 @@ struct Job {
 // DFT grid), from the basis dimensions alone.
 size_t hfg_job_footprint(const hfg_atom_desc& a, const hfg_scf_desc& s) {
   const double nn = a.nnodes, nel = a.nelem, n2 = nn * nn;
-  int lmax = 0, mmx = 0;
-  for (int i = 0; i < a.nang; ++i) {
-    lmax = std::max(lmax, a.lval[i]);
-    mmx = std::max(mmx, std::abs(a.mval[i]));
-  }
+  int lmax = 0;
+  for (int i = 0; i < a.nang; ++i) lmax = std::max(lmax, a.lval[i]);
   const double NL = 2 * lmax + 1, nang = a.nang, nrad = nel * (nn - 1) - 1, nbf = nang * nrad;
   const double rmax = std::min(n2, 2 * nn - 1);
   double b = 8.0 * NL * nel * (4 * n2 + n2 * rmax + 2 * n2 * n2);  // rs, rb (+split), factor, tensor (+split)
+  // digit planes of the exchange tensor (seven, of 128 x 16 tiles)
+  b += NL * nel * std::ceil(n2 / 128) * std::ceil(n2 / 16) * 7 * 4096;
   b += 8.0 * nel * nel * nang * nang * (2 * nn - 1);                // exchange halo
+  b += 4.0 * nel * nel * nang * nang;                               // largest values of the density tiles
   b += 8.0 * NL * NL * nel * (n2 + 2);                              // Coulomb scratch (channel bound)
   const int nspin = s.restricted ? 1 : 2;
   b += 8.0 * nbf * nbf * 13;                                        // T V H P Ps J K XC F
@@ -79,8 +80,10 @@ size_t hfg_job_footprint(const hfg_atom_desc& a, const hfg_scf_desc& s) {
   const double tab = 8.0 * NL * nel * (1.5 * n2 * n2);
   b += std::max(0.0, tab - 8.0 * nbf * nbf * (13 + 10 * nspin));
   if (s.x_func || s.c_func) {
-    const double nq = a.nquad > 0 ? a.nquad : 5 * nn, nap = (4.0 * lmax + 12) * (4.0 * mmx + 12);
-    b += 8.0 * (4 * nel * nang * nang * nq + 8 * nel * nq * nap + 8 * nel * nang * nang * nq + 3 * nang * nang * nap);
+    // per pair of angular functions: three radial densities and two potentials
+    // of each spin, polar factors; radial functions and derivatives
+    const double nq = a.nquad > 0 ? a.nquad : 5 * nn, np = 0.5 * nang * (nang + 1);
+    b += 8.0 * (10 * nel * nq * np + 3 * np * (4.0 * lmax + 12) + 2 * nel * nq * (nn + 2));
   }
   return (size_t)(b * 1.05) + (64u << 20);
 }
