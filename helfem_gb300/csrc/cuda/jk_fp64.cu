@@ -965,14 +965,16 @@ static cudaError_t launch_tiles_tc(const DevAtom& A, const DevScratch& S, const 
     // (the FP64 and float-pair kernels first: a diagonal CTA takes an SM whole)
     if (e == cudaSuccess && !tc.digits) e = pairs();
     if (e == cudaSuccess) e = launch_k_diag_tc(A, S, tc, symmetric, P, K, side->s);
-    k_zero_inactive<<<dim3(nang2, 8), 256, 0, side->s>>>(A, S, K, symmetric ? 1 : 0);
-    if (e == cudaSuccess) e = cudaEventRecord(side->join, side->s);
+    if (e == cudaSuccess) k_zero_inactive<<<dim3(nang2, 8), 256, 0, side->s>>>(A, S, K, symmetric ? 1 : 0);
+    const cudaError_t j = cudaEventRecord(side->join, side->s);
+    if (e == cudaSuccess) e = j;
     if (e == cudaSuccess && tc.digits) e = pairs();
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, side->join, 0);
+    const cudaError_t w = cudaStreamWaitEvent(st, side->join, 0);  // (joined whatever failed)
+    if (e == cudaSuccess) e = w;
   } else {
     e = pairs();
     if (e == cudaSuccess) e = launch_k_diag_tc(A, S, tc, symmetric, P, K, st);
-    k_zero_inactive<<<dim3(nang2, 8), 256, 0, st>>>(A, S, K, symmetric ? 1 : 0);
+    if (e == cudaSuccess) k_zero_inactive<<<dim3(nang2, 8), 256, 0, st>>>(A, S, K, symmetric ? 1 : 0);
   }
   return e;
 }
