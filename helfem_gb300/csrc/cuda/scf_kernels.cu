@@ -282,7 +282,13 @@ void k_add4(double* out, const double* a, const double* b, const double* c, cons
             cudaStream_t st) {
   add4<<<grid_for(n), 256, 0, st>>>(out, a, b, c, d, n);
 }
-bool thin_gemm_ok(int m, int n, int k) { return n <= 64 && (long)m * k <= (1l << 24); }
+// The line against cuBLAS, us at m = k (here, cuBLAS): one column, a matrix-vector
+// product there, 279 rows 8.2 and 6.2, 2048 28.7 and 14.4 (transposed 74 and 14);
+// 2 columns 279 rows 8.2 and 88, 4096 134 and 1063; 9 columns 279 rows 8.2 and
+// 88, 2048 131 and 281, 4096 515 and 1064; 18 columns 4096 772 and 1065; 32
+// columns 2048 260 and 267, 4096 1274 and 1067; 64 columns 140 rows 8.2 and 45,
+// 2048 516 and 557 (transposed, 1000 rows: 156 and 139).
+bool thin_gemm_ok(int m, int n, int k) { return n >= 2 && n <= 64 && (long)m * k <= (n <= 18 ? 1l << 24 : 1l << 22); }
 
 void k_thin_gemm(bool transa, int m, int n, int k, double alpha, const double* A, int lda, size_t sa, const double* B,
                  int ldb, size_t sb, double beta, double* C, int ldc, size_t sc, int batch, cudaStream_t st) {
