@@ -75,6 +75,7 @@ struct DevScratch {
   int4* oinfo;          // [nang*nang] of the first list: as jk_order
   int* ocount;          // [2]
   int* gmask;           // [ceil(nang*nang/8)]
+  unsigned char* jk_on; // [nang*nang] output block in the first list
 };
 
 // Exchange work units (int4: a, b, lo, hi), built once per atom on the host.

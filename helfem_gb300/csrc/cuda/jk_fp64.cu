@@ -480,6 +480,7 @@ __global__ void k_block_norms(DevAtom A, DevScratch S, const double* __restrict_
         S.oinfo[n + __popc(mo & below)] = info;
       }
       if (pass && half) S.olist[nang2 + nh + __popc(mh & below)] = jk;
+      if (pass && x < nang2) S.jk_on[jk] = on;
       n += __popc(mo);
       nh += __popc(mh);
     }
@@ -834,12 +835,17 @@ __global__ void __launch_bounds__(320) k_tiles_split(DevAtom A, DevScratch S, co
 }
 
 // one CTA per element pair (a,b), all output blocks: the first row/column of
-// each tile receives its neighbours' halo entries in a fixed order
-__global__ void k_fixup(DevAtom A, DevScratch S, double* __restrict__ K, int active_only) {
+// each tile receives its neighbours' halo entries in a fixed order. After the
+// tensor-core tiles, which leave out the inactive output blocks: the active
+// ones (FIX_ACTIVE), or all, those without an entry zeroed (FIX_ZERO).
+enum { FIX_ALL, FIX_ACTIVE, FIX_ZERO };
+template <int MODE>
+__global__ void k_fixup(DevAtom A, DevScratch S, double* __restrict__ K) {
   const int a = blockIdx.x % A.nel, b = blockIdx.x / A.nel;
-  const int nn = A.nn, per = 2 * nn - 3, nblk = active_only ? S.ocount[0] : A.nang * A.nang;
+  const int nn = A.nn, per = 2 * nn - 3, nang2 = A.nang * A.nang, nblk = MODE == FIX_ACTIVE ? S.ocount[0] : nang2;
   for (int w = threadIdx.x; w < per * nblk; w += blockDim.x) {
-    const int idx = w % per, jk = active_only ? S.olist[w / per] : w / per;
+    const int idx = w % per, jk = MODE == FIX_ACTIVE ? S.olist[w / per] : w / per;
+    if (MODE == FIX_ZERO && !S.jk_on[jk]) continue;
     const int j = jk % A.nang, k = jk / A.nang;
     int p, q;
     double v;
@@ -863,7 +869,23 @@ __global__ void k_fixup(DevAtom A, DevScratch S, double* __restrict__ K, int act
     if (!gvalid(A, gp) || !gvalid(A, gq)) continue;
     K[(size_t)(k * A.nrad + gq) * A.nbf + (size_t)j * A.nrad + gp] += v;
   }
+  if (MODE != FIX_ZERO) return;
+  for (int jk = 0; jk < nang2; ++jk) {
+    if (S.jk_on[jk]) continue;
+    const int j = jk % A.nang, k = jk / A.nang;
+    for (int w = threadIdx.x; w < (nn - 1) * (nn - 1); w += blockDim.x) {
+      const int gp = gfun(A, a, w % (nn - 1)), gq = gfun(A, b, w / (nn - 1));
+      if (gvalid(A, gp) && gvalid(A, gq)) K[(size_t)(k * A.nrad + gq) * A.nbf + (size_t)j * A.nrad + gp] = 0.0;
+    }
+  }
 }
+
+// Inactive output blocks: zeroed in the fix-up where K is small, otherwise by a
+// kernel of their own beside the tiles. A launch after the diagonal tiles is 3 to 4
+// us of a small build's time (l = 0, 5 elements of 6 nodes, tile stage 18.1 us
+// with it, 14.1 without; l <= 1, 10 elements of 15 nodes, whole K 62.5 and 59.2),
+// while Rn's 240 inactive blocks are 300 MB of writes.
+inline bool zero_in_fixup(const DevAtom& A) { return A.nang <= 4 && A.nbf <= 1024; }
 
 inline int threads_for(int n2) { return ((n2 + 31) / 32) * 32; }
 
@@ -943,7 +965,7 @@ cudaError_t launch_exchange_erfc(const DevAtom& A, const DevScratch& S, const do
   }
   {
     Mark m(prof, KC_K_FIXUP, st);
-    k_fixup<<<A.nel * A.nel, 256, 0, st>>>(A, S, K, 0);
+    k_fixup<FIX_ALL><<<A.nel * A.nel, 256, 0, st>>>(A, S, K);
   }
   return cudaGetLastError();
 }
@@ -956,6 +978,7 @@ template <class Pairs>
 static cudaError_t launch_tiles_tc(const DevAtom& A, const DevScratch& S, const DevTC& tc, bool symmetric,
                                    const double* P, double* K, cudaStream_t st, const SideStream* side, Pairs&& pairs) {
   const int nang2 = A.nang * A.nang;
+  const bool apart = !zero_in_fixup(A);
   cudaError_t e = cudaSuccess;
   if (side && side->s) {
     // the diagonal stage (a chain of dependent steps in 0.8 of a wave)
@@ -965,7 +988,7 @@ static cudaError_t launch_tiles_tc(const DevAtom& A, const DevScratch& S, const 
     // (the FP64 and float-pair kernels first: a diagonal CTA takes an SM whole)
     if (e == cudaSuccess && !tc.digits) e = pairs();
     if (e == cudaSuccess) e = launch_k_diag_tc(A, S, tc, symmetric, P, K, side->s);
-    if (e == cudaSuccess) k_zero_inactive<<<dim3(nang2, 8), 256, 0, side->s>>>(A, S, K, symmetric ? 1 : 0);
+    if (e == cudaSuccess && apart) k_zero_inactive<<<dim3(nang2, 8), 256, 0, side->s>>>(A, S, K, symmetric ? 1 : 0);
     const cudaError_t j = cudaEventRecord(side->join, side->s);
     if (e == cudaSuccess) e = j;
     if (e == cudaSuccess && tc.digits) e = pairs();
@@ -974,7 +997,7 @@ static cudaError_t launch_tiles_tc(const DevAtom& A, const DevScratch& S, const 
   } else {
     e = pairs();
     if (e == cudaSuccess) e = launch_k_diag_tc(A, S, tc, symmetric, P, K, st);
-    if (e == cudaSuccess) k_zero_inactive<<<dim3(nang2, 8), 256, 0, st>>>(A, S, K, symmetric ? 1 : 0);
+    if (e == cudaSuccess && apart) k_zero_inactive<<<dim3(nang2, 8), 256, 0, st>>>(A, S, K, symmetric ? 1 : 0);
   }
   return e;
 }
@@ -1006,7 +1029,7 @@ cudaError_t launch_exchange_fp64(const DevAtom& A, const DevScratch& S, const KU
     }
     {
       Mark m(prof, KC_K_FIXUP, st);
-      k_fixup<<<A.nel * A.nel, 256, 0, st>>>(A, S, K, 1);
+      (zero_in_fixup(A) ? k_fixup<FIX_ZERO> : k_fixup<FIX_ACTIVE>)<<<A.nel * A.nel, 256, 0, st>>>(A, S, K);
     }
     return cudaGetLastError();
   }
@@ -1026,7 +1049,7 @@ cudaError_t launch_exchange_fp64(const DevAtom& A, const DevScratch& S, const KU
   }
   {
     Mark m(prof, KC_K_FIXUP, st);
-    k_fixup<<<A.nel * A.nel, 256, 0, st>>>(A, S, K, 0);
+    k_fixup<FIX_ALL><<<A.nel * A.nel, 256, 0, st>>>(A, S, K);
   }
   return cudaGetLastError();
 }
@@ -1064,7 +1087,8 @@ cudaError_t launch_exchange_split(const DevAtom& A, const DevScratch& S, const K
   }
   {
     Mark m(prof, KC_K_FIXUP, st);
-    k_fixup<<<A.nel * A.nel, 256, 0, st>>>(A, S, K, tc ? 1 : 0);
+    (!tc ? k_fixup<FIX_ALL> : zero_in_fixup(A) ? k_fixup<FIX_ZERO> : k_fixup<FIX_ACTIVE>)
+        <<<A.nel * A.nel, 256, 0, st>>>(A, S, K);
   }
   return cudaGetLastError();
 }

@@ -72,6 +72,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cstdint>
 #include <type_traits>
@@ -1251,12 +1252,13 @@ cudaError_t launch_k_diag_tc(const DevAtom& A, const DevScratch& S, const DevTC&
   const int nblk = symmetric ? A.nang * (A.nang + 1) / 2 : A.nang * A.nang;
   Td.dgroups = (nblk + DSLOT - 1) / DSLOT;
   const int n = A.nel * T.dmtiles * Td.dgroups;
-  // as many stages as fit (four up to 16 nodes, three for 17)
+  // as many stages as fit (four up to 16 nodes, three for 17) and there are steps
+  // for: with less shared memory element-pair tiles run on the same SM
   int dev = 0, most = 0;
   cudaError_t e0 = cudaGetDevice(&dev);
   if (e0 == cudaSuccess) e0 = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e0 != cudaSuccess) return e0;
-  Td.dstages = DST;
+  Td.dstages = std::min(DST, A.NL * T.dksteps);
   while (Td.dstages > 2 && tc_diag_smem_bytes(A.NL, T.dksteps, A.nang, Td.dstages) > (size_t)most) --Td.dstages;
   const size_t smem = tc_diag_smem_bytes(A.NL, T.dksteps, A.nang, Td.dstages);
   const bool wide = DSLOT * 2 * T.dksteps > 512;

@@ -169,7 +169,7 @@ struct hfg_atom {
   // device copies of the tables
   DBuf d_rs, d_rb, d_cholp, d_rank, d_tk, d_chanL, d_jket_ptr, d_jket_blk, d_jket_coef, d_jbra_ptr,
       d_jbra_chan, d_jbra_coef, d_kjk_ptr, d_kent_L, d_kent_ptr, d_kterm_blk, d_kterm_off, d_kterm_coef;
-  DBuf d_order, d_kterm_L, d_kterm_ent, d_kent_sig, s_olist, s_oinfo, s_ocount, s_gmask;
+  DBuf d_order, d_kterm_L, d_kterm_ent, d_kent_sig, s_olist, s_oinfo, s_ocount, s_gmask, s_jkon;
   DBuf s_jin, s_jscal, s_khalo, s_bnorm, s_count, s_tmax, s_p2, s_act, s_entact;
   DBuf d_rs2, d_rb2, d_tk2, d_kcoef2, d_jkc2, d_jbc2, d_cholp2;
   DBuf d_units_all, d_units_sym, d_diag_all, d_diag_sym;
@@ -655,6 +655,8 @@ struct hfg_atom {
     scr.olist = s_olist.as<int>();
     scr.ocount = s_ocount.as<int>();
     scr.gmask = s_gmask.as<int>();
+    s_jkon.alloc((size_t)A.nang * A.nang);
+    scr.jk_on = s_jkon.as<unsigned char>();
     ck(cudaEventCreateWithFlags(&last_use, cudaEventDisableTiming), "cudaEventCreate");
     auto split = [](const std::vector<double>& v) {
       std::vector<float2> o(v.size());
