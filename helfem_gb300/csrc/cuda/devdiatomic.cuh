@@ -180,6 +180,9 @@ cudaError_t launch_diatomic_tx(const DevDiatomic& D, double* tx, cudaStream_t st
 // J of a pure-basis density, written to the pure-basis J (overwritten)
 cudaError_t launch_diatomic_coulomb(const DevDiatomic& D, const DevDiatomicScratch& S, const double* P, double* J,
                                     cudaStream_t st);
+// one output block per item, FP64 (short elements)
+cudaError_t launch_diatomic_exchange_items(const DevDiatomic& D, const DevDiatomicScratch& S, const double* Pd,
+                                           double* Kd, bool symmetric, cudaStream_t st);
 // tc: the in-element tiles on the tensor cores, or nullptr for the FP64 kernels (T)
 cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDia64& T,
                                      const DevDiaTC* tc, const double* Pd, double* Kd, bool symmetric, cudaStream_t st,

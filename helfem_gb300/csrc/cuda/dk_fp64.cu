@@ -19,14 +19,16 @@
 //   dk_share.cu       : the element-pair tiles (FP64 and float pairs) and the
 //                       in-element tiles (FP64), with the recoupling shared by
 //                       the output blocks of one k; dk_tc.cu: the in-element
-//                       tiles of the split form on the tensor cores.
+//                       tiles on the tensor cores.
+//   dk_tiles          : both kinds of tiles, one output block at a time (FP64,
+//                       short elements).
 //   dk_fixup          : the shared-boundary contributions of neighbouring
 //                       tiles, added in a fixed order (bitwise reproducible).
 #include <algorithm>
 #include <cfloat>
 
-#include "devdiatomic.cuh"
-#include "ff.cuh"
+#include "dk_recouple.cuh"
+#include "smem_limit.hpp"
 
 namespace hfg {
 namespace {
@@ -356,6 +358,139 @@ __device__ __forceinline__ size_t dhalo_idx(const DevDiatomic& D, int a, int b, 
   return ((size_t)(a * D.nel + b) * (D.nang * D.nang) + jk) * (2 * D.nn - 1) + h;
 }
 
+// ------------------------------------------------- one output block per item
+// Element-pair and in-element tiles in FP64, one output block per item: shares
+// nothing between the blocks of one k, but an item is short and needs a tenth of
+// the shared memory. For elements of three to five nodes, whose tiles fill less
+// than a warp, more items in flight outweigh the sharing where there are many
+// pairs (use_items64 in dcapi.cpp has the line). 12 elements of 3 nodes, l <= 4, m
+// <= 1, a density that does not mix m: 206 us, with the shared recoupling 367.
+//
+// Persistent CTAs over work items. Item w < n_off: element pair
+// pairs[w / n_act], output block jk_list[w % n_act]; the rest: diagonal
+// element e, output block from the (symmetric: j <= k) list. In symmetric
+// mode (P = P^T) only a < b pairs are items and each also writes the
+// transposed partner tile, K_kj(b,a) = K_jk(a,b)^T.
+__global__ void __launch_bounds__(320) dk_tiles(DevDiatomic D, DevDiatomicScratch S, const double* __restrict__ Pd,
+                                                double* __restrict__ Kd, int symmetric) {
+  const int nn = D.nn, n2 = nn * nn, nang2 = D.nang * D.nang;
+  const int n_act = S.counts[0], n_dact = symmetric ? S.counts[1] : S.counts[0];
+  const int* dlist = symmetric ? S.jk_list + nang2 : S.jk_list;
+  const int2* pairs = symmetric ? D.pairs_sym : D.pairs_all;
+  const long npairs = symmetric ? D.npairs_sym : D.npairs_all;
+  const long n_off = npairs * n_act, total = n_off + (long)D.nel * n_dact;
+  extern __shared__ double sm[];
+  double* X = sm;            // [4*n2]: R00, R02, R20, R22 tiles
+  double* T = X + 4 * n2;    // [2*n2]
+  double* Im = T + 2 * n2;   // [2*n2] row-element integrals (channel 0, 2)
+  double* Jm = Im + 2 * n2;  // [2*n2] column-element integrals
+  unsigned char* act = reinterpret_cast<unsigned char*>(Jm + 2 * n2);
+  for (int idx = threadIdx.x; idx < nang2; idx += blockDim.x) act[idx] = S.act[idx];
+  __syncthreads();
+  const int t = threadIdx.x;
+  const bool live = t < n2;
+  const int p = live ? t % nn : 0, q = live ? t / nn : 0;
+  for (long w = blockIdx.x; w < total; w += gridDim.x) {
+    int a, b, jk;
+    if (w < n_off) {
+      const int2 pr = pairs[w / n_act];
+      a = pr.x;
+      b = pr.y;
+      jk = S.jk_list[w % n_act];
+    } else {
+      const long w2 = w - n_off;
+      a = b = (int)(w2 / n_dact);
+      jk = dlist[w2 % n_dact];
+    }
+    const bool diag = (a == b);
+    const int j = jk % D.nang, k = jk / D.nang;
+    const int gp = dgf(D, a, p), gq = dgf(D, b, q);
+    const bool vpq = live && gp < D.nrad && gq < D.nrad;
+    double y = 0.0;
+    for (int ent = D.kjk_ptr[jk]; ent < D.kjk_ptr[jk + 1]; ++ent) {
+      if (!S.ent_act[ent]) continue;  // uniform over the CTA
+      const int L = D.kent_L[ent], Ma = D.kent_Ma[ent], ilm = D.kent_ilm[ent];
+      double x00 = 0.0, x02 = 0.0, x20 = 0.0, x22 = 0.0;
+      if (vpq) {
+        for (int sgn = 0; sgn < (Ma ? 2 : 1); ++sgn) {
+          const int M = sgn ? -Ma : Ma;
+          const int xj = al_idx(D, j, L, M), xk = al_idx(D, k, L, M);
+          const int k0 = D.al_ptr[xk], k1 = D.al_ptr[xk + 1];
+          for (int uj = D.al_ptr[xj]; uj < D.al_ptr[xj + 1]; ++uj) {
+            const int i = D.al_b[uj];
+            const double* Pi = Pd + (size_t)i * D.nrad + gp;
+            double u0 = 0.0, u2 = 0.0;
+            for (int uk = k0; uk < k1; ++uk) {
+              const int l = D.al_b[uk];
+              if (!act[i + l * D.nang]) continue;
+              const double v = Pi[(size_t)(l * D.nrad + gq) * D.nd];
+              u0 += D.al_c0[uk] * v;
+              u2 += D.al_c2[uk] * v;
+            }
+            const double c0 = D.al_c0[uj], c2 = D.al_c2[uj];
+            x00 += c0 * u0;
+            x02 += c0 * u2;
+            x20 += c2 * u0;
+            x22 += c2 * u2;
+          }
+        }
+      }
+      const double fac = (Ma & 1) ? -D.lmfac[ilm] : D.lmfac[ilm];
+      if (live) {
+        X[t] = fac * x00;
+        X[n2 + t] = -fac * x02;
+        X[2 * n2 + t] = -fac * x20;
+        X[3 * n2 + t] = fac * x22;
+        if (!diag) {
+          const size_t la = ((size_t)ilm * D.nel + a) * n2 + t, lb = ((size_t)ilm * D.nel + b) * n2 + t;
+          Im[t] = (a < b) ? D.p0[la] : D.q0[la];
+          Im[n2 + t] = (a < b) ? D.p2[la] : D.q2[la];
+          Jm[t] = (a < b) ? D.q0[lb] : D.p0[lb];
+          Jm[n2 + t] = (a < b) ? D.q2[lb] : D.p2[lb];
+        }
+      }
+      __syncthreads();
+      if (diag) {
+        if (live) {
+          const double* tx = D.tx + ((size_t)ilm * D.nel + a) * 4 * n2 * n2;
+          double s = 0.0;
+          for (int ab = 0; ab < 4; ++ab) {
+            const double* txb = tx + (size_t)ab * n2 * n2;
+            const double* Xb = X + ab * n2;
+            for (int v = 0; v < n2; ++v) s += txb[t + (size_t)v * n2] * Xb[v];
+          }
+          y += s;
+        }
+      } else {
+        if (live) {
+          double s0 = 0.0, s2 = 0.0;
+          for (int c = 0; c < nn; ++c) {
+            const double j0 = Jm[q + c * nn], j2 = Jm[n2 + q + c * nn];
+            s0 += X[p + c * nn] * j0 + X[n2 + p + c * nn] * j2;
+            s2 += X[2 * n2 + p + c * nn] * j0 + X[3 * n2 + p + c * nn] * j2;
+          }
+          T[t] = s0;
+          T[n2 + t] = s2;
+        }
+        __syncthreads();
+        if (live) {
+          double s = 0.0;
+          for (int c = 0; c < nn; ++c) s += Im[p + c * nn] * T[c + q * nn] + Im[n2 + p + c * nn] * T[n2 + c + q * nn];
+          y += s;
+        }
+      }
+      __syncthreads();
+    }
+    if (live) share_store(D, S, Kd, a, b, jk, p, q, -y);
+    if (symmetric && (!diag || j != k)) {
+      if (live) X[t] = -y;
+      __syncthreads();
+      if (live) share_store(D, S, Kd, b, a, k + j * D.nang, p, q, X[q + p * nn]);
+      __syncthreads();
+    }
+  }
+}
+
 // Shared-boundary fix-up: entry (p,q) of tile (a,b) in its first row or
 // column also receives the last row of the tile above (a-1,b), the last
 // column of the tile to the left (a,b-1) and, at the corner, the last corner
@@ -386,6 +521,19 @@ __global__ void dk_fixup(DevDiatomic D, DevDiatomicScratch S, double* __restrict
     if (gp >= D.nrad || gq >= D.nrad) continue;
     Kd[(size_t)(k * D.nrad + gq) * D.nd + (size_t)j * D.nrad + gp] += v;
   }
+}
+
+// screening: active blocks and entries, compacted lists
+cudaError_t screen(const DevDiatomic& D, const DevDiatomicScratch& S, const double* Pd, float2* pd2, double* Kd,
+                   bool symmetric, cudaStream_t st) {
+  const int nang2 = D.nang * D.nang;
+  const cudaError_t e = cudaMemsetAsync(Kd, 0, sizeof(double) * (size_t)D.nd * D.nd, st);
+  if (e != cudaSuccess) return e;
+  dk_norms<<<dim3(nang2, DNORM_SPLIT), 256, 0, st>>>(D, Pd, S.bnorm, pd2);
+  dk_act<<<(nang2 + 255) / 256, 256, 0, st>>>(D, S);
+  dk_entry_act<<<std::max(1, (D.nent + 127) / 128), 128, 0, st>>>(D, S);
+  dk_compact<<<1, 1024, 0, st>>>(D, S, symmetric ? 1 : 0);
+  return cudaGetLastError();
 }
 
 inline int dthreads(int n2) { return ((n2 + 31) / 32) * 32; }
@@ -428,13 +576,8 @@ cudaError_t launch_diatomic_coulomb(const DevDiatomic& D, const DevDiatomicScrat
 template <class Diag>
 static cudaError_t exchange_stages(const DevDiatomic& D, const DevDiatomicScratch& S, const double* Pd, float2* pd2,
                                    double* Kd, bool symmetric, cudaStream_t st, const SideStream& side, Diag&& diag) {
-  const int nang2 = D.nang * D.nang;
-  cudaError_t e = cudaMemsetAsync(Kd, 0, sizeof(double) * (size_t)D.nd * D.nd, st);
+  cudaError_t e = screen(D, S, Pd, pd2, Kd, symmetric, st);
   if (e != cudaSuccess) return e;
-  dk_norms<<<dim3(nang2, DNORM_SPLIT), 256, 0, st>>>(D, Pd, S.bnorm, pd2);
-  dk_act<<<(nang2 + 255) / 256, 256, 0, st>>>(D, S);
-  dk_entry_act<<<std::max(1, (D.nent + 127) / 128), 128, 0, st>>>(D, S);
-  dk_compact<<<1, 1024, 0, st>>>(D, S, symmetric ? 1 : 0);
   if ((e = cudaEventRecord(side.fork, st)) != cudaSuccess) return e;
   if ((e = cudaStreamWaitEvent(side.s, side.fork, 0)) != cudaSuccess) return e;
   e = diag(side.s);
@@ -444,6 +587,22 @@ static cudaError_t exchange_stages(const DevDiatomic& D, const DevDiatomicScratc
   const cudaError_t w = cudaStreamWaitEvent(st, side.join, 0);  // (joined whatever failed)
   if (e == cudaSuccess) e = w;
   if (e != cudaSuccess) return e;
+  dk_fixup<<<D.nel * D.nel, 256, 0, st>>>(D, S, Kd);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_diatomic_exchange_items(const DevDiatomic& D, const DevDiatomicScratch& S, const double* Pd,
+                                           double* Kd, bool symmetric, cudaStream_t st) {
+  cudaError_t e = screen(D, S, Pd, nullptr, Kd, symmetric, st);
+  if (e != cudaSuccess) return e;
+  const int n2 = D.nn * D.nn, th = dthreads(n2);
+  const size_t smem = sizeof(double) * 10 * n2 + (size_t)D.nang * D.nang;
+  if ((e = smem_limit(dk_tiles, smem)) != cudaSuccess) return e;
+  int dev = 0, nsm = 152, per = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dk_tiles, th, smem)) != cudaSuccess) return e;
+  dk_tiles<<<nsm * std::max(per, 1), th, smem, st>>>(D, S, Pd, Kd, symmetric ? 1 : 0);
   dk_fixup<<<D.nel * D.nel, 256, 0, st>>>(D, S, Kd);
   return cudaGetLastError();
 }

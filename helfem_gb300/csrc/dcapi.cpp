@@ -376,14 +376,36 @@ struct hfg_diatomic {
   }
 
   // scratch of the FP64 in-element tiles, on the first FP64 exchange
-  // The FP64 in-element tiles on the tensor cores. Their K steps and tiles are
-  // padded, which short elements do not pay back: K of l = 0..3 on three
-  // elements of 6 nodes 110 us on the FP64 kernels and 115 us here, of 8 nodes
-  // 131 and 121, of 15 nodes 302 and 185; l <= 5, m <= 1 on six elements of 8
-  // nodes 1711 and 1353, of 15 nodes 10.9 and 6.3 ms.
-  bool use_tc64() const { return host.nn >= 8; }
+  // The FP64 in-element tiles on the tensor cores or on the FP64 kernels. The
+  // digit form pads its K steps and tiles and fills 128 rows with output blocks,
+  // which short elements and few shells do not pay back. Measured, us, FP64
+  // kernels and this form: one shell, 5 elements of 10 nodes 69 and 93, of 15
+  // nodes 84 and 120, of 17 nodes 174 and 136; 4 shells, 3 to 5 elements of 6
+  // nodes 90 and 93, of 8 nodes 114 and 99, of 15 nodes 345 and 246; 9 shells (l
+  // <= 4, m <= 1), 5 elements of 4 nodes 159 and 156, of 5 nodes 191 and 160; 29
+  // shells (l <= 6, m <= 2), 5 elements of 3 nodes 1900 and 1827, of 7 nodes 5375
+  // and 3944.
+  bool use_tc64() const {
+    const int nn = host.nn, nang = host.nang;
+    return nang == 1 ? nn >= 16 : nang < 8 ? nn >= 8 : nang < 16 ? nn >= 5 : true;
+  }
+  // Both kinds of tiles one output block at a time: elements of up to five nodes,
+  // a warp or less per tile, with many (pair, k) items, or one shell, where there
+  // is nothing to share and the other forms' launches remain. Us, here and the
+  // better of the other two: 9 shells, 66 pairs of 3 nodes 206 and 367 (a density
+  // that does not mix m), of 5 nodes 310 and 423; 10 pairs of 3 nodes 141 and 148,
+  // of 4 nodes 172 and 156; 29 shells, 10 pairs of 5 nodes 881 and 1007; 4 shells,
+  // 66 pairs of 4 nodes 108 and 110, of 5 nodes 136 and 117; one shell, 3 elements
+  // of 3 nodes 57 and 65.
+  bool use_items64() const {
+    const int nn = host.nn, nang = host.nang, nel = host.nel;
+    if (nn > 5) return false;
+    const long items = (long)nel * (nel - 1) / 2 * nang;
+    return nang == 1 || (nn == 3 ? items >= 80 : nn == 4 ? items >= 100 : nang >= 8 && items >= 250);
+  }
   // The plain form's in-element kernels, decided by the handle's first plain
-  // exchange (they differ in the last bits of K): 1 tensor cores, 2 FP64
+  // exchange (they differ in the last bits of K): 1 tensor cores, 2 FP64, 3 one
+  // output block per item (both kinds of tiles)
   int plain_form = 0;
   // device bytes that first calls may take, 0: what is free
   size_t scratch_limit = 0;
@@ -554,7 +576,7 @@ struct hfg_diatomic {
       if (exchange) ensure_side();
       if (split) ensure_split();
       if (!split && exchange) {
-        if (!plain_form) plain_form = use_tc64() && ensure_tc(false) ? 1 : 2;
+        if (!plain_form) plain_form = use_items64() ? 3 : use_tc64() && ensure_tc(false) ? 1 : 2;
         if (plain_form == 2) ensure_fp64();
         tc64 = plain_form == 1;
       }
@@ -569,6 +591,9 @@ struct hfg_diatomic {
       ck(hfg::launch_diatomic_exchange_split(dev, scr, tc, s_Pd.as<double>(), s_Fd.as<double>(), symmetric, st,
                                              k_side, itemwise),
          "exchange (split)");
+    else if (plain_form == 3)
+      ck(hfg::launch_diatomic_exchange_items(dev, scr, s_Pd.as<double>(), s_Fd.as<double>(), symmetric, st),
+         "exchange (items)");
     else
       ck(hfg::launch_diatomic_exchange(dev, scr, t64, tc64 ? &tc : nullptr, s_Pd.as<double>(), s_Fd.as<double>(),
                                        symmetric, st, k_side),

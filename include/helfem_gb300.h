@@ -576,8 +576,8 @@ hfg_status hfg_diatomic_coulomb(hfg_diatomic* d, const double* P, double* J, voi
  * ndummy^2 float-pair density, the digit planes of the in-element kernel (14
  * bytes for each of its entries, rows padded to 64 and columns to 16) and digit
  * scratch of at most 4.7 GB. The first plain call makes the planes and that
- * scratch too or, where it uses the FP64 kernels for these tiles (elements of
- * few nodes, or less than the planes and 8 GB free), at most 2 GB. Less is taken
+ * scratch too or, where it uses the FP64 kernels for these tiles (few nodes and
+ * shells, or less than the planes and 8 GB free), at most 2 GB. Less is taken
  * where less is free; the handle keeps the kernels of its first plain call.
  * hfg_diatomic_scratch_limit: device bytes that first calls made after it may
  * take (0: what is free). */
