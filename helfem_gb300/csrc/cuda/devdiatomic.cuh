@@ -123,7 +123,7 @@ struct DevDiatomicScratch {
   int* jk_pos;            // [nang^2] position in the call's list of output blocks, or -1
   int* kg_list;           // active (k*ngrp + g), then (k*ngrp8 + g) of the in-element items
   // [0] active output blocks, [1] those with j <= k, [2] and [3] the lengths of
-  // the two kg lists, [4] and [5] item counters
+  // the two kg lists, [4] item counter
   int* counts;
   float2* pd2;            // [nd*nd] split copy of the density (split path)
   // off-diagonal pairs in parts of the multipole sum: part sums of each item's
@@ -189,7 +189,6 @@ cudaError_t launch_diatomic_exchange(const DevDiatomic& D, const DevDiatomicScra
                                      const SideStream& side);
 cudaError_t launch_dk_tc_table(const DevDiatomic& D, const DevDiaTC& T, unsigned char* tx, int* txexp, int* cexp,
                                cudaStream_t st);
-size_t dtc_gemm_smem(const DevDiatomic& D, bool f64);
 cudaError_t launch_dk_tc_diag(const DevDiatomic& D, const DevDiatomicScratch& S, const DevDiaTC& T, const double* Pd,
                               double* Kd, bool symmetric, bool itemwise, cudaStream_t st);
 // split-precision exchange: off-diagonal element pairs in float pairs, the

@@ -351,7 +351,7 @@ __global__ void dk_compact(DevDiatomic D, DevDiatomicScratch S, int symmetric) {
   for (int x = lo; x < hi; ++x)
     if (row_active(x / D.ngrp8, D.grp8_ptr, x % D.ngrp8, symmetric != 0))
       S.kg_list[(size_t)D.nang * D.ngrp + od++] = x;
-  if (threadIdx.x == 0) S.counts[4] = S.counts[5] = 0;
+  if (threadIdx.x == 0) S.counts[4] = 0;
 }
 
 __device__ __forceinline__ size_t dhalo_idx(const DevDiatomic& D, int a, int b, int jk, int h) {

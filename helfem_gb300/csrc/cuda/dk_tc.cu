@@ -646,7 +646,7 @@ cudaError_t launch_dk_tc_table(const DevDiatomic& D, const DevDiaTC& T, unsigned
   return cudaGetLastError();
 }
 
-size_t dtc_gemm_smem(const DevDiatomic& D, bool f64) {
+static size_t dtc_gemm_smem(const DevDiatomic& D, bool f64) {
   return (size_t)NSTAGE * ((f64 ? TD : XD) * APL + TD * BPL) + 8 * (2 * NSTAGE + 3) + 4 * (4 + (size_t)D.nlm);
 }
 

@@ -186,7 +186,7 @@ struct hfg_diatomic {
     s_jkpos.alloc(sizeof(int) * nang2);
     scr.jk_pos = s_jkpos.as<int>();
     s_kglist.alloc(sizeof(int) * (size_t)H.nang * (D.ngrp + D.ngrp8));
-    s_counts.alloc(sizeof(int) * 6);
+    s_counts.alloc(sizeof(int) * 5);
     s_Pd.alloc(sizeof(double) * nd * nd);
     s_Fd.alloc(sizeof(double) * nd * nd);
     scr.jin = s_jin.as<double>();

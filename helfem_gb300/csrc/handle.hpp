@@ -205,9 +205,13 @@ struct hfg_atom {
   // 63 and 59 (m-diagonal density), 95 and 98 (general mode), of 10 nodes 79 and
   // 62, 130 and 101; l <= 3, 20 elements of 8 nodes 255 and 266, dense 1016 and
   // 1517; two shells, 20 elements of 9 nodes 48 and 53, of 10 nodes 57 and 56, 60
-  // elements of 10 nodes 125 and 152, of 13 nodes 274 and 185; l = 0, 6 elements
-  // of 15 nodes 44 and 38, 20 elements 46 and 50; Kr (l <= 2, 40 elements of 15
-  // nodes, dense) 4520 and 1004.
+  // elements of 10 nodes 125 and 152, of 13 nodes 274 and 185; l = 0, 15 nodes,
+  // symmetric (general mode), 5 elements 41 (42) and 34 (34), 10 elements 45 (45)
+  // and 35 (35), 15 elements 46 (46) and 35 (45), 20 elements 45 (47) and 46 (49),
+  // 10 elements of 13 nodes 37 (38) and 32 (33), of 10 nodes 31 (31) and 31 (29);
+  // Kr (l <= 2, 40 elements of 15 nodes, dense) 4520 and 1004. Where tc_setup makes
+  // no tables (a basis that repeats angular functions, with more than 64 terms a
+  // block) every form stays on the FP64 and float-pair kernels.
   const hfg::DevTC* tc64_for(bool screened) const {
     const int nn = host.rad.nn, nang = host.nang, nel = host.rad.nel;
     const bool on = nang >= 3 ? nn >= 10 : nang == 2 ? nn >= (nel <= 24 ? 10 : 12) : nn >= 15 && nel <= 10;
