@@ -431,13 +431,15 @@ struct PairMeta {
 }  // namespace
 
 // NaN in every result of a unit whose CTA gave up, the transposed partners' too
-// (out of line: inside k_tiles_tc it cost 1 % of Kr's K)
-__device__ __noinline__ void mark_unit(const DevAtom& A, const DevScratch& S, const int4* __restrict__ units,
-                                       int symmetric, double* K) {
-  const int4 u = units[blockIdx.x];
-  const int nn = A.nn, end = min(8 * u.w, S.ocount[0]);
+// (out of line and with plain arguments: inside k_tiles_tc it cost 1 % of Kr's K)
+__device__ __noinline__ void mark_unit(int4 u, int end, int symmetric, int nn, int nel, int nrad, int nang, int nbf,
+                                       const int* __restrict__ olist, double* khalo, double* K) {
+  DevAtom A;
+  A.nn = nn, A.nel = nel, A.nrad = nrad, A.nang = nang, A.nbf = nbf;
+  DevScratch S;
+  S.khalo = khalo;
   for (int x = 8 * u.z + (int)(threadIdx.x >> 5); x < end; x += PW) {
-    const int jk = S.olist[x], kj = jk / A.nang + jk % A.nang * A.nang;
+    const int jk = olist[x], kj = jk / nang + jk % nang * nang;
     for (int i = threadIdx.x & 31; i < nn * nn; i += 32) {
       const double bad = __longlong_as_double(0x7ff8000000000000ll);
       k_store_tile(A, S, K, u.x, u.y, jk, i % nn, i / nn, bad);
@@ -863,7 +865,8 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_tiles_tc(DevAtom A, DevScratch 
       if (!tc::mbar_wait(&m.done, (uint32_t)(m.fail & 1), kWait))
         for (int i = 0; i < 100; ++i) __nanosleep(1000);
     }
-    mark_unit(A, S, units, symmetric, K);
+    const int4 v = units[blockIdx.x];
+    mark_unit(v, min(8 * v.w, S.ocount[0]), symmetric, A.nn, A.nel, A.nrad, A.nang, A.nbf, S.olist, S.khalo, K);
   }
   tc::fence_before_sync();
   __syncthreads();
