@@ -498,10 +498,11 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
 #pragma unroll
   for (int j = 0; j < 32; ++j) acc[j] = 0.0;
 
+  int copied = 0;  // K steps whose copies were started (by the copying thread)
   if (warp == 8) {
     if (lane == 0) {
       bool ok = true;
-      int it = 0;
+      int& it = copied;
       for (int a = 0; a < na && ok; ++a) {
         const unsigned char* xs = T.x + ((size_t)lu * D.nlm + act[a]) * T.ksteps * NX * APL;
         const unsigned char* ts = T.tx + (((size_t)act[a] * D.nel + e) * T.ntt + tt) * T.ksteps * TD * BPL;
@@ -516,12 +517,7 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
           tc::bulk_g2s(Bbuf + s * TD * BPL, ts + (size_t)ks * TD * BPL, TD * BPL, &full[s]);
         }
       }
-      if (!ok) {
-        atomicExch(fail, 1);
-        // the copies in flight must land before the CTA leaves
-        for (int i = max(0, it - NSTAGE); i < it; ++i)
-          tc::mbar_wait(&full[i % NSTAGE], (uint32_t)((i / NSTAGE) & 1), kWait);
-      }
+      if (!ok) atomicExch(fail, 1);
     }
   } else if (warp == 9) {
     if (lane == 0) {
@@ -608,6 +604,10 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
     for (int j = 0; j < 32; ++j)
       o[(size_t)j * 128] = bad ? __longlong_as_double(0x7ff8000000000000ll) : acc[j];
   }
+  // the copies in flight must land before the CTA leaves
+  if (fail[0] && copied > 0)
+    for (int i = max(0, copied - NSTAGE); i < copied; ++i)
+      tc::mbar_wait(&full[i % NSTAGE], (uint32_t)((i / NSTAGE) & 1), kWait);
   if (warp == 9 && lane == 0 && fail[0]) {
     atomicExch(T.err, 1);
     // products may still be running: the tensor memory is released after them

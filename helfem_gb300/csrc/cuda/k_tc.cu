@@ -1022,10 +1022,11 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = {};
 
+  int copied = 0;  // copies started (by the copying thread)
   if (warp == DW) {
     if (lane == 0) {
       bool ok = true;
-      int it = 0;
+      int& it = copied;
       for (int n = 0; n < na && ok; ++n) {
         const unsigned char* Ag =
             T.tk_digits + (((size_t)actL[n] * A.nel + a) * mtiles + mt) * ksteps * ND * APLANE;
@@ -1039,11 +1040,7 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
           tc::bulk_g2s(Abuf + s * ND * APLANE, Ag + (size_t)ks * ND * APLANE, ND * APLANE, &full[s]);
         }
       }
-      if (!ok) {
-        atomicExch(fail, 1);
-        // the copies in flight must land before the CTA leaves
-        for (int i = max(0, it - nst); i < it; ++i) tc::mbar_wait(&full[i % nst], (uint32_t)((i / nst) & 1), kWait);
-      }
+      if (!ok) atomicExch(fail, 1);
     }
   } else if (warp == DW + 1) {
     if (lane == 0) {
@@ -1207,6 +1204,10 @@ __global__ void __launch_bounds__(DTHREADS, 1) k_diag_tc(DevAtom A, DevScratch S
       if (symmetric && j0 != k0) k_store_tile(A, S, K, a, a, k0 + j0 * A.nang, q, p, y);
     }
   }
+  // the copies in flight must land before the CTA leaves
+  if (failed && copied > 0)
+    for (int i = max(0, copied - nst); i < copied; ++i)
+      tc::mbar_wait(&full[i % nst], (uint32_t)((i / nst) & 1), kWait);
   if (failed && warp == DW + 1 && lane == 0) {
     atomicExch(T.err, 1);
     // products may still be running: the tensor memory is released after them

@@ -10,10 +10,13 @@ pytestmark = pytest.mark.gpu
 DEFAULT = 1 << 17
 
 
-# two groups of output blocks per element pair, many, diagonal tiles alone
-@pytest.mark.parametrize("case", [(10, 1, 1, 6, 13), (36, 3, 3, 3, 13), (18, 1, 1, 4, 17)],
-                         ids=lambda c: f"l{c[1]}_e{c[3]}_n{c[4]}")
-@pytest.mark.parametrize("split", [False, True], ids=["plain", "split"])
+# two groups of output blocks per element pair, many, diagonal tiles alone; fewer
+# K steps than copy stages (split form only)
+@pytest.mark.parametrize("case,split", [((10, 1, 1, 6, 13), False), ((10, 1, 1, 6, 13), True),
+                                        ((36, 3, 3, 3, 13), False), ((36, 3, 3, 3, 13), True),
+                                        ((18, 1, 1, 4, 17), False), ((18, 1, 1, 4, 17), True),
+                                        ((4, 0, 0, 3, 4), True), ((10, 1, 1, 3, 4), True)],
+                         ids=lambda c: f"l{c[1]}_e{c[3]}_n{c[4]}" if isinstance(c, tuple) else "split" if c else "plain")
 @pytest.mark.parametrize("mix", [True, False], ids=["dense", "same_m"])
 def test_atomic_wait_runs_out(case, split, mix):
     torch = torch_cuda()
