@@ -59,14 +59,6 @@ constexpr int NSTAGE = 5;
 constexpr int kNoRow = (int)0x80808080;
 constexpr uint32_t kWait = DTC_WAIT;  // limit of the waits of a CTA that gives up
 
-constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: x + M - M rounds |x| < 2^22 to an integer
-__device__ __forceinline__ float rnd(float x) { return __fsub_rn(__fadd_rn(x, kMagic), kMagic); }
-__device__ __forceinline__ float rnd_mul(float x, float s) { return __fsub_rn(__fmaf_rn(x, s, kMagic), kMagic); }
-__device__ __forceinline__ float exp2i(int k) {  // 2^k, k clamped to the normal range
-  k = k < -126 ? -126 : (k > 127 ? 127 : k);
-  return __int_as_float((k + 127) << 23);
-}
-
 // six balanced base-512 digits of a float pair |x| < 2^E (weights 512^-(k+1))
 __device__ __forceinline__ void digits512(float2 x, float s27, float (&d)[XD]) {
   const float h = __fmul_rn(x.x, s27), l = __fmul_rn(x.y, s27);  // scaled to |h| < 2^27
@@ -161,11 +153,6 @@ __device__ __forceinline__ void ld_levels(uint32_t taddr, float (&v)[TD][8]) {
   for (int d = 0; d < TD; ++d)
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[d][j] = __uint_as_float(r[8 * d + j]);
-}
-
-__device__ __forceinline__ uint32_t pack_f16(float a, float b) {
-  const __half2 h = __floats2half2_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&h);
 }
 
 // the active output blocks of the call, and the units that they make

@@ -1,6 +1,8 @@
-// FP64 values as fixed-point integers and back, for the digit planes of the
-// tensor-core kernels.
+// FP64 values as fixed-point integers and back, and rounding to digits, for the
+// digit planes of the tensor-core kernels.
 #pragma once
+
+#include <cuda_fp16.h>
 
 #include <cstdint>
 
@@ -33,6 +35,21 @@ __device__ __forceinline__ double f2d_scaled(float f, int c) {
   const uint32_t bits = __float_as_uint(f), t = bits & 0x7FFFFFFFu;
   const uint32_t hi = t < 0x00800000u ? 0u : ((t >> 3) + (uint32_t)c) | (bits & 0x80000000u);
   return __hiloint2double((int)hi, t < 0x00800000u ? 0 : (int)(bits << 29));
+}
+
+constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: x + M - M rounds |x| < 2^22 to an integer
+
+__device__ __forceinline__ float rnd(float x) { return __fsub_rn(__fadd_rn(x, kMagic), kMagic); }
+// rint(x * s) with one rounding of the product
+__device__ __forceinline__ float rnd_mul(float x, float s) { return __fsub_rn(__fmaf_rn(x, s, kMagic), kMagic); }
+__device__ __forceinline__ float exp2i(int k) {  // 2^k, k clamped to the normal range
+  k = k < -126 ? -126 : (k > 127 ? 127 : k);
+  return __int_as_float((k + 127) << 23);
+}
+
+__device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
+  const __half2 v = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
 }
 
 constexpr int kBadExp = 1 << 20;  // exponent of a tile with a value that is not finite

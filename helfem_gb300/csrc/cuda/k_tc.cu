@@ -93,15 +93,6 @@ constexpr int NDX = 6;          // digits of a density tile (48 bits)
 constexpr int APLANE = 4096;    // bytes of one 128 x 16 bf16 operand plane
 constexpr int TPLANE = 512;     // bytes of one 16 x 16 bf16 table plane
 
-constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: x + M - M rounds |x| < 2^22 to an integer
-
-__device__ __forceinline__ float rnd(float x) { return __fsub_rn(__fadd_rn(x, kMagic), kMagic); }
-// rint(x * s) with one rounding of the product
-__device__ __forceinline__ float rnd_mul(float x, float s) { return __fsub_rn(__fmaf_rn(x, s, kMagic), kMagic); }
-__device__ __forceinline__ float exp2i(int k) {  // 2^k, k clamped to the normal range
-  k = k < -126 ? -126 : (k > 127 ? 127 : k);
-  return __int_as_float((k + 127) << 23);
-}
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);
@@ -225,11 +216,6 @@ __device__ __forceinline__ double pair_to_d(ffv a) {
 }
 
 // ---- element pairs: base 1024 in f16 ----
-
-__device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
-  const __half2 v = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
 
 // all six levels (16 columns apart) of 8 consecutive columns, one wait
 __device__ __forceinline__ void tmem_ld_pairs(uint32_t taddr, float (&v)[PD][4]) {

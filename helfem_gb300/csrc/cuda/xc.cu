@@ -39,28 +39,12 @@
 #include <cfloat>
 
 #include "devatom.cuh"
+#include "reduce.cuh"
 #include "smem_limit.hpp"
 #include "xc_func.cuh"
 
 namespace hfg {
 namespace {
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-__device__ double block_sum(double v, double* red) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  v = warp_sum(v);
-  __syncthreads();
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  double s = 0.0;
-  for (int i = 0; i < nw; ++i) s += red[i];
-  return s;
-}
 
 __device__ __forceinline__ bool gvalid(const DevAtom& A, int g) { return g >= 0 && g < A.nrad; }
 
