@@ -485,6 +485,7 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
 #pragma unroll
   for (int j = 0; j < 32; ++j) acc[j] = 0.0;
 
+  bool bad = false;  // this row's tile has a value that is not finite
   int copied = 0;  // K steps whose copies were started (by the copying thread)
   if (warp == 8) {
     if (lane == 0) {
@@ -545,6 +546,7 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
     for (int a = 0; a < na; ++a) {
       const int ilm = act[a];
       const int E = T.xexp[((size_t)lu * D.nlm + ilm) * 128 + row];
+      bad |= E == kBadExp;
       const int* te = T.txexp + (((size_t)ilm * D.nel + e) * T.ntt + tt) * TT + 32 * half;
       const bool ok = tc::mbar_wait(done, (uint32_t)(a & 1), T.wait);
       if (!__all_sync(0xffffffffu, ok)) {
@@ -556,15 +558,13 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
       for (int g = 0; g < 4; ++g) {
         float v[TD][8];
         ld_levels(col0 + 8 * g, v);
-        if (E != kNoRow) {
+        if (E != kNoRow && E != kBadExp) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             float lv[TD];
 #pragma unroll
             for (int d = 0; d < TD; ++d) lv[d] = v[d][j];
-            if (E == kBadExp) {
-              acc[8 * g + j] = __longlong_as_double(0x7ff8000000000000ll);
-            } else if constexpr (F64) {
+            if constexpr (F64) {
               acc[8 * g + j] += levels512_f64(lv, te[8 * g + j] + E);
             } else {
               float z0, z1, z2;
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(320, 1) dk_tc_gemm(DevDiatomic D, DevDiatomicS
   __syncthreads();
   if (warp < 8) {
     const int row = 32 * (warp & 3) + lane, half = warp >> 2;
-    const bool bad = fail[0] != 0;
+    bad |= fail[0] != 0;
     double* o = T.part + ((((size_t)lp * T.cap + lu) * T.ntt + tt) * TT + 32 * half) * 128 + row;
 #pragma unroll
     for (int j = 0; j < 32; ++j)
